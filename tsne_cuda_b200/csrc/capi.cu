@@ -10,6 +10,7 @@
 
 #include "../../include/tsnecuda_b200.h"
 #include "comm.h"
+#include "hostio.h"
 #include "peer.h"
 #include "session.h"
 
@@ -31,20 +32,26 @@ int check_device(int device)
     return 0;
 }
 struct StreamGuard {
+    StreamSet *set = nullptr;
     cudaStream_t st = nullptr;
-    int create() { B200_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)); return 0; }
-    ~StreamGuard() { if (st) cudaStreamDestroy(st); }
+    int create()
+    {
+        int device = 0;
+        B200_CUDA(cudaGetDevice(&device));
+        B200_TRY(stream_set_acquire(&set, device));
+        st = set->stream;
+        return 0;
+    }
+    ~StreamGuard() { stream_set_release(set); }
 };
 template <class T> int up(DeviceArena &a, T **d, const T *h, size_t n, cudaStream_t st)
 {
     B200_TRY(a.alloc((void **)d, sizeof(T) * std::max<size_t>(n, 1)));
-    if (n) B200_CUDA(cudaMemcpyAsync(*d, h, sizeof(T) * n, cudaMemcpyHostToDevice, st));
-    return 0;
+    return copy_in(*d, h, sizeof(T) * n, st);
 }
 template <class T> int down(T *h, const T *d, size_t n, cudaStream_t st)
 {
-    if (n) B200_CUDA(cudaMemcpyAsync(h, d, sizeof(T) * n, cudaMemcpyDeviceToHost, st));
-    return 0;
+    return copy_out(h, d, sizeof(T) * n, st);
 }
 }  // namespace
 
@@ -408,8 +415,8 @@ int b200tsne_session_set_affinities(b200tsne_session *h, const float *P_rows, co
     Session &s = h->s;
     B200_CUDA(cudaSetDevice(s.device));
     const size_t n = (size_t)s.rows() * s.K;
-    B200_CUDA(cudaMemcpyAsync(s.P, P_rows, sizeof(float) * n, cudaMemcpyHostToDevice, s.stream));
-    B200_CUDA(cudaMemcpyAsync(s.ids, ids_rows, sizeof(int32_t) * n, cudaMemcpyHostToDevice, s.stream));
+    B200_TRY(copy_in(s.P, P_rows, sizeof(float) * n, s.stream));
+    B200_TRY(copy_in(s.ids, ids_rows, sizeof(int32_t) * n, s.stream));
     B200_CUDA(cudaStreamSynchronize(s.stream));
     s.cell_order = nullptr;   // no points to order by: the blocked copy, if the graph suits it, uses the natural order
     return s.build_blocked();
@@ -421,8 +428,8 @@ int b200tsne_session_get_affinities(b200tsne_session *h, float *P_rows, int32_t 
     Session &s = h->s;
     B200_CUDA(cudaSetDevice(s.device));
     const size_t n = (size_t)s.rows() * s.K;
-    if (P_rows) B200_CUDA(cudaMemcpyAsync(P_rows, s.P, sizeof(float) * n, cudaMemcpyDeviceToHost, s.stream));
-    if (ids_rows) B200_CUDA(cudaMemcpyAsync(ids_rows, s.ids, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, s.stream));
+    if (P_rows) B200_TRY(copy_out(P_rows, s.P, sizeof(float) * n, s.stream));
+    if (ids_rows) B200_TRY(copy_out(ids_rows, s.ids, sizeof(int32_t) * n, s.stream));
     B200_CUDA(cudaStreamSynchronize(s.stream));
     return 0;
 }

@@ -31,11 +31,9 @@ bool Options::validate()
 
 GpuOptions::GpuOptions(int device_) : device(device_)
 {
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device_) == cudaSuccess) {
-        warp_size = prop.warpSize;
-        sm_count = prop.multiProcessorCount;
-    }
+    int v = 0;   // single attributes: cudaGetDeviceProperties takes about a millisecond
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrWarpSize, device_) == cudaSuccess) warp_size = v;
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device_) == cudaSuccess) sm_count = v;
     cudaSetDevice(device_);
 }
 

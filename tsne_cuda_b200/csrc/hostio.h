@@ -1,0 +1,33 @@
+// Host-side resources that outlive one call: streams, events and pinned memory, and the copies between pageable host
+// memory and the device that use them.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+#include "common.cuh"
+
+namespace b200 {
+
+// What a session or a stage call needs from the driver besides device memory.  Creating and destroying it costs one to
+// three milliseconds a time, and on a busy host single calls (pinned memory above all) stall for 0.1 to 1.2 s, so the
+// sets are kept per device and handed to the next caller: at most kMaxIdleSets idle ones,
+// b200tsne_release_cached_memory() gives them back.  Safe from several threads: a set has one user at a time.
+struct StreamSet {
+    int device = -1;
+    cudaStream_t stream = nullptr, stream2 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
+    IterState *h_state = nullptr;   // pinned
+};
+int stream_set_acquire(StreamSet **out, int device);   // makes `device` current
+void stream_set_release(StreamSet *s);                 // waits for both streams; null is fine
+
+// Copies between pageable host memory and the device on `st`.  Large ones go through pinned chunks filled (or emptied)
+// by several host threads; small ones, pinned memory and callers that cannot have staging memory use one
+// cudaMemcpyAsync.  copy_in returns once a pageable source may be changed (pinned memory is read until the stream has
+// passed the copy); copy_out returns with the data in place.
+int copy_in(void *dst_device, const void *src_host, size_t bytes, cudaStream_t st);
+int copy_out(void *dst_host, const void *src_device, size_t bytes, cudaStream_t st);
+
+void host_pools_release(int device);   // idle sets and staging memory of one device
+
+}  // namespace b200

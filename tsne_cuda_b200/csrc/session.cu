@@ -19,6 +19,7 @@
 #include <string>
 
 #include "comm.h"
+#include "hostio.h"
 #include "peer.h"
 
 namespace b200 {
@@ -61,6 +62,7 @@ int release_cached_memory()
     cudaMemPool_t pool;
     B200_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
     B200_CUDA(cudaDeviceSynchronize());
+    host_pools_release(dev);
     B200_CUDA(cudaMemPoolTrimTo(pool, 0));
     return 0;
 }
@@ -103,12 +105,10 @@ int Session::init(int64_t N_, int K_, int64_t lo, int64_t hi, int device_)
     B200_CUDA(cudaSetDevice(device));
     // (Stream priorities were measured both ways and change nothing: the attractive kernel and the grid
     // pipeline compete for the same load/store units rather than for block slots.)
-    B200_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    B200_CUDA(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking));
-    B200_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-    B200_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
-    B200_CUDA(cudaEventCreate(&ev_t0));
-    B200_CUDA(cudaEventCreate(&ev_t1));
+    B200_TRY(stream_set_acquire(&host, device));
+    stream = host->stream; stream2 = host->stream2;
+    ev_fork = host->ev_fork; ev_join = host->ev_join; ev_t0 = host->ev_t0; ev_t1 = host->ev_t1;
+    h_state = host->h_state;
     arena.serve(stream);
     arena.serve(stream2);
     blocked_arena.serve(stream);
@@ -136,7 +136,6 @@ int Session::init(int64_t N_, int K_, int64_t lo, int64_t hi, int device_)
     B200_TRY(arena.alloc((void **)&ytilde, sizeof(float4) * kG * kG));
     B200_TRY(arena.alloc(&fft_mem, fft_workspace_bytes()));
     B200_TRY(arena.alloc((void **)&state, sizeof(IterState)));
-    B200_CUDA(cudaMallocHost((void **)&h_state, sizeof(IterState)));
     B200_TRY(fft_workspace_init(&fft, fft_mem, stream));
     Y2_own = Y2;
     w_own = w;
@@ -163,20 +162,15 @@ void Session::destroy()
     blocked.clear();
     blocked_arena.release();
     arena.release();
-    if (h_state) cudaFreeHost(h_state);
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    if (ev_t0) cudaEventDestroy(ev_t0);
-    if (ev_t1) cudaEventDestroy(ev_t1);
-    if (stream) cudaStreamDestroy(stream);
-    if (stream2) cudaStreamDestroy(stream2);
+    stream_set_release(host);
+    host = nullptr;
     h_state = nullptr; stream = stream2 = nullptr; ev_fork = ev_join = ev_t0 = ev_t1 = nullptr;
 }
 
 int Session::set_embedding_soa(const float *Y_host, bool reset)
 {
     B200_CUDA(cudaSetDevice(device));
-    B200_CUDA(cudaMemcpyAsync(soa_tmp, Y_host, sizeof(float) * 2 * N, cudaMemcpyHostToDevice, stream));
+    B200_TRY(copy_in(soa_tmp, Y_host, sizeof(float) * 2 * N, stream));
     B200_TRY(launch_soa_to_aos(soa_tmp, Y2, N, stream, state_order()));
     if (reset) {
         const int64_t r = std::max<int64_t>(rows(), 1);
@@ -196,8 +190,7 @@ int Session::get_embedding_soa(float *Y_host)
 {
     B200_CUDA(cudaSetDevice(device));
     B200_TRY(launch_aos_to_soa(Y2, soa_tmp, N, stream, state_order()));
-    B200_CUDA(cudaMemcpyAsync(Y_host, soa_tmp, sizeof(float) * 2 * N, cudaMemcpyDeviceToHost, stream));
-    B200_CUDA(cudaStreamSynchronize(stream));
+    B200_TRY(copy_out(Y_host, soa_tmp, sizeof(float) * 2 * N, stream));
     launches += 1;
     return 0;
 }
@@ -209,13 +202,11 @@ int Session::get_optimizer_soa(float *momentum_host, float *gains_host)
     if (r == 0) return 0;
     if (momentum_host) {
         B200_TRY(launch_aos_to_soa(u, soa_tmp, r, stream, state_order()));
-        B200_CUDA(cudaMemcpyAsync(momentum_host, soa_tmp, sizeof(float) * 2 * r, cudaMemcpyDeviceToHost, stream));
-        B200_CUDA(cudaStreamSynchronize(stream));
+        B200_TRY(copy_out(momentum_host, soa_tmp, sizeof(float) * 2 * r, stream));
     }
     if (gains_host) {
         B200_TRY(launch_aos_to_soa(gains, soa_tmp, r, stream, state_order()));
-        B200_CUDA(cudaMemcpyAsync(gains_host, soa_tmp, sizeof(float) * 2 * r, cudaMemcpyDeviceToHost, stream));
-        B200_CUDA(cudaStreamSynchronize(stream));
+        B200_TRY(copy_out(gains_host, soa_tmp, sizeof(float) * 2 * r, stream));
     }
     return 0;
 }
@@ -226,12 +217,12 @@ int Session::set_optimizer_soa(const float *momentum_host, const float *gains_ho
     const int64_t r = rows();
     if (r == 0) return 0;
     if (momentum_host) {
-        B200_CUDA(cudaMemcpyAsync(soa_tmp, momentum_host, sizeof(float) * 2 * r, cudaMemcpyHostToDevice, stream));
+        B200_TRY(copy_in(soa_tmp, momentum_host, sizeof(float) * 2 * r, stream));
         B200_TRY(launch_soa_to_aos(soa_tmp, u, r, stream, state_order()));
         B200_CUDA(cudaStreamSynchronize(stream));
     }
     if (gains_host) {
-        B200_CUDA(cudaMemcpyAsync(soa_tmp, gains_host, sizeof(float) * 2 * r, cudaMemcpyHostToDevice, stream));
+        B200_TRY(copy_in(soa_tmp, gains_host, sizeof(float) * 2 * r, stream));
         B200_TRY(launch_soa_to_aos(soa_tmp, gains, r, stream, state_order()));
         B200_CUDA(cudaStreamSynchronize(stream));
     }
@@ -600,7 +591,7 @@ int Session::affinities_from_points(const float *X_host, int D, float perplexity
 
     StageClock clk(this);
     B200_TRY(tmp.alloc((void **)&X, sizeof(float) * N * D));
-    B200_CUDA(cudaMemcpyAsync(X, X_host, sizeof(float) * N * D, cudaMemcpyHostToDevice, stream));
+    B200_TRY(copy_in(X, X_host, sizeof(float) * N * D, stream));
     clk.begin(stream);   // the search itself: the points are on their way
     B200_TRY(tmp.alloc((void **)&d2, sizeof(float) * std::max<int64_t>(chunk, 1) * K));
     B200_TRY(tmp.alloc((void **)&max_enc, sizeof(unsigned int)));

@@ -10,6 +10,7 @@ namespace b200 {
 
 struct Comm;          // comm.h
 struct PeerExchange;  // peer.h
+struct StreamSet;     // hostio.h
 
 enum Stage { kStSpread = 0, kStConvolve, kStGather, kStAttractive, kStUpdate, kStExchange, kStKnn, kStAffinities, kStOrder };
 
@@ -28,6 +29,7 @@ struct Session {
     int64_t N = 0;           // all points
     int K = 0;
     int64_t row_lo = 0, row_hi = 0;  // owned rows
+    StreamSet *host = nullptr;       // the streams, events and pinned memory below come from here
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;  // attractive force overlaps the grid pipeline
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
