@@ -329,8 +329,10 @@ int b200tsne_repulsive(const float *Y, int64_t N, float *Frep, float *Z, float *
     const InterpConsts ic = make_interp_consts();
     B200_TRY(launch_spread(dY2, 0, N, nullptr, st, 0, ic, dw, sg.st));
     if (w_out) B200_TRY(down(w_out, reinterpret_cast<float *>(dw), (size_t)kG * kG * 4, sg.st));
+    B200_TRY(launch_kernel_spectrum(st, 0, ws, sg.st));
+    B200_TRY(launch_convolve_rows(dw, st, 0, ws, sg.st));
     B200_TRY(launch_convolve(dw, dyt, st, 0, ws, false, sg.st));
-    B200_TRY(launch_gather(dY2, 0, N, st, 0, ic, dyt, dF2, true, sg.st));
+    B200_TRY(launch_gather(dY2, 0, N, st, 0, ic, dyt, dF2, sg.st));
     B200_TRY(launch_aos_to_soa(dF2, dF, N, sg.st));
     B200_TRY(down(Frep, dF, (size_t)2 * N, sg.st));
     if (ytilde_out) B200_TRY(down(ytilde_out, reinterpret_cast<float *>(dyt), (size_t)kG * kG * 4, sg.st));

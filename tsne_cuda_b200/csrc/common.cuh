@@ -12,7 +12,7 @@ constexpr int kBoxes = 130;            // boxes per dimension (125 rounded up th
 constexpr int kInterp = 3;             // Lagrange nodes per box and dimension
 constexpr int kG = kBoxes * kInterp;   // 390 nodes per dimension
 constexpr int kTerms = 4;              // charges (1, x, y, x^2+y^2)
-constexpr int kM = 1024;               // transform length of the zero-padded convolution (>= 2*kG-1)
+constexpr int kM = 784;                // transform length of the zero-padded convolution (>= 2*kG-1)
 constexpr int kStages = 9;             // instrumented stages (== B200TSNE_N_STAGES)
 
 // ---- error plumbing ----
@@ -39,7 +39,7 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line);
 struct IterState {
     unsigned int min_enc[2];   // order-preserving encodings of min / max over all coordinates
     unsigned int max_enc[2];
-    double zsum[2];            // sum_i Z_i accumulated by the gather kernel
+    double zsum[2];            // sum_i Z_i, accumulated on the grid by the convolution's last pass
     double unorm2;             // sum of squared updates (only maintained on request)
     int bad;                   // set when a non-finite coordinate is produced
     int pad;
@@ -156,10 +156,10 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
 
 // repulsive.cu
 struct FftWorkspace {
-    float2 *A;      // [2][kG][kM] row-transformed signal planes
-    float *Rk;      // [kG][kM] row-transformed kernel plane (real part)
-    float2 *B;      // [2][kG][kM] after the fused column pass
-    float2 *tw;     // [kM] forward twiddles e^{-2 pi i k / kM}
+    float4 *A;      // [kG rows][columns 0 .. kM/2][2] row-transformed charges (see convolve.cu)
+    float4 *B;      // the same after the column pass
+    float2 *tw;     // [28][28] twiddles e^{-2 pi i k l / kM}
+    float *Rk, *Kh; // row-transformed kernel; its spectrum by column
 };
 size_t fft_workspace_bytes();
 int fft_workspace_init(FftWorkspace *ws, void *mem, cudaStream_t st);
@@ -171,11 +171,13 @@ int launch_spread(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_
 int launch_order_identity(int32_t *order, int64_t n, cudaStream_t st);
 int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order_in, int32_t *order_out,
                          int32_t *keys, int32_t *hist, const IterState *state, int slot, cudaStream_t st);
-int launch_convolve(float4 *w, float4 *ytilde, const IterState *state, int slot, const FftWorkspace &ws, bool zero_w,
-                    cudaStream_t st);
-// sum_z: add the rows' Z_i to state->zsum[slot] (off when the caller evaluates the sum on the grid)
-int launch_gather(const float2 *Y2, int64_t row_lo, int64_t row_hi, IterState *state, int slot, InterpConsts ic,
-                  const float4 *ytilde, float2 *Frep2, bool sum_z, cudaStream_t st);
+// convolve.cu: the kernel's spectrum (needs the slot's min/max only), the first pass over the charges, and the rest, which
+// needs both; the last pass adds sum_i Z_i over all charges to state->zsum[slot] and clears w when asked to
+int launch_kernel_spectrum(const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
+int launch_convolve_rows(const float4 *w, const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
+int launch_convolve(float4 *w, float4 *ytilde, IterState *state, int slot, const FftWorkspace &ws, bool zero_w, cudaStream_t st);
+int launch_gather(const float2 *Y2, int64_t row_lo, int64_t row_hi, const IterState *state, int slot, InterpConsts ic,
+                  const float4 *ytilde, float2 *Frep2, cudaStream_t st);
 
 // update.cu
 // where the updated rows go: one array (in place) or the embedding copy of every rank (peer memory)

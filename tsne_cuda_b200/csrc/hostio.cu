@@ -39,6 +39,7 @@ void set_destroy(StreamSet *s)
 {
     if (s->ev_fork) cudaEventDestroy(s->ev_fork);
     if (s->ev_join) cudaEventDestroy(s->ev_join);
+    if (s->ev_spectrum) cudaEventDestroy(s->ev_spectrum);
     if (s->ev_t0) cudaEventDestroy(s->ev_t0);
     if (s->ev_t1) cudaEventDestroy(s->ev_t1);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -53,6 +54,7 @@ int set_create(StreamSet *s)
     B200_CUDA(cudaStreamCreateWithFlags(&s->stream2, cudaStreamNonBlocking));
     B200_CUDA(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming));
     B200_CUDA(cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming));
+    B200_CUDA(cudaEventCreateWithFlags(&s->ev_spectrum, cudaEventDisableTiming));
     B200_CUDA(cudaEventCreate(&s->ev_t0));
     B200_CUDA(cudaEventCreate(&s->ev_t1));
     B200_CUDA(cudaMallocHost((void **)&s->h_state, sizeof(IterState)));

@@ -15,7 +15,7 @@ namespace b200 {
 struct StreamSet {
     int device = -1;
     cudaStream_t stream = nullptr, stream2 = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     IterState *h_state = nullptr;   // pinned
 };
 int stream_set_acquire(StreamSet **out, int device);   // makes `device` current

@@ -226,32 +226,6 @@ peer_grid_allreduce_kernel(PeerTable tab, int buf, unsigned int *epochs, int *bl
     if (threadIdx.x == 0) { epochs[kFlagSpread] = v_spread; epochs[kFlagSlice] = v_slice; }
     __threadfence_system();
 }
-
-// sum_i Z_i with Z_i = (1 + |y_i|^2) phi_count(y_i) - 2 (x_i phi_x(y_i) + y_i phi_y(y_i)) + phi_r2(y_i) and every
-// phi interpolated from the node potentials with the weights that spread the charges: summing over the
-// points first turns it into  sum_nodes  pot.count * (w.count + w.r2) - 2 (pot.x * w.x + pot.y * w.y) + pot.r2 * w.count.
-// Node layout (x, y, count, r^2) for charges and potentials alike.
-__global__ void __launch_bounds__(256)
-grid_z_kernel(const float4 *__restrict__ w_sum, const float4 *__restrict__ ytilde, IterState *state, int slot)
-{
-    const int n = kG * kG;
-    double z = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 q = w_sum[i], p = ytilde[i];
-        z += (double)p.z * ((double)q.z + (double)q.w) - 2.0 * ((double)p.x * (double)q.x + (double)p.y * (double)q.y) +
-             (double)p.w * (double)q.z;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-    __shared__ double sz[8];
-    if ((threadIdx.x & 31) == 0) sz[threadIdx.x >> 5] = z;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int k = 0; k < 8; k++) t += sz[k];
-        atomicAdd(&state->zsum[slot], t);
-    }
-}
 }  // namespace
 
 void peer_exchange_release(PeerExchange *px, Comm *comm)
@@ -458,13 +432,6 @@ int launch_peer_grid_allreduce(PeerExchange *px, int buf, cudaStream_t st)
 {
     unsigned int *epochs = reinterpret_cast<unsigned int *>(px->err) + 2;
     peer_grid_allreduce_kernel<<<kAllreduceBlocks, 256, 0, st>>>(px->tab, buf, epochs, px->err + 5, px->err, px->err_host_dev, px->timeout_ns);
-    B200_CUDA(cudaGetLastError());
-    return 0;
-}
-
-int launch_grid_z(const float4 *w_sum, const float4 *ytilde, IterState *state, int slot, cudaStream_t st)
-{
-    grid_z_kernel<<<148, 256, 0, st>>>(w_sum, ytilde, state, slot);
     B200_CUDA(cudaGetLastError());
     return 0;
 }

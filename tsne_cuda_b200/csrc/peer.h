@@ -85,7 +85,5 @@ int launch_peer_grid_reduce(PeerExchange *px, int buf, float4 *w_sum, cudaStream
 // every rank sums the nodes of its own slice from all ranks' partial grids and stores the sums into every
 // rank's summed grid (ws), then the ranks meet once more ("all slices stored").  The result is in px->ws_local().
 int launch_peer_grid_allreduce(PeerExchange *px, int buf, cudaStream_t st);
-// state->zsum[slot] += sum over nodes of the bilinear form of charges w_sum and potentials ytilde
-int launch_grid_z(const float4 *w_sum, const float4 *ytilde, IterState *state, int slot, cudaStream_t st);
 
 }  // namespace b200

@@ -107,7 +107,7 @@ int Session::init(int64_t N_, int K_, int64_t lo, int64_t hi, int device_)
     // pipeline compete for the same load/store units rather than for block slots.)
     B200_TRY(stream_set_acquire(&host, device));
     stream = host->stream; stream2 = host->stream2;
-    ev_fork = host->ev_fork; ev_join = host->ev_join; ev_t0 = host->ev_t0; ev_t1 = host->ev_t1;
+    ev_fork = host->ev_fork; ev_join = host->ev_join; ev_spectrum = host->ev_spectrum; ev_t0 = host->ev_t0; ev_t1 = host->ev_t1;
     h_state = host->h_state;
     arena.serve(stream);
     arena.serve(stream2);
@@ -164,7 +164,7 @@ void Session::destroy()
     arena.release();
     stream_set_release(host);
     host = nullptr;
-    h_state = nullptr; stream = stream2 = nullptr; ev_fork = ev_join = ev_t0 = ev_t1 = nullptr;
+    h_state = nullptr; stream = stream2 = nullptr; ev_fork = ev_join = ev_spectrum = ev_t0 = ev_t1 = nullptr;
 }
 
 int Session::set_embedding_soa(const float *Y_host, bool reset)
@@ -287,6 +287,10 @@ int Session::one_iteration(bool want_norm)
     if (!stage_timers) {
         B200_CUDA(cudaEventRecord(ev_fork, stream));
         B200_CUDA(cudaStreamWaitEvent(stream2, ev_fork, 0));
+        // the kernel's spectrum needs the bounding box only: ready long before the charges are
+        B200_TRY(launch_kernel_spectrum(state, slot, fft, stream2));
+        B200_CUDA(cudaEventRecord(ev_spectrum, stream2));
+        launches += 2;
         B200_TRY(attractive(sa));
         B200_CUDA(cudaEventRecord(ev_join, stream2));
         launches += attractive_launches();
@@ -324,21 +328,15 @@ int Session::one_iteration(bool want_norm)
         clk.end(stream, kStExchange, 0);
     }
     clk.begin(stream);
-    B200_TRY(launch_convolve(p2p ? w_sum : w, ytilde, state, slot, fft, !p2p, stream));
-    clk.end(stream, kStConvolve, 3);
+    float4 *charges = p2p ? w_sum : w;
+    if (stage_timers) B200_TRY(launch_kernel_spectrum(state, slot, fft, stream));
+    B200_TRY(launch_convolve_rows(charges, state, slot, fft, stream));
+    if (!stage_timers) B200_CUDA(cudaStreamWaitEvent(stream, ev_spectrum, 0));
+    B200_TRY(launch_convolve(charges, ytilde, state, slot, fft, !p2p, stream));   // sums Z over ALL points on the grid: no exchange
+    clk.end(stream, kStConvolve, stage_timers ? 5 : 3);
     clk.begin(stream);
-    B200_TRY(launch_gather(Y2, row_lo, row_hi, state, slot, ic, ytilde, Frep, !p2p, stream));
+    B200_TRY(launch_gather(Y2, row_lo, row_hi, state, slot, ic, ytilde, Frep, stream));
     clk.end(stream, kStGather, 1);
-    if (p2p) {
-        // sum of Z_i over ALL points from the summed grid: no exchange
-        clk.begin(stream);
-        B200_TRY(launch_grid_z(w_sum, ytilde, state, slot, stream));
-        clk.end(stream, kStGather, 1);
-    } else if (multi) {
-        clk.begin(stream);
-        B200_TRY(comm->all_reduce_sum_f64(&state->zsum[slot], 1, stream));
-        clk.end(stream, kStExchange, 0);
-    }
     if (stage_timers) {
         clk.begin(stream);
         B200_TRY(attractive(stream));

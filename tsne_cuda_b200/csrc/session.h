@@ -32,7 +32,7 @@ struct Session {
     StreamSet *host = nullptr;       // the streams, events and pinned memory below come from here
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;  // attractive force overlaps the grid pipeline
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     DeviceArena arena;
 
     // affinities (owned rows)
