@@ -1,0 +1,102 @@
+"""The gradient loop at the sizes where its kernels change, and the early stop taken on the device.
+
+Bars: one iteration against the CPU oracle.  The update is  u = m u0 - eta g (a F_attr - F_rep / Z); the forces are within
+1e-5 and 1e-4 of the oracle (relative L2, test_gpu_stages.py), so the new momentum from u0 = 0 is within their sum."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _graph(n, k, seed):
+    rng = np.random.default_rng(seed)
+    ids = rng.integers(0, n, (n, k), dtype=np.int32)
+    P = (rng.random((n, k)) / (n * k)).astype(np.float32)
+    return P, ids, rng
+
+
+def _same(a, b):
+    """Embedding and momentum up to the order of the forces' sums.  A gain takes its other value (a fifth away) where that
+    turns the sign of a gradient near zero: at most one coordinate in 10^4."""
+    assert rel_l2(a[0], b[0]) < 1e-6 and rel_l2(a[1], b[1]) < 1e-6
+    assert (np.abs(a[2] - b[2]) > 1e-5).mean() < 1e-4 and a[3] == b[3]
+
+
+# points one by one | merged in natural order | sorted, a point a lane | sorted, four a lane: both sides of every border
+@pytest.mark.parametrize("n", [1, 31, 8192, 8193, 32767, 32768, 131072, 131075])
+@pytest.mark.parametrize("spread", [1e-4, 20.0])
+def test_one_iteration_vs_oracle(engine, oracle_cpu, n, spread):
+    P, ids, rng = _graph(n, 4, n)
+    Y = rng.normal(0, spread, (2, n)).astype(np.float32)
+    Y[:, : n // 3] *= 0.02                                   # a dense part: long runs of points in one box
+    with engine.Session(n, 4) as s:
+        s.set_affinities(P, ids)
+        s.set_schedule(100.0, 12.0, 250, 0.5, 0.8)
+        s.set_embedding(Y)
+        s.run(1)
+        Y1, mom, gains, step = s.get_state()
+    Yo, gains_o, mom_o, _ = oracle_cpu.iterate(P, ids, Y, 1, 100.0)
+    assert step == 1
+    if n == 1:                                               # no neighbour but itself, Z = 0: nothing finite to compare
+        return
+    assert rel_l2(mom, mom_o) < 1.1e-4
+    # the embedding rounds once more per coordinate
+    assert np.abs(Y1 - Yo).max() < 1.1e-4 * np.linalg.norm(mom_o) + 2e-7 * np.abs(Yo).max()
+
+
+@pytest.mark.parametrize("n", [700, 40000])
+@pytest.mark.parametrize("stop_after", [1, 2, 5, 16, 17, 20])
+def test_stop_on_the_device_takes_place_where_the_host_would(engine, n, stop_after):
+    """Momentum that fades makes the update norm fall from step to step: the run ends after the first iteration whose
+    norm is below the threshold, whatever block it was queued in, and the loop goes on from there."""
+    P, ids, rng = _graph(n, 6, 5)
+    Y = rng.normal(0, 5.0, (2, n)).astype(np.float32)
+    mom = rng.normal(0, 1.0, (2, n)).astype(np.float32)
+
+    def session():
+        s = engine.Session(n, 6)
+        s.set_affinities(P, ids)
+        s.set_schedule(1e-3, 12.0, 250, 0.8, 0.8)
+        s.set_state(Y, mom, np.ones_like(mom), 0)
+        return s
+
+    with session() as s:
+        norms = []
+        for _ in range(24):
+            s.run(1, min_gradient_norm=1e-30)
+            norms.append(s.stats()["update_norm"])
+    assert all(a > b for a, b in zip(norms, norms[1:]))
+    threshold = 0.5 * (norms[stop_after - 1] + (norms[stop_after - 2] if stop_after > 1 else 2 * norms[0]))
+    with session() as s, session() as t:
+        _, done = s.run(23, min_gradient_norm=threshold)
+        assert done == stop_after and s.stats()["step"] == stop_after
+        assert abs(s.stats()["update_norm"] / norms[stop_after - 1] - 1) < 1e-5
+        t.run(stop_after)
+        _same(s.get_state(), t.get_state())
+        assert abs(s.stats()["Z"] / t.stats()["Z"] - 1) < 1e-5
+        s.run(7)
+        t.run(7)
+        _same(s.get_state(), t.get_state())
+
+
+def test_blocks_of_iterations_and_single_steps_agree(engine):
+    """Captured blocks of 16, pairs and single steps, across the phases of the schedule, against direct launches."""
+    n = 40000                                                # sorted: the late phase sorts every eighth iteration
+    P, ids, rng = _graph(n, 6, 6)
+    Y = rng.normal(0, 5.0, (2, n)).astype(np.float32)
+    out = []
+    for chunks in ([57], [1] * 57, [16, 3, 2, 1, 35], [57]):
+        with engine.Session(n, 6) as s:
+            s.set_affinities(P, ids)
+            s.set_schedule(1.0, 12.0, 18, 0.5, 0.8)
+            s.set_state(Y, np.zeros_like(Y), np.ones_like(Y), 3)
+            if len(out) == 3:
+                s.enable_stage_timers(True)                  # direct launches, the gather a kernel of its own
+            for c in chunks:
+                s.run(c)
+            out.append(s.get_state())
+    for o in out[1:]:
+        assert o[3] == out[0][3] == 60
+        assert rel_l2(o[0], out[0][0]) < 1e-6 and rel_l2(o[1], out[0][1]) < 1e-4

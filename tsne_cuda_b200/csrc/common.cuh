@@ -40,9 +40,10 @@ struct IterState {
     unsigned int min_enc[2];   // order-preserving encodings of min / max over all coordinates
     unsigned int max_enc[2];
     double zsum[2];            // sum_i Z_i, accumulated on the grid by the convolution's last pass
-    double unorm2;             // sum of squared updates (only maintained on request)
+    double unorm2[2];          // sum of squared updates (only maintained on request)
+    double z_last;             // zsum of the last iteration that changed the embedding
     int bad;                   // set when a non-finite coordinate is produced
-    int pad;
+    int done;                  // iterations that changed the embedding (counts on; the host looks at differences)
 };
 
 // Lagrange constants evaluated on the host exactly as the reference does (src/fit_tsne.cu:303-320).
@@ -164,13 +165,18 @@ struct FftWorkspace {
 size_t fft_workspace_bytes();
 int fft_workspace_init(FftWorkspace *ws, void *mem, cudaStream_t st);
 int launch_state_reset(IterState *state, cudaStream_t st);   // both slots, sums and flags
+int launch_state_swap(IterState *state, cudaStream_t st);    // exchanges the two slots (a stop between iterations of other parity)
 int launch_minmax_init(const float2 *Y2, int64_t N, IterState *state, int slot, cudaStream_t st);
+constexpr long long kSpreadDirectMax = 8192;      // up to here points are spread one by one
+constexpr long long kSortMin = 32768;             // from here on the spread order is sorted (both: repulsive.cu)
+constexpr long long kSpreadSingleMax = 131072;   // up to here a lane takes one point of the order
 // order: local row indices sorted by box (null = natural order); see launch_order_refresh
-int launch_spread(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order, const IterState *state,
+// hist (optional): the sort's counters, cleared on the way for the next sort
+int launch_spread(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order, int32_t *hist, const IterState *state,
                   int slot, InterpConsts ic, float4 *w, cudaStream_t st);
 int launch_order_identity(int32_t *order, int64_t n, cudaStream_t st);
-int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order_in, int32_t *order_out,
-                         int32_t *keys, int32_t *hist, const IterState *state, int slot, cudaStream_t st);
+int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, int32_t *order, int32_t *previous, int32_t *keys,
+                         int32_t *hist, const IterState *state, int slot, cudaStream_t st);
 // convolve.cu: the kernel's spectrum (needs the slot's min/max only), the first pass over the charges, and the rest, which
 // needs both; the last pass adds sum_i Z_i over all charges to state->zsum[slot] and clears w when asked to
 int launch_kernel_spectrum(const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
@@ -186,9 +192,10 @@ struct UpdateTargets {
     float2 *p[kMaxUpdateTargets];
     int n;
 };
-int launch_update(const float2 *Y2, const UpdateTargets &dst, const float2 *Fattr2, const float2 *Frep2, float2 *gains2, float2 *u2,
-                  int64_t N, int64_t row_lo, int64_t row_hi, IterState *state, int slot, float eta, float momentum,
-                  float exaggeration, int want_norm, cudaStream_t st);
+// ytilde given: the repulsive force is interpolated in the same kernel and Frep2 is not read; norm_mode: see update.cu
+int launch_update(const float2 *Y2, const UpdateTargets &dst, const float2 *Fattr2, const float2 *Frep2, const float4 *ytilde, InterpConsts ic,
+                  float2 *gains2, float2 *u2, int64_t N, int64_t row_lo, int64_t row_hi, IterState *state, int slot, float eta,
+                  float momentum, float exaggeration, int norm_mode, float stop_norm, cudaStream_t st);
 int launch_apply_forces_soa(float *Y, float *attr, float *rep, float *gains, float *old_forces, float eta, float Z,
                             float momentum, float exaggeration, int64_t N, cudaStream_t st);
 // perm (optional): position q of the pair array holds point perm[q] of the block-wise (x block, y block) array

@@ -381,9 +381,10 @@ fft_rows_inverse_kernel(const float4 *__restrict__ B, float4 *__restrict__ w, fl
     __syncthreads();
     if (threadIdx.x == 0) {
         atomicAdd(&state->zsum[slot], z + other);
-        if (row == 0) {   // recycle the other slot's min/max for this iteration's update
+        if (row == 0) {   // recycle the other slot's min/max and this slot's norm for this iteration's update
             state->min_enc[slot ^ 1] = 0xffffffffu;
             state->max_enc[slot ^ 1] = 0u;
+            state->unorm2[slot] = 0.0;
         }
     }
 }

@@ -13,6 +13,7 @@ namespace b200 {
 namespace {
 
 constexpr int kMaxIdleSets = 4;        // idle stream sets kept per device
+constexpr size_t kMaxKeptExecs = 16;   // executable graphs kept per set
 
 // Staging memory: kLanes host threads, each with two pinned chunks of its own, so that a thread fills one chunk while
 // the copy engine reads the other.  One thread moves pageable memory at about 10 GB/s (what a plain cudaMemcpyAsync
@@ -37,6 +38,7 @@ std::vector<Stage *> g_stages;         // idle
 
 void set_destroy(StreamSet *s)
 {
+    for (StreamSet::KeptExec &k : s->execs) cudaGraphExecDestroy(k.exec);
     if (s->ev_fork) cudaEventDestroy(s->ev_fork);
     if (s->ev_join) cudaEventDestroy(s->ev_join);
     if (s->ev_spectrum) cudaEventDestroy(s->ev_spectrum);
@@ -202,6 +204,31 @@ void stream_set_release(StreamSet *s)
         }
     }
     set_destroy(s);
+}
+
+cudaGraphExec_t graph_exec_acquire(StreamSet *s, cudaGraph_t graph, unsigned long long shape)
+{
+    for (size_t i = s->execs.size(); i-- > 0;) {
+        if (s->execs[i].shape != shape) continue;
+        cudaGraphExec_t exec = s->execs[i].exec;
+        s->execs.erase(s->execs.begin() + i);
+        cudaGraphExecUpdateResultInfo info;
+        if (cudaGraphExecUpdate(exec, graph, &info) == cudaSuccess) return exec;
+        (void)cudaGetLastError();
+        cudaGraphExecDestroy(exec);   // other nodes after all (another attractive kernel, say)
+    }
+    cudaGraphExec_t exec = nullptr;
+    if (cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    return exec;
+}
+
+void graph_exec_release(StreamSet *s, cudaGraphExec_t exec, unsigned long long shape)
+{
+    if (!s || s->execs.size() >= kMaxKeptExecs) cudaGraphExecDestroy(exec);
+    else s->execs.push_back({exec, shape});
 }
 
 int copy_in(void *dst, const void *src, size_t bytes, cudaStream_t st)

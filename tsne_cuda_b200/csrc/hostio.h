@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <vector>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -17,9 +19,21 @@ struct StreamSet {
     cudaStream_t stream = nullptr, stream2 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     IterState *h_state = nullptr;   // pinned
+    // Executable graphs that finished sessions left behind.  Instantiating one of 16 iterations takes 1.3 ms (now and
+    // then 100 on a busy host) and destroying it another; updating one of the same shape takes 0.1 ms.  They hold stale
+    // addresses and are only launched after an update.
+    struct KeptExec {
+        cudaGraphExec_t exec;
+        unsigned long long shape;
+    };
+    std::vector<KeptExec> execs;
 };
 int stream_set_acquire(StreamSet **out, int device);   // makes `device` current
 void stream_set_release(StreamSet *s);                 // waits for both streams; null is fine
+
+// An executable for `graph`: a kept one of the same shape, updated, else a new one; null if neither can be had.
+cudaGraphExec_t graph_exec_acquire(StreamSet *s, cudaGraph_t graph, unsigned long long shape);
+void graph_exec_release(StreamSet *s, cudaGraphExec_t exec, unsigned long long shape);
 
 // Copies between pageable host memory and the device on `st`.  Large ones go through pinned chunks filled (or emptied)
 // by several host threads; small ones, pinned memory and callers that cannot have staging memory use one

@@ -47,9 +47,19 @@ __global__ void state_reset_kernel(IterState *state, int slot, int all)
         state->max_enc[slot ^ 1] = 0u;
         state->zsum[0] = 0.0;
         state->zsum[1] = 0.0;
-        state->unorm2 = 0.0;
+        state->unorm2[0] = 0.0;
+        state->unorm2[1] = 0.0;
         state->bad = 0;
+        state->done = 0;
     }
+}
+
+__global__ void state_swap_kernel(IterState *state)
+{
+    const unsigned int mn = state->min_enc[0], mx = state->max_enc[0];
+    const double z = state->zsum[0];
+    state->min_enc[0] = state->min_enc[1]; state->max_enc[0] = state->max_enc[1]; state->zsum[0] = state->zsum[1];
+    state->min_enc[1] = mn; state->max_enc[1] = mx; state->zsum[1] = z;
 }
 
 __global__ void __launch_bounds__(256) minmax_kernel(const float2 *__restrict__ Y2, long long N, IterState *state, int slot)
@@ -92,6 +102,12 @@ __device__ __forceinline__ int axis_box(float c, const GridGeom &g)
 // contributions in registers; a box change inside the lane sends the finished sum to the grid directly.  The
 // lane's last (open) run is then combined with those of its neighbours as described above, so the 180
 // shuffles of the segmented reduction are paid once per 32 * kSpreadPerLane points.
+//
+// Fewer points leave most SMs idle with four points a lane: up to kSpreadSingleMax a lane takes one.  Below kSortMin
+// the points collide so rarely that sorting (three kernels, 15 us) costs more than it saves, and up to kSpreadDirectMax
+// even the shuffles do.  Whole iteration, exaggerated / settled: 5 000 points sorted every time 47 / 41 us, one by one
+// 37 / 37; 20 011 points sorted 44 / 42, merged in natural order 41 / 41, one by one 57 / 42; 60 000 points sorted
+// 54 / 49, natural order 61 / 49.
 constexpr int kSpreadPerLane = 4;
 
 __device__ __forceinline__ void spread_flush(float4 *__restrict__ w, int bx, int by, const float (&v)[kInterp][kInterp][4])
@@ -105,11 +121,20 @@ __device__ __forceinline__ void spread_flush(float4 *__restrict__ w, int bx, int
         }
 }
 
+// the counters of the next sort (a clear of its own would be one more node of the chain)
+__device__ __forceinline__ void clear_histogram(int32_t *hist)
+{
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < kBoxes * kBoxes; k += gridDim.x * blockDim.x) hist[k] = 0;
+}
+
+// hist (optional): the sort's counters, cleared here for the next one
+template <int PER_LANE>
 __global__ void __launch_bounds__(256)
 spread_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows, const int32_t *__restrict__ order,
-              const IterState *state, int slot, InterpConsts ic, float4 *__restrict__ w)
+              const IterState *state, int slot, InterpConsts ic, float4 *__restrict__ w, int32_t *__restrict__ hist)
 {
-    const long long t0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * kSpreadPerLane;
+    if (hist) clear_histogram(hist);
+    const long long t0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * PER_LANE;
     const int lane = threadIdx.x & 31;
     const GridGeom g = load_geom(state, slot);
     int key = -1, bx = 0, by = 0;
@@ -121,9 +146,9 @@ spread_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows,
 #pragma unroll
             for (int c = 0; c < 4; c++) v[a][b][c] = 0.0f;
     // all loads of the lane first: they are independent of each other
-    float2 ys[kSpreadPerLane];
+    float2 ys[PER_LANE];
 #pragma unroll
-    for (int p = 0; p < kSpreadPerLane; p++) {
+    for (int p = 0; p < PER_LANE; p++) {
         const long long t = t0 + p;
         if (t < n_rows) {
             const long long r = order ? (long long)order[t] : t;
@@ -131,7 +156,7 @@ spread_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows,
         }
     }
 #pragma unroll
-    for (int p = 0; p < kSpreadPerLane; p++) {
+    for (int p = 0; p < PER_LANE; p++) {
         if (t0 + p >= n_rows) break;
         const float2 y = ys[p];
         int kx, ky;
@@ -182,6 +207,29 @@ spread_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows,
     if (head && key >= 0) spread_flush(w, bx, by, v);
 }
 
+// No order, no merging: a point per thread (few points, see kSpreadPerLane).
+__global__ void __launch_bounds__(128)
+spread_direct_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows, const IterState *state, int slot, InterpConsts ic,
+                     float4 *__restrict__ w)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n_rows) return;
+    const GridGeom g = load_geom(state, slot);
+    const float2 y = Y2[row_lo + t];
+    int bx, by;
+    float Lx[kInterp], Ly[kInterp];
+    axis_weights(y.x, g, ic, bx, Lx);
+    axis_weights(y.y, g, ic, by, Ly);
+    const float c3 = y.x * y.x + y.y * y.y;
+#pragma unroll
+    for (int a = 0; a < kInterp; a++)
+#pragma unroll
+        for (int b = 0; b < kInterp; b++) {
+            const float l = Lx[a] * Ly[b];
+            atomicAdd(w + (size_t)(bx * kInterp + a) * kG + (by * kInterp + b), make_float4(l * y.x, l * y.y, l, l * c3));
+        }
+}
+
 // ---- counting sort of the owned points by box (order[t] = local row index) ----
 __global__ void order_identity_kernel(int32_t *order, long long n)
 {
@@ -202,10 +250,10 @@ __device__ __forceinline__ int point_key(const float2 *__restrict__ Y2, long lon
     return axis_box(y.y, g) * kBoxes + axis_box(y.x, g);
 }
 
-// keys[t] = box of point order[t]; hist[box] += 1
+// keys[t] = box of point order[t]; hist[box] += 1; previous[t] = order[t] (the scatter writes `order` anew)
 __global__ void __launch_bounds__(256)
 order_histogram_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows, const int32_t *__restrict__ order,
-                       const IterState *state, int slot, int32_t *__restrict__ keys, int32_t *__restrict__ hist)
+                       const IterState *state, int slot, int32_t *__restrict__ keys, int32_t *__restrict__ hist, int32_t *__restrict__ previous)
 {
     const long long t0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * kOrderPerThread;
     const int lane = threadIdx.x & 31;
@@ -218,12 +266,15 @@ order_histogram_kernel(const float2 *__restrict__ Y2, long long row_lo, long lon
         k[2] = point_key(Y2, row_lo + o.z, g);
         k[3] = point_key(Y2, row_lo + o.w, g);
         *reinterpret_cast<int4 *>(keys + t0) = make_int4(k[0], k[1], k[2], k[3]);
+        *reinterpret_cast<int4 *>(previous + t0) = o;
     } else {
 #pragma unroll
         for (int p = 0; p < kOrderPerThread; p++)
             if (t0 + p < n_rows) {
-                k[p] = point_key(Y2, row_lo + order[t0 + p], g);
+                const int32_t o = order[t0 + p];
+                k[p] = point_key(Y2, row_lo + o, g);
                 keys[t0 + p] = k[p];
+                previous[t0 + p] = o;
             }
     }
 #pragma unroll
@@ -349,12 +400,21 @@ int launch_state_reset(IterState *state, cudaStream_t st)
     return 0;
 }
 
-int launch_spread(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order, const IterState *state,
+int launch_state_swap(IterState *state, cudaStream_t st)
+{
+    state_swap_kernel<<<1, 1, 0, st>>>(state);
+    B200_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int launch_spread(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order, int32_t *hist, const IterState *state,
                   int slot, InterpConsts ic, float4 *w, cudaStream_t st)
 {
     const long long n = row_hi - row_lo;
     if (n <= 0) return 0;
-    spread_kernel<<<nblk((n + kSpreadPerLane - 1) / kSpreadPerLane, 256), 256, 0, st>>>(Y2, row_lo, n, order, state, slot, ic, w);
+    if (!order && n <= kSpreadDirectMax) spread_direct_kernel<<<nblk(n, 128), 128, 0, st>>>(Y2, row_lo, n, state, slot, ic, w);
+    else if (n <= kSpreadSingleMax) spread_kernel<1><<<nblk(n, 256), 256, 0, st>>>(Y2, row_lo, n, order, state, slot, ic, w, hist);
+    else spread_kernel<kSpreadPerLane><<<nblk((n + kSpreadPerLane - 1) / kSpreadPerLane, 256), 256, 0, st>>>(Y2, row_lo, n, order, state, slot, ic, w, hist);
     B200_CUDA(cudaGetLastError());
     return 0;
 }
@@ -367,20 +427,19 @@ int launch_order_identity(int32_t *order, int64_t n, cudaStream_t st)
     return 0;
 }
 
-// order_in -> order_out sorted by the box of the points' current position; keys: n ints of scratch,
-// hist: kBoxes^2 ints of scratch.
-int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order_in, int32_t *order_out,
-                         int32_t *keys, int32_t *hist, const IterState *state, int slot, cudaStream_t st)
+// `order` sorted anew by the box of the points' current position; previous, keys: n ints of scratch each,
+// hist: kBoxes^2 counters, zero on entry (the spread that follows clears them again).
+int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, int32_t *order, int32_t *previous, int32_t *keys,
+                         int32_t *hist, const IterState *state, int slot, cudaStream_t st)
 {
     const long long n = row_hi - row_lo;
     if (n <= 0) return 0;
-    B200_CUDA(cudaMemsetAsync(hist, 0, sizeof(int32_t) * kBoxes * kBoxes, st));
     const long long n_thr = (n + kOrderPerThread - 1) / kOrderPerThread;
-    order_histogram_kernel<<<nblk(n_thr, 256), 256, 0, st>>>(Y2, row_lo, n, order_in, state, slot, keys, hist);
+    order_histogram_kernel<<<nblk(n_thr, 256), 256, 0, st>>>(Y2, row_lo, n, order, state, slot, keys, hist, previous);
     B200_CUDA(cudaGetLastError());
     order_scan_kernel<<<1, 1024, 0, st>>>(hist);
     B200_CUDA(cudaGetLastError());
-    order_scatter_kernel<<<nblk(n_thr, 256), 256, 0, st>>>(order_in, keys, n, hist, order_out);
+    order_scatter_kernel<<<nblk(n_thr, 256), 256, 0, st>>>(previous, keys, n, hist, order);
     B200_CUDA(cudaGetLastError());
     return 0;
 }

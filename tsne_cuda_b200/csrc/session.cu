@@ -123,6 +123,8 @@ int Session::init(int64_t N_, int K_, int64_t lo, int64_t hi, int device_)
     B200_TRY(arena.alloc((void **)&order_keys, sizeof(int32_t) * r));
     B200_TRY(arena.alloc((void **)&box_hist, sizeof(int32_t) * kBoxes * kBoxes));
     B200_TRY(launch_order_identity(order, rows(), stream));
+    B200_CUDA(cudaMemsetAsync(box_hist, 0, sizeof(int32_t) * kBoxes * kBoxes, stream));
+    if (rows() < kSortMin) order_refresh = 0;
     if (const char *e = getenv("B200TSNE_ORDER_REFRESH")) order_refresh = atoi(e);
     if (const char *e = getenv("B200TSNE_ORDER_REFRESH_EARLY")) order_refresh_early = std::max(1, atoi(e));
     if (const char *e = getenv("B200TSNE_GRAPHS")) use_graphs = atoi(e) != 0;
@@ -179,6 +181,7 @@ int Session::set_embedding_soa(const float *Y_host, bool reset)
         step = 0;
     }
     B200_TRY(launch_state_reset(state, stream));
+    done_seen = 0;
     B200_TRY(launch_minmax_init(Y2, N, state, step & 1, stream));
     B200_CUDA(cudaMemsetAsync(w, 0, sizeof(float4) * kG * kG, stream));
     B200_CUDA(cudaStreamSynchronize(stream));
@@ -258,7 +261,8 @@ struct StageClock {
 };
 }  // namespace
 
-int Session::one_iteration(bool want_norm)
+// norm_mode, stop_norm: see launch_update
+int Session::one_iteration(int norm_mode, float stop_norm)
 {
     const int slot = step & 1;
     const bool late = step >= force_magnify_iters;
@@ -297,20 +301,18 @@ int Session::one_iteration(bool want_norm)
     }
 
     // The embedding reshuffles quickly while it is being exaggerated and slowly afterwards: sort every
-    // iteration early, every order_refresh iterations later.  (Sorting the rows for iteration t + 1 at the end of
-    // iteration t, while waiting for the other ranks, was measured on two GPUs: the next bounding box is only
+    // order_refresh_early iterations early, every order_refresh iterations later.  (Sorting the rows for iteration t + 1
+    // at the end of iteration t, while waiting for the other ranks, was measured on two GPUs: the next bounding box is only
     // known after that meeting, and boxes taken from the previous one - the embedding grows by more than a box
     // width per exaggerated iteration - break the runs of equal boxes: spread 61 us instead of 15.)
-    const bool settling = step < force_magnify_iters + 50;
-    const int refresh_every = settling ? order_refresh_early : order_refresh;
-    if (order_refresh > 0 && step % refresh_every == 0) {
+    const int refresh = refresh_period(step);
+    if (refresh > 0 && step % refresh == 0) {
         clk.begin(stream);
         B200_TRY(launch_order_refresh(Y2, row_lo, row_hi, order, order_alt, order_keys, box_hist, state, slot, stream));
-        std::swap(order, order_alt);
         clk.end(stream, kStOrder, 3);
     }
     clk.begin(stream);
-    B200_TRY(launch_spread(Y2, row_lo, row_hi, order_refresh > 0 ? order : nullptr, state, slot, ic, w, stream));
+    B200_TRY(launch_spread(Y2, row_lo, row_hi, refresh > 0 ? order : nullptr, refresh > 0 ? box_hist : nullptr, state, slot, ic, w, stream));
     clk.end(stream, kStSpread, 1);
     if (p2p) {
         clk.begin(stream);
@@ -334,9 +336,12 @@ int Session::one_iteration(bool want_norm)
     if (!stage_timers) B200_CUDA(cudaStreamWaitEvent(stream, ev_spectrum, 0));
     B200_TRY(launch_convolve(charges, ytilde, state, slot, fft, !p2p, stream));   // sums Z over ALL points on the grid: no exchange
     clk.end(stream, kStConvolve, stage_timers ? 5 : 3);
-    clk.begin(stream);
-    B200_TRY(launch_gather(Y2, row_lo, row_hi, state, slot, ic, ytilde, Frep, stream));
-    clk.end(stream, kStGather, 1);
+    const bool fused = !multi && !stage_timers;   // the update interpolates the repulsive force itself
+    if (!fused) {
+        clk.begin(stream);
+        B200_TRY(launch_gather(Y2, row_lo, row_hi, state, slot, ic, ytilde, Frep, stream));
+        clk.end(stream, kStGather, 1);
+    }
     if (stage_timers) {
         clk.begin(stream);
         B200_TRY(attractive(stream));
@@ -352,8 +357,8 @@ int Session::one_iteration(bool want_norm)
         dst.n = comm->world;
         for (int r = 0; r < comm->world; r++) dst.p[r] = px->tab.y[px->parity ^ 1][r];
     }
-    B200_TRY(launch_update(Y2, dst, Fattr, Frep, gains, u, N, row_lo, row_hi, state, slot, eta, momentum, exag,
-                           want_norm ? 1 : 0, stream));
+    B200_TRY(launch_update(Y2, dst, Fattr, Frep, fused ? ytilde : nullptr, ic, gains, u, N, row_lo, row_hi, state, slot, eta, momentum, exag,
+                           norm_mode, stop_norm, stream));
     clk.end(stream, kStUpdate, 1);
     if (p2p) {
         clk.begin(stream);
@@ -417,112 +422,136 @@ int Session::build_blocked()
 
 void Session::drop_graphs()
 {
-    for (IterGraph &g : graphs) {
-        if (g.exec) cudaGraphExecDestroy(g.exec);
-        g = IterGraph();
-    }
+    for (IterGraph &g : graphs)
+        if (g.exec) graph_exec_release(host, g.exec, g.shape());
+    graphs.clear();
 }
 
-// Which graph covers the iterations from `step` on, and how many of them; 0 when the next iteration has to be
-// launched directly (misaligned with the block, a phase boundary inside it, or a feature graphs do not carry).
-int Session::graph_block(int remaining, bool want_norm, int *kind) const
+int Session::refresh_period(int at) const
+{
+    if (order_refresh <= 0) return 0;
+    return at < force_magnify_iters + 50 ? order_refresh_early : order_refresh;
+}
+
+// How many of the next iterations one graph covers; 0 when the next one has to be launched directly.  A graph holds
+// iterations of one phase of the schedule: an even number (the state slots and the exchange buffers alternate), or a
+// single one where a caller steps one by one.
+int Session::graph_block(int remaining) const
 {
     // (a sharded run qualifies when it exchanges over peer memory: its meetings are kernels of this library)
-    if (!use_graphs || stage_timers || want_norm || (comm && comm->world > 1 && !px) || order_refresh_early != 1) return 0;
-    const int settle_end = force_magnify_iters + 50;
-    int k, block, limit;
-    if (step < force_magnify_iters) { k = 0; block = 2; limit = force_magnify_iters; }
-    else if (step < settle_end) { k = 1; block = 2; limit = settle_end; }
-    else { k = 2; block = order_refresh > 0 ? 2 * order_refresh : 2; limit = INT_MAX; }
-    if (step % block != 0 || remaining < block || (long long)step + block > limit) return 0;
-    *kind = k;
-    return block;
+    if (!use_graphs || stage_timers || (comm && comm->world > 1 && !px)) return 0;
+    long long left = remaining;
+    for (const int end : {force_magnify_iters, force_magnify_iters + 50})
+        if (step < end) left = std::min<long long>(left, (long long)end - step);
+    if (left >= kGraphIters && !(step & 1)) return kGraphIters;
+    if (left >= 2 && !(step & 1)) return 2;
+    return px ? 0 : 1;
 }
 
-int Session::run_graph_block(int kind, int iters)
+// 0: done.  1: not captured, the caller launches directly.  Negative: error.
+int Session::run_graph_block(int iters, int norm_mode, float stop_norm)
 {
-    IterGraph &g = graphs[kind];
-    const bool late = kind > 0;
-    const float momentum = late ? post_momentum : pre_momentum, exag = late ? 1.0f : exaggeration;
-    const int parity = px ? px->parity : 0;   // which exchange buffers the block starts from
-    if (g.exec && (g.iters != iters || g.eta != eta || g.exaggeration != exag || g.momentum != momentum || g.refresh != order_refresh ||
-                   g.parity != parity)) {
-        cudaGraphExecDestroy(g.exec);
-        g = IterGraph();
+    const bool late = step >= force_magnify_iters;
+    IterGraph key;
+    key.iters = iters;
+    key.parity = px ? px->parity : step & 1;
+    key.late = late;
+    key.eta = eta;
+    key.exaggeration = late ? 1.0f : exaggeration;
+    key.momentum = late ? post_momentum : pre_momentum;
+    key.norm_mode = norm_mode;
+    key.stop_norm = stop_norm;
+    for (int b = 0; b < iters; b++) {   // which of the iterations sort
+        const int r = refresh_period(step + b);
+        if (r > 0 && (step + b) % r == 0) key.sorts |= 1u << b;
     }
-    if (!g.exec) {
+    key.natural = refresh_period(step) == 0;
+    IterGraph *g = nullptr;
+    for (IterGraph &have : graphs)
+        if (have.same(key)) g = &have;
+    if (!g) {
+        if (graphs.size() >= kMaxGraphs) drop_graphs();
         // capture: the launches are recorded, not run, so the host-side counters are put back afterwards
         const int step0 = step;
         const int64_t launches0 = launches;
-        int32_t *const order0 = order;
         cudaGraph_t graph = nullptr;
         B200_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         int rc = 0;
-        for (int b = 0; b < iters && rc == 0; b++) rc = one_iteration(false);
+        for (int b = 0; b < iters && rc == 0; b++) rc = one_iteration(norm_mode, stop_norm);
         const cudaError_t end = cudaStreamEndCapture(stream, &graph);
-        g.launches = launches - launches0;
+        key.launches = launches - launches0;
         step = step0;
         launches = launches0;
-        const bool same_order = order == order0 && (!px || px->parity == parity);
-        if (order != order0) std::swap(order, order_alt);
-        if (px && px->parity != parity) { px->parity = parity; Y2 = px->y_local(parity); w = px->w_local(parity); }
-        if (rc != 0 || end != cudaSuccess || !graph || !same_order) {
-            if (graph) cudaGraphDestroy(graph);
+        const bool same_buffers = !px || px->parity == key.parity;
+        if (px && px->parity != key.parity) { px->parity = key.parity; Y2 = px->y_local(key.parity); w = px->w_local(key.parity); }
+        if (rc == 0 && end == cudaSuccess && graph && same_buffers) key.exec = graph_exec_acquire(host, graph, key.shape());
+        if (graph) cudaGraphDestroy(graph);
+        if (rc != 0 || end != cudaSuccess || !key.exec) {
             (void)cudaGetLastError();
             use_graphs = false;   // the caller falls back to direct launches
             return 1;
         }
-        const cudaError_t inst = cudaGraphInstantiate(&g.exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (inst != cudaSuccess) {
-            (void)cudaGetLastError();
-            g = IterGraph();
-            use_graphs = false;
-            return 1;
-        }
-        g.iters = iters;
-        g.eta = eta; g.exaggeration = exag; g.momentum = momentum; g.refresh = order_refresh; g.parity = parity;
+        graphs.push_back(key);
+        g = &graphs.back();
     }
-    B200_CUDA(cudaGraphLaunch(g.exec, stream));
+    B200_CUDA(cudaGraphLaunch(g->exec, stream));
     step += iters;
-    launches += g.launches;
+    launches += g->launches;
     return 0;
 }
 
 int Session::iterate(int n_iters, float min_gradient_norm, float *elapsed_ms, int *iters_done)
 {
     B200_CUDA(cudaSetDevice(device));
+    const bool multi = comm && comm->world > 1;
     const bool early_stop = min_gradient_norm > 0.0f;
-    const bool want_norm = early_stop || force_norm;
+    // One GPU checks the norm on the device: the host queues a block of iterations and learns afterwards how many of
+    // them took place (the ones after the stop change nothing).  Ranks have to take the decision together, on the host.
+    const bool device_stop = early_stop && !multi;
+    const int norm_mode = device_stop ? 2 : (early_stop || force_norm ? 1 : 0);
     int done = 0;
+    bool stopped = false;
     B200_CUDA(cudaEventRecord(ev_t0, stream));
-    for (int it = 0; it < n_iters; it++) {
+    if (device_stop) {   // no iteration of this call has a norm yet: a huge one in the slot that the first looks at
+        B200_CUDA(cudaMemsetAsync(&state->unorm2[(step & 1) ^ 1], 0x7f, sizeof(double), stream));
+    }
+    for (int it = 0; it < n_iters && !stopped;) {
         // a meeting of the ranks gave up (the kernel says so in mapped host memory): queue nothing more
         if (px && *px->err_host) break;
-        int kind = 0;
-        const int block = graph_block(n_iters - it, want_norm, &kind);
+        int block = (early_stop && multi) || (norm_mode == 1) ? 0 : graph_block(n_iters - it);
+        const int step0 = step;
         if (block > 0) {
-            const int rc = run_graph_block(kind, block);
+            const int rc = run_graph_block(block, norm_mode, min_gradient_norm);
             if (rc < 0) return rc;
-            if (rc == 0) { done += block; it += block - 1; continue; }
+            if (rc != 0) block = 0;
         }
-        if (want_norm) B200_CUDA(cudaMemsetAsync(&state->unorm2, 0, sizeof(double), stream));
-        B200_TRY(one_iteration(want_norm));
-        done++;
-        if (early_stop) {
-            B200_CUDA(cudaMemcpyAsync(h_state, state, sizeof(IterState), cudaMemcpyDeviceToHost, stream));
-            B200_CUDA(cudaStreamSynchronize(stream));
-            double n2 = h_state->unorm2;
-            if (comm && comm->world > 1) {
-                // every rank must take the same decision: sum the squared norms
-                B200_TRY(comm->all_reduce_sum_f64(&state->unorm2, 1, stream));
-                B200_CUDA(cudaMemcpyAsync(h_state, state, sizeof(IterState), cudaMemcpyDeviceToHost, stream));
-                B200_CUDA(cudaStreamSynchronize(stream));
-                n2 = h_state->unorm2;
-            }
-            last_unorm = (float)sqrt(n2);
-            if (last_unorm < min_gradient_norm) break;
+        if (block == 0) {
+            B200_TRY(one_iteration(norm_mode, min_gradient_norm));
+            block = 1;
         }
+        it += block;
+        done += block;
+        if (!early_stop) continue;
+        const int last = (step - 1) & 1;
+        B200_CUDA(cudaMemcpyAsync(h_state, state, sizeof(IterState), cudaMemcpyDeviceToHost, stream));
+        B200_CUDA(cudaStreamSynchronize(stream));
+        if (device_stop) {
+            const int took = h_state->done - done_seen;
+            done_seen = h_state->done;
+            done -= block - took;
+            step = step0 + took;
+            last_unorm = (float)sqrt(h_state->unorm2[last]);   // of the last one that took place: later ones repeat it
+            stopped = took < block || last_unorm < min_gradient_norm;
+            // the queued rest has gone through the state slots without changing anything but their turn
+            if ((block - took) & 1) B200_TRY(launch_state_swap(state, stream));
+            continue;
+        }
+        // every rank must take the same decision: sum the squared norms
+        B200_TRY(comm->all_reduce_sum_f64(&state->unorm2[last], 1, stream));
+        B200_CUDA(cudaMemcpyAsync(h_state, state, sizeof(IterState), cudaMemcpyDeviceToHost, stream));
+        B200_CUDA(cudaStreamSynchronize(stream));
+        last_unorm = (float)sqrt(h_state->unorm2[last]);
+        if (last_unorm < min_gradient_norm) stopped = true;
     }
     B200_CUDA(cudaEventRecord(ev_t1, stream));
     B200_CUDA(cudaMemcpyAsync(h_state, state, sizeof(IterState), cudaMemcpyDeviceToHost, stream));
@@ -530,8 +559,9 @@ int Session::iterate(int n_iters, float min_gradient_norm, float *elapsed_ms, in
     B200_CUDA(cudaStreamSynchronize(stream2));
     if (elapsed_ms) B200_CUDA(cudaEventElapsedTime(elapsed_ms, ev_t0, ev_t1));
     if (iters_done) *iters_done = done;
-    if (done > 0) last_Z = (float)h_state->zsum[(step - 1) & 1] - (float)N;
-    if (want_norm && !early_stop && done > 0) last_unorm = (float)sqrt(h_state->unorm2);
+    done_seen = h_state->done;
+    if (done > 0) last_Z = (float)h_state->z_last - (float)N;
+    if (norm_mode == 1 && !early_stop && done > 0) last_unorm = (float)sqrt(h_state->unorm2[(step - 1) & 1]);
     if (h_state->bad) { set_error("non-finite coordinates in the embedding"); return -3; }
     if (px) {
         int expired = 0;

@@ -99,22 +99,32 @@ struct Session {
     bool grid_two_shot = false;   // peer-memory exchange: the grid sum as slice owners (peer.h), chosen at attach
     int attach_peer_exchange();   // collective, after comm is set
 
-    // Captured iterations (single GPU or peer-memory exchange, no stage timers, no update norm): at small N the loop is bound by the
-    // launch and dependency latency of its ten kernels, so whole blocks of iterations are replayed as CUDA
-    // graphs.  One graph per phase of the schedule: [0] exaggerated, [1] the 50 iterations after, [2]
-    // settled.  A block holds an even number of iterations (the state slots alternate) and an even number
-    // of order refreshes (the two order buffers swap at each).
+    // Captured iterations (single GPU or peer-memory exchange, no stage timers): at small N the loop is bound by the
+    // launch and dependency latency of its kernels, so blocks of iterations are replayed as CUDA graphs.  What a block
+    // froze into its launches is its key.
     struct IterGraph {
         cudaGraphExec_t exec = nullptr;
-        int iters = 0;
+        int iters = 0, parity = 0, norm_mode = 0;
+        bool late = false, natural = false;
+        unsigned sorts = 0;        // bit b: the b-th iteration sorts the spread order
+        float eta = 0, exaggeration = 0, momentum = 0, stop_norm = 0;
         int64_t launches = 0;
-        float eta = 0, exaggeration = 0, momentum = 0;
-        int refresh = 0, parity = 0;
+        // what decides which nodes it has: an executable of the same shape can be updated instead of made anew
+        unsigned long long shape() const { return (unsigned long long)sorts << 32 | (unsigned)iters << 2 | (unsigned)natural << 1; }
+        bool same(const IterGraph &o) const
+        {
+            return iters == o.iters && parity == o.parity && norm_mode == o.norm_mode && late == o.late && natural == o.natural &&
+                   sorts == o.sorts && eta == o.eta && exaggeration == o.exaggeration && momentum == o.momentum && stop_norm == o.stop_norm;
+        }
     };
-    IterGraph graphs[3];
+    static constexpr int kGraphIters = 16;   // iterations of a large block; what is left of a phase goes in pairs
+    static constexpr size_t kMaxGraphs = 24;
+    std::vector<IterGraph> graphs;
     bool use_graphs = true;   // B200TSNE_GRAPHS=0 turns them off
-    int graph_block(int remaining, bool want_norm, int *kind) const;   // iterations the next graph would cover, 0 = none
-    int run_graph_block(int kind, int iters);
+    int refresh_period(int at) const;   // iterations between two sorts of the spread order at step `at` (0: natural order)
+    int graph_block(int remaining) const;
+    int run_graph_block(int iters, int norm_mode, float stop_norm);
+    int done_seen = 0;        // IterState::done as the host last saw it
     void drop_graphs();
 
     int64_t rows() const { return row_hi - row_lo; }
@@ -126,7 +136,7 @@ struct Session {
     int get_optimizer_soa(float *momentum_host, float *gains_host);
     int set_optimizer_soa(const float *momentum_host, const float *gains_host);
     int iterate(int n_iters, float min_gradient_norm, float *elapsed_ms, int *iters_done);
-    int one_iteration(bool want_norm);
+    int one_iteration(int norm_mode, float stop_norm);
     int attractive(cudaStream_t st);   // Fattr of the owned rows from the current embedding
     int attractive_launches() const { return blocked.ready ? (resident ? 1 : 3) + (blocked.extra_C > 0) : 1 + (extra.count > 0); }
     int affinities_from_points(const float *X_host, int D, float perplexity, float eps);
