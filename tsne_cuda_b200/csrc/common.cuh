@@ -78,8 +78,6 @@ __host__ __device__ inline float dec_float(unsigned int e)
 int launch_transpose(const float *X, int64_t N, int D, float *XT, cudaStream_t st);   // [N][D] -> [D][N]
 int launch_knn_exact(const float *XT, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo,
                      int64_t db_hi, int32_t *ids, float *d2, cudaStream_t st);   // ids/d2 keep (INT_MAX,+inf) in unfilled slots
-int launch_knn_exact_rows(const float *XT, int64_t N, int D, int K, const int *q_index, int64_t nq, int64_t out_base,
-                          int64_t db_lo, int64_t db_hi, int32_t *ids, float *d2, cudaStream_t st);
 // knn_tc.cu: tensor-core filter + exact re-rank + proof (nd = database rows to scan)
 bool knn_tc_supported(int64_t nd, int D, int K);
 size_t knn_tc_workspace_bytes(int D, int K, int64_t nq, int64_t nd);
@@ -95,6 +93,12 @@ struct KnnStats {
 // X: [N][D] row-major on the device; picks the path, handles the fallback rows, synchronises `st`.
 int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo, int64_t db_hi,
                int32_t *ids, float *d2, KnnStats *stats, cudaStream_t st);
+// knn_dense.cu: whole rows of distances and a selection (see that file); distances of NaN never rank
+struct DeviceArena;
+bool knn_dense_supported(int K);
+int knn_dense(const float *X, int D, int K, int64_t q_lo, int64_t nq, const int *q_index, int64_t out_base, int64_t db_lo, int64_t db_hi,
+              int32_t *ids, float *d2, DeviceArena &tmp, cudaStream_t st);
+int knn_dense_in_scratch(const float *X, int64_t N, int D, int K, float *scratch, long long floats, int32_t *ids, float *d2, cudaStream_t st);
 // knn.cu: search with the scratch in a fixed device array of the library (no allocation)
 long long knn_noalloc_max_elems();
 int knn_noalloc(const float *X, int64_t N, int D, int K, int32_t *ids, float *d2, cudaStream_t st);

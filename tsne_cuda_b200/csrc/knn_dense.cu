@@ -1,0 +1,313 @@
+// Exact k-nearest-neighbour search by whole rows of distances: every canonical distance of a group of queries is
+// written out, then a block per query selects its K smallest.
+//
+// Used where the query x database product is small: databases below the tensor-core search's range, the rows that
+// search could not certify, and callers that must not allocate.  A search that keeps a running list per query
+// (knn_exact_kernel) serves 64 queries per block and inserts survivors one at a time: at 1,500 points that is 24 blocks on
+// 148 SMs, and half of the time goes into insertions.  Here the distances are a plain tiled product over all SMs (three
+// unfused fp32 instructions per pair and dimension, the bound), and the selection is a bisection on the bits of keys
+// held in registers.  Measured on B200 (start of the path / now):
+// 4,099 points of 64 dimensions, K = 16: 1.69 / 0.31 ms; 1,500 x 20, K = 32: 1.63 / 0.06 ms; five rows of 60,000 x 784:
+// 4.4 / 0.4 ms.
+#include <limits.h>
+
+#include <algorithm>
+
+#include "session.h"
+
+namespace b200 {
+namespace {
+
+constexpr int kTileP = 128;    // database points per tile
+constexpr int kDims = 32;      // dimensions per shared-memory chunk
+constexpr int kThreads = 256;
+
+// dist[q * ld + p] = canonical distance (sequential over the dimensions, every operation rounded) of query q of the list
+// and database row db_lo + p.  QT queries and eight points a thread, 16 QT queries and 128 points a block.
+template <int QT>
+__global__ void __launch_bounds__(kThreads)
+dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long long nq, const int *__restrict__ q_index, long long db_lo,
+                      long long nd, float *__restrict__ dist, long long ld)
+{
+    constexpr int kTileQ = 16 * QT, kQs = kTileQ + 4, kPs = kTileP + 4;
+    __shared__ __align__(16) float Qs[kDims][kQs], Ps[kDims][kPs];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31, warp = tid >> 5;
+    const long long p0 = (long long)blockIdx.x * kTileP, q0 = (long long)blockIdx.y * kTileQ;
+    float acc[QT][8];
+#pragma unroll
+    for (int a = 0; a < QT; a++)
+#pragma unroll
+        for (int b = 0; b < 8; b++) acc[a][b] = 0.0f;
+    for (int d0 = 0; d0 < D; d0 += kDims) {
+        const int dlen = min(kDims, D - d0);
+        __syncthreads();
+        // a warp reads 32 dimensions of one row at a time (coalesced) and stores them as a column
+        for (int q = warp; q < kTileQ; q += kThreads / 32) {
+            const long long pos = q0 + q;
+            float v = 0.0f;
+            if (pos < nq && lane < dlen) v = X[(q_index ? (long long)q_index[pos] : q_lo + pos) * D + d0 + lane];
+            Qs[lane][q] = v;
+        }
+        for (int p = warp; p < kTileP; p += kThreads / 32) {
+            float v = 0.0f;
+            if (p0 + p < nd && lane < dlen) v = X[(db_lo + p0 + p) * D + d0 + lane];
+            Ps[lane][p] = v;
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int d = 0; d < dlen; d++) {
+            float qv[QT];
+            if constexpr (QT == 4) {
+                const float4 q4 = *reinterpret_cast<const float4 *>(&Qs[d][ty * 4]);
+                qv[0] = q4.x; qv[1] = q4.y; qv[2] = q4.z; qv[3] = q4.w;
+            } else {
+#pragma unroll
+                for (int a = 0; a < QT; a++) qv[a] = Qs[d][ty * QT + a];
+            }
+            const float4 pa = *reinterpret_cast<const float4 *>(&Ps[d][tx * 4]);
+            const float4 pb = *reinterpret_cast<const float4 *>(&Ps[d][64 + tx * 4]);
+            const float pv[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
+#pragma unroll
+            for (int a = 0; a < QT; a++)
+#pragma unroll
+                for (int b = 0; b < 8; b++) {
+                    const float t = __fsub_rn(qv[a], pv[b]);
+                    acc[a][b] = __fadd_rn(acc[a][b], __fmul_rn(t, t));
+                }
+        }
+    }
+    // (rows of dist are padded to whole tiles: every store stays inside)
+#pragma unroll
+    for (int a = 0; a < QT; a++) {
+        const long long q = q0 + ty * QT + a;
+        if (q >= nq) continue;
+        float *row = dist + q * ld + p0;
+        *reinterpret_cast<float4 *>(row + tx * 4) = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+        *reinterpret_cast<float4 *>(row + 64 + tx * 4) = make_float4(acc[a][4], acc[a][5], acc[a][6], acc[a][7]);
+    }
+}
+
+// The sum over the block, for every thread.  buf: one int per warp and parity (two calls in flight share no slot).
+__device__ __forceinline__ int block_sum(int v, int *buf)
+{
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0) buf[threadIdx.x >> 5] = v;
+    __syncthreads();
+    int t = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; w++) t += buf[w];
+    return t;
+}
+
+constexpr unsigned kInfBits = 0x7f800000u;   // distances are >= 0: their bits order like them; NaN lies above and never ranks
+constexpr int kMaxDenseK = 512;
+
+// One block per (query, segment).  The n values of segment s of query q start at val + q * ld + s * seg; with `ids` they
+// carry the ids at the same place (equal values in ascending order of id), else value j has id id_lo + s * seg + j.  The K
+// smallest by (value, id), ascending, go to out row (q * segments + s), or, with out_rows, to row out_rows[q] - out_base;
+// slots without a value get (+inf, INT_MAX).  KPT * 256 >= seg.
+template <int KPT>
+__global__ void __launch_bounds__(kThreads)
+dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ ids, long long ld, long long n_total, long long seg, int id_lo,
+                    int K, const int *__restrict__ out_rows, long long out_base, float *__restrict__ out_d, int32_t *__restrict__ out_i)
+{
+    __shared__ unsigned long long s_key[kMaxDenseK];
+    __shared__ int s_sum[2][kThreads / 32];
+    __shared__ unsigned s_lo[kThreads / 32], s_hi[kThreads / 32];
+    __shared__ int s_n, s_before;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long q = blockIdx.y, s = blockIdx.x;
+    const long long base = q * ld + s * seg;
+    const int n = (int)min(seg, n_total - s * seg);
+    unsigned key[KPT];
+    unsigned lo = 0xffffffffu, hi = 0u;
+    int valid = 0;
+#pragma unroll
+    for (int j = 0; j < KPT; j++) {
+        const int e = j * kThreads + tid;
+        key[j] = e < n ? __float_as_uint(val[base + e]) : 0xffffffffu;
+        if (key[j] <= kInfBits) { lo = min(lo, key[j]); hi = max(hi, key[j]); valid++; }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) { s_lo[warp] = lo; s_hi[warp] = hi; }
+    if (tid == 0) { s_n = 0; s_before = 0; }
+    int turn = 0;
+    valid = block_sum(valid, s_sum[turn++ & 1]);
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; w++) { lo = min(lo, s_lo[w]); hi = max(hi, s_hi[w]); }
+    // v: the smallest bound with at least K keys <= v
+    int at_most = valid;
+    unsigned v = hi;
+    if (valid > K) {
+        unsigned a = lo, b = hi;
+        while (a < b) {
+            const unsigned mid = a + ((b - a) >> 1);
+            int c = 0;
+#pragma unroll
+            for (int j = 0; j < KPT; j++) c += key[j] <= mid;
+            c = block_sum(c, s_sum[turn++ & 1]);
+            if (c >= K) { b = mid; at_most = c; if (c == K) break; }
+            else a = mid + 1;
+        }
+        v = b;
+    }
+    auto id_of = [&](int e) { return ids ? ids[base + e] : (int32_t)(id_lo + s * seg + e); };
+    auto keep = [&](int slot, int j) {
+        s_key[slot] = (unsigned long long)key[j] << 32 | (unsigned)id_of(j * kThreads + tid);
+    };
+    const bool ties = valid > K && at_most > K;   // more keys equal to v than there is room for: the first in order of id
+    if (valid > 0) {
+#pragma unroll
+        for (int j = 0; j < KPT; j++)
+            if (key[j] <= kInfBits && (ties ? key[j] < v : key[j] <= v)) keep(atomicAdd(&s_n, 1), j);
+    }
+    __syncthreads();
+    if (ties) {
+        const int room = K - s_n;
+        const int at = s_n;
+        for (int j = 0; j < KPT && s_before < room; j++) {
+            bool eq = false;
+#pragma unroll
+            for (int t = 0; t < KPT; t++) eq = t == j ? key[t] == v : eq;
+            const unsigned m = __ballot_sync(0xffffffffu, eq);
+            if (lane == 0) s_sum[0][warp] = __popc(m);
+            __syncthreads();
+            int before = s_before + __popc(m & ((1u << lane) - 1u));
+            for (int w = 0; w < warp; w++) before += s_sum[0][w];
+            if (eq && before < room) s_key[at + before] = (unsigned long long)v << 32 | (unsigned)id_of(j * kThreads + tid);
+            __syncthreads();
+            if (tid == 0)
+                for (int w = 0; w < kThreads / 32; w++) s_before += s_sum[0][w];
+            __syncthreads();
+        }
+    }
+    __syncthreads();
+    // rank by counting: K is at most a few hundred
+    const int got = min(valid, K);
+    const long long row = out_rows ? out_rows[q] - out_base : q * gridDim.x + s;
+    for (int e = tid; e < K; e += kThreads) {
+        if (e < got) {
+            const unsigned long long mine = s_key[e];
+            int rank = 0;
+            for (int u = 0; u < got; u++) rank += s_key[u] < mine;
+            out_d[row * K + rank] = __uint_as_float((unsigned)(mine >> 32));
+            out_i[row * K + rank] = (int32_t)(unsigned)mine;
+        } else {
+            out_d[row * K + e] = INFINITY;
+            out_i[row * K + e] = INT_MAX;
+        }
+    }
+}
+
+constexpr long long kMaxSegment = 48 * kThreads;   // values one block selects from (12,288)
+
+int launch_select(const float *val, const int32_t *ids, long long ld, long long n, long long seg, int segments, long long nq, int id_lo, int K,
+                  const int *out_rows, long long out_base, float *out_d, int32_t *out_i, cudaStream_t st)
+{
+    const long long longest = std::min(n, seg);
+    for (long long q = 0; q < nq; q += 65535) {   // grid.y
+        const dim3 grid((unsigned)segments, (unsigned)std::min<long long>(65535, nq - q));
+        const float *v = val + q * ld;
+        const int32_t *i = ids ? ids + q * ld : nullptr;
+        const int *r = out_rows ? out_rows + q : nullptr;
+        float *od = out_rows ? out_d : out_d + q * segments * K;
+        int32_t *oi = out_rows ? out_i : out_i + q * segments * K;
+        if (longest <= 4 * kThreads) dense_select_kernel<4><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        else if (longest <= 8 * kThreads) dense_select_kernel<8><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        else if (longest <= 16 * kThreads) dense_select_kernel<16><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        else if (longest <= 32 * kThreads) dense_select_kernel<32><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        else dense_select_kernel<48><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        B200_CUDA(cudaGetLastError());
+    }
+    return 0;
+}
+
+int launch_distances(const float *X, int D, int64_t q_lo, int64_t nq, const int *q_index, int64_t db_lo, int64_t nd, float *dist, long long ld,
+                     cudaStream_t st)
+{
+    if (nd <= 0) return 0;
+    const unsigned tiles = (unsigned)((nd + kTileP - 1) / kTileP);
+    // a short list of queries: 16 a block waste less of the tile
+    if (nq > 48) {
+        for (int64_t q = 0; q < nq; q += 65535 * 64) {
+            const int64_t m = std::min<int64_t>(65535 * 64, nq - q);
+            dense_distance_kernel<4><<<dim3(tiles, (unsigned)((m + 63) / 64)), kThreads, 0, st>>>(X, D, q_lo + q, m, q_index ? q_index + q : nullptr,
+                                                                                               db_lo, nd, dist + q * ld, ld);
+        }
+    } else {
+        dense_distance_kernel<1><<<dim3(tiles, (unsigned)((nq + 15) / 16)), kThreads, 0, st>>>(X, D, q_lo, nq, q_index, db_lo, nd, dist, ld);
+    }
+    B200_CUDA(cudaGetLastError());
+    return 0;
+}
+
+long long padded(long long nd) { return (nd + kTileP - 1) / kTileP * kTileP; }
+}  // namespace
+
+bool knn_dense_supported(int K) { return K <= kMaxDenseK; }
+
+// Queries [q_lo, q_lo + nq), or the nq rows that q_index lists, against database rows [db_lo, db_hi); the list of query
+// number p goes to row p of ids / d2, of listed row g to row g - out_base.  Queues everything on st; the buffers come
+// from tmp, which must outlive the work.
+int knn_dense(const float *X, int D, int K, int64_t q_lo, int64_t nq, const int *q_index, int64_t out_base, int64_t db_lo, int64_t db_hi,
+              int32_t *ids, float *d2, DeviceArena &tmp, cudaStream_t st)
+{
+    const long long nd = db_hi - db_lo, ld = padded(std::max<long long>(nd, 1));
+    if (nq <= 0) return 0;
+    if (!knn_dense_supported(K)) { set_error("knn_dense: K too large"); return -4; }
+    const long long seg = nd <= kMaxSegment ? std::max<long long>(nd, 1) : kMaxSegment;
+    const int segments = (int)std::max<long long>(1, (nd + seg - 1) / seg);
+    // queries per round: at most 2^26 distances (256 MB)
+    const int64_t round = std::max<int64_t>(1, std::min<int64_t>(nq, (1ll << 26) / ld));
+    float *dist = nullptr, *part_d[2] = {nullptr, nullptr};
+    int32_t *part_i[2] = {nullptr, nullptr};
+    B200_TRY(tmp.alloc((void **)&dist, sizeof(float) * (size_t)round * ld));
+    if (segments > 1)
+        for (int k = 0; k < 2; k++) {
+            B200_TRY(tmp.alloc((void **)&part_d[k], sizeof(float) * (size_t)round * segments * K));
+            B200_TRY(tmp.alloc((void **)&part_i[k], sizeof(int32_t) * (size_t)round * segments * K));
+        }
+    for (int64_t q = 0; q < nq; q += round) {
+        const int64_t m = std::min<int64_t>(round, nq - q);
+        const int *index = q_index ? q_index + q : nullptr;
+        float *final_d = q_index ? d2 : d2 + q * K;
+        int32_t *final_i = q_index ? ids : ids + q * K;
+        B200_TRY(launch_distances(X, D, q_lo + q, m, index, db_lo, nd, dist, ld, st));
+        if (segments == 1) {
+            B200_TRY(launch_select(dist, nullptr, ld, nd, seg, 1, m, (int)db_lo, K, index, out_base, final_d, final_i, st));
+            continue;
+        }
+        // the best of every segment, then of those lists (a level more while they are too long for a block)
+        B200_TRY(launch_select(dist, nullptr, ld, nd, seg, segments, m, (int)db_lo, K, nullptr, 0, part_d[0], part_i[0], st));
+        long long lists = segments;
+        int from = 0;
+        while (lists * K > kMaxSegment) {
+            const long long per = kMaxSegment / K;   // lists that one block merges
+            const long long next = (lists + per - 1) / per;
+            B200_TRY(launch_select(part_d[from], part_i[from], lists * K, lists * K, per * K, (int)next, m, 0, K, nullptr, 0, part_d[from ^ 1],
+                                   part_i[from ^ 1], st));
+            lists = next;
+            from ^= 1;
+        }
+        B200_TRY(launch_select(part_d[from], part_i[from], lists * K, lists * K, lists * K, 1, m, 0, K, index, out_base, final_d, final_i, st));
+    }
+    return 0;
+}
+
+// The same for all points against all, in scratch of `floats` floats that the caller owns; -1 when it is too small for
+// that to be worth it (the caller then searches another way).
+int knn_dense_in_scratch(const float *X, int64_t N, int D, int K, float *scratch, long long floats, int32_t *ids, float *d2, cudaStream_t st)
+{
+    const long long ld = padded(N);
+    const int64_t round = floats / ld / 64 * 64;
+    if (N > kMaxSegment || !knn_dense_supported(K) || round < 64) return -1;
+    for (int64_t q = 0; q < N; q += round) {
+        const int64_t m = std::min<int64_t>(round, N - q);
+        B200_TRY(launch_distances(X, D, q, m, nullptr, 0, N, scratch, ld, st));
+        B200_TRY(launch_select(scratch, nullptr, ld, N, N, 1, m, 0, K, nullptr, 0, d2 + q * K, ids + q * K, st));
+    }
+    return 0;
+}
+
+}  // namespace b200
