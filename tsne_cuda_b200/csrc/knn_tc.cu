@@ -311,63 +311,109 @@ __device__ __forceinline__ size_t image_offset_bf16_swizzled(int r, int k, int s
 // query and a database operand, a = a_hi + a_lo + a_r,  |dropped| <= |a_lo||b_lo| + |a - a_r||b_r| + |a_r||b - b_r|
 // + |a_r||b_r| (Cauchy-Schwarz on the leftover vectors).  Queries record |a_lo| and |a_r| (res), the database the
 // largest |b_lo|/|b| and |b_r|/|b| over its rows (rho_bits: float bits, raised with atomicMax).
-__global__ void __launch_bounds__(128)
+//
+// A block makes one tile image: 64 dimensions of its 128 rows at a time go through shared memory, so that rows are read
+// and 16-byte pieces of the image written coalesced (a thread per row, as the TF32 form has it, touches 32 sectors per
+// load: 1.2 ms for 10^6 rows of 50 dimensions, 0.56 ms for 50,000 of 1,024; now 0.12 and 0.10).  Xp (optional): the rows in
+// list order, Xp[pos] = X[list[pos]], zeros for padding: the re-rank reads ~100 candidate rows per query, and in cell order
+// the candidates of neighbouring queries share a few megabytes that stay in L2.
+constexpr int kPrepDims = 64;
+__global__ void __launch_bounds__(256)
 knn_tc_prepare_bf16_kernel(const float *__restrict__ X, const int *__restrict__ list, int D, int Dp, int KC, int sw, int db_form,
                            __nv_bfloat16 *__restrict__ img, double *__restrict__ norms, float2 *__restrict__ res,
-                           int *__restrict__ rho_bits)
+                           int *__restrict__ rho_bits, float *__restrict__ Xp)
 {
+    __shared__ float xs[TM][kPrepDims + 1];
+    __shared__ float s_nf[TM], s_rest[TM];
+    __shared__ int s_row[TM];
     const long long tile = blockIdx.x;
-    const int r = threadIdx.x;
-    const long long pos = tile * TM + r;
-    const int i = list[pos];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < TM) s_row[tid] = list[tile * TM + tid];
     __nv_bfloat16 *im_tile = img + (size_t)tile * 2 * Dp * 128;
     const size_t part = (size_t)KC * 128;
-    double n2 = 0.0;
-    for (int k = 0; k < D; k++) {
-        const float x = (i >= 0) ? X[(long long)i * D + k] : 0.0f;
-        n2 += (double)x * (double)x;
-    }
-    const float nf = (i >= 0) ? (float)n2 : 3.0e38f;
-    const float nf_hi = __bfloat162float(__float2bfloat16_rn(nf));
-    const float nf_rest = (nf - nf_hi) - __bfloat162float(__float2bfloat16_rn(nf - nf_hi));   // both differences are exact in fp32
-    double lo2 = 0.0, r2 = 0.0;   // squared norms of the lo parts and of the leftovers of the data columns
-    for (int k = 0; k < Dp; k++) {
-        float v = 0.0f;
-        if (k < D) {
-            const float x = (i >= 0) ? X[(long long)i * D + k] : 0.0f;
-            v = db_form ? -2.0f * x : x;
-        } else if (k == D) {
-            v = db_form ? nf : ((i >= 0) ? 1.0f : 0.0f);
-        } else if (k == D + 1) {
-            v = db_form ? nf_rest : ((i >= 0) ? 1.0f : 0.0f);
+    const int row = tid >> 1, half = tid & 1;   // two threads share a row's sums
+    double n2 = 0.0, lo2 = 0.0, r2 = 0.0;       // squared norms of the row, of its lo parts and of its leftovers
+    for (int k0 = 0; k0 < Dp; k0 += kPrepDims) {
+        __syncthreads();
+        for (int r = warp; r < TM; r += 8) {
+            const int i = s_row[r];
+#pragma unroll
+            for (int h = 0; h < kPrepDims; h += 32) {
+                const int k = k0 + h + lane;
+                const float x = (i >= 0 && k < D) ? X[(long long)i * D + k] : 0.0f;
+                xs[r][h + lane] = x;
+                if (Xp && k < D) Xp[(tile * TM + r) * D + k] = x;
+            }
         }
-        const __nv_bfloat16 vh = __float2bfloat16_rn(v);
-        const float rest = v - __bfloat162float(vh);
-        const __nv_bfloat16 vl = __float2bfloat16_rn(rest);
-        __nv_bfloat16 *im = im_tile + (size_t)(k / KC) * 2 * part;
-        const size_t at = sw ? image_offset_bf16_swizzled(r, k % KC, sw) : image_offset_bf16(r, k % KC);
-        im[at] = vh;
-        im[part + at] = vl;
-        if (k < D) {
-            const float left = rest - __bfloat162float(vl);
-            lo2 += (double)__bfloat162float(vl) * (double)__bfloat162float(vl);
-            r2 += (double)left * (double)left;
+        __syncthreads();
+        if (k0 < D) {
+            float lo_sum = 0.0f, left_sum = 0.0f;   // bounds, rounded up below: float sums of 32 squares will do
+            for (int m = 0; m < kPrepDims / 2; m++) {
+                const float x = xs[row][2 * m + half];
+                n2 += (double)x * (double)x;
+                const float rest = x - __bfloat162float(__float2bfloat16_rn(x));
+                const float lo = __bfloat162float(__float2bfloat16_rn(rest)), left = rest - lo;
+                lo_sum = fmaf(lo, lo, lo_sum);
+                left_sum = fmaf(left, left, left_sum);
+            }
+            lo2 += (double)lo_sum;
+            r2 += (double)left_sum;
+        }
+        if (k0 + kPrepDims > D) {   // the columns from D on carry the norm
+            const double total = n2 + __shfl_xor_sync(0xffffffffu, n2, 1);
+            const float nf = s_row[row] >= 0 ? (float)total : 3.0e38f;
+            const float hi = __bfloat162float(__float2bfloat16_rn(nf));
+            if (half == 0) {
+                s_nf[row] = nf;
+                s_rest[row] = (nf - hi) - __bfloat162float(__float2bfloat16_rn(nf - hi));   // both differences are exact in fp32
+            }
+            __syncthreads();
+        }
+        for (int idx = tid; idx < TM * (kPrepDims / 8); idx += 256) {
+            const int r = idx & (TM - 1), o = (idx >> 7) * 8, k = k0 + o;
+            if (k >= Dp) break;
+            const bool real = s_row[r] >= 0;
+            __align__(16) __nv_bfloat162 hi[4], lo[4];
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                float v[2];
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int kk = k + e + u;
+                    const float x = xs[r][o + e + u];
+                    v[u] = kk < D ? (db_form ? -2.0f * x : x) : 0.0f;
+                    if (kk == D) v[u] = db_form ? s_nf[r] : (real ? 1.0f : 0.0f);
+                    if (kk == D + 1) v[u] = db_form ? s_rest[r] : (real ? 1.0f : 0.0f);
+                }
+                hi[e / 2] = __floats2bfloat162_rn(v[0], v[1]);
+                lo[e / 2] = __floats2bfloat162_rn(v[0] - __low2float(hi[e / 2]), v[1] - __high2float(hi[e / 2]));
+            }
+            __nv_bfloat16 *im = im_tile + (size_t)(k / KC) * 2 * part;
+            const size_t at = sw ? image_offset_bf16_swizzled(r, k % KC, sw) : image_offset_bf16(r, k % KC);
+            *reinterpret_cast<uint4 *>(im + at) = *reinterpret_cast<const uint4 *>(hi);
+            *reinterpret_cast<uint4 *>(im + part + at) = *reinterpret_cast<const uint4 *>(lo);
         }
     }
-    if (norms) norms[pos] = n2;
-    if (res) res[pos] = make_float2((float)(sqrt(lo2) * 1.000001), (float)(sqrt(r2) * 1.000001));   // rounded up
+    n2 += __shfl_xor_sync(0xffffffffu, n2, 1);
+    lo2 += __shfl_xor_sync(0xffffffffu, lo2, 1);
+    r2 += __shfl_xor_sync(0xffffffffu, r2, 1);
+    const long long pos = tile * TM + row;
+    if (half == 0) {
+        if (norms) norms[pos] = n2;
+        if (res) res[pos] = make_float2((float)(sqrt(lo2) * 1.00001), (float)(sqrt(r2) * 1.00001));   // rounded up
+    }
     if (rho_bits) {
-        float rl = 0.0f, rr = 0.0f;
-        if (i >= 0 && n2 > 0.0) {
-            rl = (float)(sqrt(lo2 / (4.0 * n2)) * 1.000001);
-            rr = (float)(sqrt(r2 / (4.0 * n2)) * 1.000001);
+        float rl = 0.0f, rr = 0.0f;   // relative to the row: the factor -2 of the database form cancels
+        if (s_row[row] >= 0 && n2 > 0.0) {
+            rl = (float)(sqrt(lo2 / n2) * 1.00001);
+            rr = (float)(sqrt(r2 / n2) * 1.00001);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             rl = fmaxf(rl, __shfl_xor_sync(0xffffffffu, rl, o));
             rr = fmaxf(rr, __shfl_xor_sync(0xffffffffu, rr, o));
         }
-        if ((threadIdx.x & 31) == 0) {   // non-negative floats: integer order == float order
+        if (lane == 0) {   // non-negative floats: integer order == float order
             atomicMax(rho_bits + 0, __float_as_int(rl));
             atomicMax(rho_bits + 1, __float_as_int(rr));
         }
@@ -1349,9 +1395,8 @@ knn_tc_pick_kernel(const float *__restrict__ cand_key, const int32_t *__restrict
     for (int e = out_pos + lane; e < k; e += 32) { ok[e] = INFINITY; oi[e] = INT_MAX; }
 }
 
-// Xp[pos] = X[list[pos]] (zeros for padding): the database rows in visiting order.  The re-rank reads ~130 candidate
-// rows per query; in cell order the candidates of neighbouring queries share a few megabytes that stay in L2,
-// in the original order they are 200-byte reads scattered over the whole array.
+// Xp[pos] = X[list[pos]] (zeros for padding): the database rows in visiting order (the bf16 images' kernel writes them
+// on the way).
 __global__ void knn_gather_rows_kernel(const float *__restrict__ X, const int *__restrict__ list, int D, long long n_pos,
                                        float *__restrict__ Xp)
 {
@@ -1365,46 +1410,37 @@ __global__ void knn_gather_rows_kernel(const float *__restrict__ X, const int *_
 // ------------------------------------------------------------------------------------------------
 // exact re-rank + proof
 // ------------------------------------------------------------------------------------------------
-// The canonical distance: differences, squares and the running sum rounded one by one, in the order of the
-// dimensions.  Rows are read 16 or 8 bytes at a time where D keeps them aligned (a lane reads a row of its own,
-// so wide loads mean fewer sectors touched per instruction); the arithmetic and its order do not change.
+// The canonical distance: differences, squares and the running sum rounded one by one, in the order of the dimensions.
 __device__ __forceinline__ float canon_step(float acc, float x, float y)
 {
     const float t = __fsub_rn(x, y);
     return __fadd_rn(acc, __fmul_rn(t, t));
 }
-__device__ __forceinline__ float canon_dist(const float *__restrict__ a, const float *__restrict__ b, int D)
-{
-    float acc = 0.0f;
-    const unsigned long long both = (unsigned long long)(size_t)a | (unsigned long long)(size_t)b;
-    if ((D & 3) == 0 && (both & 15) == 0) {
-        const float4 *a4 = reinterpret_cast<const float4 *>(a), *b4 = reinterpret_cast<const float4 *>(b);
-        for (int d = 0; d < (D >> 2); d++) {
-            const float4 u = a4[d], v = b4[d];
-            acc = canon_step(acc, u.x, v.x);
-            acc = canon_step(acc, u.y, v.y);
-            acc = canon_step(acc, u.z, v.z);
-            acc = canon_step(acc, u.w, v.w);
-        }
-    } else if ((D & 1) == 0 && (both & 7) == 0) {
-        const float2 *a2 = reinterpret_cast<const float2 *>(a), *b2 = reinterpret_cast<const float2 *>(b);
-        for (int d = 0; d < (D >> 1); d++) {
-            const float2 u = a2[d], v = b2[d];
-            acc = canon_step(acc, u.x, v.x);
-            acc = canon_step(acc, u.y, v.y);
-        }
-    } else {
-        for (int d = 0; d < D; d++) acc = canon_step(acc, a[d], b[d]);
-    }
-    return acc;
-}
 
 constexpr int kRerankWarps = 4;
 constexpr int kMaxL = 256;
+constexpr int kRerankDims = 32;                  // dimensions per stage
+constexpr int kRerankStride = kRerankDims + 4;   // floats per staged row: rows 144 bytes apart, 16-byte reads without conflicts
+constexpr size_t kRerankStage = (size_t)33 * kRerankStride;   // 32 candidate rows and the query
+constexpr size_t rerank_smem(int L) { return kRerankWarps * (sizeof(float) * 2 * kRerankStage + (size_t)L * 16); }
+
+template <int BYTES> __device__ __forceinline__ void async_copy(void *dst, const void *src)
+{
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
+}
 
 // One warp per query of the list (query row qlist[q]; candidate ids are positions in dblist).  Row
 // (qlist[q] - out_base) of ids/d2 ([.][K]) receives the K best candidates by (canonical distance, row id);
 // failed[q] = 1 when the proof does not close for the query.
+//
+// Bound: the candidates' rows out of L2 (K rows per query cannot be left out: 17 GB for 60,000 queries of 784
+// dimensions, K = 90).  So only the candidates that can be among the K best are read: one whose key is more than twice
+// the filter's error above the K-th smallest key cannot (95 of 128 at K = 90, 40 at K = 32).  32 of them at a time are
+// staged 32 dimensions wide, VEC floats a copy, two stages in turn: whole 128-byte lines per request, where a lane that
+// walks its own row touches 32 lines with each.  A lane then reads its row from shared memory and sums in the canonical
+// order.  Measured: 60,000 x 784, K = 90: LATER.
+template <int VEC>
 __global__ void __launch_bounds__(kRerankWarps * 32)
 knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__ qlist, const int *__restrict__ dblist,
                      long long out_base, long long nq, const float *__restrict__ cand_key,
@@ -1415,82 +1451,183 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
                      int *__restrict__ n_failed, float *__restrict__ max_err_ratio, const float *__restrict__ Xp)
 {
     // Xp (optional): the database rows in list order, Xp[pos] = X[dblist[pos]]
-    __shared__ float s_d[kRerankWarps][kMaxL];
-    __shared__ int s_i[kRerankWarps][kMaxL];
+    extern __shared__ __align__(16) float stage_mem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long q = (long long)blockIdx.x * kRerankWarps + w;
     if (q >= nq) return;
     const long long gq = qlist[q];
     const long long orow = gq - out_base;
-    const float *xq = X + gq * D;
     const double ni = norms_exact[q];
-    float worst = 0.0f;   // largest observed |filter distance - canonical distance| among the candidates
-    float T = -INFINITY;
+    float *stage = stage_mem + (size_t)w * (2 * kRerankStage + 4 * L);
+    // evaluated candidates: distance bits and row id, list position, filter key
+    unsigned long long *s_key = reinterpret_cast<unsigned long long *>(stage + 2 * kRerankStage);
+    int *s_pos = reinterpret_cast<int *>(s_key + L);
+    float *s_fkey = reinterpret_cast<float *>(s_pos + L);
+    constexpr int kPer = kMaxL / 32;
+    float key[kPer];
+    int pos[kPer];
+    float T = -INFINITY;   // the largest key of the list: whatever is not in it has a key at least as large
     int n_valid = 0;
-    for (int e = lane; e < L; e += 32) {
-        const int pos = cand_id[q * C + e];
-        int id = (pos != INT_MAX) ? dblist[pos] : INT_MAX;
-        if (id < 0) id = INT_MAX;   // a padding position (never kept by a finite threshold)
-        const float key = cand_key[q * C + e];
-        float dist = INFINITY;
-        if (id != INT_MAX) {
-            dist = canon_dist(xq, Xp ? Xp + (long long)pos * D : X + (long long)id * D, D);
+    unsigned lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        const int e = lane + 32 * j;
+        pos[j] = e < L ? cand_id[q * C + e] : INT_MAX;
+        key[j] = e < L ? cand_key[q * C + e] : INFINITY;
+        if (pos[j] != INT_MAX && dblist[pos[j]] < 0) pos[j] = INT_MAX;   // a padding position (never kept by a finite threshold)
+        if (pos[j] != INT_MAX) {
+            T = fmaxf(T, key[j]);
             n_valid++;
-            T = fmaxf(T, key);
-            const double approx = ni + (double)key;
-            worst = fmaxf(worst, (float)fabs(approx - (double)dist));
+            lo = min(lo, enc_float(key[j]));
+            hi = max(hi, enc_float(key[j]));
         }
-        s_d[w][e] = dist;
-        s_i[w][e] = id;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        worst = fmaxf(worst, __shfl_xor_sync(0xffffffffu, worst, o));
-        T = fmaxf(T, __shfl_xor_sync(0xffffffffu, T, o));
-        n_valid += __shfl_xor_sync(0xffffffffu, n_valid, o);
+    for (int o = 16; o > 0; o >>= 1) T = fmaxf(T, __shfl_xor_sync(0xffffffffu, T, o));
+    n_valid = __reduce_add_sync(0xffffffffu, n_valid);
+    // Error bound of the filter's key for this row: it scales with |x_i||x_j|, and a point whose key is
+    // near T lies within sqrt(|x_i|^2 + T) of x_i, so |x_i||x_j| <= |x_i|^2 + (|x_i|^2 + T)+ up to a factor 2.
+    double E = (double)err_scale * (ni + fmax(0.0, ni + (double)T) + 1.0);
+    double dropped = 0.0;
+    if (res_q) {
+        // bf16 pairs: what the three products drop, bounded from the leftovers of this query and the largest
+        // relative leftovers of the database, for every point with |x_j| <= |x_i| + sqrt(|x_i|^2 + T) (a point
+        // further out cannot come closer than the threshold whatever the error of its key); the last term is
+        // the fp32 rounding of the norm column.  err_scale then covers the accumulation only.
+        const double xi = sqrt(ni), xj = xi + sqrt(fmax(0.0, ni + (double)T));
+        const float2 rq = res_q[q];
+        dropped = 1.001 * 2.0 * xj * ((double)rq.x * (double)rho[0] + xi * (double)rho[1] + (double)rq.y) + 1.2e-7 * xj * xj;
+        E += dropped;
     }
+    const double theta = (double)(D + 4) * 5.9604644775390625e-08;   // (D+4) * 2^-24
+    // The cut: a candidate with key above key_K + 2 E (and the rounding of the canonical sums) has K others before it.
+    float cut = INFINITY;
+    if (n_valid > K) {
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        while (lo < hi) {   // the K-th smallest key by bisection on the bits
+            const unsigned mid = lo + ((hi - lo) >> 1);
+            int c = 0;
+#pragma unroll
+            for (int j = 0; j < kPer; j++) c += pos[j] != INT_MAX && enc_float(key[j]) <= mid;
+            c = __reduce_add_sync(0xffffffffu, c);
+            if (c >= K) hi = mid;
+            else lo = mid + 1;
+            if (c == K) break;
+        }
+        float kth = -INFINITY;   // exactly the key: the bound may lie anywhere in the gap above it
+#pragma unroll
+        for (int j = 0; j < kPer; j++)
+            if (pos[j] != INT_MAX && enc_float(key[j]) <= hi) kth = fmaxf(kth, key[j]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) kth = fmaxf(kth, __shfl_xor_sync(0xffffffffu, kth, o));
+        const double kk = (double)kth;
+        cut = __double2float_ru(kk + 2.0 * E + 4.0 * theta * fmax(0.0, ni + kk + E) + 1e-30);
+    }
+    // the evaluated ones, close together
+    int m = 0;
+    float outside = INFINITY;   // the smallest key of a candidate that is left out
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        const bool valid = pos[j] != INT_MAX, take = valid && key[j] <= cut;
+        if (valid && !take) outside = fminf(outside, key[j]);
+        const unsigned mask = __ballot_sync(0xffffffffu, take);
+        if (take) {
+            const int at = m + __popc(mask & ((1u << lane) - 1u));
+            s_pos[at] = pos[j];
+            s_fkey[at] = key[j];
+        }
+        m += __popc(mask);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) outside = fminf(outside, __shfl_xor_sync(0xffffffffu, outside, o));
+    __syncwarp();
+    float worst = 0.0f;   // largest observed |filter distance - canonical distance|
+    const float *xq = X + gq * D;
+    const int chunks = (D + kRerankDims - 1) / kRerankDims;
+    constexpr int kLanesPerRow = kRerankDims / VEC, kRowsPerCopy = 32 / kLanesPerRow;
+    const int col = (lane % kLanesPerRow) * VEC, sub = lane / kLanesPerRow;
+    for (int g = 0; g < m; g += 32) {
+        // copies of chunk c of this group's rows and of the query
+        auto fetch = [&](int c) {
+            float *buf = stage + (size_t)(c & 1) * kRerankStage;
+            const int d = c * kRerankDims + col;
+            if (d < D) {
+                for (int r = sub; r < 33; r += kRowsPerCopy) {
+                    if (r < 32 && g + r >= m) continue;
+                    const float *row;
+                    if (r == 32) row = xq;
+                    else {
+                        const int p = s_pos[g + r];
+                        row = Xp ? Xp + (long long)p * D : X + (long long)dblist[p] * D;
+                    }
+                    async_copy<4 * VEC>(buf + r * kRerankStride + col, row + d);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        float acc = 0.0f;
+        fetch(0);
+        for (int c = 0; c < chunks; c++) {
+            if (c + 1 < chunks) {
+                fetch(c + 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncwarp();
+            const float *buf = stage + (size_t)(c & 1) * kRerankStage;
+            const float *mine = buf + lane * kRerankStride, *query = buf + 32 * kRerankStride;
+            const int len = min(kRerankDims, D - c * kRerankDims);
+            if (len == kRerankDims) {
+#pragma unroll
+                for (int d = 0; d < kRerankDims; d += 4) {
+                    const float4 u = *reinterpret_cast<const float4 *>(query + d), v = *reinterpret_cast<const float4 *>(mine + d);
+                    acc = canon_step(acc, u.x, v.x);
+                    acc = canon_step(acc, u.y, v.y);
+                    acc = canon_step(acc, u.z, v.z);
+                    acc = canon_step(acc, u.w, v.w);
+                }
+            } else {
+                for (int d = 0; d < len; d++) acc = canon_step(acc, query[d], mine[d]);
+            }
+            __syncwarp();
+        }
+        if (g + lane < m) {
+            const double approx = ni + (double)s_fkey[g + lane];
+            worst = fmaxf(worst, (float)fabs(approx - (double)acc));
+            s_key[g + lane] = (unsigned long long)__float_as_uint(acc) << 32 | (unsigned)dblist[s_pos[g + lane]];
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) worst = fmaxf(worst, __shfl_xor_sync(0xffffffffu, worst, o));
     __syncwarp();
     // rank by counting (ties by id), scatter the first K
     float dK = INFINITY;
-    for (int e = lane; e < L; e += 32) {
-        const float de = s_d[w][e];
-        const int ie = s_i[w][e];
+    for (int e = lane; e < m; e += 32) {
+        const unsigned long long mine = s_key[e];
         int rank = 0;
-        for (int u = 0; u < L; u++) {
-            const float du = s_d[w][u];
-            const int iu = s_i[w][u];
-            rank += (du < de || (du == de && iu < ie)) ? 1 : 0;
-        }
+        for (int u = 0; u < m; u++) rank += s_key[u] < mine;
+        const float de = __uint_as_float((unsigned)(mine >> 32));
         if (rank < K) {
-            ids[orow * K + rank] = (ie == INT_MAX) ? -1 : ie;
+            ids[orow * K + rank] = (int32_t)(unsigned)mine;
             d2[orow * K + rank] = de;
         }
         if (rank == K - 1) dK = de;
+    }
+    for (int e = m + lane; e < K; e += 32) {   // fewer candidates than slots: the row fails below and is searched anew
+        ids[orow * K + e] = -1;
+        d2[orow * K + e] = INFINITY;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dK = fminf(dK, __shfl_xor_sync(0xffffffffu, dK, o));
     if (lane == 0) {
         bool ok = true;
-        // Error bound of the filter's key for this row: it scales with |x_i||x_j|, and a point whose key is
-        // near T lies within sqrt(|x_i|^2 + T) of x_i, so |x_i||x_j| <= |x_i|^2 + (|x_i|^2 + T)+ up to a factor 2.
-        double E = (double)err_scale * (ni + fmax(0.0, ni + (double)T) + 1.0);
-        double dropped = 0.0;
-        if (res_q) {
-            // bf16 pairs: what the three products drop, bounded from the leftovers of this query and the largest
-            // relative leftovers of the database, for every point with |x_j| <= |x_i| + sqrt(|x_i|^2 + T) (a point
-            // further out cannot come closer than the threshold whatever the error of its key); the last term is
-            // the fp32 rounding of the norm column.  err_scale then covers the accumulation only.
-            const double xi = sqrt(ni), xj = xi + sqrt(fmax(0.0, ni + (double)T));
-            const float2 rq = res_q[q];
-            dropped = 1.001 * 2.0 * xj * ((double)rq.x * (double)rho[0] + xi * (double)rho[1] + (double)rq.y) + 1.2e-7 * xj * xj;
-            E += dropped;
-        }
-        if (n_valid == L) {
-            // outsiders: key >= T  =>  canonical distance >= (ni + T - E) * (1 - theta)
-            const double theta = (double)(D + 4) * 5.9604644775390625e-08;   // (D+4) * 2^-24
-            const double bound = (ni + (double)T - E) * (1.0 - theta);
-            ok = (double)dK < bound;
-        }
+        // outsiders (not in the list: key >= T, with a full list; left out of it: key >= outside):
+        // canonical distance >= (ni + key - E) * (1 - theta)
+        const double nearest = fmin(n_valid == L ? (double)T : (double)INFINITY, (double)outside);
+        const double bound = (ni + nearest - E) * (1.0 - theta);
+        ok = !isfinite(nearest) || (double)dK < bound;
         const float ratio = (float)(fmax(0.0, (double)worst - dropped) / (E - dropped));
         if (ratio > 0.5f) ok = false;   // the filter was less accurate than the bound assumes
         if (row_flags && row_flags[q]) ok = false;   // the fixed threshold kept too few or too many candidates
@@ -1865,17 +2002,17 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
         knn_cells_scatter_kernel<<<gd, kCellThreads, 0, st>>>(w.cell_db, db_lo, nd, cells, w.tab, 1, w.dblist);
         knn_cells_scatter_kernel<<<gq, kCellThreads, 0, st>>>(w.cell_q, q_lo, nq, cells, w.tab, 0, w.qlist);
         nd_pos = w.td * TN;
-        knn_gather_rows_kernel<<<(unsigned)((nd_pos * D + 255) / 256), 256, 0, st>>>(X, w.dblist, D, nd_pos, w.xp);
+        if (!bf16) knn_gather_rows_kernel<<<(unsigned)((nd_pos * D + 255) / 256), 256, 0, st>>>(X, w.dblist, D, nd_pos, w.xp);
     } else {
         knn_iota_kernel<<<(unsigned)((nd + 255) / 256), 256, 0, st>>>(w.dblist, db_lo, nd);
         knn_iota_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(w.qlist, q_lo, nq);
     }
     B200_CUDA(cudaGetLastError());
     if (bf16) {
-        knn_tc_prepare_bf16_kernel<<<(unsigned)w.tq, 128, 0, st>>>(X, w.qlist, D, Dp, KC, w.sw, 0, reinterpret_cast<__nv_bfloat16 *>(w.img_q),
-                                                                   w.norms_q, w.res_q, nullptr);
-        knn_tc_prepare_bf16_kernel<<<(unsigned)w.td, 128, 0, st>>>(X, w.dblist, D, Dp, KC, w.sw, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_db),
-                                                                   nullptr, nullptr, counters + 4);
+        knn_tc_prepare_bf16_kernel<<<(unsigned)w.tq, 256, 0, st>>>(X, w.qlist, D, Dp, KC, w.sw, 0, reinterpret_cast<__nv_bfloat16 *>(w.img_q),
+                                                                   w.norms_q, w.res_q, nullptr, nullptr);
+        knn_tc_prepare_bf16_kernel<<<(unsigned)w.td, 256, 0, st>>>(X, w.dblist, D, Dp, KC, w.sw, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_db),
+                                                                   nullptr, nullptr, counters + 4, w.xp);
     } else {
         knn_tc_prepare_kernel<<<(unsigned)w.tq, 128, 0, st>>>(X, w.qlist, D, Dp, KC, 0, w.img_q, w.norms_q);
         knn_tc_prepare_kernel<<<(unsigned)w.td, 128, 0, st>>>(X, w.dblist, D, Dp, KC, 1, w.img_db, nullptr);
@@ -1987,8 +2124,8 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
             const int ts = wide ? (m_a + kWideUnit - 1) / kWideUnit * 2 : (m_a + TN - 1) / TN;
             knn_sample_list_kernel<<<(unsigned)((ts * TN + 255) / 256), 256, 0, st>>>(w.slist, (long long)ts * TN, m_a, db_lo, a_stride);
             if (bf16)
-                knn_tc_prepare_bf16_kernel<<<(unsigned)ts, 128, 0, st>>>(X, w.slist, D, Dp, KC, w.sw, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_s),
-                                                                         nullptr, nullptr, nullptr);
+                knn_tc_prepare_bf16_kernel<<<(unsigned)ts, 256, 0, st>>>(X, w.slist, D, Dp, KC, w.sw, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_s),
+                                                                         nullptr, nullptr, nullptr, nullptr);
             else
                 knn_tc_prepare_kernel<<<(unsigned)ts, 128, 0, st>>>(X, w.slist, D, Dp, KC, 1, w.img_s, nullptr);
             knn_single_segment_kernel<<<1, 1, 0, st>>>(w.segs, w.nseg, wide ? ts / 2 : ts);
@@ -2057,7 +2194,12 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     // the scale covers the accumulation only.
     const float err_scale = bf16 ? std::max(1.52587890625e-05f, (float)(D + 8) * 2.384185791015625e-07f)      // max(2^-16, (D + 8) 2^-22)
                                  : std::max(6.103515625e-05f, (float)(D + 8) * 2.384185791015625e-07f);   // max(2^-14, (D + 8) 2^-22)
-    knn_tc_rerank_kernel<<<(unsigned)((nq + kRerankWarps - 1) / kRerankWarps), kRerankWarps * 32, 0, st>>>(
+    // rows are copied 16, 8 or 4 bytes at a time, as their length keeps them aligned
+    const size_t x_at = reinterpret_cast<size_t>(X);
+    const int vec = (D % 4 == 0 && x_at % 16 == 0) ? 4 : ((D % 2 == 0 && x_at % 8 == 0) ? 2 : 1);
+    auto rerank = vec == 4 ? knn_tc_rerank_kernel<4> : (vec == 2 ? knn_tc_rerank_kernel<2> : knn_tc_rerank_kernel<1>);
+    B200_CUDA(cudaFuncSetAttribute(rerank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rerank_smem(L)));
+    rerank<<<(unsigned)((nq + kRerankWarps - 1) / kRerankWarps), kRerankWarps * 32, rerank_smem(L), st>>>(
         X, D, w.qlist, w.dblist, q_lo, nq, final_key, final_id, L, final_stride, K, w.norms_q, err_scale, bf16 ? w.res_q : nullptr,
         reinterpret_cast<const float *>(counters + 4), two_pass ? row_flags : nullptr, ids, d2,
         failed, counters + 1, reinterpret_cast<float *>(counters + 3), w.xp);
