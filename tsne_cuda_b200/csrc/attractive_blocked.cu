@@ -44,109 +44,15 @@ namespace b200 {
 
 namespace {
 
-constexpr int kTileMax = 28672;        // points per tile: 224 KB of float2 (227 KB is the block limit)
+constexpr int kTileMax = kAttractiveTile;   // points per tile: 224 KB of float2 (227 KB is the block limit)
 constexpr int kChunk = 128;            // entries per warp step (4 per lane)
 constexpr int kMaxTiles = 1024;        // one bit per tile in a warp-wide bitmap
 constexpr int kBlockedThreads = 1024;
 constexpr float kMinEntriesPerGroup = 2.5f;
-constexpr int kCells = 64;
 
 // ------------------------------------------------------------------------------------------------
-// ordering of the points: nearest of kCells sample points, cells chained greedily by distance
+// ordering of the points: cells (cells.cu) chained greedily by distance
 // ------------------------------------------------------------------------------------------------
-constexpr int kDimChunk = 32;
-constexpr int kAssignThreads = 128;
-
-// centre c = row of X picked from the c-th of `cells` equal stretches at a hashed offset (an even spacing
-// would alias with a periodic ordering of the data)
-__device__ __forceinline__ long long centre_row(int c, int cells, long long N)
-{
-    const long long stretch = N / cells;
-    const unsigned long long h = ((unsigned long long)(c + 1) * 0x9E3779B97F4A7C15ull) >> 20;
-    return (long long)c * stretch + (long long)(h % (unsigned long long)stretch);
-}
-
-// cell[i] = nearest centre (ties: lower index).  A block takes 128 points; coordinates go through shared
-// memory in chunks of 32 dimensions, every thread keeps its 64 partial distances in registers.
-__global__ void __launch_bounds__(kAssignThreads)
-cell_assign_kernel(const float *__restrict__ X, long long N, int D, int cells, unsigned char *__restrict__ cell)
-{
-    __shared__ float s_x[kAssignThreads][kDimChunk + 1];
-    __shared__ float s_c[kCells][kDimChunk];
-    const long long i0 = (long long)blockIdx.x * kAssignThreads;
-    float acc[kCells];
-#pragma unroll
-    for (int c = 0; c < kCells; c++) acc[c] = 0.0f;
-    for (int d0 = 0; d0 < D; d0 += kDimChunk) {
-        const int nd = min(kDimChunk, D - d0);
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < kAssignThreads * kDimChunk; idx += kAssignThreads) {
-            const int r = idx / kDimChunk, d = idx % kDimChunk;
-            const long long i = i0 + r;
-            s_x[r][d] = (i < N && d < nd) ? X[i * D + d0 + d] : 0.0f;
-        }
-        for (int idx = threadIdx.x; idx < kCells * kDimChunk; idx += kAssignThreads) {
-            const int c = idx / kDimChunk, d = idx % kDimChunk;
-            s_c[c][d] = (c < cells && d < nd) ? X[centre_row(c, cells, N) * D + d0 + d] : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int d = 0; d < kDimChunk; d++) {
-            const float x = s_x[threadIdx.x][d];
-#pragma unroll
-            for (int c = 0; c < kCells; c++) {
-                const float t = x - s_c[c][d];
-                acc[c] = fmaf(t, t, acc[c]);
-            }
-        }
-    }
-    const long long i = i0 + threadIdx.x;
-    if (i >= N) return;
-    float best = INFINITY;
-    int bc = 0;
-#pragma unroll
-    for (int c = 0; c < kCells; c++)
-        if (c < cells && acc[c] < best) { best = acc[c]; bc = c; }
-    cell[i] = (unsigned char)bc;
-}
-
-// rank[c] = position of cell c in a greedy nearest-neighbour chain through the centres (start: cell 0), so
-// that cells of one cluster end up next to each other.  One block.
-__global__ void __launch_bounds__(kCells)
-cell_chain_kernel(const float *__restrict__ X, long long N, int D, int cells, int *__restrict__ rank)
-{
-    __shared__ float s_d[kCells][kCells + 1];
-    const int a = threadIdx.x;
-    if (a < cells) {
-        const float *xa = X + centre_row(a, cells, N) * D;
-        for (int b = 0; b < cells; b++) {
-            const float *xb = X + centre_row(b, cells, N) * D;
-            float acc = 0.0f;
-            for (int d = 0; d < D; d++) {
-                const float t = xa[d] - xb[d];
-                acc = fmaf(t, t, acc);
-            }
-            s_d[a][b] = acc;
-        }
-    }
-    __syncthreads();
-    if (a != 0) return;
-    bool used[kCells];
-    for (int c = 0; c < kCells; c++) used[c] = false;
-    int cur = 0;
-    used[0] = true;
-    rank[0] = 0;
-    for (int k = 1; k < cells; k++) {
-        int best = -1;
-        float bd = INFINITY;
-        for (int c = 0; c < cells; c++)
-            if (!used[c] && (best < 0 || s_d[cur][c] < bd)) { bd = s_d[cur][c]; best = c; }
-        used[best] = true;
-        rank[best] = k;
-        cur = best;
-    }
-}
-
 // Stable counting sort of the points by rank[cell]: a block takes kSortPerBlock consecutive points, each of
 // its warps a contiguous share of them.
 constexpr int kSortWarps = 8;
@@ -154,16 +60,16 @@ constexpr int kSortPerWarp = 512;
 constexpr int kSortPerBlock = kSortWarps * kSortPerWarp;
 
 __global__ void __launch_bounds__(kSortWarps * 32)
-cell_hist_kernel(const unsigned char *__restrict__ cell, const int *__restrict__ rank, long long N, int *__restrict__ hist /* [kCells][nblocks] */)
+cell_hist_kernel(const unsigned char *__restrict__ cell, const int *__restrict__ rank, long long N, int *__restrict__ hist /* [kMaxCells][nblocks] */)
 {
-    __shared__ int s_h[kCells];
-    for (int c = threadIdx.x; c < kCells; c += blockDim.x) s_h[c] = 0;
+    __shared__ int s_h[kMaxCells];
+    for (int c = threadIdx.x; c < kMaxCells; c += blockDim.x) s_h[c] = 0;
     __syncthreads();
     const long long lo = (long long)blockIdx.x * kSortPerBlock;
     for (int k = threadIdx.x; k < kSortPerBlock; k += blockDim.x)
         if (lo + k < N) atomicAdd(&s_h[rank[cell[lo + k]]], 1);
     __syncthreads();
-    for (int c = threadIdx.x; c < kCells; c += blockDim.x) hist[(size_t)c * gridDim.x + blockIdx.x] = s_h[c];
+    for (int c = threadIdx.x; c < kMaxCells; c += blockDim.x) hist[(size_t)c * gridDim.x + blockIdx.x] = s_h[c];
 }
 
 // exclusive scan of n ints in place; one block (the tables it serves are small)
@@ -208,16 +114,16 @@ __global__ void __launch_bounds__(kSortWarps * 32)
 cell_scatter_kernel(const unsigned char *__restrict__ cell, const int *__restrict__ rank, long long N, const int *__restrict__ offs,
                     int32_t *__restrict__ perm)
 {
-    __shared__ int s_cnt[kSortWarps][kCells], s_base[kSortWarps][kCells];
+    __shared__ int s_cnt[kSortWarps][kMaxCells], s_base[kSortWarps][kMaxCells];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int c = lane; c < kCells; c += 32) s_cnt[w][c] = 0;
+    for (int c = lane; c < kMaxCells; c += 32) s_cnt[w][c] = 0;
     __syncwarp();
     const long long lo = (long long)blockIdx.x * kSortPerBlock + (long long)w * kSortPerWarp;
     for (int k = lane; k < kSortPerWarp; k += 32)
         if (lo + k < N) atomicAdd(&s_cnt[w][rank[cell[lo + k]]], 1);
     __syncthreads();
     // first position of (block, warp, cell) = block offset + counts of the warps before this one
-    for (int c = lane; c < kCells; c += 32) {
+    for (int c = lane; c < kMaxCells; c += 32) {
         int base = offs[(size_t)c * gridDim.x + blockIdx.x];
         for (int v = 0; v < w; v++) base += s_cnt[v][c];
         s_base[w][c] = base;
@@ -242,25 +148,21 @@ cell_scatter_kernel(const unsigned char *__restrict__ cell, const int *__restric
 
 }  // namespace
 
-// perm[q] = the point at position q of the cell order.  X: [N][D] on the device.
-int order_points_by_cell(const float *X, int64_t N, int D, int32_t *perm, cudaStream_t st)
+int order_points_by_cell(const PointCells &pc, int32_t *perm, cudaStream_t st)
 {
-    if (N <= 0 || D <= 0) { set_error("order_points_by_cell: invalid sizes"); return -1; }
-    const int cells = (int)std::min<int64_t>(kCells, N);
+    const int64_t N = pc.n;
+    if (N <= 0 || pc.lo != 0) { set_error("order_points_by_cell: needs the cells of all points"); return -1; }
     const unsigned nblocks = (unsigned)((N + kSortPerBlock - 1) / kSortPerBlock);
     DeviceArena tmp;
     tmp.serve(st);
-    unsigned char *cell = nullptr;
     int *rank = nullptr, *hist = nullptr;
-    B200_TRY(tmp.alloc((void **)&cell, (size_t)N));
-    B200_TRY(tmp.alloc((void **)&rank, sizeof(int) * kCells));
-    B200_TRY(tmp.alloc((void **)&hist, sizeof(int) * (size_t)kCells * nblocks));
-    B200_CUDA(cudaMemsetAsync(rank, 0, sizeof(int) * kCells, st));
-    cell_assign_kernel<<<(unsigned)((N + kAssignThreads - 1) / kAssignThreads), kAssignThreads, 0, st>>>(X, N, D, cells, cell);
-    cell_chain_kernel<<<1, kCells, 0, st>>>(X, N, D, cells, rank);
-    cell_hist_kernel<<<nblocks, kSortWarps * 32, 0, st>>>(cell, rank, N, hist);
-    scan_inplace_kernel<<<1, 1024, 0, st>>>(hist, (long long)kCells * nblocks);
-    cell_scatter_kernel<<<nblocks, kSortWarps * 32, 0, st>>>(cell, rank, N, hist, perm);
+    B200_TRY(tmp.alloc((void **)&rank, sizeof(int) * kMaxCells));
+    B200_TRY(tmp.alloc((void **)&hist, sizeof(int) * (size_t)kMaxCells * nblocks));
+    B200_CUDA(cudaMemsetAsync(rank, 0, sizeof(int) * kMaxCells, st));
+    B200_TRY(point_cells_chain(pc, rank, st));
+    cell_hist_kernel<<<nblocks, kSortWarps * 32, 0, st>>>(pc.cell, rank, N, hist);
+    scan_inplace_kernel<<<1, 1024, 0, st>>>(hist, (long long)kMaxCells * nblocks);
+    cell_scatter_kernel<<<nblocks, kSortWarps * 32, 0, st>>>(pc.cell, rank, N, hist, perm);
     B200_CUDA(cudaGetLastError());
     B200_CUDA(cudaStreamSynchronize(st));
     return 0;

@@ -201,7 +201,9 @@ int b200tsne_attractive_blocked(const float *P, const int32_t *ids, const float 
     if (X) {
         B200_TRY(up(a, &dX, X, (size_t)N * D, sg.st));
         B200_TRY(a.alloc((void **)&perm, sizeof(int32_t) * N));
-        B200_TRY(order_points_by_cell(dX, N, D, perm, sg.st));
+        PointCells pc;
+        B200_TRY(point_cells_build(&pc, dX, D, 0, N, a, sg.st));
+        B200_TRY(order_points_by_cell(pc, perm, sg.st));
     }
     B200_CUDA(cudaMemsetAsync(dF2, 0, sizeof(float2) * N, sg.st));
     B200_TRY(launch_soa_to_aos(dY, dY2, N, sg.st));
@@ -256,7 +258,9 @@ int b200tsne_attractive_symmetric(const float *p, const int32_t *ids, const floa
     if (X) {
         B200_TRY(up(a, &dX, X, (size_t)N * D, sg.st));
         B200_TRY(a.alloc((void **)&perm, sizeof(int32_t) * N));
-        B200_TRY(order_points_by_cell(dX, N, D, perm, sg.st));
+        PointCells pc;
+        B200_TRY(point_cells_build(&pc, dX, D, 0, N, a, sg.st));
+        B200_TRY(order_points_by_cell(pc, perm, sg.st));
     }
     B200_CUDA(cudaMemsetAsync(dF2, 0, sizeof(float2) * N, sg.st));
     B200_TRY(launch_soa_to_aos(dY, dY2, N, sg.st));

@@ -78,10 +78,32 @@ __host__ __device__ inline float dec_float(unsigned int e)
 int launch_transpose(const float *X, int64_t N, int D, float *XT, cudaStream_t st);   // [N][D] -> [D][N]
 int launch_knn_exact(const float *XT, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo,
                      int64_t db_hi, int32_t *ids, float *d2, cudaStream_t st);   // ids/d2 keep (INT_MAX,+inf) in unfilled slots
-// knn_tc.cu: tensor-core filter + exact re-rank + proof (nd = database rows to scan)
+// cells.cu: nearest of at most kMaxCells sample points, for every row of a range, with the distances to all of them
+struct DeviceArena;
+constexpr int kMaxCells = 64;
+struct CellTable {
+    long long centre_row[kMaxCells];
+    unsigned int radius_bits[kMaxCells];   // the rest belongs to one neighbour search, see knn_tc.cu
+    int db_count[kMaxCells], q_count[kMaxCells];
+    int db_start[kMaxCells + 1], q_start[kMaxCells + 1];
+    int db_cursor[kMaxCells], q_cursor[kMaxCells];
+};
+struct PointCells {
+    int cells = 0;
+    int64_t lo = 0, n = 0;          // rows [lo, lo + n)
+    CellTable *tab = nullptr;
+    float *dist = nullptr;          // [n][kMaxCells]
+    unsigned char *cell = nullptr;  // [n]
+};
+inline int point_cells_count(int64_t n) { return (int)(n < 4096 ? 1 : (n / 2048 < kMaxCells ? n / 2048 : kMaxCells)); }   // see point_cells_build
+int point_cells_build(PointCells *pc, const float *X, int D, int64_t lo, int64_t n, DeviceArena &arena, cudaStream_t st);
+int point_cells_assign(const PointCells &pc, const float *X, int D, int64_t lo, int64_t n, float *dist, unsigned char *cell, cudaStream_t st);
+int point_cells_chain(const PointCells &pc, int *rank, cudaStream_t st);
+
+// knn_tc.cu: tensor-core filter + exact re-rank + proof (nd = database rows to scan); pc: the cells of the database rows
 bool knn_tc_supported(int64_t nd, int D, int K);
 size_t knn_tc_workspace_bytes(int D, int K, int64_t nq, int64_t nd);
-int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo, int64_t db_hi,
+int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo, int64_t db_hi, const PointCells &pc,
                   int32_t *ids, float *d2, void *workspace, int **failed_list, int *n_failed_host, float *err_ratio_host,
                   cudaStream_t st);
 int mbar_wait_selftest(int timeout_ms, float *waited_ms, cudaStream_t st);   // see b200tsne_selftest_bounded_waits
@@ -91,10 +113,10 @@ struct KnnStats {
     float filter_error_ratio = 0;   // largest observed filter error on the candidates / assumed bound
 };
 // X: [N][D] row-major on the device; picks the path, handles the fallback rows, synchronises `st`.
+// pc (optional): the cells of rows [db_lo, db_hi), where the caller has them
 int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo, int64_t db_hi,
-               int32_t *ids, float *d2, KnnStats *stats, cudaStream_t st);
+               int32_t *ids, float *d2, KnnStats *stats, cudaStream_t st, const PointCells *pc = nullptr);
 // knn_dense.cu: whole rows of distances and a selection (see that file); distances of NaN never rank
-struct DeviceArena;
 bool knn_dense_supported(int K);
 int knn_dense(const float *X, int D, int K, int64_t q_lo, int64_t nq, const int *q_index, int64_t out_base, int64_t db_lo, int64_t db_hi,
               int32_t *ids, float *d2, DeviceArena &tmp, cudaStream_t st);
@@ -126,7 +148,6 @@ int launch_attractive_extra(const int *ptr, const int32_t *ext_ids, const float 
                             int64_t row_hi, float2 *F2, cudaStream_t st);
 
 // attractive_blocked.cu: column-blocked copy of P whose gathers come from shared memory (see that file)
-struct DeviceArena;
 // Further stored entries of the owned rows in variable-width form: row r (0-based among the owned rows) has the
 // entries ptr[r] .. ptr[r + 1].  Used for the reverse-only edges that make P truly symmetric (affinities.cu).
 struct ExtraEntries {
@@ -135,6 +156,7 @@ struct ExtraEntries {
     const float *val = nullptr;
     int64_t count = 0;
 };
+constexpr int kAttractiveTile = 28672;   // points per tile of the blocked copy; up to here the order of the points does not matter
 struct BlockedAttractive {
     const float *ev = nullptr;
     const uint16_t *ec = nullptr;
@@ -152,7 +174,8 @@ struct BlockedAttractive {
     bool ready = false;
     void clear();
 };
-int order_points_by_cell(const float *X, int64_t N, int D, int32_t *perm, cudaStream_t st);
+// perm[q] = the point at position q of the cell order; pc: the cells of all N points
+int order_points_by_cell(const PointCells &pc, int32_t *perm, cudaStream_t st);
 int blocked_attractive_build(BlockedAttractive *b, DeviceArena &arena, const float *P_rows, const int32_t *ids_rows, int64_t N, int K,
                              int64_t row_lo, int64_t row_hi, const int32_t *perm, const ExtraEntries *extra, cudaStream_t st);
 int launch_exclusive_scan_i32(int *data, int64_t n, cudaStream_t st);   // in place; small arrays (one block)

@@ -269,7 +269,7 @@ constexpr int64_t kDenseMaxRows = 32768;
 // choosing the tensor-core path where it applies and falling back to the SIMT search for the rows it
 // cannot certify.  Unfilled slots keep (INT_MAX, +inf); see launch_knn_finalize.
 int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo, int64_t db_hi,
-               int32_t *ids, float *d2, KnnStats *stats, cudaStream_t st)
+               int32_t *ids, float *d2, KnnStats *stats, cudaStream_t st, const PointCells *pc)
 {
     KnnStats local;
     if (!stats) stats = &local;
@@ -302,6 +302,11 @@ int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_
     // Queries go through in batches of 2^20 so that the candidate buffers (about 10 KB per query) stay
     // bounded however large N is; the operand images are rebuilt per batch (a millisecond per million points).
     const int64_t batch = (int64_t)1 << 20;
+    PointCells own;
+    if (!pc || pc->lo != db_lo || pc->n != db_hi - db_lo) {
+        B200_TRY(point_cells_build(&own, X, D, db_lo, db_hi - db_lo, tmp, st));
+        pc = &own;
+    }
     void *ws = nullptr;
     B200_TRY(tmp.alloc(&ws, knn_tc_workspace_bytes(D, K, std::min(nq, batch), db_hi - db_lo)));
     stats->tensor_core = 1;
@@ -312,7 +317,7 @@ int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_
         float ratio = 0.0f;
         int32_t *ids_b = ids + (b_lo - q_lo) * K;
         float *d2_b = d2 + (b_lo - q_lo) * K;
-        B200_TRY(launch_knn_tc(X, N, D, K, b_lo, b_hi, db_lo, db_hi, ids_b, d2_b, ws, &failed_list, &n_failed, &ratio, st));
+        B200_TRY(launch_knn_tc(X, N, D, K, b_lo, b_hi, db_lo, db_hi, *pc, ids_b, d2_b, ws, &failed_list, &n_failed, &ratio, st));
         stats->rows_recomputed += n_failed;
         stats->filter_error_ratio = std::max(stats->filter_error_ratio, ratio);
         if (n_failed > 0) {

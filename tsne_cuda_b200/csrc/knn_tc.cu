@@ -424,76 +424,39 @@ knn_tc_prepare_bf16_kernel(const float *__restrict__ X, const int *__restrict__ 
 // cells: a coarse partition of the points that lets a block skip database tiles no query of it can reach
 // ------------------------------------------------------------------------------------------------
 // Both the database rows and the queries of a search are visited in the order of a partition into at
-// most kMaxCells Voronoi cells around sample points ("centres").  Database cells start on tile
+// most kMaxCells Voronoi cells around sample points (cells.cu).  Database cells start on tile
 // boundaries (padding rows in between), so a cell is a run of whole tiles; for every cell the largest
 // distance r_c of a member to its centre is known.  Once a query's threshold is fixed, no point of cell c
 // can pass it if  |x_q - centre_c| - r_c  exceeds the threshold distance (triangle inequality), and a block
 // skips the cells that none of its queries can reach.  On clustered data most tile pairs disappear; on
-// data without structure nothing is lost but the few milliseconds of these kernels.
-constexpr int kMaxCells = 64;
+// data without structure nothing is lost but a fraction of a millisecond.  The visiting order also keeps the rows that the
+// re-rank of neighbouring queries reads together in L2.
 constexpr int kCellThreads = 256;
 
-struct CellTable {
-    float centre[kMaxCells][64];      // zero beyond D
-    unsigned int radius_bits[kMaxCells];   // float bits of r_c (non-negative floats order like unsigned integers)
-    int db_count[kMaxCells], q_count[kMaxCells];
-    int db_start[kMaxCells + 1];      // first list position of the cell (multiple of TN); [cells] = end
-    int q_start[kMaxCells + 1];
-    int db_cursor[kMaxCells], q_cursor[kMaxCells];
-};
-
-__global__ void knn_cells_init_kernel(const float *__restrict__ X, int D, long long db_lo, long long nd, int cells, CellTable *tab)
+__global__ void knn_cells_reset_kernel(CellTable *tab)
 {
-    // centres = database rows, one from each of `cells` equal stretches of the range at a hashed offset (an
-    // even spacing would alias with any periodic ordering of the data and could leave whole clusters
-    // without a centre)
-    for (int idx = threadIdx.x; idx < cells * 64; idx += blockDim.x) {
-        const int c = idx >> 6, d = idx & 63;
-        const long long stretch = nd / cells;
-        const unsigned long long h = ((unsigned long long)(c + 1) * 0x9E3779B97F4A7C15ull) >> 20;
-        const long long row = db_lo + (long long)c * stretch + (long long)(h % (unsigned long long)stretch);
-        tab->centre[c][d] = (d < D) ? X[row * D + d] : 0.0f;
-    }
-    for (int c = threadIdx.x; c < kMaxCells; c += blockDim.x) {
-        tab->radius_bits[c] = 0u;
-        tab->db_count[c] = tab->q_count[c] = 0;
-        tab->db_cursor[c] = tab->q_cursor[c] = 0;
-    }
+    const int c = threadIdx.x;
+    if (c >= kMaxCells) return;
+    tab->radius_bits[c] = 0u;
+    tab->db_count[c] = tab->q_count[c] = 0;
+    tab->db_cursor[c] = tab->q_cursor[c] = 0;
 }
 
-// cell[i] = nearest centre of row lo + i; counts the members and (for the database) maintains r_c
+// members of every cell among the n rows of cell / dist and, for the database, r_c
 __global__ void __launch_bounds__(kCellThreads)
-knn_cells_assign_kernel(const float *__restrict__ X, int D, long long lo, long long n, int cells, CellTable *tab, int is_db,
-                        unsigned char *__restrict__ cell)
+knn_cells_count_kernel(const unsigned char *__restrict__ cell, const float *__restrict__ dist, long long n, CellTable *tab, int is_db)
 {
-    __shared__ float s_c[kMaxCells][65];
     __shared__ int s_cnt[kMaxCells];
     __shared__ unsigned int s_rad[kMaxCells];
-    for (int idx = threadIdx.x; idx < cells * 64; idx += kCellThreads) s_c[idx >> 6][idx & 63] = tab->centre[idx >> 6][idx & 63];
     for (int c = threadIdx.x; c < kMaxCells; c += kCellThreads) { s_cnt[c] = 0; s_rad[c] = 0u; }
     __syncthreads();
-    const long long i = (long long)blockIdx.x * kCellThreads + threadIdx.x;
-    if (i < n) {
-        float x[64];
-#pragma unroll
-        for (int d = 0; d < 64; d++) x[d] = (d < D) ? X[(lo + i) * D + d] : 0.0f;
-        float best = INFINITY;
-        int bc = 0;
-        for (int c = 0; c < cells; c++) {
-            float acc = 0.0f;
-#pragma unroll
-            for (int d = 0; d < 64; d++) {
-                const float t = x[d] - s_c[c][d];
-                acc = fmaf(t, t, acc);
-            }
-            if (acc < best) { best = acc; bc = c; }
-        }
-        cell[i] = (unsigned char)bc;
-        atomicAdd(&s_cnt[bc], 1);
-        if (is_db) atomicMax(&s_rad[bc], __float_as_uint(sqrtf(best)));
+    for (long long i = (long long)blockIdx.x * kCellThreads + threadIdx.x; i < n; i += (long long)gridDim.x * kCellThreads) {
+        const int c = cell[i];
+        atomicAdd(&s_cnt[c], 1);
+        if (is_db) atomicMax(&s_rad[c], __float_as_uint(dist[(size_t)i * kMaxCells + c]));   // >= 0: orders like the bits
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < cells; c += kCellThreads) {
+    for (int c = threadIdx.x; c < kMaxCells; c += kCellThreads) {
         if (s_cnt[c]) atomicAdd(is_db ? &tab->db_count[c] : &tab->q_count[c], s_cnt[c]);
         if (is_db && s_rad[c]) atomicMax(&tab->radius_bits[c], s_rad[c]);
     }
@@ -541,134 +504,49 @@ __global__ void knn_iota_kernel(int *__restrict__ list, long long lo, long long 
     if (i < n) list[i] = (int)(lo + i);
 }
 
-// ------------------------------------------------------------------------------------------------
-// candidate buffers: compaction by a warp-wide bitonic sort, EPL elements per lane (32*EPL = capacity)
-// ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ bool pair_less(float ka, int ia, float kb, int ib) { return ka < kb || (ka == kb && ia < ib); }
-
-// One compare-exchange step between registers r and r + J of the same lane (J < EPL).
-template <int EPL, int J>
-__device__ __forceinline__ void bitonic_in_lane(float (&k)[EPL], int (&id)[EPL], int lane, int size)
-{
-#pragma unroll
-    for (int r = 0; r < EPL; r++) {
-        if ((r & J) == 0) {
-            const bool up = ((lane * EPL + r) & size) == 0;
-            const bool swap = up ? pair_less(k[r + J], id[r + J], k[r], id[r]) : pair_less(k[r], id[r], k[r + J], id[r + J]);
-            if (swap) {
-                const float tk = k[r]; k[r] = k[r + J]; k[r + J] = tk;
-                const int ti = id[r]; id[r] = id[r + J]; id[r + J] = ti;
-            }
-        }
-    }
-}
-
-// Warp-wide bitonic sort of 32*EPL (key, id) pairs, ascending; element index = lane * EPL + r.  The two
-// outer loops are real loops (the sort runs rarely and from cold instruction cache: a fully unrolled
-// network of ~2500 instructions costs more in instruction fetch than it saves).
-template <int EPL>
-__device__ __forceinline__ void warp_bitonic_sort(float (&k)[EPL], int (&id)[EPL], int lane)
-{
-#pragma unroll 1
-    for (int size = 2; size <= 32 * EPL; size <<= 1) {
-#pragma unroll 1
-        for (int j = size >> 1; j > 0; j >>= 1) {
-            if (j >= EPL) {
-                const int lj = j / EPL;
-                const bool lower = ((lane * EPL) & j) == 0;     // same for all registers of the lane: j >= EPL
-#pragma unroll
-                for (int r = 0; r < EPL; r++) {
-                    const float ok = __shfl_xor_sync(0xffffffffu, k[r], lj);
-                    const int oi = __shfl_xor_sync(0xffffffffu, id[r], lj);
-                    const bool up = ((lane * EPL + r) & size) == 0;      // ascending block
-                    const bool keep_min = (lower == up);
-                    const bool take = keep_min ? pair_less(ok, oi, k[r], id[r]) : pair_less(k[r], id[r], ok, oi);
-                    if (take) { k[r] = ok; id[r] = oi; }
-                }
-            } else if (j == 1) {
-                bitonic_in_lane<EPL, 1>(k, id, lane, size);
-            } else if (j == 2) {
-                bitonic_in_lane<EPL, 2>(k, id, lane, size);
-            } else if (j == 4) {
-                bitonic_in_lane<EPL, 4>(k, id, lane, size);
-            } else {
-                if constexpr (EPL > 8) bitonic_in_lane<EPL, 8>(k, id, lane, size);
-            }
-        }
-    }
-}
-
-// Sort the first n entries of one query's buffer (capacity 32*EPL) and keep the L best (L = 16*EPL).
-// Whole warp; returns the new threshold (key of the L-th best, +inf while fewer than L entries exist).
-template <int EPL>
-__device__ __noinline__ float warp_compact(float *bk, int32_t *bi, int n, int lane)
-{
-    constexpr int L = 16 * EPL;
-    float k[EPL];
-    int id[EPL];
-#pragma unroll
-    for (int r = 0; r < EPL; r++) {
-        const int idx = lane * EPL + r;
-        k[r] = (idx < n) ? __ldcg(bk + idx) : INFINITY;
-        id[r] = (idx < n) ? __ldcg(bi + idx) : INT_MAX;
-    }
-    warp_bitonic_sort<EPL>(k, id, lane);
-#pragma unroll
-    for (int r = 0; r < EPL; r++) {
-        const int idx = lane * EPL + r;
-        if (idx < L) { __stcg(bk + idx, k[r]); __stcg(bi + idx, id[r]); }
-    }
-    return __shfl_sync(0xffffffffu, k[EPL - 1], 15);   // element L-1 sits in lane 15, last register
-}
-
 // One block per filter block (qpc = its queries): which cells can hold a point that passes the threshold of
-// at least one of its queries?  Their tile ranges, merged where adjacent, are the block's segments.
-// Rounding: the fp32 distances carry a relative error below 1e-5 (sums of at most 64 squares), the
-// inequality is tested with margins ten times that; a comparison that involves a NaN keeps the cell.
+// at least one of its queries?  Their tile ranges (in units of two tiles for the wide kernel), merged where adjacent, are
+// the block's segments.
+// q_dist: distances of row q_lo + r to the centres at row r.  Rounding: a distance carries a relative error of at most
+// (D + 2) 2^-25, the inequality is tested with `margin` = 1e-4 more than twice that; a comparison that involves a NaN keeps
+// the cell.
 __global__ void __launch_bounds__(kCellThreads)
-knn_cells_segments_kernel(const float *__restrict__ X, int D, const int *__restrict__ qlist, long long nq, int qpc,
-                          const float *__restrict__ tau, const double *__restrict__ norms_q, int cells,
+knn_cells_segments_kernel(const float *__restrict__ q_dist, long long q_lo, const int *__restrict__ qlist, long long nq, int qpc,
+                          const float *__restrict__ tau, const double *__restrict__ norms_q, int cells, float margin, int pair_tiles,
                           const CellTable *__restrict__ tab, int2 *__restrict__ segs, int *__restrict__ nseg)
 {
-    __shared__ float s_c[kMaxCells][65];
-    __shared__ float s_r[kMaxCells];
     __shared__ int s_keep[kMaxCells];
-    for (int idx = threadIdx.x; idx < cells * 64; idx += kCellThreads) s_c[idx >> 6][idx & 63] = tab->centre[idx >> 6][idx & 63];
-    for (int c = threadIdx.x; c < kMaxCells; c += kCellThreads) {
-        s_r[c] = __uint_as_float(tab->radius_bits[c]) * 1.00001f;
-        s_keep[c] = 0;
-    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int c = threadIdx.x; c < kMaxCells; c += kCellThreads) s_keep[c] = 0;
     __syncthreads();
-    for (int j = threadIdx.x; j < qpc; j += kCellThreads) {
+    float radius[2];
+    bool keep[2] = {false, false};
+#pragma unroll
+    for (int h = 0; h < 2; h++) radius[h] = __uint_as_float(tab->radius_bits[lane + 32 * h]) * (1.0f + margin);
+    // a warp per query, a lane per cell (and the cell 32 further on)
+    for (int j = warp; j < qpc; j += kCellThreads / 32) {
         const long long q = (long long)blockIdx.x * qpc + j;
-        if (q >= nq) continue;
+        if (q >= nq) break;
         const double R2 = norms_q[q] + (double)tau[q];   // a point passes if its squared distance is below this
-        if (!(R2 <= 0.0)) {
-            const float R = (float)sqrt(R2) * 1.0001f;
-            const int i = qlist[q];
-            float x[64];
+        if (R2 <= 0.0) continue;
+        const float R = (float)sqrt(R2) * 1.0001f;
+        const float *d = q_dist + (size_t)(qlist[q] - q_lo) * kMaxCells;
 #pragma unroll
-            for (int d = 0; d < 64; d++) x[d] = (d < D) ? X[(long long)i * D + d] : 0.0f;
-            for (int c = 0; c < cells; c++) {
-                float acc = 0.0f;
-#pragma unroll
-                for (int d = 0; d < 64; d++) {
-                    const float t = x[d] - s_c[c][d];
-                    acc = fmaf(t, t, acc);
-                }
-                const float lower = sqrtf(acc) * 0.99999f - s_r[c];
-                if (!(lower > R)) s_keep[c] = 1;
-            }
-        }
+        for (int h = 0; h < 2; h++)
+            if (!(d[lane + 32 * h] * (1.0f - margin) - radius[h] > R)) keep[h] = true;
     }
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+        if (keep[h]) s_keep[lane + 32 * h] = 1;
     __syncthreads();
     if (threadIdx.x == 0) {
         int n = 0;
         int2 *out = segs + (size_t)blockIdx.x * kMaxCells;
         for (int c = 0; c < cells; c++) {
             if (!s_keep[c] || tab->db_count[c] == 0) continue;
-            const int a = tab->db_start[c] / TN, b = tab->db_start[c + 1] / TN;
-            if (n > 0 && out[n - 1].y == a) out[n - 1].y = b;
+            int a = tab->db_start[c] / TN, b = tab->db_start[c + 1] / TN;
+            if (pair_tiles) { a /= 2; b = (b + 1) / 2; }   // a pair may hold the edge tiles of two cells
+            if (n > 0 && out[n - 1].y >= a) out[n - 1].y = max(out[n - 1].y, b);
             else out[n++] = make_int2(a, b);
         }
         nseg[blockIdx.x] = n;
@@ -779,26 +657,20 @@ __device__ __noinline__ void tc_issue_walk(TcShared *shp, volatile int *abort_fl
 // (segs + blockIdx.x * seg_stride, nseg[blockIdx.x * (seg_stride != 0)] of them; seg_stride = 0: one list shared by
 // all blocks), taking every tile_stride-th tile.  Candidate ids are database list positions; positions from
 // nd_pos on are padding and never kept.
-// cand_key / cand_id: [nq][cap] candidate buffers.  FIXED = false: threshold maintained online, cap = 32*EPL;
-// on return the first L = 16*EPL entries of each are the L best keys in ascending order ((+inf, INT_MAX)
-// where the database had fewer points).  FIXED = true: threshold tau[query] fixed, two segments of cap/2
-// entries per query; counts[2*query + buffer] receives the number of entries appended to each (bit 30 set
-// if it overflowed); knn_tc_pick_kernel finishes.
-// RANKED (with FIXED = false): no candidate buffers at all; every query thread keeps its 16 smallest keys in
+// cand_key / cand_id: [nq][cap] candidate buffers, two segments of cap/2 entries per query; threshold tau[query];
+// counts[2*query + buffer] receives the number of entries appended to each (bit 30 set if it overflowed).
+// RANKED: no candidate buffers at all; every query thread keeps its 16 smallest keys in
 // registers and rank_out[query] receives the one of rank `rank` (0-based, < 16) when the scan ends: the first
 // threshold level, a scan of a few thousand sample points.
-template <int EPL, bool FIXED, int QH, bool RANKED = false>
+template <int QH, bool RANKED>
 __global__ void __launch_bounds__(tc_threads(QH), 1)
 knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ img_db, int Dp, long long nq, long long nd_pos,
                      const int2 *__restrict__ segs, const int *__restrict__ nseg, int seg_stride, int tile_stride, int win_lo,
                      int win_hi, const float *__restrict__ tau, int cap, float *cand_key, int32_t *cand_id, int *counts,
                      int *error_flag, int bf16, int sw, int nks, int rank = 0, float *__restrict__ rank_out = nullptr)
 {
-    static_assert(!(RANKED && FIXED), "the ranked scan keeps its own threshold");
     // bf16: the images hold bf16 pairs; sw != 0: in swizzled rows of sw bytes (else core matrices without swizzle);
     // nks: K steps of 32 operand bytes per row to multiply
-    constexpr int C = 32 * EPL;   // capacity handled by one compaction
-    constexpr int L = 16 * EPL;
     constexpr int kProducerWarp = 8 * QH, kMmaWarp = 8 * QH + 1;
     constexpr uint32_t kTmemCols = kAccBufs * QH * TN;
     extern __shared__ __align__(1024) unsigned char smem[];   // swizzled images want their 8-row groups on 8 * sw bytes
@@ -820,7 +692,7 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
     if (threadIdx.x == 0) {
         mbar_init(&sh.full_a, 1);
         for (int s = 0; s < kBStages; s++) { mbar_init(&sh.full_b[s], 1); mbar_init(&sh.empty_b[s], 1); }
-        for (int b = 0; b < kAccBufs; b++) { mbar_init(&sh.acc_full[b], 1); mbar_init(&sh.acc_empty[b], (FIXED ? 8 : 4) * QH); }
+        for (int b = 0; b < kAccBufs; b++) { mbar_init(&sh.acc_full[b], 1); mbar_init(&sh.acc_empty[b], (RANKED ? 4 : 8) * QH); }
         sh.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -890,24 +762,24 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
         // takes the 64 accumulator columns buf * 64 ... (buf = g / QH) and appends to segment buf of the query's
         // candidate buffer, so the groups share nothing.  (A warp walks its keys as one dependent chain, about
         // 800 cycles per 32 keys: with all sixteen warps on a tile its epilogue takes half as long as with the
-        // groups taking whole tiles in turn, and the accumulator goes back to the MMAs that much earlier.)  With
-        // the online threshold (per-query state that cannot be shared) only the groups with buf = 0 work, on
+        // groups taking whole tiles in turn, and the accumulator goes back to the MMAs that much earlier.)  In the
+        // ranked scan (per-query state that cannot be shared) only the groups with buf = 0 work, on
         // all columns of every tile.
         const int group = warp >> 2, quarter = warp & 3;
         const int buf = group / QH, half = group % QH;
-        const bool active = FIXED || buf == 0;
-        const int seg_cap = FIXED ? cap / kAccBufs : cap;
+        const bool active = !RANKED || buf == 0;
+        const int seg_cap = cap / kAccBufs;
         const int row = quarter * 32 + lane;                    // TMEM lane
         const long long gq = (qt + half) * TM + row;
         const bool serve = gq < nq && active;
-        float *bk = cand_key + (serve ? gq : 0) * cap + (FIXED ? buf * seg_cap : 0);
-        int32_t *bi = cand_id + (serve ? gq : 0) * cap + (FIXED ? buf * seg_cap : 0);
-        float thr = serve ? (FIXED ? tau[gq] : INFINITY) : -INFINITY;
+        float *bk = cand_key + (serve ? gq : 0) * cap + buf * seg_cap;
+        int32_t *bi = cand_id + (serve ? gq : 0) * cap + buf * seg_cap;
+        float thr = serve ? (RANKED ? INFINITY : tau[gq]) : -INFINITY;
         // a fixed-threshold scan may be split into several launches (windows of the database): a launch
         // continues the buffers where the previous one stopped (counts are zeroed before the first)
         int cnt = 0;
         bool overflow = false;
-        if (FIXED && serve) {
+        if (!RANKED && serve) {
             const int c0 = counts[gq * kAccBufs + buf];
             cnt = c0 & 0x3fffffff;
             overflow = (c0 & 0x40000000) != 0;
@@ -962,23 +834,8 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
                     }
                 }
             }
-            if constexpr (RANKED) {
-                // nothing is buffered
-            } else if (FIXED) {
-                // a chunk appends at most 32 entries: stop a buffer that could overflow in the next one
-                if (cnt > seg_cap - 32) { overflow = true; thr = -INFINITY; }
-            } else {
-                // a chunk appends at most 32 entries: compact every buffer that could overflow in the next one
-                unsigned full = __ballot_sync(0xffffffffu, cnt > C - 32);
-                while (full) {
-                    const int owner = __ffs(full) - 1;
-                    full &= full - 1;
-                    const long long oq = (qt + half) * TM + quarter * 32 + owner;
-                    const int n = __shfl_sync(0xffffffffu, cnt, owner);
-                    const float nt = warp_compact<EPL>(cand_key + oq * cap, cand_id + oq * cap, n, lane);
-                    if (lane == owner) { thr = nt; cnt = L; }
-                }
-            }
+            // a chunk appends at most 32 entries: stop a buffer that could overflow in the next one
+            if (!RANKED && cnt > seg_cap - 32) { overflow = true; thr = -INFINITY; }
         };
 
         TileWalk walk(my_segs, active ? my_nseg : 0, tile_stride, win_lo, win_hi);
@@ -993,7 +850,7 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
             const uint32_t tcol = lane_base + (uint32_t)(b * QH * TN);
             // one copy of the chunk code, executed once per 32 columns: small code beats overlapping the TMEM reads
             // (16 keys per read with the next read in flight while these are compared was 4 % slower)
-            const int c_lo = FIXED ? buf * (TN / 2) : 0, c_hi = FIXED ? c_lo + TN / 2 : TN;   // this group's columns
+            const int c_lo = RANKED ? 0 : buf * (TN / 2), c_hi = RANKED ? TN : c_lo + TN / 2;   // this group's columns
 #pragma unroll 1
             for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
                 uint32_t r[32];
@@ -1007,27 +864,17 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
                 process_chunk(r, p0 + c0, inside);
             }
         }
-        if (FIXED) {
-            // The final selection is a separate kernel (one warp per query, thousands in flight): it is a chain of
-            // dependent global round trips, which the warps of this block would walk through one query at a time.
-            if (serve) counts[gq * kAccBufs + buf] = cnt | (overflow ? 0x40000000 : 0);
-        } else if (RANKED) {
+        if constexpr (RANKED) {
             if (serve) {
                 float t = top[0];
 #pragma unroll
-                for (int i = 1; i < (RANKED ? 16 : 1); i++) t = (i == rank) ? top[i] : t;
+                for (int i = 1; i < 16; i++) t = (i == rank) ? top[i] : t;
                 rank_out[gq] = t;
             }
-        } else if (active) {
-            // online threshold (small databases): one last compaction leaves the L best, sorted, in front
-            unsigned m = __ballot_sync(0xffffffffu, serve);
-            while (m) {
-                const int owner = __ffs(m) - 1;
-                m &= m - 1;
-                const long long oq = (qt + half) * TM + quarter * 32 + owner;
-                const int n = __shfl_sync(0xffffffffu, cnt, owner);
-                (void)warp_compact<EPL>(cand_key + oq * cap, cand_id + oq * cap, min(n, C), lane);
-            }
+        } else {
+            // The final selection is a separate kernel (one warp per query, thousands in flight): it is a chain of
+            // dependent global round trips, which the warps of this block would walk through one query at a time.
+            if (serve) counts[gq * kAccBufs + buf] = cnt | (overflow ? 0x40000000 : 0);
         }
     }
     // ---------------- teardown ----------------
@@ -1067,7 +914,7 @@ struct WideShared {
 
 // RANKED: the first threshold level (see the narrow kernel): no buffers, the warps of the unit's first database tile
 // read both tiles and keep the 16 smallest keys of their queries in registers; positions from n_pos on are padding.
-template <int EPL, bool RANKED = false>
+template <bool RANKED>
 __global__ void __launch_bounds__(tc_threads(2), 1)
 knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ img_db, int n_chunks, long long nq,
                    const int2 *__restrict__ segs, const int *__restrict__ nseg, int seg_stride, int unit_stride, int win_lo,
@@ -1297,102 +1144,88 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
 }
 
 // ------------------------------------------------------------------------------------------------
-// final selection after a fixed-threshold scan: one warp per query
+// selection after a scan: one warp per query
 // ------------------------------------------------------------------------------------------------
 // Buffer of query q: two segments of cap/2 entries with counts[2q], counts[2q+1] valid entries (bit 30 of a
-// count: the segment overflowed, i.e. keys below tau were lost).
-// The k smallest keys of the buffer by selection rather than sorting (a warp-wide bitonic sort of the buffer
-// was measured at ~17 000 issue slots per query, this takes ~1 500).  The warp holds the keys in
-// registers as order-preserving integers, finds the k-th smallest value v by bisection on the 32 bits (each
-// step counts the keys <= mid), keeps every key below v and as many of the keys equal to v as are needed.
-// kth[q] (optional) = v, or -inf when the buffer lost keys or holds fewer than k; out_* (optional) receive
-// the k kept pairs in buffer order, padded with (+inf, INT_MAX); row_flags[q]: bit 0 = a segment overflowed,
-// bit 1 = fewer than k candidates.
-template <int SLOTS>
-__global__ void __launch_bounds__(128)
-knn_tc_pick_kernel(const float *__restrict__ cand_key, const int32_t *__restrict__ cand_id, int cap, const int *__restrict__ counts,
-                   long long nq, int k, float *__restrict__ out_key, int32_t *__restrict__ out_id, int out_stride,
-                   float *__restrict__ kth, int *__restrict__ row_flags)
+// count: the segment overflowed, i.e. keys below tau were lost).  The warp holds the keys in registers as
+// order-preserving integers (SLOTS a lane, the two segments one after the other) and finds the k-th smallest by bisection on
+// the bits between the smallest and the largest key of the buffer: they share their leading bits, so about half of 32
+// steps are enough, 1,500 issue slots (a warp-wide bitonic sort: 17,000).
+struct CandidateBuffer {
+    const float *key;
+    const int32_t *id;
+    int n0, n, half;
+    bool lost;
+    __device__ CandidateBuffer(const float *cand_key, const int32_t *cand_id, int cap, const int *counts, long long q)
+        : key(cand_key + q * cap), id(cand_id + q * cap), half(cap / 2)
+    {
+        const int c0 = counts[2 * q], c1 = counts[2 * q + 1];
+        lost = ((c0 | c1) & 0x40000000) != 0;
+        n0 = c0 & 0x3fffffff;
+        n = n0 + (c1 & 0x3fffffff);
+    }
+    __device__ int at(int e) const { return e < n0 ? e : half + (e - n0); }
+};
+template <int SLOTS> __device__ __forceinline__ void load_keys(const CandidateBuffer &b, int lane, unsigned (&enc)[SLOTS], unsigned &lo, unsigned &hi)
 {
-    const int lane = threadIdx.x & 31;
-    const long long q = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (q >= nq) return;
-    const int c0 = counts[2 * q], c1 = counts[2 * q + 1];
-    const bool ovf = ((c0 | c1) & 0x40000000) != 0;
-    const int n0 = c0 & 0x3fffffff, n1 = c1 & 0x3fffffff, n = n0 + n1;
-    const int jmax = (n + 31) / 32;
-    const float *bk = cand_key + q * cap;
-    const int32_t *bi = cand_id + q * cap;
-    unsigned int enc[SLOTS];
+    lo = 0xffffffffu;
+    hi = 0u;
 #pragma unroll
     for (int j = 0; j < SLOTS; j++) {
         const int e = lane + 32 * j;
         enc[j] = 0xffffffffu;
-        if (e < n) enc[j] = enc_float(__ldcg(bk + (e < n0 ? e : cap / 2 + (e - n0))));
+        if (e < b.n) {
+            enc[j] = enc_float(__ldcg(b.key + b.at(e)));
+            lo = min(lo, enc[j]);
+            hi = max(hi, enc[j]);
+        }
     }
-    unsigned int v = 0xffffffffu;   // with fewer than k keys everything is kept
-    if (n > k) {
-        // bisection between the smallest and the largest key of the buffer: they share their leading bits, so about
-        // half of the 32 steps of a search over all encodings are enough
-        unsigned int lo = 0xffffffffu, hi = 0u;
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+}
+// the smallest value with at least k keys at or below it; 0 < k <= n
+template <int SLOTS> __device__ __forceinline__ unsigned kth_key(const unsigned (&enc)[SLOTS], int n, int k, unsigned lo, unsigned hi)
+{
+    const int jmax = (n + 31) / 32;
+#pragma unroll 1
+    while (lo < hi) {
+        const unsigned mid = lo + ((hi - lo) >> 1);
+        int c = 0;
 #pragma unroll
         for (int j = 0; j < SLOTS; j++) {
             if (j >= jmax) break;
-            if (lane + 32 * j < n) { lo = min(lo, enc[j]); hi = max(hi, enc[j]); }
+            c += (enc[j] <= mid) ? 1 : 0;
         }
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-#pragma unroll 1
-        for (int it = 0; it < 32 && lo < hi; it++) {
-            const unsigned int mid = lo + ((hi - lo) >> 1);
-            int cnt = 0;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c >= k) hi = mid;
+        else lo = mid + 1;
+        if (c == k) {   // exactly those: the largest of them
+            unsigned v = 0u;
 #pragma unroll
-            for (int j = 0; j < SLOTS; j++) {
-                if (j >= jmax) break;
-                cnt += (enc[j] <= mid) ? 1 : 0;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-            if (cnt >= k) hi = mid;
-            else lo = mid + 1;
+            for (int j = 0; j < SLOTS; j++)
+                if (enc[j] <= hi) v = max(v, enc[j]);
+            return __reduce_max_sync(0xffffffffu, v);
         }
-        v = lo;
     }
-    const bool short_list = n < k;
-    if (kth && lane == 0) kth[q] = (ovf || short_list) ? -INFINITY : dec_float(v);
-    if (lane == 0) row_flags[q] = (ovf ? 1 : 0) | (short_list ? 2 : 0);
-    if (!out_key) return;
-    // keys below v, then as many keys equal to v as fit
-    int below = 0;
-#pragma unroll
-    for (int j = 0; j < SLOTS; j++) {
-        if (j >= jmax) break;
-        below += (enc[j] < v) ? 1 : 0;
+    return lo;
+}
+
+// kth[q] = the k-th smallest key of the buffer, or -inf when it lost keys or holds fewer than k
+template <int SLOTS>
+__global__ void __launch_bounds__(128)
+knn_tc_pick_kernel(const float *__restrict__ cand_key, int cap, const int *__restrict__ counts, long long nq, int k, float *__restrict__ kth)
+{
+    const int lane = threadIdx.x & 31;
+    const long long q = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (q >= nq) return;
+    const CandidateBuffer b(cand_key, nullptr, cap, counts, q);
+    float v = -INFINITY;
+    if (!b.lost && b.n >= k) {
+        unsigned enc[SLOTS], lo, hi;
+        load_keys(b, lane, enc, lo, hi);
+        v = dec_float(kth_key(enc, b.n, k, lo, hi));
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
-    int room_eq = min(k, n) - below;     // keys equal to v still to take (n <= k: v is above every key, all are "below")
-    int out_pos = 0;
-    float *ok = out_key + q * out_stride;
-    int32_t *oi = out_id + q * out_stride;
-    const unsigned int lt = (1u << lane) - 1u;
-#pragma unroll
-    for (int j = 0; j < SLOTS; j++) {
-        if (j >= jmax) break;
-        const int e = lane + 32 * j;
-        const bool is_eq = enc[j] == v && e < n;
-        const unsigned int eqmask = __ballot_sync(0xffffffffu, is_eq);
-        const bool keep = (e < n) && (enc[j] < v || (is_eq && __popc(eqmask & lt) < room_eq));
-        const unsigned int keepmask = __ballot_sync(0xffffffffu, keep);
-        if (keep) {
-            const int slot = e < n0 ? e : cap / 2 + (e - n0);
-            ok[out_pos + __popc(keepmask & lt)] = dec_float(enc[j]);
-            oi[out_pos + __popc(keepmask & lt)] = __ldcg(bi + slot);
-        }
-        out_pos += __popc(keepmask);
-        room_eq -= min(room_eq, __popc(eqmask));
-    }
-    for (int e = out_pos + lane; e < k; e += 32) { ok[e] = INFINITY; oi[e] = INT_MAX; }
+    if (lane == 0) kth[q] = v;
 }
 
 // Xp[pos] = X[list[pos]] (zeros for padding): the database rows in visiting order (the bf16 images' kernel writes them
@@ -1419,10 +1252,14 @@ __device__ __forceinline__ float canon_step(float acc, float x, float y)
 
 constexpr int kRerankWarps = 4;
 constexpr int kMaxL = 256;
-constexpr int kRerankDims = 32;                  // dimensions per stage
-constexpr int kRerankStride = kRerankDims + 4;   // floats per staged row: rows 144 bytes apart, 16-byte reads without conflicts
-constexpr size_t kRerankStage = (size_t)33 * kRerankStride;   // 32 candidate rows and the query
-constexpr size_t rerank_smem(int L) { return kRerankWarps * (sizeof(float) * 2 * kRerankStage + (size_t)L * 16); }
+constexpr int kRerankDims = 32;   // dimensions per stage of wide rows
+constexpr int kRerankWhole = 64;  // rows of up to this many dimensions are staged whole
+
+// Staged rows are `stride` floats apart: a multiple of 4, but not of 8, so that 32 lanes read 16 bytes of a row of their own
+// without bank conflicts.
+__host__ __device__ constexpr int rerank_stride(int D) { const int d = D <= kRerankWhole ? (D + 3) / 4 * 4 : kRerankDims; return d % 8 == 0 ? d + 4 : d; }
+// one warp: one stage (two where the row is walked) of 32 candidate rows and the query; L evaluated candidates
+__host__ __device__ constexpr size_t rerank_floats(int D, int L) { return (size_t)(D <= kRerankWhole ? 1 : 2) * 33 * rerank_stride(D) + 4 * (size_t)L; }
 
 template <int BYTES> __device__ __forceinline__ void async_copy(void *dst, const void *src)
 {
@@ -1432,59 +1269,46 @@ template <int BYTES> __device__ __forceinline__ void async_copy(void *dst, const
 
 // One warp per query of the list (query row qlist[q]; candidate ids are positions in dblist).  Row
 // (qlist[q] - out_base) of ids/d2 ([.][K]) receives the K best candidates by (canonical distance, row id);
-// failed[q] = 1 when the proof does not close for the query.
+// failed[q] = 1 when the proof does not close for the query (its output is then unspecified).
 //
 // Bound: the candidates' rows out of L2 (K rows per query cannot be left out: 17 GB for 60,000 queries of 784
-// dimensions, K = 90).  So only the candidates that can be among the K best are read: one whose key is more than twice
-// the filter's error above the K-th smallest key cannot (95 of 128 at K = 90, 40 at K = 32).  32 of them at a time are
-// staged 32 dimensions wide, VEC floats a copy, two stages in turn: whole 128-byte lines per request, where a lane that
-// walks its own row touches 32 lines with each.  A lane then reads its row from shared memory and sums in the canonical
-// order.  Measured: 60,000 x 784, K = 90: LATER.
-template <int VEC>
-__global__ void __launch_bounds__(kRerankWarps * 32)
+// dimensions, K = 90).  So of the buffer's ~3 L candidates only those are read that can be among the K best: one whose key
+// is more than twice the filter's error above the K-th smallest key cannot (95 at K = 90, 40 at K = 32); where the error
+// is so large that more than L remain, the L smallest.  32 rows at a time are staged with asynchronous copies, VEC floats
+// each, whole or 32 dimensions wide in two stages: whole lines per request, where a lane that walks a row of its own
+// touches 32 lines with each.  A lane then reads its row from shared memory and sums in the canonical order.
+// Measured with the pass that used to write the L best out first: LATER.
+template <int VEC, int SLOTS>
+__global__ void __launch_bounds__(kRerankWarps * 32, SLOTS <= 32 ? 6 : 4)
 knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__ qlist, const int *__restrict__ dblist,
-                     long long out_base, long long nq, const float *__restrict__ cand_key,
-                     const int32_t *__restrict__ cand_id, int L, int C, int K, const double *__restrict__ norms_exact,
-                     float err_scale, const float2 *__restrict__ res_q, const float *__restrict__ rho, const int *__restrict__ row_flags,
-                     int32_t *__restrict__ ids, float *__restrict__ d2,
-                     int *__restrict__ failed,
-                     int *__restrict__ n_failed, float *__restrict__ max_err_ratio, const float *__restrict__ Xp)
+                     long long out_base, long long nq, const float *__restrict__ cand_key, const int32_t *__restrict__ cand_id, int cap,
+                     const int *__restrict__ counts, const float *__restrict__ tau, int L, int K, const double *__restrict__ norms_exact,
+                     float err_scale, const float2 *__restrict__ res_q, const float *__restrict__ rho, int32_t *__restrict__ ids,
+                     float *__restrict__ d2, int *__restrict__ failed, int *__restrict__ n_failed, float *__restrict__ max_err_ratio,
+                     const float *__restrict__ Xp)
 {
     // Xp (optional): the database rows in list order, Xp[pos] = X[dblist[pos]]
     extern __shared__ __align__(16) float stage_mem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long q = (long long)blockIdx.x * kRerankWarps + w;
     if (q >= nq) return;
+    const CandidateBuffer b(cand_key, cand_id, cap, counts, q);
+    if (b.lost || b.n < K) {   // the fixed threshold kept too few or too many
+        if (lane == 0) { failed[q] = 1; atomicAdd(n_failed, 1); }
+        return;
+    }
     const long long gq = qlist[q];
     const long long orow = gq - out_base;
     const double ni = norms_exact[q];
-    float *stage = stage_mem + (size_t)w * (2 * kRerankStage + 4 * L);
-    // evaluated candidates: distance bits and row id, list position, filter key
-    unsigned long long *s_key = reinterpret_cast<unsigned long long *>(stage + 2 * kRerankStage);
-    int *s_pos = reinterpret_cast<int *>(s_key + L);
-    float *s_fkey = reinterpret_cast<float *>(s_pos + L);
-    constexpr int kPer = kMaxL / 32;
-    float key[kPer];
-    int pos[kPer];
-    float T = -INFINITY;   // the largest key of the list: whatever is not in it has a key at least as large
-    int n_valid = 0;
-    unsigned lo = 0xffffffffu, hi = 0u;
-#pragma unroll
-    for (int j = 0; j < kPer; j++) {
-        const int e = lane + 32 * j;
-        pos[j] = e < L ? cand_id[q * C + e] : INT_MAX;
-        key[j] = e < L ? cand_key[q * C + e] : INFINITY;
-        if (pos[j] != INT_MAX && dblist[pos[j]] < 0) pos[j] = INT_MAX;   // a padding position (never kept by a finite threshold)
-        if (pos[j] != INT_MAX) {
-            T = fmaxf(T, key[j]);
-            n_valid++;
-            lo = min(lo, enc_float(key[j]));
-            hi = max(hi, enc_float(key[j]));
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) T = fmaxf(T, __shfl_xor_sync(0xffffffffu, T, o));
-    n_valid = __reduce_add_sync(0xffffffffu, n_valid);
+    const int stride = rerank_stride(D);
+    const bool whole = D <= kRerankWhole;
+    float *stage = stage_mem + (size_t)w * rerank_floats(D, L);
+    // evaluated candidates: distance bits and row id, row of `base`, filter key
+    unsigned long long *s_key = reinterpret_cast<unsigned long long *>(stage + (whole ? 1 : 2) * 33 * stride);
+    int *s_src = reinterpret_cast<int *>(s_key + L);
+    float *s_fkey = reinterpret_cast<float *>(s_src + L);
+    const float *base = Xp ? Xp : X;
+    const float T = tau[q];   // every database point with a key below this is in the buffer
     // Error bound of the filter's key for this row: it scales with |x_i||x_j|, and a point whose key is
     // near T lies within sqrt(|x_i|^2 + T) of x_i, so |x_i||x_j| <= |x_i|^2 + (|x_i|^2 + T)+ up to a factor 2.
     double E = (double)err_scale * (ni + fmax(0.0, ni + (double)T) + 1.0);
@@ -1500,69 +1324,61 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
         E += dropped;
     }
     const double theta = (double)(D + 4) * 5.9604644775390625e-08;   // (D+4) * 2^-24
-    // The cut: a candidate with key above key_K + 2 E (and the rounding of the canonical sums) has K others before it.
-    float cut = INFINITY;
-    if (n_valid > K) {
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-        while (lo < hi) {   // the K-th smallest key by bisection on the bits
-            const unsigned mid = lo + ((hi - lo) >> 1);
-            int c = 0;
-#pragma unroll
-            for (int j = 0; j < kPer; j++) c += pos[j] != INT_MAX && enc_float(key[j]) <= mid;
-            c = __reduce_add_sync(0xffffffffu, c);
-            if (c >= K) hi = mid;
-            else lo = mid + 1;
-            if (c == K) break;
-        }
-        float kth = -INFINITY;   // exactly the key: the bound may lie anywhere in the gap above it
-#pragma unroll
-        for (int j = 0; j < kPer; j++)
-            if (pos[j] != INT_MAX && enc_float(key[j]) <= hi) kth = fmaxf(kth, key[j]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) kth = fmaxf(kth, __shfl_xor_sync(0xffffffffu, kth, o));
-        const double kk = (double)kth;
-        cut = __double2float_ru(kk + 2.0 * E + 4.0 * theta * fmax(0.0, ni + kk + E) + 1e-30);
-    }
-    // the evaluated ones, close together
     int m = 0;
-    float outside = INFINITY;   // the smallest key of a candidate that is left out
+    float outside = T;   // what is not evaluated has a key of at least this
+    {
+        unsigned enc[SLOTS], lo, hi;
+        load_keys(b, lane, enc, lo, hi);
+        const double kk = (double)dec_float(kth_key(enc, b.n, K, lo, hi));
+        // one with a key above key_K + 2 E (and the rounding of the canonical sums) has K others before it
+        unsigned cut = enc_float(__double2float_ru(kk + 2.0 * E + 4.0 * theta * fmax(0.0, ni + kk + E) + 1e-30));
+        int c = 0;
 #pragma unroll
-    for (int j = 0; j < kPer; j++) {
-        const bool valid = pos[j] != INT_MAX, take = valid && key[j] <= cut;
-        if (valid && !take) outside = fminf(outside, key[j]);
-        const unsigned mask = __ballot_sync(0xffffffffu, take);
-        if (take) {
-            const int at = m + __popc(mask & ((1u << lane) - 1u));
-            s_pos[at] = pos[j];
-            s_fkey[at] = key[j];
+        for (int j = 0; j < SLOTS; j++) c += (lane + 32 * j < b.n && enc[j] <= cut) ? 1 : 0;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c > L) {
+            cut = kth_key(enc, b.n, L, lo, hi);
+            c = 0;
+#pragma unroll
+            for (int j = 0; j < SLOTS; j++) c += (lane + 32 * j < b.n && enc[j] <= cut) ? 1 : 0;
+            c = __reduce_add_sync(0xffffffffu, c);
+            if (c > L) cut--;   // ties beyond the last place stay out
         }
-        m += __popc(mask);
+        const int jmax = (b.n + 31) / 32;
+#pragma unroll
+        for (int j = 0; j < SLOTS; j++) {
+            if (j >= jmax) break;
+            const int e = lane + 32 * j;
+            const bool take = e < b.n && enc[j] <= cut;
+            if (e < b.n && !take) outside = fminf(outside, dec_float(enc[j]));
+            const unsigned mask = __ballot_sync(0xffffffffu, take);
+            if (take) {
+                const int at = m + __popc(mask & ((1u << lane) - 1u));
+                const int p = __ldcg(b.id + b.at(e));
+                s_src[at] = Xp ? p : dblist[p];
+                s_fkey[at] = dec_float(enc[j]);
+            }
+            m += __popc(mask);
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) outside = fminf(outside, __shfl_xor_sync(0xffffffffu, outside, o));
     __syncwarp();
     float worst = 0.0f;   // largest observed |filter distance - canonical distance|
     const float *xq = X + gq * D;
-    const int chunks = (D + kRerankDims - 1) / kRerankDims;
-    constexpr int kLanesPerRow = kRerankDims / VEC, kRowsPerCopy = 32 / kLanesPerRow;
-    const int col = (lane % kLanesPerRow) * VEC, sub = lane / kLanesPerRow;
+    const int width = whole ? D : kRerankDims, chunks = whole ? 1 : (D + kRerankDims - 1) / kRerankDims;
+    // lanes per row of a copy: the power of two that covers the width, at most the warp
+    const int lanes_log = width <= 8 * VEC ? 3 : (width <= 16 * VEC ? 4 : 5);
+    const int col = (lane & ((1 << lanes_log) - 1)) * VEC, sub = lane >> lanes_log, rows_per_copy = 32 >> lanes_log;
     for (int g = 0; g < m; g += 32) {
-        // copies of chunk c of this group's rows and of the query
-        auto fetch = [&](int c) {
-            float *buf = stage + (size_t)(c & 1) * kRerankStage;
-            const int d = c * kRerankDims + col;
-            if (d < D) {
-                for (int r = sub; r < 33; r += kRowsPerCopy) {
-                    if (r < 32 && g + r >= m) continue;
-                    const float *row;
-                    if (r == 32) row = xq;
-                    else {
-                        const int p = s_pos[g + r];
-                        row = Xp ? Xp + (long long)p * D : X + (long long)dblist[p] * D;
-                    }
-                    async_copy<4 * VEC>(buf + r * kRerankStride + col, row + d);
-                }
+        const int rows = min(32, m - g);
+        auto fetch = [&](int c) {   // the group's rows and, in row 32, the query
+            float *buf = stage + (size_t)(c & 1) * 33 * stride;
+            const int d0 = c * width, d1 = min(width, D - d0);
+            for (int r = sub; r <= rows; r += rows_per_copy) {
+                const int to = r == rows ? 32 : r;
+                const float *row = (r == rows ? xq : base + (size_t)s_src[g + r] * D) + d0;
+                for (int d = col; d < d1; d += 32 * VEC) async_copy<4 * VEC>(buf + to * stride + d, row + d);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
@@ -1576,27 +1392,26 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
                 asm volatile("cp.async.wait_group 0;" ::: "memory");
             }
             __syncwarp();
-            const float *buf = stage + (size_t)(c & 1) * kRerankStage;
-            const float *mine = buf + lane * kRerankStride, *query = buf + 32 * kRerankStride;
-            const int len = min(kRerankDims, D - c * kRerankDims);
-            if (len == kRerankDims) {
-#pragma unroll
-                for (int d = 0; d < kRerankDims; d += 4) {
-                    const float4 u = *reinterpret_cast<const float4 *>(query + d), v = *reinterpret_cast<const float4 *>(mine + d);
-                    acc = canon_step(acc, u.x, v.x);
-                    acc = canon_step(acc, u.y, v.y);
-                    acc = canon_step(acc, u.z, v.z);
-                    acc = canon_step(acc, u.w, v.w);
-                }
-            } else {
-                for (int d = 0; d < len; d++) acc = canon_step(acc, query[d], mine[d]);
+            const float *buf = stage + (size_t)(c & 1) * 33 * stride;
+            const float *mine = buf + lane * stride, *query = buf + 32 * stride;
+            const int len = min(width, D - c * width);
+            int d = 0;
+#pragma unroll 4
+            for (; d + 4 <= len; d += 4) {
+                const float4 u = *reinterpret_cast<const float4 *>(query + d), v = *reinterpret_cast<const float4 *>(mine + d);
+                acc = canon_step(acc, u.x, v.x);
+                acc = canon_step(acc, u.y, v.y);
+                acc = canon_step(acc, u.z, v.z);
+                acc = canon_step(acc, u.w, v.w);
             }
+            for (; d < len; d++) acc = canon_step(acc, query[d], mine[d]);
             __syncwarp();
         }
-        if (g + lane < m) {
+        if (lane < rows) {
             const double approx = ni + (double)s_fkey[g + lane];
             worst = fmaxf(worst, (float)fabs(approx - (double)acc));
-            s_key[g + lane] = (unsigned long long)__float_as_uint(acc) << 32 | (unsigned)dblist[s_pos[g + lane]];
+            const int src = s_src[g + lane];
+            s_key[g + lane] = (unsigned long long)__float_as_uint(acc) << 32 | (unsigned)(Xp ? dblist[src] : src);
         }
     }
 #pragma unroll
@@ -1607,6 +1422,7 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
     for (int e = lane; e < m; e += 32) {
         const unsigned long long mine = s_key[e];
         int rank = 0;
+#pragma unroll 4
         for (int u = 0; u < m; u++) rank += s_key[u] < mine;
         const float de = __uint_as_float((unsigned)(mine >> 32));
         if (rank < K) {
@@ -1615,22 +1431,14 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
         }
         if (rank == K - 1) dK = de;
     }
-    for (int e = m + lane; e < K; e += 32) {   // fewer candidates than slots: the row fails below and is searched anew
-        ids[orow * K + e] = -1;
-        d2[orow * K + e] = INFINITY;
-    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dK = fminf(dK, __shfl_xor_sync(0xffffffffu, dK, o));
     if (lane == 0) {
-        bool ok = true;
-        // outsiders (not in the list: key >= T, with a full list; left out of it: key >= outside):
-        // canonical distance >= (ni + key - E) * (1 - theta)
-        const double nearest = fmin(n_valid == L ? (double)T : (double)INFINITY, (double)outside);
-        const double bound = (ni + nearest - E) * (1.0 - theta);
-        ok = !isfinite(nearest) || (double)dK < bound;
+        // outsiders: key >= outside  =>  canonical distance >= (ni + outside - E) * (1 - theta)
+        const double bound = (ni + (double)outside - E) * (1.0 - theta);
+        bool ok = (double)dK < bound;
         const float ratio = (float)(fmax(0.0, (double)worst - dropped) / (E - dropped));
-        if (ratio > 0.5f) ok = false;   // the filter was less accurate than the bound assumes
-        if (row_flags && row_flags[q]) ok = false;   // the fixed threshold kept too few or too many candidates
+        if (!(ratio <= 0.5f)) ok = false;   // the filter was less accurate than the bound assumes
         failed[q] = ok ? 0 : 1;
         if (!ok) atomicAdd(n_failed, 1);
         atomicMax(reinterpret_cast<int *>(max_err_ratio), __float_as_int(ratio));   // ratio >= 0: int order == float order
@@ -1818,27 +1626,24 @@ static bool tc_bf16()
     const char *e = getenv("B200TSNE_KNN_FILTER");
     return !(e && strcmp(e, "tf32") == 0);
 }
-constexpr long long kWideMinRows = 16384;   // the wide kernel has fixed thresholds only: it needs a database to sample
 
 // nd: database rows the search will scan
 bool knn_tc_supported(int64_t nd, int D, int K)
 {
     if (K + 32 > kMaxL || D > 8192) return false;
-    if (tc_wide(D)) return nd >= kWideMinRows;
-    return nd >= 2048;   // below this the SIMT search is faster than the set-up of this one
+    return nd >= 2048;   // below this whole rows of distances are faster than the set-up of this one (knn_dense.cu)
 }
 
 // candidate buffer entries per query in a fixed-threshold pass: 8 L (two halves of 4 L for ~1.5 L expected each)
 static int fixed_cap(int K) { return (K + 32 <= 128) ? 1024 : 2048; }
 constexpr int kSampleStride = 16;    // the sample pass looks at every 16th database tile
 constexpr int kMaxSampleTiles = 128; // first threshold level: at most 16 384 sample points
-constexpr long long kTwoPassMinTiles = 512;   // below this many database tiles the online pass alone is used
 
 // Device workspace of launch_knn_tc, carved in this order.
 struct TcWorkspace {
     bool wide, bf16;
     size_t image_bytes;        // one tile's image (hi and lo)
-    int Dp, cells;
+    int Dp;
     int sw, nks;               // narrow kernel: bytes of a swizzled image row (0: core matrices without swizzle), K steps
     long long tq, td;          // tiles allocated for the query list / the database list
     float *img_q, *img_db;
@@ -1848,13 +1653,13 @@ struct TcWorkspace {
     int *slist;
     int *qlist, *dblist;
     float *xp;   // database rows in list order (cells only)
-    unsigned char *cell_q, *cell_db;
-    CellTable *tab;
+    unsigned char *cell_q;     // queries outside the database range: their cells
+    float *dist_q;             // and distances to the centres
     int2 *segs;
     int *nseg;
-    float *cand_key, *fix_key, *tau;
-    int32_t *cand_id, *fix_id;
-    int *row_flags, *counts, *failed, *flist, *counters;
+    float *cand_key, *tau;
+    int32_t *cand_id;
+    int *counts, *failed, *flist, *counters;
     size_t bytes;
 };
 
@@ -1879,14 +1684,9 @@ static TcWorkspace tc_carve(void *base, int D, int K, long long nq, long long nd
         w.nks = w.Dp / 8;
     }
     w.image_bytes = (size_t)w.Dp * (w.bf16 ? 512 : 1024);
-    const bool two_pass = nd >= (w.wide ? kWideMinRows : kTwoPassMinTiles * TN);
-    // cells of at least 16384 points: the padding between them stays below 1 % of the database
-    // (wide points are not visited by cells: the cell kernels keep a point in registers)
-    w.cells = (two_pass && !w.wide) ? (int)std::min<long long>(kMaxCells, std::max<long long>(1, nd / 16384)) : 1;
     w.tq = (nq + TM - 1) / TM + 1;                 // one padding tile: a block may hold two query tiles
-    w.td = (nd + TN - 1) / TN + w.cells;           // every cell may end in a partly filled tile
+    w.td = (nd + TN - 1) / TN + point_cells_count(nd);   // every cell may end in a partly filled tile
     if (w.wide) w.td = (w.td + 1) / 2 * 2;         // the wide kernel takes the database two tiles at a time
-    const int C = (K + 32 <= 128) ? 256 : 512;
     char *p = static_cast<char *>(base);
     auto take = [&](size_t bytes) { char *r = p; p += (bytes + 255) / 256 * 256; return r; };
     w.img_q = reinterpret_cast<float *>(take((size_t)w.tq * w.image_bytes));
@@ -1895,27 +1695,17 @@ static TcWorkspace tc_carve(void *base, int D, int K, long long nq, long long nd
     w.res_q = reinterpret_cast<float2 *>(take(sizeof(float2) * (size_t)w.tq * TM));
     w.qlist = reinterpret_cast<int *>(take(sizeof(int) * (size_t)w.tq * TM));
     w.dblist = reinterpret_cast<int *>(take(sizeof(int) * (size_t)w.td * TN));
-    w.xp = (w.cells > 1) ? reinterpret_cast<float *>(take(sizeof(float) * (size_t)w.td * TN * D)) : nullptr;
-    w.img_s = nullptr; w.slist = nullptr;
-    if (two_pass) {
-        w.img_s = reinterpret_cast<float *>(take((size_t)kMaxSampleTiles * w.image_bytes));
-        w.slist = reinterpret_cast<int *>(take(sizeof(int) * (size_t)kMaxSampleTiles * TN));
-    }
+    w.xp = w.wide ? nullptr : reinterpret_cast<float *>(take(sizeof(float) * (size_t)w.td * TN * D));
+    w.img_s = reinterpret_cast<float *>(take((size_t)kMaxSampleTiles * w.image_bytes));
+    w.slist = reinterpret_cast<int *>(take(sizeof(int) * (size_t)kMaxSampleTiles * TN));
     w.cell_q = reinterpret_cast<unsigned char *>(take((size_t)nq));
-    w.cell_db = reinterpret_cast<unsigned char *>(take((size_t)nd));
-    w.tab = reinterpret_cast<CellTable *>(take(sizeof(CellTable)));
+    w.dist_q = reinterpret_cast<float *>(take(sizeof(float) * kMaxCells * (size_t)nq));
     w.segs = reinterpret_cast<int2 *>(take(sizeof(int2) * (size_t)w.tq * kMaxCells));
     w.nseg = reinterpret_cast<int *>(take(sizeof(int) * (size_t)w.tq));
-    w.cand_key = reinterpret_cast<float *>(take(sizeof(float) * (size_t)nq * C));
-    w.cand_id = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * (size_t)nq * C));
-    w.fix_key = nullptr; w.fix_id = nullptr; w.tau = nullptr; w.row_flags = nullptr; w.counts = nullptr;
-    if (two_pass) {
-        w.fix_key = reinterpret_cast<float *>(take(sizeof(float) * (size_t)nq * fixed_cap(K)));
-        w.fix_id = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * (size_t)nq * fixed_cap(K)));
-        w.tau = reinterpret_cast<float *>(take(sizeof(float) * (size_t)nq));
-        w.row_flags = reinterpret_cast<int *>(take(sizeof(int) * (size_t)nq));
-        w.counts = reinterpret_cast<int *>(take(sizeof(int) * (size_t)nq * 2));
-    }
+    w.cand_key = reinterpret_cast<float *>(take(sizeof(float) * (size_t)nq * fixed_cap(K)));
+    w.cand_id = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * (size_t)nq * fixed_cap(K)));
+    w.tau = reinterpret_cast<float *>(take(sizeof(float) * (size_t)nq));
+    w.counts = reinterpret_cast<int *>(take(sizeof(int) * (size_t)nq * 2));
     w.failed = reinterpret_cast<int *>(take(sizeof(int) * (size_t)nq));
     w.flist = reinterpret_cast<int *>(take(sizeof(int) * (size_t)nq));
     w.counters = reinterpret_cast<int *>(take(sizeof(int) * 16));   // [0] wait time-out flag, [1] failed rows, [2] listed rows, [3] max error ratio (float bits), [4], [5] largest relative lo part / leftover of a database row (float bits)
@@ -1966,7 +1756,7 @@ size_t knn_tc_workspace_bytes(int D, int K, int64_t nq, int64_t nd) { return tc_
 // whose proof did not close; their global row indices are in failed_list (device, first n entries) and
 // the caller recomputes them with the SIMT search.  Returns after the kernels are queued, except for
 // the small synchronous read of the counters.
-int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo, int64_t db_hi,
+int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo, int64_t db_hi, const PointCells &pc,
                   int32_t *ids, float *d2, void *workspace, int **failed_list, int *n_failed_host, float *err_ratio_host,
                   cudaStream_t st)
 {
@@ -1974,17 +1764,16 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     const long long nq = q_hi - q_lo, nd = db_hi - db_lo;
     *n_failed_host = 0;
     if (nq <= 0) return 0;
-    TcWorkspace w = tc_carve(workspace, D, K, nq, nd);
-    const int Dp = w.Dp, cells = w.cells;
+    const TcWorkspace w = tc_carve(workspace, D, K, nq, nd);
+    const int Dp = w.Dp, cells = pc.cells;
     const bool wide = w.wide;
     const int bf16 = w.bf16 ? 1 : 0;
     const int KC = wide ? (bf16 ? 2 * kWideKC : kWideKC) : Dp;   // inner dimensions per image chunk
-    const int EPL = (K + 32 <= 128) ? 8 : 16, C = 32 * EPL, L = 16 * EPL;
-    const int kFixedCap = fixed_cap(K);
-    const bool two_pass = w.fix_key != nullptr;
-    float *cand_key = w.cand_key, *fix_key = w.fix_key, *tau = w.tau;
-    int32_t *cand_id = w.cand_id, *fix_id = w.fix_id;
-    int *row_flags = w.row_flags, *counts = w.counts, *failed = w.failed, *flist = w.flist, *counters = w.counters;
+    const int L = (K + 32 <= 128) ? 128 : 256;                   // candidates that may be evaluated per query; about 3 L pass a scan
+    const int cap = fixed_cap(K);
+    float *cand_key = w.cand_key, *tau = w.tau;
+    int32_t *cand_id = w.cand_id;
+    int *counts = w.counts, *failed = w.failed, *flist = w.flist, *counters = w.counters;
     B200_CUDA(cudaMemsetAsync(counters, 0, sizeof(int) * 16, st));
     PhaseTimer phases(st);
     phases.mark("start");
@@ -1993,26 +1782,37 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     B200_CUDA(cudaMemsetAsync(w.qlist, 0xff, sizeof(int) * (size_t)w.tq * TM, st));    // -1 = padding
     B200_CUDA(cudaMemsetAsync(w.dblist, 0xff, sizeof(int) * (size_t)w.td * TN, st));
     long long nd_pos = nd;   // database list positions in use (an upper bound when the cells are padded)
+    const float *q_dist = nullptr;   // the queries' distances to the centres
     if (cells > 1) {
         const unsigned gq = (unsigned)((nq + kCellThreads - 1) / kCellThreads), gd = (unsigned)((nd + kCellThreads - 1) / kCellThreads);
-        knn_cells_init_kernel<<<1, 256, 0, st>>>(X, D, db_lo, nd, cells, w.tab);
-        knn_cells_assign_kernel<<<gd, kCellThreads, 0, st>>>(X, D, db_lo, nd, cells, w.tab, 1, w.cell_db);
-        knn_cells_assign_kernel<<<gq, kCellThreads, 0, st>>>(X, D, q_lo, nq, cells, w.tab, 0, w.cell_q);
-        knn_cells_layout_kernel<<<1, 32, 0, st>>>(cells, w.tab);
-        knn_cells_scatter_kernel<<<gd, kCellThreads, 0, st>>>(w.cell_db, db_lo, nd, cells, w.tab, 1, w.dblist);
-        knn_cells_scatter_kernel<<<gq, kCellThreads, 0, st>>>(w.cell_q, q_lo, nq, cells, w.tab, 0, w.qlist);
+        const unsigned char *cell_q = nullptr;
+        if (q_lo >= pc.lo && q_hi <= pc.lo + pc.n) {
+            q_dist = pc.dist + (size_t)(q_lo - pc.lo) * kMaxCells;
+            cell_q = pc.cell + (q_lo - pc.lo);
+        } else {   // queries that are not database rows
+            q_dist = w.dist_q;
+            cell_q = w.cell_q;
+            B200_TRY(point_cells_assign(pc, X, D, q_lo, nq, w.dist_q, w.cell_q, st));
+        }
+        knn_cells_reset_kernel<<<1, kMaxCells, 0, st>>>(pc.tab);
+        knn_cells_count_kernel<<<std::min(gd, 592u), kCellThreads, 0, st>>>(pc.cell, pc.dist, nd, pc.tab, 1);
+        knn_cells_count_kernel<<<std::min(gq, 592u), kCellThreads, 0, st>>>(cell_q, q_dist, nq, pc.tab, 0);
+        knn_cells_layout_kernel<<<1, 32, 0, st>>>(cells, pc.tab);
+        knn_cells_scatter_kernel<<<gd, kCellThreads, 0, st>>>(pc.cell, db_lo, nd, cells, pc.tab, 1, w.dblist);
+        knn_cells_scatter_kernel<<<gq, kCellThreads, 0, st>>>(cell_q, q_lo, nq, cells, pc.tab, 0, w.qlist);
         nd_pos = w.td * TN;
-        if (!bf16) knn_gather_rows_kernel<<<(unsigned)((nd_pos * D + 255) / 256), 256, 0, st>>>(X, w.dblist, D, nd_pos, w.xp);
+        if (!bf16 && w.xp) knn_gather_rows_kernel<<<(unsigned)((nd_pos * D + 255) / 256), 256, 0, st>>>(X, w.dblist, D, nd_pos, w.xp);
     } else {
         knn_iota_kernel<<<(unsigned)((nd + 255) / 256), 256, 0, st>>>(w.dblist, db_lo, nd);
         knn_iota_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(w.qlist, q_lo, nq);
     }
+    float *const xp = cells > 1 ? w.xp : nullptr;
     B200_CUDA(cudaGetLastError());
     if (bf16) {
         knn_tc_prepare_bf16_kernel<<<(unsigned)w.tq, 256, 0, st>>>(X, w.qlist, D, Dp, KC, w.sw, 0, reinterpret_cast<__nv_bfloat16 *>(w.img_q),
                                                                    w.norms_q, w.res_q, nullptr, nullptr);
         knn_tc_prepare_bf16_kernel<<<(unsigned)w.td, 256, 0, st>>>(X, w.dblist, D, Dp, KC, w.sw, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_db),
-                                                                   nullptr, nullptr, counters + 4, w.xp);
+                                                                   nullptr, nullptr, counters + 4, xp);
     } else {
         knn_tc_prepare_kernel<<<(unsigned)w.tq, 128, 0, st>>>(X, w.qlist, D, Dp, KC, 0, w.img_q, w.norms_q);
         knn_tc_prepare_kernel<<<(unsigned)w.td, 128, 0, st>>>(X, w.dblist, D, Dp, KC, 1, w.img_db, nullptr);
@@ -2025,14 +1825,15 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     const int QH = ((size_t)(2 + kBStages) * w.image_bytes + 1024 <= 227 * 1024) ? 2 : 1;
     const long long q_tiles = (nq + TM - 1) / TM;
     // Segments of the blocks: all database tiles (one shared list) unless the cells prune (per block).
-    // The blocks of an online pass hold one query tile, those of a fixed-threshold pass QH.
-    knn_single_segment_kernel<<<1, 1, 0, st>>>(w.segs, w.nseg, wide ? (int)(w.td / 2) : (int)((nd + TN - 1) / TN));
+    const int all_tiles = wide ? (int)(w.td / 2) : (int)((cells > 1 ? nd_pos : nd + TN - 1) / TN);   // wide: pairs of tiles
+    knn_single_segment_kernel<<<1, 1, 0, st>>>(w.segs, w.nseg, all_tiles);
     B200_CUDA(cudaGetLastError());
     int seg_stride = 0;
     auto prune = [&]() -> int {   // segments from the current thresholds
         if (cells <= 1) return 0;
-        knn_cells_segments_kernel<<<(unsigned)((q_tiles + QH - 1) / QH), kCellThreads, 0, st>>>(X, D, w.qlist, nq, QH * TM, tau, w.norms_q,
-                                                                                              cells, w.tab, w.segs, w.nseg);
+        const int per_block = wide ? 2 : QH;
+        knn_cells_segments_kernel<<<(unsigned)((q_tiles + per_block - 1) / per_block), kCellThreads, 0, st>>>(
+            q_dist, q_lo, w.qlist, nq, per_block * TM, tau, w.norms_q, cells, 1e-4f + (float)(D + 2) * 5.97e-8f, wide ? 1 : 0, pc.tab, w.segs, w.nseg);
         B200_CUDA(cudaGetLastError());
         seg_stride = kMaxCells;
         return 0;
@@ -2044,147 +1845,105 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     const long long db_image_bytes = (long long)w.td * (long long)w.image_bytes;
     int window_tiles = db_image_bytes > (512ll << 20) ? (int)((60ll << 20) / (long long)w.image_bytes) : INT_MAX;
     if (const char *e = getenv("B200TSNE_KNN_WINDOW_TILES")) window_tiles = std::max(1, atoi(e));   // for tests
-#define B200_KNN_FILTER_V(EPL_, FIXED_, QH_, stride_, tau_, cap_, key_, id_, counts_)                                           \
-    do {                                                                                                                        \
-        const size_t smem_ = (size_t)(QH_ + kBStages) * w.image_bytes;                                                          \
-        B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<EPL_, FIXED_, QH_>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
-                                       (int)smem_));                                                                            \
-        if (FIXED_) B200_CUDA(cudaMemsetAsync(counts_, 0, sizeof(int) * (size_t)nq * kAccBufs, st));                            \
-        const long long win_ = FIXED_ ? (long long)window_tiles * (stride_) : (long long)INT_MAX;                               \
-        for (long long lo_ = 0; lo_ < w.td; lo_ += win_) {                                                                      \
-            const int hi_ = (int)std::min<long long>(w.td, lo_ + win_);                                                         \
-            knn_tc_filter_kernel<EPL_, FIXED_, QH_><<<(unsigned)((q_tiles + QH_ - 1) / QH_), tc_threads(QH_), smem_, st>>>(      \
-                w.img_q, w.img_db, Dp, nq, nd_pos, w.segs, w.nseg, seg_stride, stride_, (int)lo_, hi_, tau_, cap_, key_, id_,   \
-                counts_, counters + 0, bf16, w.sw, w.nks);                                                                      \
-            B200_CUDA(cudaGetLastError());                                                                                      \
-        }                                                                                                                       \
-    } while (0)
-    // wide points: the same scan by the chunked kernel, in units of two database tiles
-#define B200_KNN_FILTER_WIDE(EPL_, stride_, tau_, cap_, key_, id_, counts_)                                                      \
-    do {                                                                                                                        \
-        const size_t smem_ = (size_t)kWideStages * 4 * kWideChunkBytes;                                                         \
-        B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<EPL_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_));      \
-        B200_CUDA(cudaMemsetAsync(counts_, 0, sizeof(int) * (size_t)nq * 2, st));                                               \
-        const long long units_ = w.td / 2;                                                                                      \
-        const long long win_ = (long long)std::max(1, window_tiles / 2) * (stride_);                                            \
-        for (long long lo_ = 0; lo_ < units_; lo_ += win_) {                                                                    \
-            const int hi_ = (int)std::min<long long>(units_, lo_ + win_);                                                       \
-            knn_tc_wide_kernel<EPL_><<<(unsigned)((q_tiles + 1) / 2), tc_threads(2), smem_, st>>>(                               \
-                w.img_q, w.img_db, Dp / KC, nq, w.segs, w.nseg, seg_stride, stride_, (int)lo_, hi_, tau_, cap_, key_, id_,       \
-                counts_, counters + 0, bf16);                                                                                   \
-            B200_CUDA(cudaGetLastError());                                                                                      \
-        }                                                                                                                       \
-    } while (0)
-    // the online threshold keeps one group per query busy: one query tile per block is enough there
-#define B200_KNN_FILTER(EPL_, FIXED_, stride_, tau_, cap_, key_, id_, counts_)                                                   \
-    do {                                                                                                                        \
-        if (FIXED_ && wide) B200_KNN_FILTER_WIDE(EPL_, stride_, tau_, cap_, key_, id_, counts_);                                 \
-        else if (!FIXED_ || QH == 1) B200_KNN_FILTER_V(EPL_, FIXED_, 1, stride_, tau_, cap_, key_, id_, counts_);                \
-        else B200_KNN_FILTER_V(EPL_, FIXED_, (FIXED_ ? 2 : 1), stride_, tau_, cap_, key_, id_, counts_);                         \
-    } while (0)
-    const float *final_key = cand_key;
-    const int32_t *final_id = cand_id;
-    int final_stride = C;
-    if (!two_pass) {
-        if (EPL == 8) B200_KNN_FILTER(8, false, 1, nullptr, C, cand_key, cand_id, nullptr);
-        else B200_KNN_FILTER(16, false, 1, nullptr, C, cand_key, cand_id, nullptr);
-    } else {
-        // Three levels, each fixing the threshold of the next:
-        //  A  (CUDA cores) rank ~10 of a few thousand sample points spread over the database -> tau_A,
-        //     chosen so that ~300 points of sample B beat it;
-        //  B  every kSampleStride-th tile against tau_A;
-        //  C  everything against tau_B = the key of rank ~3L/kSampleStride in sample B: ~3L points beat it.
-        // Before each scan the cells are tested against the thresholds it will use; a skipped cell holds no
-        // point below them, so the candidate sets (and the sample statistics) are those of a full scan.
-        // (the wide kernel strides over units of two tiles: the same 1/kSampleStride of the database)
-        const long long n_db_tiles = (nd + TN - 1) / TN;
-        const double b_points = wide ? (double)((n_db_tiles / 2 + kSampleStride - 1) / kSampleStride) * kWideUnit
-                                     : (double)((n_db_tiles + kSampleStride - 1) / kSampleStride) * TN;
-        const long long db_n = nd;
-        // Up to ~400k points the sample of level A is large enough (16 N / 3L points, rank ~16) to fix the
-        // threshold of level C directly; beyond that level B refines it.
-        const bool direct = db_n <= 393216;
-        const int m_a = direct ? (int)std::min<long long>(16384, std::max<long long>(256, 16 * db_n / (3 * L)))
-                               : (int)std::min<long long>(16384, std::max<long long>(2048, (long long)(b_points / 32)));
-        const long long a_stride = std::max<long long>(1, db_n / m_a);
-        const double a_target = direct ? 3.0 * L * m_a / (double)db_n : 300.0 * m_a / b_points;
-        const int rank_a = std::min(16, std::max(4, (int)(a_target + 0.5))) - 1;
-        const int rank_b = std::max(4, (3 * L + kSampleStride - 1) / kSampleStride) - 1;
-        if (getenv("B200TSNE_KNN_LEVEL_A") && strcmp(getenv("B200TSNE_KNN_LEVEL_A"), "simt") == 0) {
+    // One scan of every stride-th tile against tau.  The attribute and the launch of the instantiation that fits the images:
+    auto scan = [&](int stride) -> int {
+        B200_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)nq * 2, st));
+        const long long tiles = wide ? w.td / 2 : w.td;
+        const long long win = (long long)(wide ? std::max(1, window_tiles / 2) : window_tiles) * stride;
+        const size_t smem = wide ? (size_t)kWideStages * 4 * kWideChunkBytes : (size_t)(QH + kBStages) * w.image_bytes;
+        if (wide) B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        else if (QH == 1) B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        else B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        for (long long lo = 0; lo < tiles; lo += win) {
+            const int hi = (int)std::min<long long>(tiles, lo + win);
             if (wide)
-                knn_sample_tau_wide_kernel<<<(unsigned)((nq + kTauThreads - 1) / kTauThreads), kTauThreads, 0, st>>>(X, D, w.qlist, nq, db_lo,
-                                                                                                             a_stride, m_a, rank_a, tau);
+                knn_tc_wide_kernel<false><<<(unsigned)((q_tiles + 1) / 2), tc_threads(2), smem, st>>>(
+                    w.img_q, w.img_db, Dp / KC, nq, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand_key, cand_id, counts,
+                    counters + 0, bf16);
+            else if (QH == 1)
+                knn_tc_filter_kernel<1, false><<<(unsigned)q_tiles, tc_threads(1), smem, st>>>(
+                    w.img_q, w.img_db, Dp, nq, nd_pos, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand_key, cand_id, counts,
+                    counters + 0, bf16, w.sw, w.nks);
             else
-                knn_sample_tau_kernel<<<(unsigned)((nq + kTauThreads - 1) / kTauThreads), kTauThreads, 0, st>>>(X, D, w.qlist, nq, db_lo,
-                                                                                                        a_stride, m_a, rank_a, tau);
+                knn_tc_filter_kernel<2, false><<<(unsigned)((q_tiles + 1) / 2), tc_threads(2), smem, st>>>(
+                    w.img_q, w.img_db, Dp, nq, nd_pos, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand_key, cand_id, counts,
+                    counters + 0, bf16, w.sw, w.nks);
+            B200_CUDA(cudaGetLastError());
+        }
+        return 0;
+    };
+    // Three levels, each fixing the threshold of the next:
+    //  A  rank ~10 of a few thousand sample points spread over the database -> tau_A,
+    //     chosen so that ~300 points of sample B beat it;
+    //  B  every kSampleStride-th tile against tau_A;
+    //  C  everything against tau_B = the key of rank ~3L/kSampleStride in sample B: ~3L points beat it.
+    // Before each scan the cells are tested against the thresholds it will use; a skipped cell holds no
+    // point below them, so the candidate sets (and the sample statistics) are those of a full scan.
+    // (the wide kernel strides over units of two tiles: the same 1/kSampleStride of the database)
+    const long long n_db_tiles = (nd + TN - 1) / TN;
+    const double b_points = wide ? (double)((n_db_tiles / 2 + kSampleStride - 1) / kSampleStride) * kWideUnit
+                                 : (double)((n_db_tiles + kSampleStride - 1) / kSampleStride) * TN;
+    // Up to ~400k points the sample of level A is large enough (16 N / 3L points, rank ~16) to fix the
+    // threshold of level C directly; beyond that level B refines it.  The rank decides how far the number of points that
+    // pass strays (3 L times a Beta(16, .) variate: fewer than L or more than 8 L in about one of 10^4 rows).
+    const bool direct = nd <= 393216;
+    const int m_a = direct ? (int)std::min<long long>(16384, std::max<long long>(32, 16 * nd / (3 * L)))
+                           : (int)std::min<long long>(16384, std::max<long long>(2048, (long long)(b_points / 32)));
+    const long long a_stride = std::max<long long>(1, nd / m_a);
+    const double a_target = direct ? 3.0 * L * m_a / (double)nd : 300.0 * m_a / b_points;
+    const int rank_a = std::min(16, std::max(4, (int)(a_target + 0.5))) - 1;
+    const int rank_b = std::max(4, (3 * L + kSampleStride - 1) / kSampleStride) - 1;
+    if (getenv("B200TSNE_KNN_LEVEL_A") && strcmp(getenv("B200TSNE_KNN_LEVEL_A"), "simt") == 0) {
+        if (wide)
+            knn_sample_tau_wide_kernel<<<(unsigned)((nq + kTauThreads - 1) / kTauThreads), kTauThreads, 0, st>>>(X, D, w.qlist, nq, db_lo,
+                                                                                                         a_stride, m_a, rank_a, tau);
+        else
+            knn_sample_tau_kernel<<<(unsigned)((nq + kTauThreads - 1) / kTauThreads), kTauThreads, 0, st>>>(X, D, w.qlist, nq, db_lo,
+                                                                                                    a_stride, m_a, rank_a, tau);
+    } else {
+        // the same sample on the tensor cores: its points as a few tile images, every query thread keeping its
+        // 16 smallest keys in registers (the keys differ from the fp32 sums of the CUDA-core kernels by the
+        // filter's error only, and this threshold has to be roughly right, no more)
+        const int ts = wide ? (m_a + kWideUnit - 1) / kWideUnit * 2 : (m_a + TN - 1) / TN;
+        knn_sample_list_kernel<<<(unsigned)((ts * TN + 255) / 256), 256, 0, st>>>(w.slist, (long long)ts * TN, m_a, db_lo, a_stride);
+        if (bf16)
+            knn_tc_prepare_bf16_kernel<<<(unsigned)ts, 256, 0, st>>>(X, w.slist, D, Dp, KC, w.sw, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_s),
+                                                                     nullptr, nullptr, nullptr, nullptr);
+        else
+            knn_tc_prepare_kernel<<<(unsigned)ts, 128, 0, st>>>(X, w.slist, D, Dp, KC, 1, w.img_s, nullptr);
+        knn_single_segment_kernel<<<1, 1, 0, st>>>(w.segs, w.nseg, wide ? ts / 2 : ts);
+        B200_CUDA(cudaGetLastError());
+        if (wide) {
+            const size_t smem_a = (size_t)kWideStages * 4 * kWideChunkBytes;
+            B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+            knn_tc_wide_kernel<true><<<(unsigned)((q_tiles + 1) / 2), tc_threads(2), smem_a, st>>>(
+                w.img_q, w.img_s, Dp / KC, nq, w.segs, w.nseg, 0, 1, 0, ts / 2, nullptr, 0, nullptr, nullptr, nullptr, counters + 0, bf16,
+                rank_a, tau, (long long)m_a);
         } else {
-            // the same sample on the tensor cores: its points as a few tile images, every query thread keeping its
-            // 16 smallest keys in registers (the keys differ from the fp32 sums of the CUDA-core kernels by the
-            // filter's error only, and this threshold has to be roughly right, no more)
-            const int ts = wide ? (m_a + kWideUnit - 1) / kWideUnit * 2 : (m_a + TN - 1) / TN;
-            knn_sample_list_kernel<<<(unsigned)((ts * TN + 255) / 256), 256, 0, st>>>(w.slist, (long long)ts * TN, m_a, db_lo, a_stride);
-            if (bf16)
-                knn_tc_prepare_bf16_kernel<<<(unsigned)ts, 256, 0, st>>>(X, w.slist, D, Dp, KC, w.sw, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_s),
-                                                                         nullptr, nullptr, nullptr, nullptr);
-            else
-                knn_tc_prepare_kernel<<<(unsigned)ts, 128, 0, st>>>(X, w.slist, D, Dp, KC, 1, w.img_s, nullptr);
-            knn_single_segment_kernel<<<1, 1, 0, st>>>(w.segs, w.nseg, wide ? ts / 2 : ts);
-            B200_CUDA(cudaGetLastError());
-            if (wide) {
-                const size_t smem_a = (size_t)kWideStages * 4 * kWideChunkBytes;
-                B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
-                knn_tc_wide_kernel<8, true><<<(unsigned)((q_tiles + 1) / 2), tc_threads(2), smem_a, st>>>(
-                    w.img_q, w.img_s, Dp / KC, nq, w.segs, w.nseg, 0, 1, 0, ts / 2, nullptr, 0, nullptr, nullptr, nullptr, counters + 0, bf16,
-                    rank_a, tau, (long long)m_a);
-            } else {
-                const size_t smem_a = (size_t)(1 + kBStages) * w.image_bytes;
-                B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<8, false, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
-                knn_tc_filter_kernel<8, false, 1, true><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
-                    w.img_q, w.img_s, Dp, nq, (long long)m_a, w.segs, w.nseg, 0, 1, 0, ts, nullptr, 0, nullptr, nullptr, nullptr, counters + 0,
-                    bf16, w.sw, w.nks, rank_a, tau);
-            }
-            B200_CUDA(cudaGetLastError());
-            // back to all database tiles
-            knn_single_segment_kernel<<<1, 1, 0, st>>>(w.segs, w.nseg, wide ? (int)(w.td / 2) : (int)((nd + TN - 1) / TN));
+            const size_t smem_a = (size_t)(1 + kBStages) * w.image_bytes;
+            B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+            knn_tc_filter_kernel<1, true><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
+                w.img_q, w.img_s, Dp, nq, (long long)m_a, w.segs, w.nseg, 0, 1, 0, ts, nullptr, 0, nullptr, nullptr, nullptr, counters + 0,
+                bf16, w.sw, w.nks, rank_a, tau);
         }
         B200_CUDA(cudaGetLastError());
-        phases.mark("level_A");
-        B200_TRY(prune());
-        const unsigned sel_grid = (unsigned)((nq + 3) / 4);
-        if (!direct) {
-            // level B: only the key of rank rank_b among the sample's candidates is needed
-            if (EPL == 8) {
-                B200_KNN_FILTER(8, true, kSampleStride, tau, kFixedCap, fix_key, fix_id, counts);
-                knn_tc_pick_kernel<32><<<sel_grid, 128, 0, st>>>(fix_key, fix_id, kFixedCap, counts, nq, rank_b + 1, nullptr, nullptr, 0, tau,
-                                                                 row_flags);
-            } else {
-                B200_KNN_FILTER(16, true, kSampleStride, tau, kFixedCap, fix_key, fix_id, counts);
-                knn_tc_pick_kernel<64><<<sel_grid, 128, 0, st>>>(fix_key, fix_id, kFixedCap, counts, nq, rank_b + 1, nullptr, nullptr, 0, tau,
-                                                                 row_flags);
-            }
-            B200_CUDA(cudaGetLastError());
-            phases.mark("level_B+pick");
-            B200_TRY(prune());
-        }
-        // level C: the L best go to the (otherwise unused) online buffers, in no particular order
-        if (EPL == 8) {
-            B200_KNN_FILTER(8, true, 1, tau, kFixedCap, fix_key, fix_id, counts);
-            phases.mark("level_C");
-            knn_tc_pick_kernel<32><<<sel_grid, 128, 0, st>>>(fix_key, fix_id, kFixedCap, counts, nq, L, cand_key, cand_id, C, nullptr, row_flags);
-        } else {
-            B200_KNN_FILTER(16, true, 1, tau, kFixedCap, fix_key, fix_id, counts);
-            phases.mark("level_C");
-            knn_tc_pick_kernel<64><<<sel_grid, 128, 0, st>>>(fix_key, fix_id, kFixedCap, counts, nq, L, cand_key, cand_id, C, nullptr, row_flags);
-        }
-        phases.mark("pick");
-        B200_CUDA(cudaGetLastError());
-        final_key = cand_key;
-        final_id = cand_id;
-        final_stride = C;
+        knn_single_segment_kernel<<<1, 1, 0, st>>>(w.segs, w.nseg, all_tiles);   // back to all database tiles
     }
-#undef B200_KNN_FILTER
-#undef B200_KNN_FILTER_V
-#undef B200_KNN_FILTER_WIDE
+    B200_CUDA(cudaGetLastError());
+    phases.mark("level_A");
+    B200_TRY(prune());
+    if (!direct) {
+        // level B: only the key of rank rank_b among the sample's candidates is needed
+        B200_TRY(scan(kSampleStride));
+        const unsigned sel_grid = (unsigned)((nq + 3) / 4);
+        if (cap <= 1024) knn_tc_pick_kernel<32><<<sel_grid, 128, 0, st>>>(cand_key, cap, counts, nq, rank_b + 1, tau);
+        else knn_tc_pick_kernel<64><<<sel_grid, 128, 0, st>>>(cand_key, cap, counts, nq, rank_b + 1, tau);
+        B200_CUDA(cudaGetLastError());
+        phases.mark("level_B+pick");
+        B200_TRY(prune());
+    }
+    B200_TRY(scan(1));   // level C
+    phases.mark("level_C");
     // Error bound of the filter relative to (|x_i|^2 + d^2 + 1): 3xTF32 drops terms of order 2^-22 |x_i||x_j|,
     // and the fp32 accumulation of D products (not IEEE in the tensor core: take two units in the last place
     // per addition) adds up to 2 D 2^-24 |x_i||x_j| in the worst case.  2^-14 covers both with a wide margin
@@ -2197,12 +1956,13 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     // rows are copied 16, 8 or 4 bytes at a time, as their length keeps them aligned
     const size_t x_at = reinterpret_cast<size_t>(X);
     const int vec = (D % 4 == 0 && x_at % 16 == 0) ? 4 : ((D % 2 == 0 && x_at % 8 == 0) ? 2 : 1);
-    auto rerank = vec == 4 ? knn_tc_rerank_kernel<4> : (vec == 2 ? knn_tc_rerank_kernel<2> : knn_tc_rerank_kernel<1>);
-    B200_CUDA(cudaFuncSetAttribute(rerank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rerank_smem(L)));
-    rerank<<<(unsigned)((nq + kRerankWarps - 1) / kRerankWarps), kRerankWarps * 32, rerank_smem(L), st>>>(
-        X, D, w.qlist, w.dblist, q_lo, nq, final_key, final_id, L, final_stride, K, w.norms_q, err_scale, bf16 ? w.res_q : nullptr,
-        reinterpret_cast<const float *>(counters + 4), two_pass ? row_flags : nullptr, ids, d2,
-        failed, counters + 1, reinterpret_cast<float *>(counters + 3), w.xp);
+    auto rerank = cap <= 1024 ? (vec == 4 ? knn_tc_rerank_kernel<4, 32> : (vec == 2 ? knn_tc_rerank_kernel<2, 32> : knn_tc_rerank_kernel<1, 32>))
+                              : (vec == 4 ? knn_tc_rerank_kernel<4, 64> : (vec == 2 ? knn_tc_rerank_kernel<2, 64> : knn_tc_rerank_kernel<1, 64>));
+    const size_t rerank_smem = sizeof(float) * kRerankWarps * rerank_floats(D, L);
+    B200_CUDA(cudaFuncSetAttribute(rerank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rerank_smem));
+    rerank<<<(unsigned)((nq + kRerankWarps - 1) / kRerankWarps), kRerankWarps * 32, rerank_smem, st>>>(
+        X, D, w.qlist, w.dblist, q_lo, nq, cand_key, cand_id, cap, counts, tau, L, K, w.norms_q, err_scale, bf16 ? w.res_q : nullptr,
+        reinterpret_cast<const float *>(counters + 4), ids, d2, failed, counters + 1, reinterpret_cast<float *>(counters + 3), xp);
     B200_CUDA(cudaGetLastError());
     knn_tc_collect_failed_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(failed, nq, w.qlist, flist, counters + 2);
     B200_CUDA(cudaGetLastError());

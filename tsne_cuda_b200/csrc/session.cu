@@ -640,8 +640,13 @@ int Session::affinities_from_points(const float *X_host, int D, float perplexity
         const int64_t batch = std::min<int64_t>(std::max<int64_t>(r, 1), 1 << 20);
         if (knn_tc_workspace_bytes(D, K, batch, N) > total_b / 2) db_sharded = true;
     }
+    // the cells of the points: the search visits by them, and the blocked copy of P numbers the points by them
+    const char *attr_mode = getenv("B200TSNE_ATTRACTIVE");
+    const bool want_order = N > kAttractiveTile && !(attr_mode && strcmp(attr_mode, "rows") == 0);
+    PointCells cells;
+    if (want_order || (!db_sharded && knn_tc_supported(N, D, K))) B200_TRY(point_cells_build(&cells, X, D, 0, N, tmp, stream));
     if (!db_sharded) {
-        B200_TRY(knn_search(X, N, D, K, row_lo, row_hi, 0, N, ids, d2, &knn_stats, stream));
+        B200_TRY(knn_search(X, N, D, K, row_lo, row_hi, 0, N, ids, d2, &knn_stats, stream, cells.cells ? &cells : nullptr));
     } else {
         int32_t *part_i = nullptr, *recv_i = nullptr;
         float *part_d = nullptr, *recv_d = nullptr;
@@ -661,12 +666,9 @@ int Session::affinities_from_points(const float *X_host, int D, float perplexity
 
     clk.begin(stream);
     // the order in which the attractive force's blocked copy of P numbers the points (every rank computes the same)
-    {
-        const char *mode = getenv("B200TSNE_ATTRACTIVE");
-        if (!(mode && strcmp(mode, "rows") == 0)) {
-            if (!cell_order) B200_TRY(arena.alloc((void **)&cell_order, sizeof(int32_t) * N));
-            B200_TRY(order_points_by_cell(X, N, D, cell_order, stream));
-        }
+    if (want_order) {
+        if (!cell_order) B200_TRY(arena.alloc((void **)&cell_order, sizeof(int32_t) * N));
+        B200_TRY(order_points_by_cell(cells, cell_order, stream));
     }
 
     clk.begin(stream);
