@@ -1192,9 +1192,9 @@ template <int SLOTS> __device__ __forceinline__ unsigned kth_key(const unsigned 
         const unsigned mid = lo + ((hi - lo) >> 1);
         int c = 0;
 #pragma unroll
-        for (int j = 0; j < SLOTS; j++) {
+        for (int j = 0; j < SLOTS; j += 4) {
             if (j >= jmax) break;
-            c += (enc[j] <= mid) ? 1 : 0;
+            c += (enc[j] <= mid) + (enc[j + 1] <= mid) + (enc[j + 2] <= mid) + (enc[j + 3] <= mid);   // (empty slots hold the maximum)
         }
         c = __reduce_add_sync(0xffffffffu, c);
         if (c >= k) hi = mid;
@@ -1258,13 +1258,43 @@ constexpr int kRerankWhole = 64;  // rows of up to this many dimensions are stag
 // Staged rows are `stride` floats apart: a multiple of 4, but not of 8, so that 32 lanes read 16 bytes of a row of their own
 // without bank conflicts.
 __host__ __device__ constexpr int rerank_stride(int D) { const int d = D <= kRerankWhole ? (D + 3) / 4 * 4 : kRerankDims; return d % 8 == 0 ? d + 4 : d; }
-// one warp: one stage (two where the row is walked) of 32 candidate rows and the query; L evaluated candidates
-__host__ __device__ constexpr size_t rerank_floats(int D, int L) { return (size_t)(D <= kRerankWhole ? 1 : 2) * 33 * rerank_stride(D) + 4 * (size_t)L; }
+// one warp: one stage (two where the row is walked) of 32 candidate rows and the query; L evaluated candidates; 34 row
+// addresses
+__host__ __device__ constexpr size_t rerank_floats(int D, int L) { return (size_t)(D <= kRerankWhole ? 1 : 2) * 33 * rerank_stride(D) + 4 * (size_t)L + 68; }
 
 template <int BYTES> __device__ __forceinline__ void async_copy(void *dst, const void *src)
 {
     if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
     else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+
+// Warp-wide bitonic sort of 32 EPL keys, ascending; element lane * EPL + r in k[r].
+template <int EPL> __device__ __forceinline__ void warp_sort(unsigned long long (&k)[EPL], int lane)
+{
+#pragma unroll
+    for (int size = 2; size <= 32 * EPL; size <<= 1) {
+#pragma unroll
+        for (int j = size >> 1; j > 0; j >>= 1) {
+            if (j >= EPL) {
+                const bool lower = ((lane * EPL) & j) == 0, up = ((lane * EPL) & size) == 0;   // alike for all registers: j, size >= EPL
+#pragma unroll
+                for (int r = 0; r < EPL; r++) {
+                    const unsigned long long o = __shfl_xor_sync(0xffffffffu, k[r], j / EPL);
+                    if ((o < k[r]) == (lower == up)) k[r] = o;
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < EPL; r++) {
+                    if (r & j) continue;
+                    const bool up = ((lane * EPL + r) & size) == 0;
+                    const unsigned long long a = k[r], c = k[r + j];
+                    const bool swap = (c < a) == up;
+                    k[r] = swap ? c : a;
+                    k[r + j] = swap ? a : c;
+                }
+            }
+        }
+    }
 }
 
 // One warp per query of the list (query row qlist[q]; candidate ids are positions in dblist).  Row
@@ -1278,16 +1308,18 @@ template <int BYTES> __device__ __forceinline__ void async_copy(void *dst, const
 // each, whole or 32 dimensions wide in two stages: whole lines per request, where a lane that walks a row of its own
 // touches 32 lines with each.  A lane then reads its row from shared memory and sums in the canonical order.
 // Measured with the pass that used to write the L best out first: LATER.
-template <int VEC, int SLOTS>
-__global__ void __launch_bounds__(kRerankWarps * 32, SLOTS <= 32 ? 6 : 4)
+// EPL: evaluated candidates a lane sorts (L = 32 EPL); the buffer holds up to 8 L.
+template <int VEC, int EPL>
+__global__ void __launch_bounds__(kRerankWarps * 32, EPL <= 4 ? 6 : 4)
 knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__ qlist, const int *__restrict__ dblist,
                      long long out_base, long long nq, const float *__restrict__ cand_key, const int32_t *__restrict__ cand_id, int cap,
-                     const int *__restrict__ counts, const float *__restrict__ tau, int L, int K, const double *__restrict__ norms_exact,
+                     const int *__restrict__ counts, const float *__restrict__ tau, int K, const double *__restrict__ norms_exact,
                      float err_scale, const float2 *__restrict__ res_q, const float *__restrict__ rho, int32_t *__restrict__ ids,
                      float *__restrict__ d2, int *__restrict__ failed, int *__restrict__ n_failed, float *__restrict__ max_err_ratio,
                      const float *__restrict__ Xp)
 {
     // Xp (optional): the database rows in list order, Xp[pos] = X[dblist[pos]]
+    constexpr int L = 32 * EPL, SLOTS = 8 * EPL;
     extern __shared__ __align__(16) float stage_mem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long q = (long long)blockIdx.x * kRerankWarps + w;
@@ -1307,6 +1339,7 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
     unsigned long long *s_key = reinterpret_cast<unsigned long long *>(stage + (whole ? 1 : 2) * 33 * stride);
     int *s_src = reinterpret_cast<int *>(s_key + L);
     float *s_fkey = reinterpret_cast<float *>(s_src + L);
+    const float **s_row = reinterpret_cast<const float **>(s_fkey + L);   // the rows of a group, then the query
     const float *base = Xp ? Xp : X;
     const float T = tau[q];   // every database point with a key below this is in the buffer
     // Error bound of the filter's key for this row: it scales with |x_i||x_j|, and a point whose key is
@@ -1370,15 +1403,23 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
     // lanes per row of a copy: the power of two that covers the width, at most the warp
     const int lanes_log = width <= 8 * VEC ? 3 : (width <= 16 * VEC ? 4 : 5);
     const int col = (lane & ((1 << lanes_log) - 1)) * VEC, sub = lane >> lanes_log, rows_per_copy = 32 >> lanes_log;
+    const float *mine = stage + lane * stride, *query = stage + 32 * stride;
+    if (lane == 0) s_row[32] = xq;
     for (int g = 0; g < m; g += 32) {
         const int rows = min(32, m - g);
-        auto fetch = [&](int c) {   // the group's rows and, in row 32, the query
-            float *buf = stage + (size_t)(c & 1) * 33 * stride;
-            const int d0 = c * width, d1 = min(width, D - d0);
-            for (int r = sub; r <= rows; r += rows_per_copy) {
-                const int to = r == rows ? 32 : r;
-                const float *row = (r == rows ? xq : base + (size_t)s_src[g + r] * D) + d0;
-                for (int d = col; d < d1; d += 32 * VEC) async_copy<4 * VEC>(buf + to * stride + d, row + d);
+        // lanes without a candidate point at the query: their copies and sums are done and not used
+        s_row[lane] = lane < rows ? base + (size_t)s_src[g + lane] * D : xq;
+        __syncwarp();
+        auto fetch = [&](int c) {
+            float *to = stage + (size_t)(c & 1) * 33 * stride + sub * stride + col;
+            const int d = c * width + col;
+            if (col < width && d < D) {
+#pragma unroll 4
+                for (int r = sub; r < 32; r += rows_per_copy, to += rows_per_copy * stride) async_copy<4 * VEC>(to, s_row[r] + d);
+                if (sub == 0) async_copy<4 * VEC>(to, s_row[32] + d);
+                if (VEC == 1 && width > 32 && d + 32 < D) {   // an odd row of up to 64 dimensions: its second half
+                    for (int r = 0; r < 33; r++) async_copy<4>(stage + r * stride + col + 32, s_row[r] + d + 32);
+                }
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
@@ -1392,19 +1433,24 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
                 asm volatile("cp.async.wait_group 0;" ::: "memory");
             }
             __syncwarp();
-            const float *buf = stage + (size_t)(c & 1) * 33 * stride;
-            const float *mine = buf + lane * stride, *query = buf + 32 * stride;
-            const int len = min(width, D - c * width);
-            int d = 0;
-#pragma unroll 4
-            for (; d + 4 <= len; d += 4) {
-                const float4 u = *reinterpret_cast<const float4 *>(query + d), v = *reinterpret_cast<const float4 *>(mine + d);
+            const float *x = query + (size_t)(c & 1) * 33 * stride, *y = mine + (size_t)(c & 1) * 33 * stride;
+            auto four = [&](int d) {
+                const float4 u = *reinterpret_cast<const float4 *>(x + d), v = *reinterpret_cast<const float4 *>(y + d);
                 acc = canon_step(acc, u.x, v.x);
                 acc = canon_step(acc, u.y, v.y);
                 acc = canon_step(acc, u.z, v.z);
                 acc = canon_step(acc, u.w, v.w);
+            };
+            const int len = min(width, D - c * width);
+            if (len == kRerankDims) {
+#pragma unroll
+                for (int d = 0; d < kRerankDims; d += 4) four(d);
+            } else {
+                int d = 0;
+#pragma unroll 4
+                for (; d + 4 <= len; d += 4) four(d);
+                for (; d < len; d++) acc = canon_step(acc, x[d], y[d]);
             }
-            for (; d < len; d++) acc = canon_step(acc, query[d], mine[d]);
             __syncwarp();
         }
         if (lane < rows) {
@@ -1417,22 +1463,23 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) worst = fmaxf(worst, __shfl_xor_sync(0xffffffffu, worst, o));
     __syncwarp();
-    // rank by counting (ties by id), scatter the first K
-    float dK = INFINITY;
-    for (int e = lane; e < m; e += 32) {
-        const unsigned long long mine = s_key[e];
-        int rank = 0;
-#pragma unroll 4
-        for (int u = 0; u < m; u++) rank += s_key[u] < mine;
-        const float de = __uint_as_float((unsigned)(mine >> 32));
-        if (rank < K) {
-            ids[orow * K + rank] = (int32_t)(unsigned)mine;
-            d2[orow * K + rank] = de;
-        }
-        if (rank == K - 1) dK = de;
-    }
+    // in order of (distance, id)
+    unsigned long long key[EPL];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dK = fminf(dK, __shfl_xor_sync(0xffffffffu, dK, o));
+    for (int r = 0; r < EPL; r++) key[r] = lane * EPL + r < m ? s_key[lane * EPL + r] : ~0ull;
+    warp_sort<EPL>(key, lane);
+    float dK = INFINITY;
+#pragma unroll
+    for (int r = 0; r < EPL; r++) {
+        const int e = lane * EPL + r;
+        const float de = __uint_as_float((unsigned)(key[r] >> 32));
+        if (e < K) {
+            ids[orow * K + e] = (int32_t)(unsigned)key[r];
+            d2[orow * K + e] = de;
+        }
+        if (e == K - 1) dK = de;
+    }
+    dK = __shfl_sync(0xffffffffu, dK, (K - 1) / EPL);
     if (lane == 0) {
         // outsiders: key >= outside  =>  canonical distance >= (ni + outside - E) * (1 - theta)
         const double bound = (ni + (double)outside - E) * (1.0 - theta);
@@ -1956,12 +2003,12 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     // rows are copied 16, 8 or 4 bytes at a time, as their length keeps them aligned
     const size_t x_at = reinterpret_cast<size_t>(X);
     const int vec = (D % 4 == 0 && x_at % 16 == 0) ? 4 : ((D % 2 == 0 && x_at % 8 == 0) ? 2 : 1);
-    auto rerank = cap <= 1024 ? (vec == 4 ? knn_tc_rerank_kernel<4, 32> : (vec == 2 ? knn_tc_rerank_kernel<2, 32> : knn_tc_rerank_kernel<1, 32>))
-                              : (vec == 4 ? knn_tc_rerank_kernel<4, 64> : (vec == 2 ? knn_tc_rerank_kernel<2, 64> : knn_tc_rerank_kernel<1, 64>));
+    auto rerank = L == 128 ? (vec == 4 ? knn_tc_rerank_kernel<4, 4> : (vec == 2 ? knn_tc_rerank_kernel<2, 4> : knn_tc_rerank_kernel<1, 4>))
+                           : (vec == 4 ? knn_tc_rerank_kernel<4, 8> : (vec == 2 ? knn_tc_rerank_kernel<2, 8> : knn_tc_rerank_kernel<1, 8>));
     const size_t rerank_smem = sizeof(float) * kRerankWarps * rerank_floats(D, L);
     B200_CUDA(cudaFuncSetAttribute(rerank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rerank_smem));
     rerank<<<(unsigned)((nq + kRerankWarps - 1) / kRerankWarps), kRerankWarps * 32, rerank_smem, st>>>(
-        X, D, w.qlist, w.dblist, q_lo, nq, cand_key, cand_id, cap, counts, tau, L, K, w.norms_q, err_scale, bf16 ? w.res_q : nullptr,
+        X, D, w.qlist, w.dblist, q_lo, nq, cand_key, cand_id, cap, counts, tau, K, w.norms_q, err_scale, bf16 ? w.res_q : nullptr,
         reinterpret_cast<const float *>(counters + 4), ids, d2, failed, counters + 1, reinterpret_cast<float *>(counters + 3), xp);
     B200_CUDA(cudaGetLastError());
     knn_tc_collect_failed_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(failed, nq, w.qlist, flist, counters + 2);
