@@ -232,7 +232,8 @@ __device__ __forceinline__ uint64_t make_desc_swizzled(uint32_t saddr, uint32_t 
 constexpr uint32_t kInstrDesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 // the same with bf16 A and B (format 1 of kind::f16); one K step is 32 operand bytes per row in either kind
 constexpr uint32_t kInstrDescBf16 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
-
+// two database tiles at once: 128 x 256 x 16
+constexpr uint32_t kInstrDescBf16Pair = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(2 * TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 
 // ------------------------------------------------------------------------------------------------
 // operand preparation
@@ -285,20 +286,14 @@ knn_tc_prepare_kernel(const float *__restrict__ X, const int *__restrict__ list,
     if (norms) norms[pos] = n2;
 }
 
-// The bf16 form of the images: v = hi + lo + r with hi, lo in bf16 (round to nearest) and |r| <= 2^-16 |v|; the
-// same byte geometry as the TF32 images (a K step is 16 values = 32 bytes per row, core matrices of 8 rows x 16
-// bytes), so the shared-memory descriptors are the same and an image has half the bytes per inner dimension.
-// [tiles][Dp/KC chunks][2 (hi, lo)][KC/16][2048 values].  Two columns carry the norm (its bf16 pair and the pair of
-// what that pair leaves over: 32 significant bits), against 1, 1 in the query form.
-__device__ __forceinline__ size_t image_offset_bf16(int r, int k)
-{
-    return (size_t)(k >> 4) * 2048 + (size_t)(r >> 3) * 128 + (size_t)((k >> 3) & 1) * 64 + (size_t)(r & 7) * 8 + (k & 7);
-}
-// The swizzled form (narrow kernel): rows of sw bytes (sw / 2 values), blocks of 128 rows one after the other along
+// The bf16 form of the images: v = hi + lo + r with hi, lo in bf16 (round to nearest) and |r| <= 2^-16 |v|; an image
+// has half the bytes per inner dimension of a TF32 one, [tiles][Dp/KC chunks][2 (hi, lo)][KC * 128 values].  Two columns
+// carry the norm (its bf16 pair and the pair of what that pair leaves over: 32 significant bits), against 1, 1 in the
+// query form.  A part is rows of sw bytes (sw / 2 values), blocks of 128 rows one after the other along
 // the inner dimension; inside a block the 16-byte piece p of row r sits where piece p ^ ((r * sw / 128) mod (sw / 16))
 // would (the shared-memory swizzle of that width, which the tensor core undoes when it reads: operands in this
 // form are fetched about twice as fast as core matrices without swizzle, measured).  Offset in values.
-__device__ __forceinline__ size_t image_offset_bf16_swizzled(int r, int k, int sw)
+__device__ __forceinline__ size_t image_offset_bf16(int r, int k, int sw)
 {
     const int per_row = sw >> 1;
     const int block = k / per_row;
@@ -389,7 +384,7 @@ knn_tc_prepare_bf16_kernel(const float *__restrict__ X, const int *__restrict__ 
                 lo[e / 2] = __floats2bfloat162_rn(v[0] - __low2float(hi[e / 2]), v[1] - __high2float(hi[e / 2]));
             }
             __nv_bfloat16 *im = im_tile + (size_t)(k / KC) * 2 * part;
-            const size_t at = sw ? image_offset_bf16_swizzled(r, k % KC, sw) : image_offset_bf16(r, k % KC);
+            const size_t at = image_offset_bf16(r, k % KC, sw);
             *reinterpret_cast<uint4 *>(im + at) = *reinterpret_cast<const uint4 *>(hi);
             *reinterpret_cast<uint4 *>(im + part + at) = *reinterpret_cast<const uint4 *>(lo);
         }
@@ -892,15 +887,19 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
 // ------------------------------------------------------------------------------------------------
 // A block multiplies two query tiles with two database tiles (a "unit" of 256 database rows) at a time,
 // walking the inner dimension in chunks of kWideKC: a stage holds the chunk images of the four tiles
-// (4 x 24 KB), two stages alternate, the four 128 x 128 accumulators fill the 512 TMEM columns.  Operand
-// bytes per MMA are those of the narrow kernel with two query tiles, but the query images are streamed
-// again for every unit, so the kernel leans on L2 bandwidth (24 KB per tile pair and chunk).  After the
+// (4 x 16 KB), three stages alternate, the four 128 x 128 accumulators fill the 512 TMEM columns.  The query
+// images are streamed again for every unit, so the kernel leans on L2 bandwidth (64 KB per 12.6 Mi products).
+// bf16 images are in rows of 64 bytes with the 64-byte swizzle, and one MMA multiplies a query tile with both
+// database tiles (N = 256): their parts are placed one after the other in the stage, which costs the producer
+// two more copies and saves a third of what the tensor core reads from shared memory (no swizzle, N = 128, two
+// stages of 96 KB: 5 to 9 % slower, 50 000 x 1 024 14.4 against 13.8 ms a scan).  After the
 // last chunk of a unit the sixteen epilogue warps (query tile x database tile x TMEM lane quarter) compare
 // the keys with the fixed thresholds exactly as in the narrow kernel; the next unit's MMAs wait until the
 // accumulators have been read.  Fixed thresholds only (a small database goes to the SIMT search).
-constexpr int kWideKC = 24;                       // inner dimensions per chunk = 3 MMA K steps
+constexpr int kWideKC = 16;                       // words of 32 bits per row, chunk and part (32 bf16 values, 16 TF32) = 2 MMA K steps
+constexpr int kWideSwizzle = 64;                  // bytes of such a row: the swizzle of the bf16 images
 constexpr uint32_t kWideChunkBytes = kWideKC * 1024;   // hi + lo of one tile and chunk
-constexpr int kWideStages = 2;
+constexpr int kWideStages = 3;
 constexpr int kWideUnit = 2 * TN;                 // database rows per unit
 
 struct WideShared {
@@ -937,8 +936,9 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
     }
     volatile int *abort_flag = &sh.abort_flag;
     const size_t tile_floats = (size_t)n_chunks * (kWideChunkBytes / 4);   // one tile's image, all chunks
-    // stage layout: [A0 chunk][A1 chunk][B0 chunk][B1 chunk], each hi then lo
-    auto stage_ptr = [&](int s, int which) { return smem + ((size_t)s * 4 + which) * kWideChunkBytes; };
+    // stage layout: [A0 hi][A0 lo][A1 hi][A1 lo][B0 hi][B1 hi][B0 lo][B1 lo]
+    constexpr uint32_t kPartBytes = kWideChunkBytes / 2;
+    auto stage_ptr = [&](int s, int part) { return smem + ((size_t)s * 8 + part) * kPartBytes; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kWideStages; s++) { mbar_init(&sh.full[s], 1); mbar_init(&sh.empty[s], 1); }
@@ -973,10 +973,13 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
                     mbar_expect_tx(&sh.full[s], 4 * kWideChunkBytes);
                     const size_t coff = (size_t)c * (kWideChunkBytes / 4);
                     bulk_load(stage_ptr(s, 0), img_q + (size_t)qt * tile_floats + coff, kWideChunkBytes, &sh.full[s]);
-                    bulk_load(stage_ptr(s, 1), img_q + (size_t)(qt + 1) * tile_floats + coff, kWideChunkBytes, &sh.full[s]);
-                    bulk_load(stage_ptr(s, 2), img_db + (size_t)(2 * (long long)unit) * tile_floats + coff, kWideChunkBytes, &sh.full[s]);
-                    bulk_load(stage_ptr(s, 3), img_db + (size_t)(2 * (long long)unit + 1) * tile_floats + coff, kWideChunkBytes,
-                              &sh.full[s]);
+                    bulk_load(stage_ptr(s, 2), img_q + (size_t)(qt + 1) * tile_floats + coff, kWideChunkBytes, &sh.full[s]);
+#pragma unroll
+                    for (int g = 0; g < 2; g++) {
+                        const float *b = img_db + (size_t)(2 * (long long)unit + g) * tile_floats + coff;
+                        bulk_load(stage_ptr(s, 4 + g), b, kPartBytes, &sh.full[s]);
+                        bulk_load(stage_ptr(s, 6 + g), b + kPartBytes / 4, kPartBytes, &sh.full[s]);
+                    }
                 }
             }
         }
@@ -986,8 +989,8 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
             int unit;
             long long it = 0, n_unit = 0;
             bool ok = true;
-            const uint64_t no_addr = make_desc(0u);
-            const uint32_t stage16 = smem_u32(smem) >> 4, chunk16 = kWideChunkBytes >> 4;
+            const uint64_t no_addr = bf16 ? make_desc_swizzled(0u, kWideSwizzle) : make_desc(0u);
+            const uint32_t stage16 = smem_u32(smem) >> 4, part16 = kPartBytes >> 4;
             while (ok && walk.next(unit)) {
                 // the accumulators of the previous unit must have been read
                 if (!mbar_wait(&sh.acc_empty, (uint32_t)((n_unit & 1) ^ 1), abort_flag)) break;
@@ -996,27 +999,32 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
                     const uint32_t ph = (uint32_t)((it / kWideStages) & 1);
                     if (!mbar_wait(&sh.full[s], ph, abort_flag)) { ok = false; break; }
                     tc_fence_after();
-                    // descriptors by addition only (see the narrow kernel's issuer); a stage's four chunk images
-                    // are kWideChunkBytes apart, lo follows hi after kSteps blocks of 4 KB
-                    const uint64_t st0 = no_addr + (uint64_t)(stage16 + (uint32_t)s * 4u * chunk16);
+                    // descriptors by addition only (see the narrow kernel's issuer)
+                    const uint64_t st0 = no_addr + (uint64_t)(stage16 + (uint32_t)s * 8u * part16);
+                    const uint32_t acc0 = (c > 0) ? 1u : 0u;
+                    if (bf16) {
 #pragma unroll
-                    for (int pair = 0; pair < 4; pair++) {
-                        const int h = pair >> 1, g = pair & 1;
-                        const uint64_t a_hi = st0 + (uint64_t)((uint32_t)h * chunk16), a_lo = a_hi + kSteps * 256u;
-                        const uint64_t b_hi = st0 + (uint64_t)((uint32_t)(2 + g) * chunk16), b_lo = b_hi + kSteps * 256u;
-                        const uint32_t d_tmem = tmem_base + (uint32_t)((h * 2 + g) * TN);
-                        const uint32_t acc0 = (c > 0) ? 1u : 0u;
-                        if (bf16) {
+                        for (int h = 0; h < 2; h++) {   // both database tiles at once; a K step is 32 bytes of a row
+                            const uint64_t a_hi = st0 + (uint64_t)(2u * (uint32_t)h * part16), a_lo = a_hi + part16;
+                            const uint64_t b_hi = st0 + (uint64_t)(4u * part16), b_lo = b_hi + 2u * part16;
+                            const uint32_t d_tmem = tmem_base + (uint32_t)(h * 2 * TN);
 #pragma unroll
                             for (int ks = 0; ks < kSteps; ks++)        // hi . hi
-                                tc_mma_bf16(d_tmem, a_hi + ks * 256u, b_hi + ks * 256u, kInstrDescBf16, ks ? 1u : acc0);
+                                tc_mma_bf16(d_tmem, a_hi + ks * 2u, b_hi + ks * 2u, kInstrDescBf16Pair, ks ? 1u : acc0);
 #pragma unroll
                             for (int ks = 0; ks < kSteps; ks++)        // lo . hi
-                                tc_mma_bf16(d_tmem, a_lo + ks * 256u, b_hi + ks * 256u, kInstrDescBf16, 1u);
+                                tc_mma_bf16(d_tmem, a_lo + ks * 2u, b_hi + ks * 2u, kInstrDescBf16Pair, 1u);
 #pragma unroll
                             for (int ks = 0; ks < kSteps; ks++)        // hi . lo
-                                tc_mma_bf16(d_tmem, a_hi + ks * 256u, b_lo + ks * 256u, kInstrDescBf16, 1u);
-                        } else {
+                                tc_mma_bf16(d_tmem, a_hi + ks * 2u, b_lo + ks * 2u, kInstrDescBf16Pair, 1u);
+                        }
+                    } else {
+#pragma unroll
+                        for (int pair = 0; pair < 4; pair++) {   // a K step is a block of 4 KB
+                            const int h = pair >> 1, g = pair & 1;
+                            const uint64_t a_hi = st0 + (uint64_t)(2u * (uint32_t)h * part16), a_lo = a_hi + part16;
+                            const uint64_t b_hi = st0 + (uint64_t)((4u + (uint32_t)g) * part16), b_lo = b_hi + 2u * part16;
+                            const uint32_t d_tmem = tmem_base + (uint32_t)((h * 2 + g) * TN);
 #pragma unroll
                             for (int ks = 0; ks < kSteps; ks++)        // hi . hi
                                 tc_mma_tf32(d_tmem, a_hi + ks * 256u, b_hi + ks * 256u, kInstrDesc, ks ? 1u : acc0);
@@ -1724,6 +1732,7 @@ static TcWorkspace tc_carve(void *base, int D, int K, long long nq, long long nd
         w.Dp = (need + w.sw / 2 - 1) / (w.sw / 2) * (w.sw / 2);
         w.nks = (need + 15) / 16;
     } else if (w.bf16) {
+        w.sw = kWideSwizzle;
         w.Dp = (D + 2 + 2 * kWideKC - 1) / (2 * kWideKC) * (2 * kWideKC);
         w.nks = w.Dp / 16;
     } else {
