@@ -1,0 +1,49 @@
+"""Scans whose database tiles several blocks divide (few query blocks on many SMs): the blocks append to the same candidate
+buffers.  The lists are defined operation by operation, so they equal the SIMT search's bit for bit."""
+import numpy as np
+import pytest
+
+from conftest import mixture
+
+pytestmark = pytest.mark.gpu
+
+
+def both(engine, monkeypatch, X, k, **ranges):
+    a = engine.knn(X, k, **ranges)
+    st = engine.knn_last_stats()
+    assert st["tensor_core"] == 1
+    monkeypatch.setenv("B200TSNE_KNN", "simt")
+    b = engine.knn(X, k, **ranges)
+    assert engine.knn_last_stats()["tensor_core"] == 0
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    return st
+
+
+# one block of queries and up to sixteen; narrow and wide points; the last unit, tile and chunk partly filled
+@pytest.mark.parametrize("n,d,k", [(2048, 7, 5), (2049, 63, 90), (2177, 64, 64), (4095, 30, 150), (5003, 257, 224), (9001, 784, 90)])
+def test_few_query_blocks(engine, monkeypatch, n, d, k):
+    from tsne_cuda_b200 import datasets
+    X = datasets.mnist_shaped(n, d, seed=n) if d == 784 else mixture(n, d, n + d)
+    st = both(engine, monkeypatch, X, k)
+    assert st["rows_recomputed"] <= 0.02 * n
+
+
+@pytest.mark.parametrize("d", [20, 100])
+@pytest.mark.parametrize("q_lo,q_hi,db_lo,db_hi", [(0, 1, 0, 30000), (777, 906, 5, 29990), (0, 700, 15000, 30000)])
+def test_short_query_ranges(engine, monkeypatch, d, q_lo, q_hi, db_lo, db_hi):
+    both(engine, monkeypatch, mixture(30000, d, d), 40, q_lo=q_lo, q_hi=q_hi, db_lo=db_lo, db_hi=db_hi)
+
+
+@pytest.mark.parametrize("d", [20, 100])
+def test_windows(engine, monkeypatch, d):
+    monkeypatch.setenv("B200TSNE_KNN_WINDOW_TILES", "33")
+    both(engine, monkeypatch, mixture(17000, d, 3), 33, q_lo=100, q_hi=1500)
+
+
+@pytest.mark.parametrize("d", [20, 100])
+def test_full_buffers(engine, monkeypatch, d):
+    """3 000 copies of one point: more candidates than a buffer holds arrive from all blocks at once."""
+    X = mixture(9000, d, 4)
+    X[2000:5000] = X[2000]
+    st = both(engine, monkeypatch, X, 50)
+    assert st["rows_recomputed"] >= 3000

@@ -554,27 +554,79 @@ __global__ void knn_single_segment_kernel(int2 *segs, int *nseg, int tiles)
     nseg[0] = 1;
 }
 
+// How many blocks divide the tiles of one block of queries: `most` are launched, and as the cells leave a block of queries
+// anything between all tiles and a handful, each decides by what is left of its walk: shares of at least `share` tiles, or
+// of four where that only takes SMs that would idle (`idle` blocks a block of queries).
+struct ScanParts {
+    int most = 1, idle = 1, share = 1;
+    __host__ __device__ int of(int tiles) const
+    {
+        int n = tiles / share;
+        const int free = tiles / 4 < idle ? tiles / 4 : idle;
+        if (n < free) n = free;
+        if (n > most) n = most;
+        return n < 1 ? 1 : n;
+    }
+};
 // The database tiles of a block in scan order: the tiles of its segments that are multiples of `stride` and lie
-// in the window [win_lo, win_hi) of the launch.
+// in the window [win_lo, win_hi) of the launch, and of these the share of block `part` where several blocks divide them.
 // The producer, the MMA issuer and the epilogue each walk the same sequence.
+template <bool DIVIDED>
 struct TileWalk {
     const int2 *segs;
-    int nseg, stride, win_lo, win_hi, s, t, end;
-    __device__ TileWalk(const int2 *segs_, int nseg_, int stride_, int win_lo_, int win_hi_)
-        : segs(segs_), nseg(nseg_), stride(stride_), win_lo(win_lo_), win_hi(win_hi_), s(-1), t(0), end(0) {}
+    int nseg, stride, win_lo, win_hi, s, t, end, skip, left, parts;
+    __device__ TileWalk(const int2 *segs_, int nseg_, int stride_, int win_lo_, int win_hi_, int part = 0, ScanParts p = ScanParts())
+        : segs(segs_), nseg(nseg_), stride(stride_), win_lo(win_lo_), win_hi(win_hi_), s(-1), t(0), end(0), skip(0), left(INT_MAX), parts(1)
+    {
+        if (DIVIDED && p.most > 1) {
+            long long total = 0;
+            for (int i = 0; i < nseg; i++) {
+                open(i);
+                total += tiles();
+            }
+            t = end = 0;
+            parts = p.of((int)total);
+            skip = part < parts ? (int)(total * part / parts) : 0;
+            left = part < parts ? (int)(total * (part + 1) / parts) - skip : 0;
+        }
+    }
+    __device__ void open(int i)
+    {
+        const int2 g = segs[i];
+        t = (max(g.x, win_lo) + stride - 1) / stride * stride;
+        end = min(g.y, win_hi);
+    }
+    __device__ int tiles() const { return t < end ? (end - t + stride - 1) / stride : 0; }
     __device__ bool next(int &tile)
     {
+        if (DIVIDED && left <= 0) return false;
         while (t >= end) {
             if (++s >= nseg) return false;
-            const int2 g = segs[s];
-            t = (max(g.x, win_lo) + stride - 1) / stride * stride;
-            end = min(g.y, win_hi);
+            open(s);
+            if (DIVIDED && skip > 0) {
+                const int over = min(skip, tiles());
+                skip -= over;
+                t += over * stride;
+            }
         }
+        if (DIVIDED) left--;
         tile = t;
         t += stride;
         return true;
     }
 };
+
+// Where several blocks share a query's buffer, the slots for the n keys of a chunk that passed are taken with one atomic
+// addition.  Returns the first; `room` = how many of them exist.  A count beyond the segment says that keys were lost (and
+// bit 30, which the thread that met the end sets, stops every block that starts on the query later).
+__device__ __forceinline__ int take_slots(int *count, int n, int seg_cap, int &room)
+{
+    const int c = atomicAdd(count, n);
+    const int first = c & 0x3fffffff;
+    room = seg_cap - first;
+    if (room < n && !(c & 0x40000000)) atomicOr(count, 0x40000000);
+    return first;
+}
 
 // ------------------------------------------------------------------------------------------------
 // filter kernel
@@ -616,8 +668,8 @@ __device__ __forceinline__ void tc_issue_products(uint32_t d_tmem, uint64_t a_hi
 // The MMA issuer's walk over the block's database tiles (one thread).  a16 / b16 / end16: the block's images in
 // 16-byte units of shared memory; span16: what one K step reads beyond its start.  Every tile's descriptors are
 // checked against that range before they are used (an MMA that reads outside the block's shared memory is a fault).
-template <int QH, bool BF16, int NKS>
-__device__ __noinline__ void tc_issue_walk(TcShared *shp, volatile int *abort_flag, TileWalk walk, uint32_t tmem_base, uint64_t no_addr,
+template <int QH, bool BF16, int NKS, bool DIVIDED>
+__device__ __noinline__ void tc_issue_walk(TcShared *shp, volatile int *abort_flag, TileWalk<DIVIDED> walk, uint32_t tmem_base, uint64_t no_addr,
                                            uint32_t a16, uint32_t b16, uint32_t image16, uint32_t spr_log, uint32_t block16,
                                            uint32_t in_row16, uint32_t span16, uint32_t end16)
 {
@@ -657,12 +709,13 @@ __device__ __noinline__ void tc_issue_walk(TcShared *shp, volatile int *abort_fl
 // RANKED: no candidate buffers at all; every query thread keeps its 16 smallest keys in
 // registers and rank_out[query] receives the one of rank `rank` (0-based, < 16) when the scan ends: the first
 // threshold level, a scan of a few thousand sample points.
-template <int QH, bool RANKED>
+// SHARED: the tiles of a block of queries are dealt to gridDim.y blocks, which append to the same buffers (take_slots).
+template <int QH, bool RANKED, bool SHARED>
 __global__ void __launch_bounds__(tc_threads(QH), 1)
 knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ img_db, int Dp, long long nq, long long nd_pos,
                      const int2 *__restrict__ segs, const int *__restrict__ nseg, int seg_stride, int tile_stride, int win_lo,
                      int win_hi, const float *__restrict__ tau, int cap, float *cand_key, int32_t *cand_id, int *counts,
-                     int *error_flag, int bf16, int sw, int nks, int rank = 0, float *__restrict__ rank_out = nullptr)
+                     int *error_flag, int bf16, int sw, int nks, ScanParts parts, int rank = 0, float *__restrict__ rank_out = nullptr)
 {
     // bf16: the images hold bf16 pairs; sw != 0: in swizzled rows of sw bytes (else core matrices without swizzle);
     // nks: K steps of 32 operand bytes per row to multiply
@@ -677,8 +730,9 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
     const long long qt = (long long)blockIdx.x * QH;   // first query tile of the block
     const int2 *my_segs = segs + (size_t)blockIdx.x * seg_stride;
     const int my_nseg = nseg[seg_stride ? blockIdx.x : 0];
+    const int part = SHARED ? blockIdx.y : 0;
     {   // nothing of this block's segments in the window: leave before any barrier or TMEM is set up
-        TileWalk probe(my_segs, my_nseg, tile_stride, win_lo, win_hi);
+        TileWalk<SHARED> probe(my_segs, my_nseg, tile_stride, win_lo, win_hi, part, parts);
         int first;
         if (!probe.next(first)) return;
     }
@@ -711,7 +765,7 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
             mbar_expect_tx(&sh.full_a, QH * image_bytes);
             for (int h = 0; h < QH; h++)
                 bulk_load(sA + (size_t)h * (image_bytes / 4), img_q + (size_t)(qt + h) * (image_bytes / 4), image_bytes, &sh.full_a);
-            TileWalk walk(my_segs, my_nseg, tile_stride, win_lo, win_hi);
+            TileWalk<SHARED> walk(my_segs, my_nseg, tile_stride, win_lo, win_hi, part, parts);
             int tile;
             for (long long t = 0; walk.next(tile); t++) {
                 const int s = (int)(t % kBStages);
@@ -736,12 +790,12 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
             const uint64_t no_addr = sw ? make_desc_swizzled(0u, (uint32_t)sw) : make_desc(0u);
             const uint32_t a16 = smem_u32(sA) >> 4, b16 = smem_u32(sB) >> 4, image16 = image_bytes >> 4;
             const uint32_t end16 = (smem_u32(smem) + (uint32_t)(QH + kBStages) * image_bytes) >> 4;
-            const TileWalk walk(my_segs, my_nseg, tile_stride, win_lo, win_hi);
+            const TileWalk<SHARED> walk(my_segs, my_nseg, tile_stride, win_lo, win_hi, part, parts);
 #define B200_ISSUE(NKS_)                                                                                                        \
     case NKS_:                                                                                                                  \
-        if (bf16) tc_issue_walk<QH, true, NKS_>(&sh, abort_flag, walk, tmem_base, no_addr, a16, b16, image16, spr_log, block16,  \
+        if (bf16) tc_issue_walk<QH, true, NKS_, SHARED>(&sh, abort_flag, walk, tmem_base, no_addr, a16, b16, image16, spr_log, block16,  \
                                                 in_row16, span16, end16);                                                       \
-        else tc_issue_walk<QH, false, NKS_>(&sh, abort_flag, walk, tmem_base, no_addr, a16, b16, image16, spr_log, block16,      \
+        else tc_issue_walk<QH, false, NKS_, SHARED>(&sh, abort_flag, walk, tmem_base, no_addr, a16, b16, image16, spr_log, block16,      \
                                             in_row16, span16, end16);                                                           \
         break;
             switch (nks) {
@@ -800,6 +854,15 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
             }
             const float mn = fminf(min3(m4[0], m4[1], m4[2]), m4[3]);
             if (mn < thr) {
+                int end = 0;
+                if constexpr (SHARED) {
+                    int n = 0, room = 0;
+#pragma unroll
+                    for (int c = 0; c < 32; c++) n += (__uint_as_float(r[c]) < thr && (tile_inside || col0 + c < nd_pos)) ? 1 : 0;
+                    if (n > 0) cnt = take_slots(counts + gq * kAccBufs + buf, n, seg_cap, room);
+                    if (room < n) overflow = true;
+                    end = cnt + room;
+                }
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     if (m4[q] < thr) {
@@ -809,7 +872,15 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
                             const float key = __uint_as_float(r[c]);
                             const long long cid = col0 + c;
                             const bool pass = key < thr && (tile_inside || cid < nd_pos);
-                            if constexpr (RANKED) {
+                            if constexpr (SHARED) {
+                                if (pass) {
+                                    if (cnt < end) {
+                                        __stcg(bk + cnt, key);
+                                        __stcg(bi + cnt, (int32_t)cid);
+                                    }
+                                    cnt++;
+                                }
+                            } else if constexpr (RANKED) {
                                 if (pass) {   // replaces the largest of the 16 and sinks to its place
                                     top[15] = key;
 #pragma unroll
@@ -830,10 +901,10 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
                 }
             }
             // a chunk appends at most 32 entries: stop a buffer that could overflow in the next one
-            if (!RANKED && cnt > seg_cap - 32) { overflow = true; thr = -INFINITY; }
+            if (!RANKED && (SHARED ? overflow : cnt > seg_cap - 32)) { overflow = true; thr = -INFINITY; }
         };
 
-        TileWalk walk(my_segs, active ? my_nseg : 0, tile_stride, win_lo, win_hi);
+        TileWalk<SHARED> walk(my_segs, active ? my_nseg : 0, tile_stride, win_lo, win_hi, part, parts);
         int tile;
         for (long long t = 0; walk.next(tile); t++) {
             const int b = (int)(t % kAccBufs);
@@ -866,7 +937,7 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
                 for (int i = 1; i < 16; i++) t = (i == rank) ? top[i] : t;
                 rank_out[gq] = t;
             }
-        } else {
+        } else if constexpr (!SHARED) {
             // The final selection is a separate kernel (one warp per query, thousands in flight): it is a chain of
             // dependent global round trips, which the warps of this block would walk through one query at a time.
             if (serve) counts[gq * kAccBufs + buf] = cnt | (overflow ? 0x40000000 : 0);
@@ -918,7 +989,7 @@ __global__ void __launch_bounds__(tc_threads(2), 1)
 knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ img_db, int n_chunks, long long nq,
                    const int2 *__restrict__ segs, const int *__restrict__ nseg, int seg_stride, int unit_stride, int win_lo,
                    int win_hi, const float *__restrict__ tau, int cap, float *cand_key, int32_t *cand_id, int *counts,
-                   int *error_flag, int bf16, int rank = 0, float *__restrict__ rank_out = nullptr, long long n_pos = 0)
+                   int *error_flag, int bf16, ScanParts parts, int rank = 0, float *__restrict__ rank_out = nullptr, long long n_pos = 0)
 {
     constexpr int kProducerWarp = 16, kMmaWarp = 17;
     constexpr uint32_t kTmemCols = 512;
@@ -929,8 +1000,9 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
     const long long qt = (long long)blockIdx.x * 2;   // first query tile of the block
     const int2 *my_segs = segs + (size_t)blockIdx.x * seg_stride;
     const int my_nseg = nseg[seg_stride ? blockIdx.x : 0];
+    const int part = RANKED ? 0 : blockIdx.y;
     {   // nothing of this block's segments in the window
-        TileWalk probe(my_segs, my_nseg, unit_stride, win_lo, win_hi);
+        TileWalk<!RANKED> probe(my_segs, my_nseg, unit_stride, win_lo, win_hi, part, parts);
         int first;
         if (!probe.next(first)) return;
     }
@@ -961,7 +1033,7 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
 
     if (warp == kProducerWarp) {
         if (lane == 0) {
-            TileWalk walk(my_segs, my_nseg, unit_stride, win_lo, win_hi);
+            TileWalk<!RANKED> walk(my_segs, my_nseg, unit_stride, win_lo, win_hi, part, parts);
             int unit;
             long long it = 0;   // stage counter over (unit, chunk)
             bool ok = true;
@@ -985,7 +1057,7 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
         }
     } else if (warp == kMmaWarp) {
         if (lane == 0) {
-            TileWalk walk(my_segs, my_nseg, unit_stride, win_lo, win_hi);
+            TileWalk<!RANKED> walk(my_segs, my_nseg, unit_stride, win_lo, win_hi, part, parts);
             int unit;
             long long it = 0, n_unit = 0;
             bool ok = true;
@@ -1061,6 +1133,9 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
             overflow = (c0 & 0x40000000) != 0;
             if (overflow) thr = -INFINITY;
         }
+        TileWalk<!RANKED> walk(my_segs, active ? my_nseg : 0, unit_stride, win_lo, win_hi, part, parts);
+        const bool alone = walk.parts == 1;   // as in the narrow kernel
+        int unit;
         float top[RANKED ? 16 : 1];
 #pragma unroll
         for (int i = 0; i < (RANKED ? 16 : 1); i++) top[i] = INFINITY;
@@ -1076,6 +1151,15 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
             }
             const float mn = fminf(min3(m4[0], m4[1], m4[2]), m4[3]);
             if (mn < thr) {
+                int end = seg_cap;
+                if (!RANKED && !alone) {
+                    int n = 0, room = 0;
+#pragma unroll
+                    for (int c = 0; c < 32; c++) n += __uint_as_float(r[c]) < thr ? 1 : 0;
+                    cnt = take_slots(counts + gq * 2 + g, n, seg_cap, room);
+                    if (room < n) overflow = true;
+                    end = cnt + room;
+                }
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     if (m4[q] < thr) {
@@ -1095,19 +1179,19 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
                                     thr = top[15];
                                 }
                             } else if (key < thr) {   // padding rows carry a huge norm and never pass a finite threshold
-                                __stcg(bk + cnt, key);
-                                __stcg(bi + cnt, (int32_t)(pos0 + c));
+                                if (cnt < end) {
+                                    __stcg(bk + cnt, key);
+                                    __stcg(bi + cnt, (int32_t)(pos0 + c));
+                                }
                                 cnt++;
                             }
                         }
                     }
                 }
             }
-            if (!RANKED && cnt > seg_cap - 32) { overflow = true; thr = -INFINITY; }
+            if (!RANKED && (overflow || (alone && cnt > seg_cap - 32))) { overflow = true; thr = -INFINITY; }
         };
         const uint32_t tlane = tmem_base + ((uint32_t)(quarter * 32) << 16);
-        TileWalk walk(my_segs, active ? my_nseg : 0, unit_stride, win_lo, win_hi);
-        int unit;
         for (long long n_unit = 0; walk.next(unit); n_unit++) {
             if (!mbar_wait(&sh.acc_full, (uint32_t)(n_unit & 1), abort_flag, 32)) break;
             tc_fence_after();
@@ -1138,7 +1222,7 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
                 rank_out[gq] = t;
             }
         } else {
-            if (serve) counts[gq * 2 + g] = cnt | (overflow ? 0x40000000 : 0);
+            if (serve && alone) counts[gq * 2 + g] = cnt | (overflow ? 0x40000000 : 0);
         }
     }
     // ---------------- teardown ----------------
@@ -1808,6 +1892,29 @@ struct PhaseTimer {
 // Workspace (device, 256-byte aligned) needed by launch_knn_tc for nq queries against nd database rows.
 size_t knn_tc_workspace_bytes(int D, int K, int64_t nq, int64_t nd) { return tc_carve(nullptr, D, K, nq, nd).bytes; }
 
+// Into how many parts the database tiles of every block of queries are dealt, one block a part.  A block holds a whole SM,
+// so `blocks` blocks of equal work take ceil(blocks / SMs) turns: 196 on 148 SMs leave a third of the chip idle, 20 seven
+// eighths of it.  One part unless more save 3 %.
+// The narrow kernel's epilogue is most of its time, and slots taken in memory make it a third longer (30 011 x 32: 0.47
+// against 0.61 ms): its tiles are dealt only where half of the SMs would idle.
+// Scans, one part and by this rule: 50 000 x 1 024 13.8 -> 10.7 ms, 60 000 x 784 2.26 -> 1.80, 20 011 x 784 2.13 -> 1.23,
+// 8 000 x 512 0.76 -> 0.28, 5 000 x 50 0.21 -> 0.10.
+static ScanParts scan_parts(int blocks, int tiles, int share, int limit, int sms)
+{
+    auto cost = [&](int parts) {   // a part's set-up is about a tenth of a share
+        const long long turns = ((long long)blocks * parts + sms - 1) / sms;
+        return (double)turns * ((double)((tiles + parts - 1) / parts) + 0.1 * share);
+    };
+    ScanParts p;
+    p.idle = std::max(1, sms / blocks);
+    p.share = share;
+    const int most = std::min(limit, std::max(p.idle, tiles / share));
+    double least = 0.97 * cost(1);
+    for (int parts = 2; parts <= most; parts++)
+        if (cost(parts) < least) { p.most = parts; least = cost(parts); }
+    return p;
+}
+
 // X: [N][D] row-major (device).  ids/d2: [(q_hi-q_lo)][K].  n_failed_host receives the number of rows
 // whose proof did not close; their global row indices are in failed_list (device, first n entries) and
 // the caller recomputes them with the SIMT search.  Returns after the kernels are queued, except for
@@ -1901,29 +2008,34 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     const long long db_image_bytes = (long long)w.td * (long long)w.image_bytes;
     int window_tiles = db_image_bytes > (512ll << 20) ? (int)((60ll << 20) / (long long)w.image_bytes) : INT_MAX;
     if (const char *e = getenv("B200TSNE_KNN_WINDOW_TILES")) window_tiles = std::max(1, atoi(e));   // for tests
+    int device = 0, sm_count = 0;
+    B200_CUDA(cudaGetDevice(&device));
+    B200_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
     // One scan of every stride-th tile against tau.  The attribute and the launch of the instantiation that fits the images:
     auto scan = [&](int stride) -> int {
         B200_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)nq * 2, st));
         const long long tiles = wide ? w.td / 2 : w.td;
         const long long win = (long long)(wide ? std::max(1, window_tiles / 2) : window_tiles) * stride;
         const size_t smem = wide ? (size_t)kWideStages * 4 * kWideChunkBytes : (size_t)(QH + kBStages) * w.image_bytes;
+        const int blocks = (int)((q_tiles + (wide ? 2 : QH) - 1) / (wide ? 2 : QH));
+        // a share is worth its block's barriers, TMEM, first loads and last epilogue (6 us) ten times over
+        const ScanParts parts = scan_parts(blocks, (int)((std::min(tiles, win) + stride - 1) / stride), wide ? (63 + Dp / KC) / (Dp / KC) : 32,
+                                            wide || 2 * blocks <= sm_count ? 16 : 1, sm_count);
+        const dim3 grid((unsigned)blocks, (unsigned)parts.most);
+        auto narrow = parts.most > 1 ? (QH == 1 ? knn_tc_filter_kernel<1, false, true> : knn_tc_filter_kernel<2, false, true>)
+                                : (QH == 1 ? knn_tc_filter_kernel<1, false, false> : knn_tc_filter_kernel<2, false, false>);
         if (wide) B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        else if (QH == 1) B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        else B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        else B200_CUDA(cudaFuncSetAttribute(narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         for (long long lo = 0; lo < tiles; lo += win) {
             const int hi = (int)std::min<long long>(tiles, lo + win);
             if (wide)
-                knn_tc_wide_kernel<false><<<(unsigned)((q_tiles + 1) / 2), tc_threads(2), smem, st>>>(
+                knn_tc_wide_kernel<false><<<grid, tc_threads(2), smem, st>>>(
                     w.img_q, w.img_db, Dp / KC, nq, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand_key, cand_id, counts,
-                    counters + 0, bf16);
-            else if (QH == 1)
-                knn_tc_filter_kernel<1, false><<<(unsigned)q_tiles, tc_threads(1), smem, st>>>(
-                    w.img_q, w.img_db, Dp, nq, nd_pos, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand_key, cand_id, counts,
-                    counters + 0, bf16, w.sw, w.nks);
+                    counters + 0, bf16, parts);
             else
-                knn_tc_filter_kernel<2, false><<<(unsigned)((q_tiles + 1) / 2), tc_threads(2), smem, st>>>(
+                narrow<<<grid, tc_threads(QH), smem, st>>>(
                     w.img_q, w.img_db, Dp, nq, nd_pos, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand_key, cand_id, counts,
-                    counters + 0, bf16, w.sw, w.nks);
+                    counters + 0, bf16, w.sw, w.nks, parts, 0, nullptr);
             B200_CUDA(cudaGetLastError());
         }
         return 0;
@@ -1974,13 +2086,13 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
             B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
             knn_tc_wide_kernel<true><<<(unsigned)((q_tiles + 1) / 2), tc_threads(2), smem_a, st>>>(
                 w.img_q, w.img_s, Dp / KC, nq, w.segs, w.nseg, 0, 1, 0, ts / 2, nullptr, 0, nullptr, nullptr, nullptr, counters + 0, bf16,
-                rank_a, tau, (long long)m_a);
+                ScanParts(), rank_a, tau, (long long)m_a);
         } else {
             const size_t smem_a = (size_t)(1 + kBStages) * w.image_bytes;
-            B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
-            knn_tc_filter_kernel<1, true><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
+            B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+            knn_tc_filter_kernel<1, true, false><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
                 w.img_q, w.img_s, Dp, nq, (long long)m_a, w.segs, w.nseg, 0, 1, 0, ts, nullptr, 0, nullptr, nullptr, nullptr, counters + 0,
-                bf16, w.sw, w.nks, rank_a, tau);
+                bf16, w.sw, w.nks, ScanParts(), rank_a, tau);
         }
         B200_CUDA(cudaGetLastError());
         knn_single_segment_kernel<<<1, 1, 0, st>>>(w.segs, w.nseg, all_tiles);   // back to all database tiles
