@@ -81,6 +81,9 @@ constexpr int kAccBufs = 2;
 // from L2 once per 128 * QH queries.  8 * QH epilogue warps, then the producer warp and the MMA warp;
 // TMEM columns = kAccBufs * QH * TN.
 constexpr int tc_threads(int QH) { return (8 * QH + 2) * 32; }
+// Thresholds stay below the keys of padding rows, whose norm is 3e38: without the limit a sample of infinite keys (norms
+// beyond the range of floats) lets padding pass.  Rows that find too few candidates below it are recomputed.
+constexpr float kTauLimit = 2.9e38f;
 
 // ------------------------------------------------------------------------------------------------
 // PTX helpers
@@ -704,7 +707,7 @@ __device__ __noinline__ void tc_issue_walk(TcShared *shp, volatile int *abort_fl
 // (segs + blockIdx.x * seg_stride, nseg[blockIdx.x * (seg_stride != 0)] of them; seg_stride = 0: one list shared by
 // all blocks), taking every tile_stride-th tile.  Candidate ids are database list positions; positions from
 // nd_pos on are padding and never kept.
-// cand_key / cand_id: [nq][cap] candidate buffers, two segments of cap/2 entries per query; threshold tau[query];
+// cand: [nq][cap] candidate buffers (key bits, list position), two segments of cap/2 entries per query; threshold tau[query];
 // counts[2*query + buffer] receives the number of entries appended to each (bit 30 set if it overflowed).
 // RANKED: no candidate buffers at all; every query thread keeps its 16 smallest keys in
 // registers and rank_out[query] receives the one of rank `rank` (0-based, < 16) when the scan ends: the first
@@ -714,7 +717,7 @@ template <int QH, bool RANKED, bool SHARED>
 __global__ void __launch_bounds__(tc_threads(QH), 1)
 knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ img_db, int Dp, long long nq, long long nd_pos,
                      const int2 *__restrict__ segs, const int *__restrict__ nseg, int seg_stride, int tile_stride, int win_lo,
-                     int win_hi, const float *__restrict__ tau, int cap, float *cand_key, int32_t *cand_id, int *counts,
+                     int win_hi, const float *__restrict__ tau, int cap, uint2 *cand, int *counts,
                      int *error_flag, int bf16, int sw, int nks, ScanParts parts, int rank = 0, float *__restrict__ rank_out = nullptr)
 {
     // bf16: the images hold bf16 pairs; sw != 0: in swizzled rows of sw bytes (else core matrices without swizzle);
@@ -821,16 +824,15 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
         const int row = quarter * 32 + lane;                    // TMEM lane
         const long long gq = (qt + half) * TM + row;
         const bool serve = gq < nq && active;
-        float *bk = cand_key + (serve ? gq : 0) * cap + buf * seg_cap;
-        int32_t *bi = cand_id + (serve ? gq : 0) * cap + buf * seg_cap;
+        uint2 *const segment = cand + (serve ? gq : 0) * cap + buf * seg_cap;
+        uint2 *next = segment;   // where the next candidate goes
         float thr = serve ? (RANKED ? INFINITY : tau[gq]) : -INFINITY;
         // a fixed-threshold scan may be split into several launches (windows of the database): a launch
         // continues the buffers where the previous one stopped (counts are zeroed before the first)
-        int cnt = 0;
         bool overflow = false;
         if (!RANKED && serve) {
             const int c0 = counts[gq * kAccBufs + buf];
-            cnt = c0 & 0x3fffffff;
+            next += c0 & 0x3fffffff;
             overflow = (c0 & 0x40000000) != 0;
             if (overflow) thr = -INFINITY;
         }
@@ -840,6 +842,9 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
         // independent three-input min operations and one comparison.  Only if the minimum beats the
         // threshold (rare once the scan is under way) are the quarters whose minimum does so compared
         // element by element; everything is indexed statically, so the keys never leave the registers.
+        // What a survivor costs decides the scan: nearly every chunk of a warp has one.  Comparison, one 8-byte store, one
+        // addition to the pointer; with key and id in two arrays, an index and a test for padding the scans took 80.3
+        // instead of 63.2 ms (10^6 x 50), 7.16 instead of 4.34 (300 000 x 20), 0.48 instead of 0.31 (30 011 x 32).
         float top[RANKED ? 16 : 1];
 #pragma unroll
         for (int i = 0; i < (RANKED ? 16 : 1); i++) top[i] = INFINITY;
@@ -854,14 +859,12 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
             }
             const float mn = fminf(min3(m4[0], m4[1], m4[2]), m4[3]);
             if (mn < thr) {
-                int end = 0;
                 if constexpr (SHARED) {
                     int n = 0, room = 0;
 #pragma unroll
-                    for (int c = 0; c < 32; c++) n += (__uint_as_float(r[c]) < thr && (tile_inside || col0 + c < nd_pos)) ? 1 : 0;
-                    if (n > 0) cnt = take_slots(counts + gq * kAccBufs + buf, n, seg_cap, room);
-                    if (room < n) overflow = true;
-                    end = cnt + room;
+                    for (int c = 0; c < 32; c++) n += __uint_as_float(r[c]) < thr ? 1 : 0;
+                    next = segment + take_slots(counts + gq * kAccBufs + buf, n, seg_cap, room);
+                    if (room < n) { overflow = true; thr = -INFINITY; }   // the row is lost: nothing more is written
                 }
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
@@ -870,18 +873,8 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
                         for (int e = 0; e < 8; e++) {
                             const int c = q * 8 + e;
                             const float key = __uint_as_float(r[c]);
-                            const long long cid = col0 + c;
-                            const bool pass = key < thr && (tile_inside || cid < nd_pos);
-                            if constexpr (SHARED) {
-                                if (pass) {
-                                    if (cnt < end) {
-                                        __stcg(bk + cnt, key);
-                                        __stcg(bi + cnt, (int32_t)cid);
-                                    }
-                                    cnt++;
-                                }
-                            } else if constexpr (RANKED) {
-                                if (pass) {   // replaces the largest of the 16 and sinks to its place
+                            if constexpr (RANKED) {
+                                if (key < thr && (tile_inside || col0 + c < nd_pos)) {   // replaces the largest of the 16 and sinks to its place
                                     top[15] = key;
 #pragma unroll
                                     for (int i = 15; i > 0; i--) {
@@ -891,17 +884,16 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
                                     }
                                     thr = top[15];
                                 }
-                            } else if (pass) {
-                                __stcg(bk + cnt, key);
-                                __stcg(bi + cnt, (int32_t)cid);
-                                cnt++;
+                            } else if (key < thr) {   // padding rows carry a huge norm and never pass (kTauLimit)
+                                __stcg(next, make_uint2(r[c], (unsigned)col0 + c));
+                                next++;
                             }
                         }
                     }
                 }
             }
             // a chunk appends at most 32 entries: stop a buffer that could overflow in the next one
-            if (!RANKED && (SHARED ? overflow : cnt > seg_cap - 32)) { overflow = true; thr = -INFINITY; }
+            if (!RANKED && !SHARED && next > segment + (seg_cap - 32)) { overflow = true; thr = -INFINITY; }
         };
 
         TileWalk<SHARED> walk(my_segs, active ? my_nseg : 0, tile_stride, win_lo, win_hi, part, parts);
@@ -935,12 +927,12 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
                 float t = top[0];
 #pragma unroll
                 for (int i = 1; i < 16; i++) t = (i == rank) ? top[i] : t;
-                rank_out[gq] = t;
+                rank_out[gq] = fminf(t, kTauLimit);
             }
         } else if constexpr (!SHARED) {
             // The final selection is a separate kernel (one warp per query, thousands in flight): it is a chain of
             // dependent global round trips, which the warps of this block would walk through one query at a time.
-            if (serve) counts[gq * kAccBufs + buf] = cnt | (overflow ? 0x40000000 : 0);
+            if (serve) counts[gq * kAccBufs + buf] = (int)(next - segment) | (overflow ? 0x40000000 : 0);
         }
     }
     // ---------------- teardown ----------------
@@ -988,7 +980,7 @@ template <bool RANKED>
 __global__ void __launch_bounds__(tc_threads(2), 1)
 knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ img_db, int n_chunks, long long nq,
                    const int2 *__restrict__ segs, const int *__restrict__ nseg, int seg_stride, int unit_stride, int win_lo,
-                   int win_hi, const float *__restrict__ tau, int cap, float *cand_key, int32_t *cand_id, int *counts,
+                   int win_hi, const float *__restrict__ tau, int cap, uint2 *cand, int *counts,
                    int *error_flag, int bf16, ScanParts parts, int rank = 0, float *__restrict__ rank_out = nullptr, long long n_pos = 0)
 {
     constexpr int kProducerWarp = 16, kMmaWarp = 17;
@@ -1122,14 +1114,13 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
         const long long gq = (qt + half) * TM + row;
         const bool active = !RANKED || g == 0;
         const bool serve = gq < nq && active;
-        float *bk = cand_key + (serve ? gq : 0) * cap + g * seg_cap;
-        int32_t *bi = cand_id + (serve ? gq : 0) * cap + g * seg_cap;
+        uint2 *const segment = cand + (serve ? gq : 0) * cap + g * seg_cap;
+        uint2 *next = segment;
         float thr = serve ? (RANKED ? INFINITY : tau[gq]) : -INFINITY;
-        int cnt = 0;
         bool overflow = false;
         if (!RANKED && serve) {
             const int c0 = counts[gq * 2 + g];
-            cnt = c0 & 0x3fffffff;
+            next += c0 & 0x3fffffff;
             overflow = (c0 & 0x40000000) != 0;
             if (overflow) thr = -INFINITY;
         }
@@ -1151,14 +1142,12 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
             }
             const float mn = fminf(min3(m4[0], m4[1], m4[2]), m4[3]);
             if (mn < thr) {
-                int end = seg_cap;
                 if (!RANKED && !alone) {
                     int n = 0, room = 0;
 #pragma unroll
                     for (int c = 0; c < 32; c++) n += __uint_as_float(r[c]) < thr ? 1 : 0;
-                    cnt = take_slots(counts + gq * 2 + g, n, seg_cap, room);
-                    if (room < n) overflow = true;
-                    end = cnt + room;
+                    next = segment + take_slots(counts + gq * 2 + g, n, seg_cap, room);
+                    if (room < n) { overflow = true; thr = -INFINITY; }   // the row is lost: nothing more is written
                 }
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
@@ -1178,18 +1167,15 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
                                     }
                                     thr = top[15];
                                 }
-                            } else if (key < thr) {   // padding rows carry a huge norm and never pass a finite threshold
-                                if (cnt < end) {
-                                    __stcg(bk + cnt, key);
-                                    __stcg(bi + cnt, (int32_t)(pos0 + c));
-                                }
-                                cnt++;
+                            } else if (key < thr) {   // padding rows carry a huge norm and never pass (kTauLimit)
+                                __stcg(next, make_uint2(r[c], (unsigned)pos0 + c));
+                                next++;
                             }
                         }
                     }
                 }
             }
-            if (!RANKED && (overflow || (alone && cnt > seg_cap - 32))) { overflow = true; thr = -INFINITY; }
+            if (!RANKED && alone && next > segment + (seg_cap - 32)) { overflow = true; thr = -INFINITY; }
         };
         const uint32_t tlane = tmem_base + ((uint32_t)(quarter * 32) << 16);
         for (long long n_unit = 0; walk.next(unit); n_unit++) {
@@ -1219,10 +1205,10 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
                 float t = top[0];
 #pragma unroll
                 for (int i = 1; i < 16; i++) t = (i == rank) ? top[i] : t;
-                rank_out[gq] = t;
+                rank_out[gq] = fminf(t, kTauLimit);
             }
         } else {
-            if (serve && alone) counts[gq * 2 + g] = cnt | (overflow ? 0x40000000 : 0);
+            if (serve && alone) counts[gq * 2 + g] = (int)(next - segment) | (overflow ? 0x40000000 : 0);
         }
     }
     // ---------------- teardown ----------------
@@ -1244,12 +1230,10 @@ knn_tc_wide_kernel(const float *__restrict__ img_q, const float *__restrict__ im
 // the bits between the smallest and the largest key of the buffer: they share their leading bits, so about half of 32
 // steps are enough, 1,500 issue slots (a warp-wide bitonic sort: 17,000).
 struct CandidateBuffer {
-    const float *key;
-    const int32_t *id;
+    const uint2 *entry;   // (key bits, list position)
     int n0, n, half;
     bool lost;
-    __device__ CandidateBuffer(const float *cand_key, const int32_t *cand_id, int cap, const int *counts, long long q)
-        : key(cand_key + q * cap), id(cand_id + q * cap), half(cap / 2)
+    __device__ CandidateBuffer(const uint2 *cand, int cap, const int *counts, long long q) : entry(cand + q * cap), half(cap / 2)
     {
         const int c0 = counts[2 * q], c1 = counts[2 * q + 1];
         lost = ((c0 | c1) & 0x40000000) != 0;
@@ -1267,7 +1251,7 @@ template <int SLOTS> __device__ __forceinline__ void load_keys(const CandidateBu
         const int e = lane + 32 * j;
         enc[j] = 0xffffffffu;
         if (e < b.n) {
-            enc[j] = enc_float(__ldcg(b.key + b.at(e)));
+            enc[j] = enc_float(__uint_as_float(__ldcg(&b.entry[b.at(e)].x)));
             lo = min(lo, enc[j]);
             hi = max(hi, enc[j]);
         }
@@ -1305,12 +1289,12 @@ template <int SLOTS> __device__ __forceinline__ unsigned kth_key(const unsigned 
 // kth[q] = the k-th smallest key of the buffer, or -inf when it lost keys or holds fewer than k
 template <int SLOTS>
 __global__ void __launch_bounds__(128)
-knn_tc_pick_kernel(const float *__restrict__ cand_key, int cap, const int *__restrict__ counts, long long nq, int k, float *__restrict__ kth)
+knn_tc_pick_kernel(const uint2 *__restrict__ cand, int cap, const int *__restrict__ counts, long long nq, int k, float *__restrict__ kth)
 {
     const int lane = threadIdx.x & 31;
     const long long q = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (q >= nq) return;
-    const CandidateBuffer b(cand_key, nullptr, cap, counts, q);
+    const CandidateBuffer b(cand, cap, counts, q);
     float v = -INFINITY;
     if (!b.lost && b.n >= k) {
         unsigned enc[SLOTS], lo, hi;
@@ -1404,7 +1388,7 @@ template <int EPL> __device__ __forceinline__ void warp_sort(unsigned long long 
 template <int VEC, int EPL>
 __global__ void __launch_bounds__(kRerankWarps * 32, EPL <= 4 ? 6 : 4)
 knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__ qlist, const int *__restrict__ dblist,
-                     long long out_base, long long nq, const float *__restrict__ cand_key, const int32_t *__restrict__ cand_id, int cap,
+                     long long out_base, long long nq, const uint2 *__restrict__ cand, int cap,
                      const int *__restrict__ counts, const float *__restrict__ tau, int K, const double *__restrict__ norms_exact,
                      float err_scale, const float2 *__restrict__ res_q, const float *__restrict__ rho, int32_t *__restrict__ ids,
                      float *__restrict__ d2, int *__restrict__ failed, int *__restrict__ n_failed, float *__restrict__ max_err_ratio,
@@ -1416,7 +1400,7 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long q = (long long)blockIdx.x * kRerankWarps + w;
     if (q >= nq) return;
-    const CandidateBuffer b(cand_key, cand_id, cap, counts, q);
+    const CandidateBuffer b(cand, cap, counts, q);
     if (b.lost || b.n < K) {   // the fixed threshold kept too few or too many
         if (lane == 0) { failed[q] = 1; atomicAdd(n_failed, 1); }
         return;
@@ -1479,7 +1463,7 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
             const unsigned mask = __ballot_sync(0xffffffffu, take);
             if (take) {
                 const int at = m + __popc(mask & ((1u << lane) - 1u));
-                const int p = __ldcg(b.id + b.at(e));
+                const int p = (int)__ldcg(&b.entry[b.at(e)].y);
                 s_src[at] = Xp ? p : dblist[p];
                 s_fkey[at] = dec_float(enc[j]);
             }
@@ -1662,7 +1646,7 @@ knn_sample_tau_kernel(const float *__restrict__ X, int D, const int *__restrict_
         float t = top[0];
 #pragma unroll
         for (int i = 1; i < 16; i++) t = (i == rank) ? top[i] : t;
-        tau[q] = t;
+        tau[q] = fminf(t, kTauLimit);
     }
 }
 
@@ -1727,7 +1711,7 @@ knn_sample_tau_wide_kernel(const float *__restrict__ X, int D, const int *__rest
         float t = top[0];
 #pragma unroll
         for (int i = 1; i < 16; i++) t = (i == rank) ? top[i] : t;
-        tau[q] = t;
+        tau[q] = fminf(t, kTauLimit);
     }
 }
 
@@ -1796,8 +1780,8 @@ struct TcWorkspace {
     float *dist_q;             // and distances to the centres
     int2 *segs;
     int *nseg;
-    float *cand_key, *tau;
-    int32_t *cand_id;
+    uint2 *cand;
+    float *tau;
     int *counts, *failed, *flist, *counters;
     size_t bytes;
 };
@@ -1842,8 +1826,7 @@ static TcWorkspace tc_carve(void *base, int D, int K, long long nq, long long nd
     w.dist_q = reinterpret_cast<float *>(take(sizeof(float) * kMaxCells * (size_t)nq));
     w.segs = reinterpret_cast<int2 *>(take(sizeof(int2) * (size_t)w.tq * kMaxCells));
     w.nseg = reinterpret_cast<int *>(take(sizeof(int) * (size_t)w.tq));
-    w.cand_key = reinterpret_cast<float *>(take(sizeof(float) * (size_t)nq * fixed_cap(K)));
-    w.cand_id = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * (size_t)nq * fixed_cap(K)));
+    w.cand = reinterpret_cast<uint2 *>(take(sizeof(uint2) * (size_t)nq * fixed_cap(K)));
     w.tau = reinterpret_cast<float *>(take(sizeof(float) * (size_t)nq));
     w.counts = reinterpret_cast<int *>(take(sizeof(int) * (size_t)nq * 2));
     w.failed = reinterpret_cast<int *>(take(sizeof(int) * (size_t)nq));
@@ -1934,8 +1917,8 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     const int KC = wide ? (bf16 ? 2 * kWideKC : kWideKC) : Dp;   // inner dimensions per image chunk
     const int L = (K + 32 <= 128) ? 128 : 256;                   // candidates that may be evaluated per query; about 3 L pass a scan
     const int cap = fixed_cap(K);
-    float *cand_key = w.cand_key, *tau = w.tau;
-    int32_t *cand_id = w.cand_id;
+    uint2 *cand = w.cand;
+    float *tau = w.tau;
     int *counts = w.counts, *failed = w.failed, *flist = w.flist, *counters = w.counters;
     B200_CUDA(cudaMemsetAsync(counters, 0, sizeof(int) * 16, st));
     PhaseTimer phases(st);
@@ -2030,11 +2013,11 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
             const int hi = (int)std::min<long long>(tiles, lo + win);
             if (wide)
                 knn_tc_wide_kernel<false><<<grid, tc_threads(2), smem, st>>>(
-                    w.img_q, w.img_db, Dp / KC, nq, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand_key, cand_id, counts,
+                    w.img_q, w.img_db, Dp / KC, nq, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand, counts,
                     counters + 0, bf16, parts);
             else
                 narrow<<<grid, tc_threads(QH), smem, st>>>(
-                    w.img_q, w.img_db, Dp, nq, nd_pos, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand_key, cand_id, counts,
+                    w.img_q, w.img_db, Dp, nq, nd_pos, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand, counts,
                     counters + 0, bf16, w.sw, w.nks, parts, 0, nullptr);
             B200_CUDA(cudaGetLastError());
         }
@@ -2085,13 +2068,13 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
             const size_t smem_a = (size_t)kWideStages * 4 * kWideChunkBytes;
             B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
             knn_tc_wide_kernel<true><<<(unsigned)((q_tiles + 1) / 2), tc_threads(2), smem_a, st>>>(
-                w.img_q, w.img_s, Dp / KC, nq, w.segs, w.nseg, 0, 1, 0, ts / 2, nullptr, 0, nullptr, nullptr, nullptr, counters + 0, bf16,
+                w.img_q, w.img_s, Dp / KC, nq, w.segs, w.nseg, 0, 1, 0, ts / 2, nullptr, 0, nullptr, nullptr, counters + 0, bf16,
                 ScanParts(), rank_a, tau, (long long)m_a);
         } else {
             const size_t smem_a = (size_t)(1 + kBStages) * w.image_bytes;
             B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
             knn_tc_filter_kernel<1, true, false><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
-                w.img_q, w.img_s, Dp, nq, (long long)m_a, w.segs, w.nseg, 0, 1, 0, ts, nullptr, 0, nullptr, nullptr, nullptr, counters + 0,
+                w.img_q, w.img_s, Dp, nq, (long long)m_a, w.segs, w.nseg, 0, 1, 0, ts, nullptr, 0, nullptr, nullptr, counters + 0,
                 bf16, w.sw, w.nks, ScanParts(), rank_a, tau);
         }
         B200_CUDA(cudaGetLastError());
@@ -2104,8 +2087,8 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
         // level B: only the key of rank rank_b among the sample's candidates is needed
         B200_TRY(scan(kSampleStride));
         const unsigned sel_grid = (unsigned)((nq + 3) / 4);
-        if (cap <= 1024) knn_tc_pick_kernel<32><<<sel_grid, 128, 0, st>>>(cand_key, cap, counts, nq, rank_b + 1, tau);
-        else knn_tc_pick_kernel<64><<<sel_grid, 128, 0, st>>>(cand_key, cap, counts, nq, rank_b + 1, tau);
+        if (cap <= 1024) knn_tc_pick_kernel<32><<<sel_grid, 128, 0, st>>>(cand, cap, counts, nq, rank_b + 1, tau);
+        else knn_tc_pick_kernel<64><<<sel_grid, 128, 0, st>>>(cand, cap, counts, nq, rank_b + 1, tau);
         B200_CUDA(cudaGetLastError());
         phases.mark("level_B+pick");
         B200_TRY(prune());
@@ -2129,7 +2112,7 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     const size_t rerank_smem = sizeof(float) * kRerankWarps * rerank_floats(D, L);
     B200_CUDA(cudaFuncSetAttribute(rerank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rerank_smem));
     rerank<<<(unsigned)((nq + kRerankWarps - 1) / kRerankWarps), kRerankWarps * 32, rerank_smem, st>>>(
-        X, D, w.qlist, w.dblist, q_lo, nq, cand_key, cand_id, cap, counts, tau, K, w.norms_q, err_scale, bf16 ? w.res_q : nullptr,
+        X, D, w.qlist, w.dblist, q_lo, nq, cand, cap, counts, tau, K, w.norms_q, err_scale, bf16 ? w.res_q : nullptr,
         reinterpret_cast<const float *>(counters + 4), ids, d2, failed, counters + 1, reinterpret_cast<float *>(counters + 3), xp);
     B200_CUDA(cudaGetLastError());
     knn_tc_collect_failed_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(failed, nq, w.qlist, flist, counters + 2);
