@@ -47,3 +47,12 @@ def test_full_buffers(engine, monkeypatch, d):
     X[2000:5000] = X[2000]
     st = both(engine, monkeypatch, X, 50)
     assert st["rows_recomputed"] >= 3000
+
+
+@pytest.mark.parametrize("pairs", ["bf16", "tf32"])
+@pytest.mark.parametrize("d", [1, 4, 5, 9, 10, 15, 16, 20, 21, 25, 26, 31, 32, 36, 37, 42, 47, 48, 52, 53, 57, 58, 63])
+def test_every_number_of_k_steps(engine, monkeypatch, d, pairs):
+    """The narrow kernel's images: none to three groups of 16 dimensions and one to three steps for what is left."""
+    monkeypatch.setenv("B200TSNE_KNN_FILTER", pairs)
+    st = both(engine, monkeypatch, mixture(2300, d, 70 + d), 20)
+    assert st["filter_error_ratio"] < 0.5 and st["rows_recomputed"] <= 46

@@ -305,6 +305,12 @@ __device__ __forceinline__ size_t image_offset_bf16(int r, int k, int sw)
     return (size_t)block * 64 * sw + (off >> 1);
 }
 
+// The narrow kernel's images are packed (whole >= 0): K steps of 16 columns, first the hi parts of the `whole` full groups of 16
+// dimensions, then their lo parts, then the r = D mod 16 dimensions left over with all three products side by side:
+//   query     [x_hi | x_lo | x_hi | 1 1 1]        database  [b_hi | b_hi | b_lo | the norm in three pieces]
+// in ceil((3 r + 3) / 16) steps that are multiplied once.  With whole steps for what is left (and the norm's pair of columns)
+// 50 dimensions took 12 MMAs a tile pair instead of 10, 20 took 6 instead of 4, and 57 to 63 an image of 64 KB.
+
 // What the three products drop is bounded per pair from the actual leftovers: with a, b the data columns of a
 // query and a database operand, a = a_hi + a_lo + a_r,  |dropped| <= |a_lo||b_lo| + |a - a_r||b_r| + |a_r||b - b_r|
 // + |a_r||b_r| (Cauchy-Schwarz on the leftover vectors).  Queries record |a_lo| and |a_r| (res), the database the
@@ -317,7 +323,7 @@ __device__ __forceinline__ size_t image_offset_bf16(int r, int k, int sw)
 // the candidates of neighbouring queries share a few megabytes that stay in L2.
 constexpr int kPrepDims = 64;
 __global__ void __launch_bounds__(256)
-knn_tc_prepare_bf16_kernel(const float *__restrict__ X, const int *__restrict__ list, int D, int Dp, int KC, int sw, int db_form,
+knn_tc_prepare_bf16_kernel(const float *__restrict__ X, const int *__restrict__ list, int D, int Dp, int KC, int sw, int whole, int db_form,
                            __nv_bfloat16 *__restrict__ img, double *__restrict__ norms, float2 *__restrict__ res,
                            int *__restrict__ rho_bits, float *__restrict__ Xp)
 {
@@ -331,7 +337,8 @@ knn_tc_prepare_bf16_kernel(const float *__restrict__ X, const int *__restrict__ 
     const size_t part = (size_t)KC * 128;
     const int row = tid >> 1, half = tid & 1;   // two threads share a row's sums
     double n2 = 0.0, lo2 = 0.0, r2 = 0.0;       // squared norms of the row, of its lo parts and of its leftovers
-    for (int k0 = 0; k0 < Dp; k0 += kPrepDims) {
+    const int k_end = whole >= 0 ? kPrepDims : Dp;   // (a packed row has fewer than 64 dimensions)
+    for (int k0 = 0; k0 < k_end; k0 += kPrepDims) {
         __syncthreads();
         for (int r = warp; r < TM; r += 8) {
             const int i = s_row[r];
@@ -366,6 +373,38 @@ knn_tc_prepare_bf16_kernel(const float *__restrict__ X, const int *__restrict__ 
                 s_rest[row] = (nf - hi) - __bfloat162float(__float2bfloat16_rn(nf - hi));   // both differences are exact in fp32
             }
             __syncthreads();
+        }
+        if (whole >= 0) {
+            const int n16 = 16 * whole, rest = D - n16;
+            for (int idx = tid; idx < TM * (Dp / 4); idx += 256) {
+                const int r = idx & (TM - 1), c0 = (idx >> 7) * 8;
+                __align__(16) __nv_bfloat16 out[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const int c = c0 + e, j = c - 2 * n16;   // j: column of the remainder's steps
+                    int k = c < n16 ? c : c - n16;
+                    bool low = c >= n16;
+                    if (j >= 0) {
+                        const int third = j < rest ? 0 : (j < 2 * rest ? 1 : (j < 3 * rest ? 2 : 3));
+                        k = third < 3 ? n16 + j - third * rest : -1;
+                        low = third == (db_form ? 2 : 1);
+                    }
+                    float v = 0.0f;
+                    if (k >= 0) {
+                        v = db_form ? -2.0f * xs[r][k] : xs[r][k];
+                        const float hi = __bfloat162float(__float2bfloat16_rn(v));
+                        v = low ? v - hi : hi;
+                    } else if (j < 3 * rest + 3) {   // the norm in three pieces of 8 bits, against ones
+                        const float nf = s_nf[r], hi = __bfloat162float(__float2bfloat16_rn(nf));
+                        const int piece = j - 3 * rest;
+                        v = piece == 0 ? hi : (piece == 1 ? nf - hi : s_rest[r]);
+                        if (!db_form) v = s_row[r] >= 0 ? 1.0f : 0.0f;
+                    }
+                    out[e] = __float2bfloat16_rn(v);
+                }
+                *reinterpret_cast<uint4 *>(im_tile + image_offset_bf16(r, c0, sw)) = *reinterpret_cast<const uint4 *>(out);
+            }
+            break;
         }
         for (int idx = tid; idx < TM * (kPrepDims / 8); idx += 256) {
             const int r = idx & (TM - 1), o = (idx >> 7) * 8, k = k0 + o;
@@ -644,61 +683,61 @@ struct TcShared {
     int abort_flag;
 };
 
-// The MMAs of one accumulator tile: three products over NKS K steps, every descriptor a register plus a register.
-// NKS is a template argument so that the loops unroll into independent instruction sequences: one thread issues
+// The MMAs of one accumulator tile: three products over F K steps, then S K steps once (the packed remainder of bf16
+// images); off16: offsets of the image's K steps, hi, lo, remainder.  Every descriptor is a register plus a register.
+// F and S are template arguments so that the loops unroll into independent instruction sequences: one thread issues
 // every MMA of the block, and whatever it computes per MMA shows in the kernel's time.
-template <bool BF16, int NKS>
-__device__ __forceinline__ void tc_issue_products(uint32_t d_tmem, uint64_t a_hi, uint64_t a_lo, uint64_t b_hi, uint64_t b_lo,
-                                                  const uint32_t (&off16)[NKS])
+template <bool BF16, int F, int S>
+__device__ __forceinline__ void tc_issue_products(uint32_t d_tmem, uint64_t a, uint64_t b, const uint32_t (&off16)[2 * F + S])
 {
+    auto mma = [&](int i, int j, uint32_t accumulate) {
+        if (BF16) tc_mma_bf16(d_tmem, a + off16[i], b + off16[j], kInstrDescBf16, accumulate);
+        else tc_mma_tf32(d_tmem, a + off16[i], b + off16[j], kInstrDesc, accumulate);
+    };
 #pragma unroll
-    for (int ks = 0; ks < NKS; ks++) {      // hi . hi
-        if (BF16) tc_mma_bf16(d_tmem, a_hi + off16[ks], b_hi + off16[ks], kInstrDescBf16, ks ? 1u : 0u);
-        else tc_mma_tf32(d_tmem, a_hi + off16[ks], b_hi + off16[ks], kInstrDesc, ks ? 1u : 0u);
-    }
+    for (int ks = 0; ks < F; ks++) mma(ks, ks, ks ? 1u : 0u);      // hi . hi
 #pragma unroll
-    for (int ks = 0; ks < NKS; ks++) {      // lo . hi
-        if (BF16) tc_mma_bf16(d_tmem, a_lo + off16[ks], b_hi + off16[ks], kInstrDescBf16, 1u);
-        else tc_mma_tf32(d_tmem, a_lo + off16[ks], b_hi + off16[ks], kInstrDesc, 1u);
-    }
+    for (int ks = 0; ks < F; ks++) mma(F + ks, ks, 1u);            // lo . hi
 #pragma unroll
-    for (int ks = 0; ks < NKS; ks++) {      // hi . lo
-        if (BF16) tc_mma_bf16(d_tmem, a_hi + off16[ks], b_lo + off16[ks], kInstrDescBf16, 1u);
-        else tc_mma_tf32(d_tmem, a_hi + off16[ks], b_lo + off16[ks], kInstrDesc, 1u);
-    }
+    for (int ks = 0; ks < F; ks++) mma(ks, F + ks, 1u);            // hi . lo
+#pragma unroll
+    for (int ks = 0; ks < S; ks++) mma(2 * F + ks, 2 * F + ks, (F || ks) ? 1u : 0u);
 }
 
 // The MMA issuer's walk over the block's database tiles (one thread).  a16 / b16 / end16: the block's images in
 // 16-byte units of shared memory; span16: what one K step reads beyond its start.  Every tile's descriptors are
 // checked against that range before they are used (an MMA that reads outside the block's shared memory is a fault).
-template <int QH, bool BF16, int NKS, bool DIVIDED>
+template <int QH, bool BF16, int F, int S, bool DIVIDED>
 __device__ __noinline__ void tc_issue_walk(TcShared *shp, volatile int *abort_flag, TileWalk<DIVIDED> walk, uint32_t tmem_base, uint64_t no_addr,
                                            uint32_t a16, uint32_t b16, uint32_t image16, uint32_t spr_log, uint32_t block16,
                                            uint32_t in_row16, uint32_t span16, uint32_t end16)
 {
     TcShared &sh = *shp;
-    const uint32_t part16 = image16 >> 1, spr_mask = (1u << spr_log) - 1u;
-    uint32_t off16[NKS];
+    const uint32_t spr_mask = (1u << spr_log) - 1u;
+    uint32_t off16[2 * F + S];
+    uint32_t reach16 = 0;   // the furthest an image's K steps read
 #pragma unroll
-    for (int ks = 0; ks < NKS; ks++) off16[ks] = ((uint32_t)ks >> spr_log) * block16 + ((uint32_t)ks & spr_mask) * in_row16;
-    const uint32_t reach16 = off16[NKS - 1] + span16;   // the furthest a part's K steps read
+    for (int ks = 0; ks < 2 * F + S; ks++) {
+        off16[ks] = ((uint32_t)ks >> spr_log) * block16 + ((uint32_t)ks & spr_mask) * in_row16;
+        reach16 = max(reach16, off16[ks] + span16);
+    }
     int tile;
     for (long long t = 0; walk.next(tile); t++) {
-        const int s = (int)(t % kBStages), b = (int)(t % kAccBufs);
+        const int s = (int)(t % kBStages), acc = (int)(t % kAccBufs);
         const uint32_t ph_s = (uint32_t)((t / kBStages) & 1), ph_b = (uint32_t)((t / kAccBufs) & 1);
-        if (!mbar_wait(&sh.acc_empty[b], ph_b ^ 1u, abort_flag)) break;
+        if (!mbar_wait(&sh.acc_empty[acc], ph_b ^ 1u, abort_flag)) break;
         if (!mbar_wait(&sh.full_b[s], ph_s, abort_flag)) break;
         tc_fence_after();
         const uint32_t bs16 = b16 + (uint32_t)s * image16;
-        if (reach16 > part16 || a16 + QH * image16 > b16 || bs16 + image16 > end16) { *abort_flag = 1; break; }
-        const uint64_t b_hi = no_addr + (uint64_t)bs16, b_lo = b_hi + part16;
+        if (reach16 > image16 || a16 + QH * image16 > b16 || bs16 + image16 > end16) { *abort_flag = 1; break; }
+        const uint64_t b = no_addr + (uint64_t)bs16;
 #pragma unroll
         for (int h = 0; h < QH; h++) {
-            const uint64_t a_hi = no_addr + (uint64_t)(a16 + (uint32_t)h * image16), a_lo = a_hi + part16;
-            tc_issue_products<BF16, NKS>(tmem_base + (uint32_t)((b * QH + h) * TN), a_hi, a_lo, b_hi, b_lo, off16);
+            const uint64_t a = no_addr + (uint64_t)(a16 + (uint32_t)h * image16);
+            tc_issue_products<BF16, F, S>(tmem_base + (uint32_t)((acc * QH + h) * TN), a, b, off16);
         }
         tc_commit(&sh.empty_b[s]);    // the stage may be refilled once these MMAs have read it
-        tc_commit(&sh.acc_full[b]);   // the accumulator tiles are complete
+        tc_commit(&sh.acc_full[acc]);   // the accumulator tiles are complete
     }
 }
 
@@ -718,10 +757,10 @@ __global__ void __launch_bounds__(tc_threads(QH), 1)
 knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ img_db, int Dp, long long nq, long long nd_pos,
                      const int2 *__restrict__ segs, const int *__restrict__ nseg, int seg_stride, int tile_stride, int win_lo,
                      int win_hi, const float *__restrict__ tau, int cap, uint2 *cand, int *counts,
-                     int *error_flag, int bf16, int sw, int nks, ScanParts parts, int rank = 0, float *__restrict__ rank_out = nullptr)
+                     int *error_flag, int bf16, int sw, int nks, int n_rest, ScanParts parts, int rank = 0, float *__restrict__ rank_out = nullptr)
 {
     // bf16: the images hold bf16 pairs; sw != 0: in swizzled rows of sw bytes (else core matrices without swizzle);
-    // nks: K steps of 32 operand bytes per row to multiply
+    // nks: K steps of 32 operand bytes per row to multiply threefold, n_rest: once (packed remainder)
     constexpr int kProducerWarp = 8 * QH, kMmaWarp = 8 * QH + 1;
     constexpr uint32_t kTmemCols = kAccBufs * QH * TN;
     extern __shared__ __align__(1024) unsigned char smem[];   // swizzled images want their 8-row groups on 8 * sw bytes
@@ -794,16 +833,25 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
             const uint32_t a16 = smem_u32(sA) >> 4, b16 = smem_u32(sB) >> 4, image16 = image_bytes >> 4;
             const uint32_t end16 = (smem_u32(smem) + (uint32_t)(QH + kBStages) * image_bytes) >> 4;
             const TileWalk<SHARED> walk(my_segs, my_nseg, tile_stride, win_lo, win_hi, part, parts);
-#define B200_ISSUE(NKS_)                                                                                                        \
-    case NKS_:                                                                                                                  \
-        if (bf16) tc_issue_walk<QH, true, NKS_, SHARED>(&sh, abort_flag, walk, tmem_base, no_addr, a16, b16, image16, spr_log, block16,  \
-                                                in_row16, span16, end16);                                                       \
-        else tc_issue_walk<QH, false, NKS_, SHARED>(&sh, abort_flag, walk, tmem_base, no_addr, a16, b16, image16, spr_log, block16,      \
-                                            in_row16, span16, end16);                                                           \
+#define B200_ISSUE(BF16_, F_, S_)                                                                                               \
+    case (F_) * 4 + (S_):                                                                                                       \
+        tc_issue_walk<QH, BF16_, F_, S_, SHARED>(&sh, abort_flag, walk, tmem_base, no_addr, a16, b16, image16, spr_log, block16, \
+                                                 in_row16, span16, end16);                                                      \
         break;
-            switch (nks) {
-                B200_ISSUE(1) B200_ISSUE(2) B200_ISSUE(3) B200_ISSUE(4) B200_ISSUE(5) B200_ISSUE(6) B200_ISSUE(7) B200_ISSUE(8)
-                default: sh.abort_flag = 1; break;   // more K steps than a narrow image holds
+            if (bf16) {
+                switch (nks * 4 + n_rest) {
+                    B200_ISSUE(true, 0, 1) B200_ISSUE(true, 0, 2) B200_ISSUE(true, 0, 3)
+                    B200_ISSUE(true, 1, 1) B200_ISSUE(true, 1, 2) B200_ISSUE(true, 1, 3)
+                    B200_ISSUE(true, 2, 1) B200_ISSUE(true, 2, 2) B200_ISSUE(true, 2, 3)
+                    B200_ISSUE(true, 3, 1) B200_ISSUE(true, 3, 2) B200_ISSUE(true, 3, 3)
+                    default: sh.abort_flag = 1; break;   // more K steps than a narrow image holds
+                }
+            } else {
+                switch (nks * 4 + n_rest) {
+                    B200_ISSUE(false, 1, 0) B200_ISSUE(false, 2, 0) B200_ISSUE(false, 3, 0) B200_ISSUE(false, 4, 0)
+                    B200_ISSUE(false, 5, 0) B200_ISSUE(false, 6, 0) B200_ISSUE(false, 7, 0) B200_ISSUE(false, 8, 0)
+                    default: sh.abort_flag = 1; break;
+                }
             }
 #undef B200_ISSUE
         }
@@ -1767,7 +1815,8 @@ struct TcWorkspace {
     bool wide, bf16;
     size_t image_bytes;        // one tile's image (hi and lo)
     int Dp;
-    int sw, nks;               // narrow kernel: bytes of a swizzled image row (0: core matrices without swizzle), K steps
+    int sw, nks, n_rest;       // bytes of a swizzled image row (0: core matrices without swizzle), K steps of the narrow kernel
+    int whole;                 // full groups of 16 dimensions of a packed image, -1: not packed
     long long tq, td;          // tiles allocated for the query list / the database list
     float *img_q, *img_db;
     double *norms_q;
@@ -1792,13 +1841,15 @@ static TcWorkspace tc_carve(void *base, int D, int K, long long nq, long long nd
     w.wide = tc_wide(D);
     w.bf16 = tc_bf16();
     // one extra inner column carries the norm (two in bf16); wide points are chunked along the inner dimension
-    w.sw = 0;
+    w.sw = w.n_rest = 0;
+    w.whole = w.bf16 && !w.wide ? D / 16 : -1;
     if (w.bf16 && !w.wide) {
-        // swizzled rows of 32, 64 or 128 bytes (16, 32 or 64 values); more inner dimensions: blocks of 128-byte rows
-        const int need = D + 2;
-        w.sw = need <= 16 ? 32 : (need <= 32 ? 64 : 128);
-        w.Dp = (need + w.sw / 2 - 1) / (w.sw / 2) * (w.sw / 2);
-        w.nks = (need + 15) / 16;
+        // packed K steps of 16 columns in swizzled rows of 32, 64 or 128 bytes; more of them: blocks of 128-byte rows
+        w.nks = D / 16;
+        w.n_rest = (3 * (D % 16) + 3 + 15) / 16;
+        const int steps = 2 * w.nks + w.n_rest;
+        w.sw = steps == 1 ? 32 : (steps == 2 ? 64 : 128);
+        w.Dp = (steps * 32 + w.sw - 1) / w.sw * w.sw / 4;   // half the columns
     } else if (w.bf16) {
         w.sw = kWideSwizzle;
         w.Dp = (D + 2 + 2 * kWideKC - 1) / (2 * kWideKC) * (2 * kWideKC);
@@ -1955,9 +2006,9 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     float *const xp = cells > 1 ? w.xp : nullptr;
     B200_CUDA(cudaGetLastError());
     if (bf16) {
-        knn_tc_prepare_bf16_kernel<<<(unsigned)w.tq, 256, 0, st>>>(X, w.qlist, D, Dp, KC, w.sw, 0, reinterpret_cast<__nv_bfloat16 *>(w.img_q),
+        knn_tc_prepare_bf16_kernel<<<(unsigned)w.tq, 256, 0, st>>>(X, w.qlist, D, Dp, KC, w.sw, w.whole, 0, reinterpret_cast<__nv_bfloat16 *>(w.img_q),
                                                                    w.norms_q, w.res_q, nullptr, nullptr);
-        knn_tc_prepare_bf16_kernel<<<(unsigned)w.td, 256, 0, st>>>(X, w.dblist, D, Dp, KC, w.sw, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_db),
+        knn_tc_prepare_bf16_kernel<<<(unsigned)w.td, 256, 0, st>>>(X, w.dblist, D, Dp, KC, w.sw, w.whole, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_db),
                                                                    nullptr, nullptr, counters + 4, xp);
     } else {
         knn_tc_prepare_kernel<<<(unsigned)w.tq, 128, 0, st>>>(X, w.qlist, D, Dp, KC, 0, w.img_q, w.norms_q);
@@ -2018,7 +2069,7 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
             else
                 narrow<<<grid, tc_threads(QH), smem, st>>>(
                     w.img_q, w.img_db, Dp, nq, nd_pos, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand, counts,
-                    counters + 0, bf16, w.sw, w.nks, parts, 0, nullptr);
+                    counters + 0, bf16, w.sw, w.nks, w.n_rest, parts, 0, nullptr);
             B200_CUDA(cudaGetLastError());
         }
         return 0;
@@ -2058,7 +2109,7 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
         const int ts = wide ? (m_a + kWideUnit - 1) / kWideUnit * 2 : (m_a + TN - 1) / TN;
         knn_sample_list_kernel<<<(unsigned)((ts * TN + 255) / 256), 256, 0, st>>>(w.slist, (long long)ts * TN, m_a, db_lo, a_stride);
         if (bf16)
-            knn_tc_prepare_bf16_kernel<<<(unsigned)ts, 256, 0, st>>>(X, w.slist, D, Dp, KC, w.sw, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_s),
+            knn_tc_prepare_bf16_kernel<<<(unsigned)ts, 256, 0, st>>>(X, w.slist, D, Dp, KC, w.sw, w.whole, 1, reinterpret_cast<__nv_bfloat16 *>(w.img_s),
                                                                      nullptr, nullptr, nullptr, nullptr);
         else
             knn_tc_prepare_kernel<<<(unsigned)ts, 128, 0, st>>>(X, w.slist, D, Dp, KC, 1, w.img_s, nullptr);
@@ -2075,7 +2126,7 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
             B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
             knn_tc_filter_kernel<1, true, false><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
                 w.img_q, w.img_s, Dp, nq, (long long)m_a, w.segs, w.nseg, 0, 1, 0, ts, nullptr, 0, nullptr, nullptr, counters + 0,
-                bf16, w.sw, w.nks, ScanParts(), rank_a, tau);
+                bf16, w.sw, w.nks, w.n_rest, ScanParts(), rank_a, tau);
         }
         B200_CUDA(cudaGetLastError());
         knn_single_segment_kernel<<<1, 1, 0, st>>>(w.segs, w.nseg, all_tiles);   // back to all database tiles
