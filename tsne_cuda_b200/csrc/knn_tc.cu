@@ -30,16 +30,11 @@
 // step 128 bytes apart; 8-row groups 256 bytes apart).  A tile is therefore ONE contiguous bulk
 // copy (cp.async.bulk + mbarrier complete_tx) with no tensor map and no swizzle.
 //
-// Thresholds.  For a small database the threshold is maintained online: the L-th best key at the last
-// compaction of the query's buffer (a warp-wide bitonic sort).  That appends about L ln(N/L) candidates per
-// query, which is rare per thread but not per warp of 32 queries, and each compaction costs thousands of
-// issue slots.  For a large database (>= 512 tiles) the threshold is therefore FIXED per query, in three
-// levels, each sizing the candidate set of the next: (A) on the CUDA cores, the key of rank ~10 among a
-// few thousand jittered sample points; (B) every 16th tile against tau_A (~300 candidates); (C) all
-// tiles against tau_B = the key of rank ~3L/16 of sample B, which about 3L points beat.  Nothing is
-// compacted during a fixed-threshold scan; the L best are selected once at the end (by bisection on the
-// key bits, not by sorting).  A row whose buffer
-// overflows or ends with fewer than L candidates is flagged and recomputed by the SIMT search.
+// Thresholds are FIXED per query before the scan that uses them.  Up to 393,216 rows a sample (16 N / 3 L points, spread over
+// the database and scanned with a top-16 epilogue in registers) sets it at the key of rank ~16; beyond, in two further
+// steps: every 16th tile against the sample's threshold (~300 candidates), then all tiles against the key of rank
+// ~3L/16 of those, which about 3L points beat.  Nothing is compacted during a scan; the re-rank picks from the buffer by
+// bisection on the key bits.  A row whose buffer overflows or ends with too few candidates is recomputed.
 //
 // Epilogue: a thread first reduces its 32 keys of a chunk to their minimum (a tree of independent
 // min operations); only if that minimum beats the threshold, which becomes rare as the scan
@@ -54,9 +49,10 @@
 // that) against every database tile, so a database image is fetched from L2 once per 256 queries.
 // Warps 0 .. 8 QH - 1 are the epilogue, in 2 QH groups of four (TMEM lane quarter = warp % 4), then the
 // bulk-copy producer warp and the MMA issuer / TMEM owner warp.  Two database stages and two accumulator
-// buffers (of QH tiles each), so the MMAs of tile t+1 overlap the epilogue of tile t.  Measured on the
-// full pass at N = 10^6, D = 50: with the epilogue's comparisons removed the kernel takes 89 % of its
-// time, i.e. it is bound by the tensor pipe (42 MMAs 128x128x8 per tile pair at ~105 cycles each).
+// buffers (of QH tiles each), so the MMAs of tile t+1 overlap the epilogue of tile t.  Measured at 400,000 x 50 before the
+// last change of the epilogue: issue slots 77 % busy (390 instructions per MMA, most of them survivors' stores in divergent
+// warps), tensor pipe 50 %: the epilogue bounds the narrow kernel; the wide one runs at the tensor pipe's rate
+// (50,000 x 1,024: 15.4 TFLOP in 10.4 ms).
 // Every wait has a time limit; on expiry the kernel sets an error flag, drains and frees its TMEM.
 #include <limits.h>
 #include <stdio.h>
@@ -752,7 +748,8 @@ __device__ __noinline__ void tc_issue_walk(TcShared *shp, volatile int *abort_fl
 // registers and rank_out[query] receives the one of rank `rank` (0-based, < 16) when the scan ends: the first
 // threshold level, a scan of a few thousand sample points.
 // SHARED: the tiles of a block of queries are dealt to gridDim.y blocks, which append to the same buffers (take_slots).
-template <int QH, bool RANKED, bool SHARED>
+// SPARSE: survivors are rare (see the dispatch).
+template <int QH, bool RANKED, bool SHARED, bool SPARSE>
 __global__ void __launch_bounds__(tc_threads(QH), 1)
 knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ img_db, int Dp, long long nq, long long nd_pos,
                      const int2 *__restrict__ segs, const int *__restrict__ nseg, int seg_stride, int tile_stride, int win_lo,
@@ -917,11 +914,11 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     if (m4[q] < thr) {
+                        if constexpr (RANKED) {
 #pragma unroll
-                        for (int e = 0; e < 8; e++) {
-                            const int c = q * 8 + e;
-                            const float key = __uint_as_float(r[c]);
-                            if constexpr (RANKED) {
+                            for (int e = 0; e < 8; e++) {
+                                const int c = q * 8 + e;
+                                const float key = __uint_as_float(r[c]);
                                 if (key < thr && (tile_inside || col0 + c < nd_pos)) {   // replaces the largest of the 16 and sinks to its place
                                     top[15] = key;
 #pragma unroll
@@ -932,9 +929,25 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
                                     }
                                     thr = top[15];
                                 }
-                            } else if (key < thr) {   // padding rows carry a huge norm and never pass (kTauLimit)
-                                __stcg(next, make_uint2(r[c], (unsigned)col0 + c));
+                            }
+                        } else {   // padding rows carry a huge norm and never pass (kTauLimit)
+                            unsigned which = 16u;   // 8 + index of the survivor when there is one, 16 or more when there are several
+                            if constexpr (SPARSE) {
+                                which = 0u;
+#pragma unroll
+                                for (int e = 0; e < 8; e++) which += __uint_as_float(r[q * 8 + e]) < thr ? 8u + e : 0u;
+                            }
+                            if (SPARSE && which < 16u) {   // its key is the minimum
+                                __stcg(next, make_uint2(__float_as_uint(m4[q]), (unsigned)col0 + q * 8 - 8 + which));
                                 next++;
+                            } else {
+#pragma unroll
+                                for (int e = 0; e < 8; e++) {
+                                    if (__uint_as_float(r[q * 8 + e]) < thr) {
+                                        __stcg(next, make_uint2(r[q * 8 + e], (unsigned)col0 + q * 8 + e));
+                                        next++;
+                                    }
+                                }
                             }
                         }
                     }
@@ -2056,8 +2069,12 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
         const ScanParts parts = scan_parts(blocks, (int)((std::min(tiles, win) + stride - 1) / stride), wide ? (63 + Dp / KC) / (Dp / KC) : 32,
                                             wide || 2 * blocks <= sm_count ? 16 : 1, sm_count);
         const dim3 grid((unsigned)blocks, (unsigned)parts.most);
-        auto narrow = parts.most > 1 ? (QH == 1 ? knn_tc_filter_kernel<1, false, true> : knn_tc_filter_kernel<2, false, true>)
-                                : (QH == 1 ? knn_tc_filter_kernel<1, false, false> : knn_tc_filter_kernel<2, false, false>);
+        // SPARSE: survivors so rare that eight keys with one mostly hold no second: one store behind a search for its place
+        // (scan of 10^6 x 50: 60.0 -> 54.6 ms, 300 000 x 20: 4.29 -> 3.72); below, a test and a store per key are faster
+        // (30 011 x 32, one key in eight passes: 0.29 against 0.33)
+        auto narrow = parts.most > 1 ? (QH == 1 ? knn_tc_filter_kernel<1, false, true, false> : knn_tc_filter_kernel<2, false, true, false>)
+                      : nd >= 131072 ? (QH == 1 ? knn_tc_filter_kernel<1, false, false, true> : knn_tc_filter_kernel<2, false, false, true>)
+                                     : (QH == 1 ? knn_tc_filter_kernel<1, false, false, false> : knn_tc_filter_kernel<2, false, false, false>);
         if (wide) B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         else B200_CUDA(cudaFuncSetAttribute(narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         for (long long lo = 0; lo < tiles; lo += win) {
@@ -2123,8 +2140,8 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
                 ScanParts(), rank_a, tau, (long long)m_a);
         } else {
             const size_t smem_a = (size_t)(1 + kBStages) * w.image_bytes;
-            B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
-            knn_tc_filter_kernel<1, true, false><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
+            B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+            knn_tc_filter_kernel<1, true, false, false><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
                 w.img_q, w.img_s, Dp, nq, (long long)m_a, w.segs, w.nseg, 0, 1, 0, ts, nullptr, 0, nullptr, nullptr, counters + 0,
                 bf16, w.sw, w.nks, w.n_rest, ScanParts(), rank_a, tau);
         }
