@@ -748,13 +748,13 @@ __device__ __noinline__ void tc_issue_walk(TcShared *shp, volatile int *abort_fl
 // registers and rank_out[query] receives the one of rank `rank` (0-based, < 16) when the scan ends: the first
 // threshold level, a scan of a few thousand sample points.
 // SHARED: the tiles of a block of queries are dealt to gridDim.y blocks, which append to the same buffers (take_slots).
-// SPARSE: survivors are rare (see the dispatch).
-template <int QH, bool RANKED, bool SHARED, bool SPARSE>
+// sparse: survivors are rare (see the dispatch).
+template <int QH, bool RANKED, bool SHARED>
 __global__ void __launch_bounds__(tc_threads(QH), 1)
 knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ img_db, int Dp, long long nq, long long nd_pos,
                      const int2 *__restrict__ segs, const int *__restrict__ nseg, int seg_stride, int tile_stride, int win_lo,
                      int win_hi, const float *__restrict__ tau, int cap, uint2 *cand, int *counts,
-                     int *error_flag, int bf16, int sw, int nks, int n_rest, ScanParts parts, int rank = 0, float *__restrict__ rank_out = nullptr)
+                     int *error_flag, int bf16, int sw, int nks, int n_rest, ScanParts parts, int sparse, int rank = 0, float *__restrict__ rank_out = nullptr)
 {
     // bf16: the images hold bf16 pairs; sw != 0: in swizzled rows of sw bytes (else core matrices without swizzle);
     // nks: K steps of 32 operand bytes per row to multiply threefold, n_rest: once (packed remainder)
@@ -932,12 +932,12 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
                             }
                         } else {   // padding rows carry a huge norm and never pass (kTauLimit)
                             unsigned which = 16u;   // 8 + index of the survivor when there is one, 16 or more when there are several
-                            if constexpr (SPARSE) {
+                            if (!SHARED && sparse) {
                                 which = 0u;
 #pragma unroll
                                 for (int e = 0; e < 8; e++) which += __uint_as_float(r[q * 8 + e]) < thr ? 8u + e : 0u;
                             }
-                            if (SPARSE && which < 16u) {   // its key is the minimum
+                            if (!SHARED && which < 16u) {   // its key is the minimum
                                 __stcg(next, make_uint2(__float_as_uint(m4[q]), (unsigned)col0 + q * 8 - 8 + which));
                                 next++;
                             } else {
@@ -2069,12 +2069,14 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
         const ScanParts parts = scan_parts(blocks, (int)((std::min(tiles, win) + stride - 1) / stride), wide ? (63 + Dp / KC) / (Dp / KC) : 32,
                                             wide || 2 * blocks <= sm_count ? 16 : 1, sm_count);
         const dim3 grid((unsigned)blocks, (unsigned)parts.most);
-        // SPARSE: survivors so rare that eight keys with one mostly hold no second: one store behind a search for its place
-        // (scan of 10^6 x 50: 60.0 -> 54.6 ms, 300 000 x 20: 4.29 -> 3.72); below, a test and a store per key are faster
-        // (30 011 x 32, one key in eight passes: 0.29 against 0.33)
-        auto narrow = parts.most > 1 ? (QH == 1 ? knn_tc_filter_kernel<1, false, true, false> : knn_tc_filter_kernel<2, false, true, false>)
-                      : nd >= 131072 ? (QH == 1 ? knn_tc_filter_kernel<1, false, false, true> : knn_tc_filter_kernel<2, false, false, true>)
-                                     : (QH == 1 ? knn_tc_filter_kernel<1, false, false, false> : knn_tc_filter_kernel<2, false, false, false>);
+        // sparse: survivors so rare that eight keys with one mostly hold no second: one store behind a search for its place
+        // (scan of 10^6 x 50: 60.0 -> 54.6 ms, 300 000 x 20: 4.30 -> 3.83); below, a test and a store per key
+        // (30 011 x 32, one key in eight passes: 0.30 -> 0.32 by the test for the flag, 0.33 with the search).  As an
+        // instantiation of its own the sparse form took 61 to 62 ms at 10^6 x 50, in every run: the kernel's code is large,
+        // and where it comes to lie counts.
+        const int sparse = nd >= 131072;
+        auto narrow = parts.most > 1 ? (QH == 1 ? knn_tc_filter_kernel<1, false, true> : knn_tc_filter_kernel<2, false, true>)
+                                     : (QH == 1 ? knn_tc_filter_kernel<1, false, false> : knn_tc_filter_kernel<2, false, false>);
         if (wide) B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         else B200_CUDA(cudaFuncSetAttribute(narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         for (long long lo = 0; lo < tiles; lo += win) {
@@ -2086,7 +2088,7 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
             else
                 narrow<<<grid, tc_threads(QH), smem, st>>>(
                     w.img_q, w.img_db, Dp, nq, nd_pos, w.segs, w.nseg, seg_stride, stride, (int)lo, hi, tau, cap, cand, counts,
-                    counters + 0, bf16, w.sw, w.nks, w.n_rest, parts, 0, nullptr);
+                    counters + 0, bf16, w.sw, w.nks, w.n_rest, parts, sparse, 0, nullptr);
             B200_CUDA(cudaGetLastError());
         }
         return 0;
@@ -2140,10 +2142,10 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
                 ScanParts(), rank_a, tau, (long long)m_a);
         } else {
             const size_t smem_a = (size_t)(1 + kBStages) * w.image_bytes;
-            B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
-            knn_tc_filter_kernel<1, true, false, false><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
+            B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+            knn_tc_filter_kernel<1, true, false><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
                 w.img_q, w.img_s, Dp, nq, (long long)m_a, w.segs, w.nseg, 0, 1, 0, ts, nullptr, 0, nullptr, nullptr, counters + 0,
-                bf16, w.sw, w.nks, w.n_rest, ScanParts(), rank_a, tau);
+                bf16, w.sw, w.nks, w.n_rest, ScanParts(), 0, rank_a, tau);
         }
         B200_CUDA(cudaGetLastError());
         knn_single_segment_kernel<<<1, 1, 0, st>>>(w.segs, w.nseg, all_tiles);   // back to all database tiles
