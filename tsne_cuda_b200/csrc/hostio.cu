@@ -225,6 +225,13 @@ cudaGraphExec_t graph_exec_acquire(StreamSet *s, cudaGraph_t graph, unsigned lon
     return exec;
 }
 
+bool graph_exec_kept(const StreamSet *s, unsigned long long shape)
+{
+    for (const auto &e : s->execs)
+        if (e.shape == shape) return true;
+    return false;
+}
+
 void graph_exec_release(StreamSet *s, cudaGraphExec_t exec, unsigned long long shape)
 {
     if (!s || s->execs.size() >= kMaxKeptExecs) cudaGraphExecDestroy(exec);

@@ -33,6 +33,7 @@ void stream_set_release(StreamSet *s);                 // waits for both streams
 
 // An executable for `graph`: a kept one of the same shape, updated, else a new one; null if neither can be had.
 cudaGraphExec_t graph_exec_acquire(StreamSet *s, cudaGraph_t graph, unsigned long long shape);
+bool graph_exec_kept(const StreamSet *s, unsigned long long shape);   // one of that shape waits to be updated
 void graph_exec_release(StreamSet *s, cudaGraphExec_t exec, unsigned long long shape);
 
 // Copies between pageable host memory and the device on `st`.  Large ones go through pinned chunks filled (or emptied)

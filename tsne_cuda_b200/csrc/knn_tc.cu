@@ -9,7 +9,7 @@
 //     query operand is [x_i, 1], the database operand [-2 x_j, |x_j|^2] (padding columns of the inner
 //     dimension carry the norm), each value split in a pair v = hi + lo and multiplied as three products
 //     hi.hi + lo.hi + hi.lo accumulated in fp32 in TMEM.  By default the pairs are bf16 (kind::f16, K steps
-//     of 16, keys accurate to 3 * 2^-16 of sum_k |x_ik||2 x_jk|; the norm travels in two column pairs);
+//     of 16, keys accurate to 3 * 2^-16 of sum_k |x_ik||2 x_jk|; the norm travels in three or four columns);
 //     B200TSNE_KNN_FILTER=tf32 selects TF32 pairs (K steps of 8, about 2^-20 of |x_i||x_j|) at nearly twice
 //     the tensor-core time.  Either error is covered by the proof of step 3.  A block owns 256 queries (one
 //     TMEM lane each per query tile) and
@@ -22,13 +22,12 @@
 //     canonical distance >= (|x_i|^2 + T - E)(1 - theta) with E bounding the filter's error and theta the
 //     rounding of the canonical sum.  If the K-th candidate distance is strictly below that bound the
 //     first K candidates are provably the exact answer; otherwise the row is flagged and recomputed by
-//     the SIMT search.  The observed filter error on the candidates is checked against E as well.
+//     an exact search.  The observed filter error on the candidates is checked against E as well.
 //
-// Operand staging: the prepared operands live in global memory as ready-made shared-memory images,
-// one per 128-row tile: for hi then lo, for every 8-wide K step, the 128 x 8 block in the
-// no-swizzle K-major core-matrix order (8 rows x 16 bytes contiguous; the two 16-byte halves of a K
-// step 128 bytes apart; 8-row groups 256 bytes apart).  A tile is therefore ONE contiguous bulk
-// copy (cp.async.bulk + mbarrier complete_tx) with no tensor map and no swizzle.
+// Operand staging: the prepared operands live in global memory as ready-made shared-memory images, one per 128-row tile
+// (and chunk of the inner dimension for wide points), bf16 pairs in swizzled rows, TF32 pairs in no-swizzle core matrices
+// (8 rows x 16 bytes contiguous; the two 16-byte halves of a K step 128 bytes apart; 8-row groups 256 bytes apart).  A
+// tile is therefore ONE contiguous bulk copy (cp.async.bulk + mbarrier complete_tx) with no tensor map.
 //
 // Thresholds are FIXED per query before the scan that uses them.  Up to 393,216 rows a sample (16 N / 3 L points, spread over
 // the database and scanned with a top-16 epilogue in registers) sets it at the key of rank ~16; beyond, in two further

@@ -448,8 +448,9 @@ int Session::graph_block(int remaining) const
     return px ? 0 : 1;
 }
 
-// 0: done.  1: not captured, the caller launches directly.  Negative: error.
-int Session::run_graph_block(int iters, int norm_mode, float stop_norm)
+// 0: done, `iters` iterations of at most the number asked for.  1: not captured, the caller launches directly.  Negative:
+// error.  remaining: iterations left in the call.
+int Session::run_graph_block(int &iters, int remaining, int norm_mode, float stop_norm)
 {
     const bool late = step >= force_magnify_iters;
     IterGraph key;
@@ -469,6 +470,13 @@ int Session::run_graph_block(int iters, int norm_mode, float stop_norm)
     IterGraph *g = nullptr;
     for (IterGraph &have : graphs)
         if (have.same(key)) g = &have;
+    if (!g && !graph_exec_kept(host, key.shape())) {
+        if (iters == kGraphIters && remaining < kLargeFrom) {
+            iters = 2;
+            return run_graph_block(iters, remaining, norm_mode, stop_norm);
+        }
+        if (iters == 1 && remaining > 1) return 1;   // the odd one before a block: an executable would serve it alone
+    }
     if (!g) {
         if (graphs.size() >= kMaxGraphs) drop_graphs();
         // capture: the launches are recorded, not run, so the host-side counters are put back afterwards
@@ -521,7 +529,7 @@ int Session::iterate(int n_iters, float min_gradient_norm, float *elapsed_ms, in
         int block = (early_stop && multi) || (norm_mode == 1) ? 0 : graph_block(n_iters - it);
         const int step0 = step;
         if (block > 0) {
-            const int rc = run_graph_block(block, norm_mode, min_gradient_norm);
+            const int rc = run_graph_block(block, n_iters - it, norm_mode, min_gradient_norm);
             if (rc < 0) return rc;
             if (rc != 0) block = 0;
         }

@@ -118,12 +118,15 @@ struct Session {
         }
     };
     static constexpr int kGraphIters = 16;   // iterations of a large block; what is left of a phase goes in pairs
+    // A large block's first executable of a process costs 3 to 20 ms: calls of fewer iterations go in pairs until one exists
+    // (20 iterations at 10^6 points after a warm-up of 3: 23.3 ms with it, 5.6 in pairs).
+    static constexpr int kLargeFrom = 64;
     static constexpr size_t kMaxGraphs = 24;
     std::vector<IterGraph> graphs;
     bool use_graphs = true;   // B200TSNE_GRAPHS=0 turns them off
     int refresh_period(int at) const;   // iterations between two sorts of the spread order at step `at` (0: natural order)
     int graph_block(int remaining) const;
-    int run_graph_block(int iters, int norm_mode, float stop_norm);
+    int run_graph_block(int &iters, int remaining, int norm_mode, float stop_norm);
     int done_seen = 0;        // IterState::done as the host last saw it
     void drop_graphs();
 
