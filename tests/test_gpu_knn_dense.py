@@ -2,9 +2,14 @@
 tiles, of the keys a thread holds and of its segments, with exact ties, with fewer points than slots and for the rows the
 tensor-core search hands over."""
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
+
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +63,47 @@ def test_rows_handed_over_in_segments(engine, oracle_cpu, n, k):
     for lo in (0, n // 2 - 20, n - 60):
         ids_o, d2_o = oracle_cpu.knn(X, k, q_lo=lo, q_hi=lo + 60)
         assert np.array_equal(ids[lo:lo + 60], ids_o) and np.array_equal(d2[lo:lo + 60], d2_o)
+
+
+@pytest.mark.parametrize("n", [12288, 12289, 20011, 30000])
+def test_rows_without_neighbours(n):
+    """A row of NaN has no neighbours at any size: ids -1, distances +inf, in memory filled with other bits before (in a
+    process of its own).  Nor does it change the others' affinities, which scale by 1 / 2N."""
+    code = """
+import numpy as np
+from tsne_cuda_b200 import _lib as e
+n, k = %d, 30
+X = np.random.default_rng(n).normal(0, 1, (n, 20)).astype(np.float32)
+X[-1] = np.nan
+ids, d2 = e.knn(X, k)
+assert (ids[-1] == -1).all() and np.isposinf(d2[-1]).all(), (ids[-1], d2[-1])
+ids_r, d2_r = e.knn(X[:-1], k)
+assert np.array_equal(ids[:-1], ids_r) and np.array_equal(d2[:-1], d2_r)
+P = []
+for x in (X, X[:-1]):
+    with e.Session(len(x), k) as s:
+        s.affinities_from_points(x, 10.0, 1e-4)
+        P.append(s.get_affinities()[0][:n - 1].astype(np.float64) * len(x))
+assert np.isfinite(P[0]).all() and np.abs(P[0] - P[1]).max() <= 2e-7 * P[1].max()
+Y, Z = e.fit(X, num_neighbors=k, perplexity=10.0, iterations=20, random_seed=1)
+assert np.isfinite(Y).all()
+""" % n
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT, timeout=120, env=dict(os.environ, B200TSNE_POISON="1"))
+
+
+def test_infinitely_far_neighbours_in_segments(engine):
+    """Distances beyond the range of floats rank by id behind the finite ones, and before the slots that a segment of
+    nothing but NaN leaves empty."""
+    n, k, lo, hi = 25000, 24, 13000, 13040
+    X = np.random.default_rng(2).normal(0, 1, (n, 8)).astype(np.float32) * np.float32(1e20)   # squared differences overflow
+    X[:12500] = np.nan
+    X[lo + 5] = X[lo + 4]
+    ids, d2 = engine.knn(X, k, q_lo=lo, q_hi=hi)
+    with np.errstate(over="ignore", invalid="ignore"):
+        dist = np.zeros((hi - lo, n), np.float32)
+        for d in range(8):
+            t = X[lo:hi, None, d] - X[None, :, d]
+            dist += t * t
+    want = np.argsort(dist, axis=1, kind="stable")[:, :k]    # NaN last, equal distances by index
+    assert np.array_equal(ids, want) and np.array_equal(d2, np.take_along_axis(dist, want, 1))
+    assert (np.isfinite(d2).sum(1) < 4).all()

@@ -105,7 +105,8 @@ constexpr int kMaxDenseK = 512;
 // One block per (query, segment).  The n values of segment s of query q start at val + q * ld + s * seg; with `ids` they
 // carry the ids at the same place (equal values in ascending order of id), else value j has id id_lo + s * seg + j.  The K
 // smallest by (value, id), ascending, go to out row (q * segments + s), or, with out_rows, to row out_rows[q] - out_base;
-// slots without a value get (+inf, INT_MAX).  KPT * 256 >= seg.
+// slots without a value get (+inf, INT_MAX), and where such slots of shorter lists come in again (ids given) they are no
+// values: a neighbour infinitely far away is one, and precedes them.  KPT * 256 >= seg.
 template <int KPT>
 __global__ void __launch_bounds__(kThreads)
 dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ ids, long long ld, long long n_total, long long seg, int id_lo,
@@ -126,6 +127,7 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
     for (int j = 0; j < KPT; j++) {
         const int e = j * kThreads + tid;
         key[j] = e < n ? __float_as_uint(val[base + e]) : 0xffffffffu;
+        if (ids && key[j] == kInfBits && ids[base + e] == INT_MAX) key[j] = 0xffffffffu;
         if (key[j] <= kInfBits) { lo = min(lo, key[j]); hi = max(hi, key[j]); valid++; }
     }
     lo = __reduce_min_sync(0xffffffffu, lo);
