@@ -268,3 +268,14 @@ def test_knn_tensor_core_exact_whatever_the_norms(engine, monkeypatch, shift, sc
     b = engine.knn(X, 30)
     assert engine.knn_last_stats()["tensor_core"] == 0
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("n,spread,offset", [(300, 3.0, 0.0), (2000, 60.0, 300.0), (20011, 10.0, 50.0), (20011, 1e-4, 0.0)])
+def test_normalisation_sums_the_grid_in_double(engine, n, spread, offset):
+    """Z + N is the bilinear form of the charges and potentials that the call hands out, whose terms are of order |y|^2
+    and cancel: evaluated in double, what is left is the rounding of Z + N and of Z to float."""
+    Y = (np.random.default_rng(n).normal(0, spread, (2, n)) + offset).astype(np.float32)
+    _, Z, w, yt = engine.repulsive(Y, True)
+    w, yt = w.astype(np.float64), yt.astype(np.float64)
+    z = ((w[..., 0] + w[..., 3]) * yt[..., 0] - 2 * w[..., 1] * yt[..., 1] - 2 * w[..., 2] * yt[..., 2] + w[..., 0] * yt[..., 3]).sum()
+    assert abs((Z + n) - z) <= 2.0 ** -23 * z

@@ -369,9 +369,10 @@ fft_rows_inverse_kernel(const float4 *__restrict__ B, float4 *__restrict__ w, fl
             out[2 * j] = p;
             // node = (x, y, count, r^2) charges and potentials:
             // pot.count (w.count + w.r2) - 2 (pot.x w.x + pot.y w.y) + pot.r2 w.count
+            // The two planes' terms are of order |y|^2 and cancel down to Z: products and sums in double.
             const float2 q = reinterpret_cast<const float2 *>(charge + j)[plane];
-            // (products rounded to float like the points' own Z_i were, the sum in double)
-            z += (double)(plane == 0 ? -2.0f * fmaf(p.x, q.x, p.y * q.y) : fmaf(p.x, q.x + q.y, p.y * q.x));
+            const double px = p.x, py = p.y, qx = q.x, qy = q.y;
+            z += plane == 0 ? -2.0 * fma(px, qx, py * qy) : fma(px, qx + qy, py * qx);
         }
     }
 #pragma unroll
