@@ -175,12 +175,8 @@ __device__ __forceinline__ float kernel_value(int row, int j, float h, float cmi
     // node coordinates in float exactly as the reference forms them, summed and inverted in double (nbodyfft.cu:175-195)
     const float x1 = cmin + h / 2, y1 = cmin + h / 2 + row * h, y2 = cmin + h / 2 + j * h;
     const float da = x1 - y1, db = x1 - y2;
-    const double s = 1.0 + (double)(da * da) + (double)(db * db), t = s * s;
-    if (t > 1e37) return (float)(1.0 / t);
-    // 1 / t by one Newton step from the float reciprocal: 2^-44 from exact before the rounding to float (a double
-    // division is thirty dependent instructions, and a lane evaluates 28 of these)
-    const double r = (double)__fdividef(1.0f, (float)t);
-    return (float)fma(r, fma(-t, r, 1.0), r);
+    const double s = 1.0 + (double)(da * da) + (double)(db * db);
+    return (float)(1.0 / (s * s));
 }
 // completes a lane's half of an even sequence: v[r], r < 14, holds x[28 r + l]; the rest is x[784 - (28 r + l)]
 __device__ __forceinline__ void mirror_input(float2 (&v)[kR], int lane)
