@@ -245,9 +245,10 @@ int launch_perplexity(const float *d2, int64_t n_rows, int K, float perplexity, 
 {
     if (n_rows <= 0) return 0;
     const size_t smem = (size_t)kPerpWarps * K * sizeof(float);
-    if (smem > 200 * 1024) { set_error("perplexity: num_neighbors too large for the shared-memory row buffer"); return -4; }
-    if (smem > 48 * 1024)
-        B200_CUDA(cudaFuncSetAttribute(perplexity_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr size_t most = 200 * 1024;
+    if (smem > most) { set_error("perplexity: num_neighbors too large for the shared-memory row buffer"); return -4; }
+    // always to the most: another thread may be between this and its launch
+    if (smem > 48 * 1024) B200_CUDA(cudaFuncSetAttribute(perplexity_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     perplexity_kernel<<<nblk(n_rows, kPerpWarps), kPerpWarps * 32, smem, st>>>(d2, n_rows, K, perplexity, eps, max_enc, p,
                                                                               betas);
     B200_CUDA(cudaGetLastError());

@@ -1398,6 +1398,9 @@ __host__ __device__ constexpr int rerank_stride(int D) { const int d = D <= kRer
 // addresses
 __host__ __device__ constexpr size_t rerank_floats(int D, int L) { return (size_t)(D <= kRerankWhole ? 1 : 2) * 33 * rerank_stride(D) + 4 * (size_t)L + 68; }
 
+__host__ __device__ constexpr size_t rerank_floats_max(int L) { return rerank_floats(kRerankWhole + 1, L); }
+static_assert(rerank_floats_max(0) >= rerank_floats(kRerankWhole, 0), "rows that are walked take the most");
+
 template <int BYTES> __device__ __forceinline__ void async_copy(void *dst, const void *src)
 {
     if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
@@ -1811,6 +1814,16 @@ static bool tc_bf16()
 }
 
 // nd: database rows the search will scan
+// The limit of a kernel's dynamic shared memory is one value per function and device, shared by all threads of the
+// process: a call that set it to its own need could lower it between another's call here and its launch.  So every call
+// sets the most that any size needs, and launches with its own.
+constexpr int kFilterSmemMax = 227 * 1024 - 1024;   // beside the kernels' static 0.1 KB
+template <class Kernel> static int allow_smem(Kernel kernel, size_t most)
+{
+    B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    return 0;
+}
+
 bool knn_tc_supported(int64_t nd, int D, int K)
 {
     if (K + 32 > kMaxL || D > 8192) return false;
@@ -2076,8 +2089,8 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
         const int sparse = nd >= 131072;
         auto narrow = parts.most > 1 ? (QH == 1 ? knn_tc_filter_kernel<1, false, true> : knn_tc_filter_kernel<2, false, true>)
                                      : (QH == 1 ? knn_tc_filter_kernel<1, false, false> : knn_tc_filter_kernel<2, false, false>);
-        if (wide) B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        else B200_CUDA(cudaFuncSetAttribute(narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (wide) B200_TRY(allow_smem(knn_tc_wide_kernel<false>, kFilterSmemMax));
+        else B200_TRY(allow_smem(narrow, kFilterSmemMax));
         for (long long lo = 0; lo < tiles; lo += win) {
             const int hi = (int)std::min<long long>(tiles, lo + win);
             if (wide)
@@ -2135,13 +2148,13 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
         B200_CUDA(cudaGetLastError());
         if (wide) {
             const size_t smem_a = (size_t)kWideStages * 4 * kWideChunkBytes;
-            B200_CUDA(cudaFuncSetAttribute(knn_tc_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+            B200_TRY(allow_smem(knn_tc_wide_kernel<true>, kFilterSmemMax));
             knn_tc_wide_kernel<true><<<(unsigned)((q_tiles + 1) / 2), tc_threads(2), smem_a, st>>>(
                 w.img_q, w.img_s, Dp / KC, nq, w.segs, w.nseg, 0, 1, 0, ts / 2, nullptr, 0, nullptr, nullptr, counters + 0, bf16,
                 ScanParts(), rank_a, tau, (long long)m_a);
         } else {
             const size_t smem_a = (size_t)(1 + kBStages) * w.image_bytes;
-            B200_CUDA(cudaFuncSetAttribute(knn_tc_filter_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+            B200_TRY(allow_smem(knn_tc_filter_kernel<1, true, false>, kFilterSmemMax));
             knn_tc_filter_kernel<1, true, false><<<(unsigned)q_tiles, tc_threads(1), smem_a, st>>>(
                 w.img_q, w.img_s, Dp, nq, (long long)m_a, w.segs, w.nseg, 0, 1, 0, ts, nullptr, 0, nullptr, nullptr, counters + 0,
                 bf16, w.sw, w.nks, w.n_rest, ScanParts(), 0, rank_a, tau);
@@ -2179,7 +2192,7 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     auto rerank = L == 128 ? (vec == 4 ? knn_tc_rerank_kernel<4, 4> : (vec == 2 ? knn_tc_rerank_kernel<2, 4> : knn_tc_rerank_kernel<1, 4>))
                            : (vec == 4 ? knn_tc_rerank_kernel<4, 8> : (vec == 2 ? knn_tc_rerank_kernel<2, 8> : knn_tc_rerank_kernel<1, 8>));
     const size_t rerank_smem = sizeof(float) * kRerankWarps * rerank_floats(D, L);
-    B200_CUDA(cudaFuncSetAttribute(rerank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rerank_smem));
+    B200_TRY(allow_smem(rerank, sizeof(float) * kRerankWarps * rerank_floats_max(L)));
     rerank<<<(unsigned)((nq + kRerankWarps - 1) / kRerankWarps), kRerankWarps * 32, rerank_smem, st>>>(
         X, D, w.qlist, w.dblist, q_lo, nq, cand, cap, counts, tau, K, w.norms_q, err_scale, bf16 ? w.res_q : nullptr,
         reinterpret_cast<const float *>(counters + 4), ids, d2, failed, counters + 1, reinterpret_cast<float *>(counters + 3), xp);
