@@ -107,3 +107,22 @@ def test_infinitely_far_neighbours_in_segments(engine):
     want = np.argsort(dist, axis=1, kind="stable")[:, :k]    # NaN last, equal distances by index
     assert np.array_equal(ids, want) and np.array_equal(d2, np.take_along_axis(dist, want, 1))
     assert (np.isfinite(d2).sum(1) < 4).all()
+
+
+@pytest.mark.parametrize("n,k,copies", [(70001, 8, 2), (60000, 5, 2), (70001, 5, 24), (200003, 32, 2)])
+def test_many_rows_handed_over_to_the_list_search(engine, oracle_cpu, n, k, copies):
+    """Every `copies`-th point is one of sixteen corners: so many rows and pairs that lists are kept for them, over the whole
+    database or in slices that are merged; a row of NaN among them stays empty."""
+    X = np.random.default_rng(3).normal(0.5, 1, (n, 4)).astype(np.float32)
+    X[::copies] = np.random.default_rng(4).integers(0, 2, (len(X[::copies]), 4))
+    X[5 * copies] = np.nan
+    ids, d2 = engine.knn(X, k)
+    st = engine.knn_last_stats()
+    assert st["tensor_core"] == 1 and st["rows_recomputed"] * n > 1e7 * k ** 1.5
+    assert (ids[5 * copies] == -1).all() and np.isposinf(d2[5 * copies]).all()
+    Xo = np.delete(X, 5 * copies, axis=0)                    # (the oracle takes no NaN)
+    back = np.delete(np.arange(n), 5 * copies)
+    for lo in (0, n // 2, n - 61):
+        ids_o, d2_o = oracle_cpu.knn(Xo, k, q_lo=lo, q_hi=lo + 60)
+        rows = back[lo:lo + 60]
+        assert np.array_equal(ids[rows], back[ids_o]) and np.array_equal(d2[rows], d2_o)

@@ -15,6 +15,7 @@
 // k-th best; the rare survivors are inserted into the sorted result rows by the whole warp.
 // No N x N matrix is ever written.
 #include <limits.h>
+#include <math.h>
 #include <stdlib.h>
 #include <string.h>
 
@@ -90,12 +91,22 @@ __device__ __forceinline__ void warp_insert(volatile float *ld, volatile int32_t
     __syncwarp();
 }
 
-// XT: dimension-major copy of X ([D][N]).  The nq queries are rows q_lo, q_lo+1, ...; database rows [db_lo,db_hi).
-// The list of query q_lo + r is row r of ids/d2 ([.][K], pre-set to (INT_MAX, +inf)).
+// XT: dimension-major copy of X ([D][N]).  The nq queries are rows q_lo, q_lo+1, ... or, when q_index is
+// given, the rows it lists; database rows [db_lo,db_hi).  The list of query row g is written to row
+// (g - out_base) of ids/d2 ([.][K], pre-set to (INT_MAX, +inf)).
 __global__ void __launch_bounds__(kThreads, 2)
-knn_exact_kernel(const float *__restrict__ XT, long long N, int D, int K, long long q_lo, long long nq, long long db_lo, long long db_hi,
-                 int32_t *ids, float *d2)
+knn_exact_kernel(const float *__restrict__ XT, long long N, int D, int K, long long q_lo, long long nq,
+                 const int *__restrict__ q_index, long long out_base, long long db_lo, long long db_hi, int32_t *ids,
+                 float *d2, long long slice_step, long long slice_out_stride)
 {
+    // slice_step > 0: block row y searches the database slice [db_lo + y * slice_step, ... + slice_step) and
+    // writes its lists slice_out_stride elements after those of row y - 1
+    if (slice_step > 0) {
+        db_lo += (long long)blockIdx.y * slice_step;
+        db_hi = min(db_hi, db_lo + slice_step);
+        ids += (long long)blockIdx.y * slice_out_stride;
+        d2 += (long long)blockIdx.y * slice_out_stride;
+    }
     extern __shared__ __align__(16) float sm[];
     float *Qs = sm;                          // [DCH][BQ]
     float *Ps = Qs + DCH * BQ;               // [DCH][BP]
@@ -111,7 +122,7 @@ knn_exact_kernel(const float *__restrict__ XT, long long N, int D, int K, long l
         thr_d[tid] = INFINITY;
         thr_i[tid] = INT_MAX;
         const long long pos = q0 + tid;
-        q_row[tid] = (pos < nq) ? (int)(q_lo + pos) : -1;
+        q_row[tid] = (pos < nq) ? (q_index ? q_index[pos] : (int)(q_lo + pos)) : -1;
     }
     __syncthreads();
 
@@ -179,7 +190,7 @@ knn_exact_kernel(const float *__restrict__ XT, long long N, int D, int K, long l
                     const float cd = __shfl_sync(0xffffffffu, dl[c], src);
                     const int ci = (int)(p0 + src * 4 + c);
                     if (cd < td || (cd == td && ci < ti)) {   // the threshold may have moved since the ballot
-                        const long long orow = gq - q_lo;
+                        const long long orow = (out_base < 0) ? (q0 + q) : (gq - out_base);   // out_base < 0: by list position
                         volatile float *ld = d2 + orow * K;
                         volatile int32_t *li = ids + orow * K;
                         warp_insert(ld, li, K, cd, ci, lane);
@@ -218,7 +229,62 @@ __global__ void knn_merge_kernel(const int32_t *__restrict__ ids_parts, const fl
     }
 }
 
+// The same merge for many short lists (up to 1024 parts): one warp per row, lane l owns the parts
+// l, l + 32, ...; every round each lane offers the best head among its parts and the warp takes the
+// smallest offer by (distance, id).
+__global__ void __launch_bounds__(128)
+knn_merge_many_kernel(const int32_t *__restrict__ ids_parts, const float *__restrict__ d2_parts, int parts,
+                      long long part_stride, long long n_rows, int K, const int *__restrict__ row_index, long long out_base,
+                      int32_t *__restrict__ ids, float *__restrict__ d2)
+{
+    const int lane = threadIdx.x & 31;
+    const long long r = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (r >= n_rows) return;
+    const long long orow = row_index ? (row_index[r] - out_base) : r;
+    int head[32];
+#pragma unroll
+    for (int j = 0; j < 32; j++) head[j] = 0;
+    for (int s = 0; s < K; s++) {
+        float bd = INFINITY;
+        int bi = INT_MAX, bj = -1;
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+            const int p = lane + 32 * j;
+            if (p < parts && head[j] < K) {
+                const long long o = (long long)p * part_stride + r * K + head[j];
+                const float cd = d2_parts[o];
+                const int ci = ids_parts[o];
+                if (cd < bd || (cd == bd && ci < bi)) { bd = cd; bi = ci; bj = j; }
+            }
+        }
+        float wd = bd;
+        int wi = bi;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float od = __shfl_xor_sync(0xffffffffu, wd, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, wi, o);
+            if (od < wd || (od == wd && oi < wi)) { wd = od; wi = oi; }
+        }
+        // ids are unique across the parts (disjoint database slices), so exactly one lane holds the winner
+        if (bj >= 0 && bd == wd && bi == wi) {
+#pragma unroll
+            for (int j = 0; j < 32; j++)
+                if (j == bj) head[j]++;
+        }
+        if (lane == 0) { ids[orow * K + s] = wi; d2[orow * K + s] = wd; }
+    }
+}
+
 constexpr size_t kKnnSmem = sizeof(float) * (DCH * BQ + DCH * BP + BQ * DSTR + BQ) + sizeof(int) * 2 * BQ;
+
+__global__ void knn_init_rows_kernel(int32_t *ids, float *d2, const int *__restrict__ q_index, long long nq, long long out_base, int K)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nq * K) return;
+    const long long row = (out_base < 0) ? (t / K) : (q_index[t / K] - out_base);
+    ids[row * K + t % K] = INT_MAX;
+    d2[row * K + t % K] = INFINITY;
+}
 }  // namespace
 
 int launch_knn_finalize(int32_t *ids, float *d2, int64_t n, cudaStream_t st)
@@ -258,12 +324,68 @@ int launch_knn_exact(const float *XT, int64_t N, int D, int K, int64_t q_lo, int
     knn_init_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ids, d2, n);
     B200_CUDA(cudaGetLastError());
     B200_CUDA(cudaFuncSetAttribute(knn_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKnnSmem));
-    knn_exact_kernel<<<(unsigned)((nq + BQ - 1) / BQ), kThreads, kKnnSmem, st>>>(XT, N, D, K, q_lo, nq, db_lo, db_hi, ids, d2);
+    knn_exact_kernel<<<(unsigned)((nq + BQ - 1) / BQ), kThreads, kKnnSmem, st>>>(XT, N, D, K, q_lo, nq, nullptr, q_lo, db_lo, db_hi,
+                                                                                 ids, d2, 0, 0);
+    B200_CUDA(cudaGetLastError());
+    return 0;
+}
+
+// Same search for an explicit list of query rows (device array q_index of nq global row ids); the list
+// of row g replaces row (g - out_base) of ids/d2.
+int launch_knn_exact_rows(const float *XT, int64_t N, int D, int K, const int *q_index, int64_t nq, int64_t out_base,
+                          int64_t db_lo, int64_t db_hi, int32_t *ids, float *d2, cudaStream_t st)
+{
+    if (nq <= 0) return 0;
+    const long long n = nq * K;
+    knn_init_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ids, d2, q_index, nq, out_base, K);
+    B200_CUDA(cudaGetLastError());
+    B200_CUDA(cudaFuncSetAttribute(knn_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKnnSmem));
+    knn_exact_kernel<<<(unsigned)((nq + BQ - 1) / BQ), kThreads, kKnnSmem, st>>>(XT, N, D, K, 0, nq, q_index, out_base, db_lo, db_hi,
+                                                                                 ids, d2, 0, 0);
+    B200_CUDA(cudaGetLastError());
+    return 0;
+}
+
+
+// The list search for listed rows.  A block serves 64 queries against the whole database, so a few rows would occupy a
+// few SMs for the whole scan: the database is cut into slices searched by the block rows of one launch (enough of them to
+// fill the GPU four times over), and the partial lists are merged.
+static int knn_list_rows(const float *XT, int64_t N, int D, int K, const int *rows, int64_t n_rows, int64_t out_base,
+                              int64_t db_lo, int64_t db_hi, int32_t *ids, float *d2, DeviceArena &tmp, cudaStream_t st)
+{
+    const int64_t span = db_hi - db_lo;
+    const int64_t q_blocks = (n_rows + BQ - 1) / BQ;
+    const int slices = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(span / 2048, 1024), 592 / q_blocks));
+    if (slices == 1)
+        return launch_knn_exact_rows(XT, N, D, K, rows, n_rows, out_base, db_lo, db_hi, ids, d2, st);
+    int32_t *pi = nullptr;
+    float *pd = nullptr;
+    const long long per_slice = (long long)n_rows * K;
+    B200_TRY(tmp.alloc((void **)&pi, sizeof(int32_t) * (size_t)slices * per_slice));
+    B200_TRY(tmp.alloc((void **)&pd, sizeof(float) * (size_t)slices * per_slice));
+    const int64_t step = (span + slices - 1) / slices;
+    knn_init_kernel<<<(unsigned)((slices * per_slice + 255) / 256), 256, 0, st>>>(pi, pd, slices * per_slice);
+    B200_CUDA(cudaGetLastError());
+    B200_CUDA(cudaFuncSetAttribute(knn_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKnnSmem));
+    knn_exact_kernel<<<dim3((unsigned)q_blocks, (unsigned)slices), kThreads, kKnnSmem, st>>>(XT, N, D, K, 0, n_rows, rows, -1, db_lo, db_hi,
+                                                                                            pi, pd, step, per_slice);
+    B200_CUDA(cudaGetLastError());
+    knn_merge_many_kernel<<<(unsigned)((n_rows + 3) / 4), 128, 0, st>>>(pi, pd, slices, per_slice, n_rows, K, rows, out_base, ids, d2);
     B200_CUDA(cudaGetLastError());
     return 0;
 }
 
 constexpr int64_t kDenseMaxRows = 32768;
+
+// Rows that the filter could not certify: whole rows of distances write and read eight bytes a pair, a list kept per row
+// while the database streams by costs its insertions, about log N of them a row, in which a block's other queries wait.  So
+// the list pays from a number of pairs on that grows with K.  Measured, dense / list in ms, rows x database:
+//   K = 32, points of 20 dimensions drawn from few:  3,000 x 10^6  44 / 17, 30,000 x 200,000  95 / 30, 3,000 x 200,000  9.5 / 6.4
+//           all different:                           3,000 x 10^6  21 / 19, 30,000 x 200,000  43 / 36, 3,000 x 200,000  4.3 / 7.7
+//   K = 90, points of 50 dimensions drawn from few:  60,000 x 200,000  227 / 131, 30,000 x 60,000  33 / 30, 3,000 x 60,000  3.3 / 15
+//           all different:                           60,000 x 200,000  133 / 161, 30,000 x 60,000  20 / 42, 3,000 x 60,000  2.0 / 17
+// (many uncertified rows mostly are points that repeat, many neighbours as near as the K-th).
+static bool list_pays(int64_t rows, int64_t nd, int K) { return (double)rows * (double)nd > 1e7 * K * sqrt((double)K); }
 
 // Exact search of queries [q_lo,q_hi) against database rows [db_lo,db_hi) of X ([N][D], device),
 // choosing the tensor-core path where it applies and falling back to the SIMT search for the rows it
@@ -286,8 +408,8 @@ int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_
         B200_TRY(tmp.alloc((void **)&XT, sizeof(float) * (size_t)N * D));
         return launch_transpose(X, N, D, XT, st);
     };
-    // Below the tensor-core range the distances of all pairs fit in memory a few thousand queries at a time; a list kept
-    // per query while the database streams by pays from about 30,000 rows on (its insertions grow with log N only).
+    // Without the tensor cores (few rows, or K beyond their range) the distances of all pairs are written out a few thousand
+    // queries at a time: 32,768 x 50 with K = 300 20 ms, by lists 147.  Larger databases keep lists (135 ms at 32,769).
     if (!want_tc && db_hi - db_lo <= kDenseMaxRows && knn_dense_supported(K)) {
         B200_TRY(knn_dense(X, D, K, q_lo, nq, nullptr, 0, db_lo, db_hi, ids, d2, tmp, st));
         B200_CUDA(cudaStreamSynchronize(st));   // its buffers are released on return
@@ -321,7 +443,12 @@ int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_
         stats->rows_recomputed += n_failed;
         stats->filter_error_ratio = std::max(stats->filter_error_ratio, ratio);
         if (n_failed > 0) {
-            B200_TRY(knn_dense(X, D, K, 0, n_failed, failed_list, b_lo, db_lo, db_hi, ids_b, d2_b, tmp, st));
+            if (list_pays(n_failed, db_hi - db_lo, K)) {
+                B200_TRY(ensure_xt());
+                B200_TRY(knn_list_rows(XT, N, D, K, failed_list, n_failed, b_lo, db_lo, db_hi, ids_b, d2_b, tmp, st));
+            } else {
+                B200_TRY(knn_dense(X, D, K, 0, n_failed, failed_list, b_lo, db_lo, db_hi, ids_b, d2_b, tmp, st));
+            }
             B200_CUDA(cudaStreamSynchronize(st));   // the failed list lives in the workspace the next batch reuses
         }
     }
