@@ -448,6 +448,23 @@ int Session::graph_block(int remaining) const
     return px ? 0 : 1;
 }
 
+// Capturing a block and having an executable for it costs 100 us (updated) to 400 (new) more than the launches it saves cost
+// once, so it has to serve again: blocks that this call repeats or that an earlier one asked for, single iterations (50 us
+// saved) that were asked for kSingleFrom times.  A caller that steps one by one and changes the schedule every time
+// never gets there (2,000 / 60,000 points, us per step: 286 / 436 with a capture each, 119 / 118 launched directly); the odd
+// iteration at the end of a short call does not pay for an executable of its own.
+bool Session::worth_capturing(const IterGraph &key, int remaining)
+{
+    if (key.iters > 2 || (key.iters == 2 && remaining >= 4)) return true;
+    if (key.iters == 1 && remaining > 1) return false;   // the odd one before a block
+    for (IterGraph &m : missed)
+        if (m.same(key)) return ++m.asked >= (key.iters > 1 ? 2 : kSingleFrom);
+    if (missed.size() >= kMaxGraphs) missed.erase(missed.begin());
+    missed.push_back(key);
+    missed.back().asked = 1;
+    return false;
+}
+
 // 0: done, `iters` iterations of at most the number asked for.  1: not captured, the caller launches directly.  Negative:
 // error.  remaining: iterations left in the call.
 int Session::run_graph_block(int &iters, int remaining, int norm_mode, float stop_norm)
@@ -470,12 +487,12 @@ int Session::run_graph_block(int &iters, int remaining, int norm_mode, float sto
     IterGraph *g = nullptr;
     for (IterGraph &have : graphs)
         if (have.same(key)) g = &have;
-    if (!g && !graph_exec_kept(host, key.shape())) {
-        if (iters == kGraphIters && remaining < kLargeFrom) {
+    if (!g) {
+        if (iters == kGraphIters && remaining < kLargeFrom && !graph_exec_kept(host, key.shape())) {
             iters = 2;
             return run_graph_block(iters, remaining, norm_mode, stop_norm);
         }
-        if (iters == 1 && remaining > 1) return 1;   // the odd one before a block: an executable would serve it alone
+        if (!worth_capturing(key, remaining)) return 1;
     }
     if (!g) {
         if (graphs.size() >= kMaxGraphs) drop_graphs();

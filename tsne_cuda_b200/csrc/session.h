@@ -109,6 +109,7 @@ struct Session {
         unsigned sorts = 0;        // bit b: the b-th iteration sorts the spread order
         float eta = 0, exaggeration = 0, momentum = 0, stop_norm = 0;
         int64_t launches = 0;
+        int asked = 0;             // of one without an executable: how many calls asked for it
         // what decides which nodes it has: an executable of the same shape can be updated instead of made anew
         unsigned long long shape() const { return (unsigned long long)sorts << 32 | (unsigned)iters << 2 | (unsigned)natural << 1; }
         bool same(const IterGraph &o) const
@@ -121,11 +122,13 @@ struct Session {
     // A large block's first executable of a process costs 3 to 20 ms: calls of fewer iterations go in pairs until one exists
     // (20 iterations at 10^6 points after a warm-up of 3: 23.3 ms with it, 5.6 in pairs).
     static constexpr int kLargeFrom = 64;
+    static constexpr int kSingleFrom = 6;
     static constexpr size_t kMaxGraphs = 24;
-    std::vector<IterGraph> graphs;
+    std::vector<IterGraph> graphs, missed;   // with an executable; asked for lately, without one
     bool use_graphs = true;   // B200TSNE_GRAPHS=0 turns them off
     int refresh_period(int at) const;   // iterations between two sorts of the spread order at step `at` (0: natural order)
     int graph_block(int remaining) const;
+    bool worth_capturing(const IterGraph &key, int remaining);
     int run_graph_block(int &iters, int remaining, int norm_mode, float stop_norm);
     int done_seen = 0;        // IterState::done as the host last saw it
     void drop_graphs();
