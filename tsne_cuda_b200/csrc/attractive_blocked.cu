@@ -939,13 +939,7 @@ int blocked_attractive_build(BlockedAttractive *b, DeviceArena &arena, const flo
     else B200_TRY(arena.alloc((void **)&Yown, sizeof(float2) * rows));
     B200_TRY(arena.alloc((void **)&Fp, sizeof(float2) * rows));
     B200_CUDA(cudaMemsetAsync(Yp, 0, sizeof(float2) * (size_t)ntiles * T, st));
-    static bool attr_set[64] = {false};
-    int dev = 0;
-    B200_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        B200_CUDA(cudaFuncSetAttribute(attractive_blocked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileMax * (int)sizeof(float2)));
-        attr_set[dev] = true;
-    }
+    B200_CUDA(cudaFuncSetAttribute(attractive_blocked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileMax * (int)sizeof(float2)));
     B200_CUDA(cudaStreamSynchronize(st));   // the temporaries go away with `tmp`
 
     b->ev = main_stream.ev; b->ec = main_stream.ec; b->chunk_row0 = main_stream.chunk_row0; b->tile_chunk0 = main_stream.tile_chunk0;

@@ -401,14 +401,7 @@ int fft_workspace_init(FftWorkspace *ws, void *mem, cudaStream_t st)
     ws->tw = reinterpret_cast<float2 *>(p); p += sizeof(float2) * kM;
     ws->Kh = reinterpret_cast<float *>(p); p += sizeof(float) * (size_t)kC * kM;
     ws->Rk = reinterpret_cast<float *>(p);
-    static_assert(kColsSmem <= 48 * 1024 + 2048, "columns pass: three blocks to an SM");
-    static bool done[64] = {false};
-    int dev = 0;
-    B200_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !done[dev]) {
-        B200_CUDA(cudaFuncSetAttribute(fft_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColsSmem));
-        if (dev >= 0 && dev < 64) done[dev] = true;
-    }
+    static_assert(kColsSmem <= 48 * 1024, "columns pass: three blocks to an SM, and no more than a kernel may have unasked");
     twiddle_init_kernel<<<(kM + 255) / 256, 256, 0, st>>>(ws->tw);
     B200_CUDA(cudaGetLastError());
     return 0;

@@ -1,6 +1,7 @@
 // Kept streams and pinned memory, and the host <-> device copies (see hostio.h).
 #include "hostio.h"
 
+#include <cuda.h>
 #include <string.h>
 
 #include <algorithm>
@@ -26,6 +27,7 @@ constexpr int kMaxIdleStages = 2;                // 16 MiB of pinned memory each
 
 struct Stage {
     int device = -1;
+    unsigned long long context = 0;
     char *mem = nullptr;               // [kLanes][2][kChunk], pinned
     cudaEvent_t ev[kLanes][2] = {};
     cudaEvent_t begin = nullptr;
@@ -86,20 +88,30 @@ int stage_create(Stage *g)
     return 0;
 }
 
+// An idle one of this device and context, or null.  Those of a context that is gone are forgotten: their handles went
+// with it.
+template <class T> T *take_idle(std::vector<T *> &idle, int device, unsigned long long context)
+{
+    std::lock_guard<std::mutex> hold(g_lock);
+    T *found = nullptr;
+    for (size_t i = idle.size(); i-- > 0;) {
+        T *t = idle[i];
+        if (t->device != device || (found && t->context == context)) continue;
+        idle.erase(idle.begin() + i);
+        if (t->context == context) found = t;
+        else delete t;
+    }
+    return found;
+}
+
 // null when it cannot be had (not an error: the caller copies without it)
 Stage *stage_acquire(int device)
 {
-    {
-        std::lock_guard<std::mutex> hold(g_lock);
-        for (size_t i = 0; i < g_stages.size(); i++)
-            if (g_stages[i]->device == device) {
-                Stage *g = g_stages[i];
-                g_stages.erase(g_stages.begin() + i);
-                return g;
-            }
-    }
+    const unsigned long long context = context_id();
+    if (Stage *kept = take_idle(g_stages, device, context)) return kept;
     Stage *g = new Stage();
     g->device = device;
+    g->context = context;
     if (stage_create(g) != 0) {
         stage_destroy(g);
         (void)cudaGetLastError();
@@ -166,21 +178,32 @@ template <class F> cudaError_t on_lanes(int lanes, int device, F body)
 
 }  // namespace
 
+unsigned long long context_id()
+{
+    using GetId = CUresult (*)(CUcontext, unsigned long long *);
+    static const GetId get = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &found) != cudaSuccess) {
+            (void)cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<GetId>(f);
+    }();
+    unsigned long long id = 0;
+    return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 int stream_set_acquire(StreamSet **out, int device)
 {
     *out = nullptr;
     B200_CUDA(cudaSetDevice(device));
-    {
-        std::lock_guard<std::mutex> hold(g_lock);
-        for (size_t i = 0; i < g_sets.size(); i++)
-            if (g_sets[i]->device == device) {
-                *out = g_sets[i];
-                g_sets.erase(g_sets.begin() + i);
-                return 0;
-            }
-    }
+    const unsigned long long context = context_id();
+    *out = take_idle(g_sets, device, context);
+    if (*out) return 0;
     StreamSet *s = new StreamSet();
     s->device = device;
+    s->context = context;
     const int rc = set_create(s);
     if (rc != 0) {
         set_destroy(s);
@@ -190,9 +213,19 @@ int stream_set_acquire(StreamSet **out, int device)
     return 0;
 }
 
+bool stream_set_alive(const StreamSet *s)
+{
+    if (cudaSetDevice(s->device) != cudaSuccess) (void)cudaGetLastError();   // an error that stays: the handles are still valid
+    return s->context == context_id();
+}
+
 void stream_set_release(StreamSet *s)
 {
     if (!s) return;
+    if (!stream_set_alive(s)) {
+        delete s;
+        return;
+    }
     const bool fine = cudaStreamSynchronize(s->stream) == cudaSuccess && cudaStreamSynchronize(s->stream2) == cudaSuccess;
     if (fine) {
         std::lock_guard<std::mutex> hold(g_lock);
@@ -321,17 +354,9 @@ int copy_out(void *dst, const void *src, size_t bytes, cudaStream_t st)
 
 void host_pools_release(int device)
 {
-    std::vector<StreamSet *> sets;
-    std::vector<Stage *> stages;
-    {
-        std::lock_guard<std::mutex> hold(g_lock);
-        for (size_t i = g_sets.size(); i-- > 0;)
-            if (g_sets[i]->device == device) { sets.push_back(g_sets[i]); g_sets.erase(g_sets.begin() + i); }
-        for (size_t i = g_stages.size(); i-- > 0;)
-            if (g_stages[i]->device == device) { stages.push_back(g_stages[i]); g_stages.erase(g_stages.begin() + i); }
-    }
-    for (StreamSet *s : sets) set_destroy(s);
-    for (Stage *g : stages) stage_destroy(g);
+    const unsigned long long context = context_id();
+    while (StreamSet *s = take_idle(g_sets, device, context)) set_destroy(s);
+    while (Stage *g = take_idle(g_stages, device, context)) stage_destroy(g);
 }
 
 }  // namespace b200

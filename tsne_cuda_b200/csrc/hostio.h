@@ -10,12 +10,17 @@
 
 namespace b200 {
 
+// Which context of the current device this is: another one after cudaDeviceReset, which takes streams, events, pinned
+// memory, executables and function attributes with it (a stale handle is not refused but crashes).  0: cannot be told.
+unsigned long long context_id();
+
 // What a session or a stage call needs from the driver besides device memory.  Creating and destroying it costs one to
 // three milliseconds a time, and on a busy host single calls (pinned memory above all) stall for 0.1 to 1.2 s, so the
 // sets are kept per device and handed to the next caller: at most kMaxIdleSets idle ones,
 // b200tsne_release_cached_memory() gives them back.  Safe from several threads: a set has one user at a time.
 struct StreamSet {
     int device = -1;
+    unsigned long long context = 0;   // its handles are of this context
     cudaStream_t stream = nullptr, stream2 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     IterState *h_state = nullptr;   // pinned
@@ -30,6 +35,7 @@ struct StreamSet {
 };
 int stream_set_acquire(StreamSet **out, int device);   // makes `device` current
 void stream_set_release(StreamSet *s);                 // waits for both streams; null is fine
+bool stream_set_alive(const StreamSet *s);             // its context still is the device's; makes the device current
 
 // An executable for `graph`: a kept one of the same shape, updated, else a new one; null if neither can be had.
 cudaGraphExec_t graph_exec_acquire(StreamSet *s, cudaGraph_t graph, unsigned long long shape);

@@ -25,6 +25,7 @@
 #include "common.cuh"
 
 #include <atomic>
+#include "hostio.h"
 #include "session.h"
 
 namespace b200 {
@@ -471,17 +472,20 @@ constexpr long long kNoAllocMaxElems = 4ll << 20;   // N * D may not exceed this
 static __device__ __align__(256) float g_noalloc_xt[kNoAllocMaxElems];
 
 // In host code `g_noalloc_xt` is only a handle; the address a kernel can use comes from the runtime and
-// differs per device.  Looked up once per device, with that device current.
+// differs per device and context.  Looked up once in each, with the device current.
 static int noalloc_scratch(float **out)
 {
     static std::atomic<float *> cached[64];   // zero-initialised; two threads racing here store the same address
+    static std::atomic<unsigned long long> cached_in[64];
     int dev = 0;
     B200_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) { set_error("knn_noalloc: device ordinal out of range"); return -4; }
-    float *p = cached[dev].load(std::memory_order_acquire);
+    const unsigned long long context = context_id();
+    float *p = cached_in[dev].load(std::memory_order_acquire) == context ? cached[dev].load(std::memory_order_relaxed) : nullptr;
     if (!p) {
         B200_CUDA(cudaGetSymbolAddress((void **)&p, g_noalloc_xt));
-        cached[dev].store(p, std::memory_order_release);
+        cached[dev].store(p, std::memory_order_relaxed);
+        cached_in[dev].store(context_id(), std::memory_order_release);   // (the look-up may have made the context)
     }
     *out = p;
     return 0;

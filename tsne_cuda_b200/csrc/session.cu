@@ -16,6 +16,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <string>
 
 #include "comm.h"
@@ -43,15 +44,16 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line)
 // handed to any stream afterwards.  b200tsne_release_cached_memory() returns the pool to the driver.
 static int configure_pool()
 {
-    static bool done[64] = {false};
+    static std::atomic<unsigned long long> done[64];   // the context (plus one) that it was done in
     int dev = 0;
     B200_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || done[dev]) return 0;
+    const unsigned long long context = context_id() + 1;
+    if (dev < 0 || dev >= 64 || done[dev].load(std::memory_order_relaxed) == context) return 0;
     cudaMemPool_t pool;
     B200_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
     unsigned long long keep = ~0ull;
     B200_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-    done[dev] = true;
+    done[dev].store(context, std::memory_order_relaxed);
     return 0;
 }
 
@@ -84,6 +86,11 @@ int DeviceArena::alloc(void **p, size_t bytes)
         B200_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
     }
     return 0;
+}
+void DeviceArena::forget()
+{
+    consumers.clear();
+    ptrs.clear();
 }
 void DeviceArena::release()
 {
@@ -156,6 +163,12 @@ int Session::init(int64_t N_, int K_, int64_t lo, int64_t hi, int device_)
 void Session::destroy()
 {
     cudaSetDevice(device);
+    if (host && !stream_set_alive(host)) {   // the device was reset: memory, streams and executables are gone already
+        graphs.clear();
+        blocked_arena.forget();
+        arena.forget();
+        stream = stream2 = nullptr;
+    }
     if (stream) cudaStreamSynchronize(stream);
     if (stream2) cudaStreamSynchronize(stream2);
     drop_graphs();

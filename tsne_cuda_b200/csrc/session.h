@@ -22,6 +22,7 @@ struct DeviceArena {
     void serve(cudaStream_t st) { consumers.push_back(st); }
     int alloc(void **p, size_t bytes);
     void release();
+    void forget();   // the memory went with its context
 };
 
 struct Session {
