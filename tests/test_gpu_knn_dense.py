@@ -126,3 +126,15 @@ def test_many_rows_handed_over_to_the_list_search(engine, oracle_cpu, n, k, copi
         ids_o, d2_o = oracle_cpu.knn(Xo, k, q_lo=lo, q_hi=lo + 60)
         rows = back[lo:lo + 60]
         assert np.array_equal(ids[rows], back[ids_o]) and np.array_equal(d2[rows], d2_o)
+
+
+@pytest.mark.parametrize("ties", [False, True])
+@pytest.mark.parametrize("n,d,k", [(300, 20, 10), (2047, 50, 90), (9000, 20, 300), (12289, 7, 256), (32768, 5, 230)])
+def test_against_the_list_search_on_every_row(engine, monkeypatch, n, d, k, ties):
+    """Whole rows of distances against the search that keeps lists (forced at any size), which shares no kernel with it."""
+    X = _points(n, d, n + k, ties)
+    ids, d2 = engine.knn(X, k)
+    assert engine.knn_last_stats()["tensor_core"] == 0
+    monkeypatch.setenv("B200TSNE_KNN", "simt")
+    ids_l, d2_l = engine.knn(X, k)
+    assert np.array_equal(ids, ids_l) and np.array_equal(d2, d2_l)

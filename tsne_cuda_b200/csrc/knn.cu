@@ -399,8 +399,11 @@ int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_
     *stats = KnnStats();
     const int64_t nq = q_hi - q_lo;
     if (nq <= 0) return 0;
+    // B200TSNE_KNN=simt: the list-keeping search whatever the sizes.  It shares no kernel with the other two, and so
+    // checks the rows that whole rows of distances are computed for as well.
     const char *force = getenv("B200TSNE_KNN");
-    const bool want_tc = knn_tc_supported(db_hi - db_lo, D, K) && !(force && strcmp(force, "simt") == 0);
+    const bool lists = force && strcmp(force, "simt") == 0;
+    const bool want_tc = knn_tc_supported(db_hi - db_lo, D, K) && !lists;
     DeviceArena tmp;
     tmp.serve(st);
     float *XT = nullptr;
@@ -411,7 +414,7 @@ int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_
     };
     // Without the tensor cores (few rows, or K beyond their range) the distances of all pairs are written out a few thousand
     // queries at a time: 32,768 x 50 with K = 300 20 ms, by lists 147.  Larger databases keep lists (135 ms at 32,769).
-    if (!want_tc && db_hi - db_lo <= kDenseMaxRows && knn_dense_supported(K)) {
+    if (!want_tc && !lists && db_hi - db_lo <= kDenseMaxRows && knn_dense_supported(K)) {
         B200_TRY(knn_dense(X, D, K, q_lo, nq, nullptr, 0, db_lo, db_hi, ids, d2, tmp, st));
         B200_CUDA(cudaStreamSynchronize(st));   // its buffers are released on return
         return 0;
