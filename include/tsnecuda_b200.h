@@ -125,15 +125,17 @@ int b200tsne_knn_last_stats(int *tensor_core, int *rows_recomputed, float *filte
  * hands out all device memory from its own pool, a service whose footprint is fixed at start-up, a
  * latency-bound loop where cudaMalloc's implicit synchronisation is unacceptable.  X_device ([N][D]),
  * ids_device and d2_device ([N][K]) are DEVICE pointers on the current device, owned by the caller; the
- * one piece of scratch the search needs (a dimension-major copy of X) lives in a fixed array inside the
- * library, so N * D must not exceed b200tsne_knn_noalloc_max_elements() (4 Mi floats = 16 MiB, resident
- * on every GPU that loads the library); larger inputs are rejected with B200TSNE_ERR_UNSUPPORTED.
+ * one piece of scratch the search needs (distances of a group of queries, or above 12,288 points or 512
+ * neighbours a dimension-major copy of X) lives in a fixed array inside the library, so N * D must not
+ * exceed b200tsne_knn_noalloc_max_elements() (4 Mi floats = 16 MiB, resident on every GPU that loads the
+ * library); larger inputs are rejected with B200TSNE_ERR_UNSUPPORTED.
  * The work is queued on cuda_stream (a cudaStream_t, NULL = default stream) and the call returns without
- * waiting, on the device that is current (cuda_stream must belong to it).  The first call on a device looks up
- * the array's device address and sets kernel attributes, which may load the library's device code: make that
- * call once at start-up, before any stream capture.  All calls share the one array, which keeps the previous
- * call's contents (every element the search reads is rewritten first): two calls whose GPU work overlaps, on different streams or from
- * different threads, race on it.  Results equal b200tsne_knn's (SIMT search; whole database, all queries). */
+ * waiting, on the device that is current (cuda_stream must belong to it).  The first call on a device, of any
+ * size, looks up the array's device address and loads all the kernels that later calls may launch: make it
+ * once at start-up, before any stream capture; later calls of any size may be captured.  All calls share the
+ * one array, which keeps the previous call's contents (every element the search reads is rewritten first):
+ * two calls whose GPU work overlaps, on different streams or from different threads, race on it.  Results
+ * equal b200tsne_knn's (whole database, all queries). */
 int b200tsne_knn_noalloc(const float *X_device, int64_t N, int D, int K, int32_t *ids_device, float *d2_device,
                          void *cuda_stream);
 int64_t b200tsne_knn_noalloc_max_elements(void);

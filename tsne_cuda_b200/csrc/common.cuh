@@ -120,6 +120,7 @@ int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_
 bool knn_dense_supported(int K);
 int knn_dense(const float *X, int D, int K, int64_t q_lo, int64_t nq, const int *q_index, int64_t out_base, int64_t db_lo, int64_t db_hi,
               int32_t *ids, float *d2, DeviceArena &tmp, cudaStream_t st);
+int knn_dense_load();
 int knn_dense_in_scratch(const float *X, int64_t N, int D, int K, float *scratch, long long floats, int32_t *ids, float *d2, cudaStream_t st);
 // knn.cu: search with the scratch in a fixed device array of the library (no allocation)
 long long knn_noalloc_max_elems();

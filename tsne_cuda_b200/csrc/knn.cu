@@ -475,7 +475,8 @@ constexpr long long kNoAllocMaxElems = 4ll << 20;   // N * D may not exceed this
 static __device__ __align__(256) float g_noalloc_xt[kNoAllocMaxElems];
 
 // In host code `g_noalloc_xt` is only a handle; the address a kernel can use comes from the runtime and
-// differs per device and context.  Looked up once in each, with the device current.
+// differs per device and context.  Looked up once in each, with the device current; the same call loads every kernel that
+// any later one may launch, whatever its sizes.
 static int noalloc_scratch(float **out)
 {
     static std::atomic<float *> cached[64];   // zero-initialised; two threads racing here store the same address
@@ -487,6 +488,10 @@ static int noalloc_scratch(float **out)
     float *p = cached_in[dev].load(std::memory_order_acquire) == context ? cached[dev].load(std::memory_order_relaxed) : nullptr;
     if (!p) {
         B200_CUDA(cudaGetSymbolAddress((void **)&p, g_noalloc_xt));
+        B200_TRY(knn_dense_load());
+        cudaFuncAttributes a;
+        for (const void *k : {(const void *)transpose_kernel, (const void *)knn_init_kernel, (const void *)knn_exact_kernel, (const void *)knn_finalize_kernel})
+            B200_CUDA(cudaFuncGetAttributes(&a, k));
         cached[dev].store(p, std::memory_order_relaxed);
         cached_in[dev].store(context_id(), std::memory_order_release);   // (the look-up may have made the context)
     }

@@ -299,6 +299,17 @@ int knn_dense(const float *X, int D, int K, int64_t q_lo, int64_t nq, const int 
     return 0;
 }
 
+// loads every kernel that knn_dense_in_scratch may launch (a look at its attributes does)
+int knn_dense_load()
+{
+    cudaFuncAttributes a;
+    const void *kernels[] = {(const void *)dense_distance_kernel<1>, (const void *)dense_distance_kernel<4>, (const void *)dense_select_kernel<4>,
+                             (const void *)dense_select_kernel<8>,   (const void *)dense_select_kernel<16>,  (const void *)dense_select_kernel<32>,
+                             (const void *)dense_select_kernel<48>};
+    for (const void *k : kernels) B200_CUDA(cudaFuncGetAttributes(&a, k));
+    return 0;
+}
+
 // The same for all points against all, in scratch of `floats` floats that the caller owns; -1 when it is too small for
 // that to be worth it (the caller then searches another way).
 int knn_dense_in_scratch(const float *X, int64_t N, int D, int K, float *scratch, long long floats, int32_t *ids, float *d2, cudaStream_t st)
