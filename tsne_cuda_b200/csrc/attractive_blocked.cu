@@ -148,7 +148,7 @@ cell_scatter_kernel(const unsigned char *__restrict__ cell, const int *__restric
 
 }  // namespace
 
-int order_points_by_cell(const PointCells &pc, int32_t *perm, cudaStream_t st)
+int order_points_by_cell(const PointCells &pc, const float *X, int D, int32_t *perm, cudaStream_t st)
 {
     const int64_t N = pc.n;
     if (N <= 0 || pc.lo != 0) { set_error("order_points_by_cell: needs the cells of all points"); return -1; }
@@ -159,7 +159,7 @@ int order_points_by_cell(const PointCells &pc, int32_t *perm, cudaStream_t st)
     B200_TRY(tmp.alloc((void **)&rank, sizeof(int) * kMaxCells));
     B200_TRY(tmp.alloc((void **)&hist, sizeof(int) * (size_t)kMaxCells * nblocks));
     B200_CUDA(cudaMemsetAsync(rank, 0, sizeof(int) * kMaxCells, st));
-    B200_TRY(point_cells_chain(pc, rank, st));
+    B200_TRY(point_cells_chain(pc, X, D, rank, tmp, st));
     cell_hist_kernel<<<nblocks, kSortWarps * 32, 0, st>>>(pc.cell, rank, N, hist);
     scan_inplace_kernel<<<1, 1024, 0, st>>>(hist, (long long)kMaxCells * nblocks);
     cell_scatter_kernel<<<nblocks, kSortWarps * 32, 0, st>>>(pc.cell, rank, N, hist, perm);

@@ -202,8 +202,8 @@ int b200tsne_attractive_blocked(const float *P, const int32_t *ids, const float 
         B200_TRY(up(a, &dX, X, (size_t)N * D, sg.st));
         B200_TRY(a.alloc((void **)&perm, sizeof(int32_t) * N));
         PointCells pc;
-        B200_TRY(point_cells_build(&pc, dX, D, 0, N, a, sg.st));
-        B200_TRY(order_points_by_cell(pc, perm, sg.st));
+        B200_TRY(point_cells_build(&pc, dX, D, 0, N, false, a, sg.st));
+        B200_TRY(order_points_by_cell(pc, dX, D, perm, sg.st));
     }
     B200_CUDA(cudaMemsetAsync(dF2, 0, sizeof(float2) * N, sg.st));
     B200_TRY(launch_soa_to_aos(dY, dY2, N, sg.st));
@@ -259,8 +259,8 @@ int b200tsne_attractive_symmetric(const float *p, const int32_t *ids, const floa
         B200_TRY(up(a, &dX, X, (size_t)N * D, sg.st));
         B200_TRY(a.alloc((void **)&perm, sizeof(int32_t) * N));
         PointCells pc;
-        B200_TRY(point_cells_build(&pc, dX, D, 0, N, a, sg.st));
-        B200_TRY(order_points_by_cell(pc, perm, sg.st));
+        B200_TRY(point_cells_build(&pc, dX, D, 0, N, false, a, sg.st));
+        B200_TRY(order_points_by_cell(pc, dX, D, perm, sg.st));
     }
     B200_CUDA(cudaMemsetAsync(dF2, 0, sizeof(float2) * N, sg.st));
     B200_TRY(launch_soa_to_aos(dY, dY2, N, sg.st));

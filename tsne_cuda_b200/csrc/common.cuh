@@ -78,7 +78,7 @@ __host__ __device__ inline float dec_float(unsigned int e)
 int launch_transpose(const float *X, int64_t N, int D, float *XT, cudaStream_t st);   // [N][D] -> [D][N]
 int launch_knn_exact(const float *XT, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo,
                      int64_t db_hi, int32_t *ids, float *d2, cudaStream_t st);   // ids/d2 keep (INT_MAX,+inf) in unfilled slots
-// cells.cu: nearest of at most kMaxCells sample points, for every row of a range, with the distances to all of them
+// cells.cu: nearest of at most kMaxCells sample points, for every row of a range, with the distance to it
 struct DeviceArena;
 constexpr int kMaxCells = 64;
 struct CellTable {
@@ -92,17 +92,20 @@ struct PointCells {
     int cells = 0;
     int64_t lo = 0, n = 0;          // rows [lo, lo + n)
     CellTable *tab = nullptr;
-    float *dist = nullptr;          // [n][kMaxCells]
+    float *own = nullptr;           // [n] distance to the own cell's sample point
     unsigned char *cell = nullptr;  // [n]
+    float *dist = nullptr;          // [n][kMaxCells] the distances to all of them, where they are kept
 };
+constexpr int64_t kCellRowsMax = (int64_t)1 << 20;   // rows whose distances to all sample points are kept (256 MB)
 inline int point_cells_count(int64_t n) { return (int)(n < 4096 ? 1 : (n / 2048 < kMaxCells ? n / 2048 : kMaxCells)); }   // see point_cells_build
-int point_cells_build(PointCells *pc, const float *X, int D, int64_t lo, int64_t n, DeviceArena &arena, cudaStream_t st);
-int point_cells_assign(const PointCells &pc, const float *X, int D, int64_t lo, int64_t n, float *dist, unsigned char *cell, cudaStream_t st);
-int point_cells_chain(const PointCells &pc, int *rank, cudaStream_t st);
+int point_cells_build(PointCells *pc, const float *X, int D, int64_t lo, int64_t n, bool distances, DeviceArena &arena, cudaStream_t st);
+int point_cells_assign(const PointCells &pc, const float *X, int D, int64_t lo, int64_t n, float *dist, float *own, unsigned char *cell, cudaStream_t st);
+int point_cells_chain(const PointCells &pc, const float *X, int D, int *rank, DeviceArena &arena, cudaStream_t st);
 
 // knn_tc.cu: tensor-core filter + exact re-rank + proof (nd = database rows to scan); pc: the cells of the database rows
 bool knn_tc_supported(int64_t nd, int D, int K);
-size_t knn_tc_workspace_bytes(int D, int K, int64_t nq, int64_t nd);
+// cells_kept: the queries' distances to the cells are at hand (PointCells::dist)
+size_t knn_tc_workspace_bytes(int D, int K, int64_t nq, int64_t nd, bool cells_kept);
 int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo, int64_t db_hi, const PointCells &pc,
                   int32_t *ids, float *d2, void *workspace, int **failed_list, int *n_failed_host, float *err_ratio_host,
                   cudaStream_t st);
@@ -176,7 +179,7 @@ struct BlockedAttractive {
     void clear();
 };
 // perm[q] = the point at position q of the cell order; pc: the cells of all N points
-int order_points_by_cell(const PointCells &pc, int32_t *perm, cudaStream_t st);
+int order_points_by_cell(const PointCells &pc, const float *X, int D, int32_t *perm, cudaStream_t st);
 int blocked_attractive_build(BlockedAttractive *b, DeviceArena &arena, const float *P_rows, const int32_t *ids_rows, int64_t N, int K,
                              int64_t row_lo, int64_t row_hi, const int32_t *perm, const ExtraEntries *extra, cudaStream_t st);
 int launch_exclusive_scan_i32(int *data, int64_t n, cudaStream_t st);   // in place; small arrays (one block)

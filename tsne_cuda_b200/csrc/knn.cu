@@ -427,14 +427,14 @@ int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_
     }
     // Queries go through in batches of 2^20 so that the candidate buffers (about 10 KB per query) stay
     // bounded however large N is; the operand images are rebuilt per batch (a millisecond per million points).
-    const int64_t batch = (int64_t)1 << 20;
+    const int64_t batch = kCellRowsMax;
     PointCells own;
     if (!pc || pc->lo != db_lo || pc->n != db_hi - db_lo) {
-        B200_TRY(point_cells_build(&own, X, D, db_lo, db_hi - db_lo, tmp, st));
+        B200_TRY(point_cells_build(&own, X, D, db_lo, db_hi - db_lo, true, tmp, st));
         pc = &own;
     }
     void *ws = nullptr;
-    B200_TRY(tmp.alloc(&ws, knn_tc_workspace_bytes(D, K, std::min(nq, batch), db_hi - db_lo)));
+    B200_TRY(tmp.alloc(&ws, knn_tc_workspace_bytes(D, K, std::min(nq, batch), db_hi - db_lo, pc->dist && q_lo >= db_lo && q_hi <= db_hi)));
     stats->tensor_core = 1;
     for (int64_t b_lo = q_lo; b_lo < q_hi; b_lo += batch) {
         const int64_t b_hi = std::min(q_hi, b_lo + batch);

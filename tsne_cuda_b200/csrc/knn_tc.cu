@@ -474,9 +474,9 @@ __global__ void knn_cells_reset_kernel(CellTable *tab)
     tab->db_cursor[c] = tab->q_cursor[c] = 0;
 }
 
-// members of every cell among the n rows of cell / dist and, for the database, r_c
+// members of every cell among the n rows of cell and, for the database, r_c from the rows' distances to their own centre
 __global__ void __launch_bounds__(kCellThreads)
-knn_cells_count_kernel(const unsigned char *__restrict__ cell, const float *__restrict__ dist, long long n, CellTable *tab, int is_db)
+knn_cells_count_kernel(const unsigned char *__restrict__ cell, const float *__restrict__ own, long long n, CellTable *tab, int is_db)
 {
     __shared__ int s_cnt[kMaxCells];
     __shared__ unsigned int s_rad[kMaxCells];
@@ -485,7 +485,7 @@ knn_cells_count_kernel(const unsigned char *__restrict__ cell, const float *__re
     for (long long i = (long long)blockIdx.x * kCellThreads + threadIdx.x; i < n; i += (long long)gridDim.x * kCellThreads) {
         const int c = cell[i];
         atomicAdd(&s_cnt[c], 1);
-        if (is_db) atomicMax(&s_rad[c], __float_as_uint(dist[(size_t)i * kMaxCells + c]));   // >= 0: orders like the bits
+        if (is_db) atomicMax(&s_rad[c], __float_as_uint(own[i]));   // >= 0: orders like the bits
     }
     __syncthreads();
     for (int c = threadIdx.x; c < kMaxCells; c += kCellThreads) {
@@ -1850,8 +1850,8 @@ struct TcWorkspace {
     int *slist;
     int *qlist, *dblist;
     float *xp;   // database rows in list order (cells only)
-    unsigned char *cell_q;     // queries outside the database range: their cells
-    float *dist_q;             // and distances to the centres
+    unsigned char *cell_q;     // queries whose distances to the centres are not kept: their cells
+    float *dist_q;             // and the distances
     int2 *segs;
     int *nseg;
     uint2 *cand;
@@ -1860,7 +1860,7 @@ struct TcWorkspace {
     size_t bytes;
 };
 
-static TcWorkspace tc_carve(void *base, int D, int K, long long nq, long long nd)
+static TcWorkspace tc_carve(void *base, int D, int K, long long nq, long long nd, bool cells_kept)
 {
     TcWorkspace w;
     w.wide = tc_wide(D);
@@ -1898,8 +1898,8 @@ static TcWorkspace tc_carve(void *base, int D, int K, long long nq, long long nd
     w.xp = w.wide ? nullptr : reinterpret_cast<float *>(take(sizeof(float) * (size_t)w.td * TN * D));
     w.img_s = reinterpret_cast<float *>(take((size_t)kMaxSampleTiles * w.image_bytes));
     w.slist = reinterpret_cast<int *>(take(sizeof(int) * (size_t)kMaxSampleTiles * TN));
-    w.cell_q = reinterpret_cast<unsigned char *>(take((size_t)nq));
-    w.dist_q = reinterpret_cast<float *>(take(sizeof(float) * kMaxCells * (size_t)nq));
+    w.cell_q = cells_kept ? nullptr : reinterpret_cast<unsigned char *>(take((size_t)nq));
+    w.dist_q = cells_kept ? nullptr : reinterpret_cast<float *>(take(sizeof(float) * kMaxCells * (size_t)nq));
     w.segs = reinterpret_cast<int2 *>(take(sizeof(int2) * (size_t)w.tq * kMaxCells));
     w.nseg = reinterpret_cast<int *>(take(sizeof(int) * (size_t)w.tq));
     w.cand = reinterpret_cast<uint2 *>(take(sizeof(uint2) * (size_t)nq * fixed_cap(K)));
@@ -1949,7 +1949,7 @@ struct PhaseTimer {
 };
 
 // Workspace (device, 256-byte aligned) needed by launch_knn_tc for nq queries against nd database rows.
-size_t knn_tc_workspace_bytes(int D, int K, int64_t nq, int64_t nd) { return tc_carve(nullptr, D, K, nq, nd).bytes; }
+size_t knn_tc_workspace_bytes(int D, int K, int64_t nq, int64_t nd, bool cells_kept) { return tc_carve(nullptr, D, K, nq, nd, cells_kept).bytes; }
 
 // Into how many parts the database tiles of every block of queries are dealt, one block a part.  A block holds a whole SM,
 // so `blocks` blocks of equal work take ceil(blocks / SMs) turns: 196 on 148 SMs leave a third of the chip idle, 20 seven
@@ -1986,7 +1986,8 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     const long long nq = q_hi - q_lo, nd = db_hi - db_lo;
     *n_failed_host = 0;
     if (nq <= 0) return 0;
-    const TcWorkspace w = tc_carve(workspace, D, K, nq, nd);
+    const bool cells_kept = pc.dist && q_lo >= pc.lo && q_hi <= pc.lo + pc.n;
+    const TcWorkspace w = tc_carve(workspace, D, K, nq, nd, cells_kept);
     const int Dp = w.Dp, cells = pc.cells;
     const bool wide = w.wide;
     const int bf16 = w.bf16 ? 1 : 0;
@@ -2008,17 +2009,17 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     if (cells > 1) {
         const unsigned gq = (unsigned)((nq + kCellThreads - 1) / kCellThreads), gd = (unsigned)((nd + kCellThreads - 1) / kCellThreads);
         const unsigned char *cell_q = nullptr;
-        if (q_lo >= pc.lo && q_hi <= pc.lo + pc.n) {
+        if (cells_kept) {
             q_dist = pc.dist + (size_t)(q_lo - pc.lo) * kMaxCells;
             cell_q = pc.cell + (q_lo - pc.lo);
-        } else {   // queries that are not database rows
+        } else {   // queries that are not database rows, or one batch of very many
             q_dist = w.dist_q;
             cell_q = w.cell_q;
-            B200_TRY(point_cells_assign(pc, X, D, q_lo, nq, w.dist_q, w.cell_q, st));
+            B200_TRY(point_cells_assign(pc, X, D, q_lo, nq, w.dist_q, nullptr, w.cell_q, st));
         }
         knn_cells_reset_kernel<<<1, kMaxCells, 0, st>>>(pc.tab);
-        knn_cells_count_kernel<<<std::min(gd, 592u), kCellThreads, 0, st>>>(pc.cell, pc.dist, nd, pc.tab, 1);
-        knn_cells_count_kernel<<<std::min(gq, 592u), kCellThreads, 0, st>>>(cell_q, q_dist, nq, pc.tab, 0);
+        knn_cells_count_kernel<<<std::min(gd, 592u), kCellThreads, 0, st>>>(pc.cell, pc.own, nd, pc.tab, 1);
+        knn_cells_count_kernel<<<std::min(gq, 592u), kCellThreads, 0, st>>>(cell_q, nullptr, nq, pc.tab, 0);
         knn_cells_layout_kernel<<<1, 32, 0, st>>>(cells, pc.tab);
         knn_cells_scatter_kernel<<<gd, kCellThreads, 0, st>>>(pc.cell, db_lo, nd, cells, pc.tab, 1, w.dblist);
         knn_cells_scatter_kernel<<<gq, kCellThreads, 0, st>>>(cell_q, q_lo, nq, cells, pc.tab, 0, w.qlist);

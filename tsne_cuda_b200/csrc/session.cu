@@ -676,13 +676,14 @@ int Session::affinities_from_points(const float *X_host, int D, float perplexity
         size_t free_b = 0, total_b = 0;
         B200_CUDA(cudaMemGetInfo(&free_b, &total_b));
         const int64_t batch = std::min<int64_t>(std::max<int64_t>(r, 1), 1 << 20);
-        if (knn_tc_workspace_bytes(D, K, batch, N) > total_b / 2) db_sharded = true;
+        if (knn_tc_workspace_bytes(D, K, batch, N, N <= kCellRowsMax) > total_b / 2) db_sharded = true;
     }
     // the cells of the points: the search visits by them, and the blocked copy of P numbers the points by them
     const char *attr_mode = getenv("B200TSNE_ATTRACTIVE");
     const bool want_order = N > kAttractiveTile && !(attr_mode && strcmp(attr_mode, "rows") == 0);
     PointCells cells;
-    if (want_order || (!db_sharded && knn_tc_supported(N, D, K))) B200_TRY(point_cells_build(&cells, X, D, 0, N, tmp, stream));
+    const bool cells_search = !db_sharded && knn_tc_supported(N, D, K);
+    if (want_order || cells_search) B200_TRY(point_cells_build(&cells, X, D, 0, N, cells_search, tmp, stream));
     if (!db_sharded) {
         B200_TRY(knn_search(X, N, D, K, row_lo, row_hi, 0, N, ids, d2, &knn_stats, stream, cells.cells ? &cells : nullptr));
     } else {
@@ -706,7 +707,7 @@ int Session::affinities_from_points(const float *X_host, int D, float perplexity
     // the order in which the attractive force's blocked copy of P numbers the points (every rank computes the same)
     if (want_order) {
         if (!cell_order) B200_TRY(arena.alloc((void **)&cell_order, sizeof(int32_t) * N));
-        B200_TRY(order_points_by_cell(cells, cell_order, stream));
+        B200_TRY(order_points_by_cell(cells, X, D, cell_order, stream));
     }
 
     clk.begin(stream);
