@@ -301,7 +301,8 @@ def test_frame_feed_has_the_reference_wire_format(engine):
 
 def test_full_size_properties_one_million_points(engine, oracle_cpu):
     """Size-independent properties at the benchmark's N = 10^6: exact neighbours on sampled queries, charge
-    conservation through the spread, and the grid identity for the normalisation."""
+    conservation through the spread, and the grid's normalisation against the points'."""
+    from oracle import np64
     from tsne_cuda_b200 import datasets
     N = 1000000
     rng = np.random.default_rng(0)
@@ -311,9 +312,16 @@ def test_full_size_properties_one_million_points(engine, oracle_cpu):
     expect = np.array([N, Y[0].astype(np.float64).sum(), Y[1].astype(np.float64).sum(),
                        (Y[0].astype(np.float64) ** 2 + Y[1].astype(np.float64) ** 2).sum()])
     assert np.allclose(tot, expect, rtol=2e-4, atol=2.0)
-    w64, yt64 = w.astype(np.float64), yt.astype(np.float64)
-    zs = ((w64[..., 0] + w64[..., 3]) * yt64[..., 0] - 2 * w64[..., 1] * yt64[..., 1] - 2 * w64[..., 2] * yt64[..., 2]
-          + w64[..., 0] * yt64[..., 3]).sum()
+    # Z from the points, in float64: each point's Z_i interpolated from the potentials (the engine sums charges times
+    # potentials over the grid instead)
+    x, y = Y.astype(np.float64)
+    cmin, bw = Y.astype(np.float64).min(), (Y.astype(np.float64).max() - Y.astype(np.float64).min()) / np64.N_BOXES
+    (bx, Lx), (by, Ly) = np64._weights(x, cmin, bw), np64._weights(y, cmin, bw)
+    phi = np.zeros((N, 4))
+    for a in range(3):
+        for b in range(3):
+            phi += (Lx[a] * Ly[b])[:, None] * yt[bx * 3 + a, by * 3 + b]
+    zs = ((1 + x * x + y * y) * phi[:, 0] - 2 * (x * phi[:, 1] + y * phi[:, 2]) + phi[:, 3]).sum()
     assert abs((zs - N) - Z) / abs(Z) < 1e-4
     assert np.isfinite(F).all() and abs(F.astype(np.float64).sum()) < 1e-3 * np.abs(F).sum()   # momentum conservation
     X = datasets.gaussian_mixture(200000, 50, seed=9)
