@@ -56,3 +56,13 @@ def test_every_number_of_k_steps(engine, monkeypatch, d, pairs):
     monkeypatch.setenv("B200TSNE_KNN_FILTER", pairs)
     st = both(engine, monkeypatch, mixture(2300, d, 70 + d), 20)
     assert st["filter_error_ratio"] < 0.5 and st["rows_recomputed"] <= 46
+
+
+@pytest.mark.parametrize("n,k", [(49151, 20), (49152, 20), (98303, 97), (98304, 97)])
+def test_both_sides_of_rare_survivors(engine, monkeypatch, n, k):
+    """From one key in 128 down the scan stores a lone survivor of eight behind a search for its place: every row, with
+    points that repeat, so that survivors come alone, in pairs and in runs."""
+    X = mixture(n, 5, k)
+    X[: n // 7] = X[n // 2 : n // 2 + n // 7]
+    st = both(engine, monkeypatch, X, k)
+    assert st["rows_recomputed"] <= 0.02 * n

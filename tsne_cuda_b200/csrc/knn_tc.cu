@@ -2082,12 +2082,13 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
         const ScanParts parts = scan_parts(blocks, (int)((std::min(tiles, win) + stride - 1) / stride), wide ? (63 + Dp / KC) / (Dp / KC) : 32,
                                             wide || 2 * blocks <= sm_count ? 16 : 1, sm_count);
         const dim3 grid((unsigned)blocks, (unsigned)parts.most);
-        // sparse: survivors so rare that eight keys with one mostly hold no second: one store behind a search for its place
-        // (scan of 10^6 x 50: 60.0 -> 54.6 ms, 300 000 x 20: 4.30 -> 3.83); below, a test and a store per key
-        // (30 011 x 32, one key in eight passes: 0.30 -> 0.32 by the test for the flag, 0.33 with the search).  As an
-        // instantiation of its own the sparse form took 61 to 62 ms at 10^6 x 50, in every run: the kernel's code is large,
-        // and where it comes to lie counts.
-        const int sparse = nd >= 131072;
+        // sparse: about 3 L of nd keys pass; where eight keys with one mostly hold no second, it is stored once behind a
+        // search for its place, else there is a test and a store per key.  Both forms, scan in ms (D = 20; 50 is alike):
+        //   L = 128 (K <= 96): 40 000 rows 0.56 / 0.56, 65 536 0.78 / 0.87, 131 072 2.08 / 2.58, 10^6 47.7 / 59.5
+        //   L = 256:           40 000 rows 0.68 / 0.60, 65 536 0.98 / 0.92, 100 000 1.72 / 1.79, 131 072 2.59 / 2.86, 10^6 58.6 / 76.4
+        // so the line is at one key in 128.  As an instantiation of its own the sparse form took 61 to 62 ms at 10^6 x 50, 53 by
+        // this flag: the kernel's code is large, and where it comes to lie counts.
+        const int sparse = nd >= 128ll * 3 * L;
         auto narrow = parts.most > 1 ? (QH == 1 ? knn_tc_filter_kernel<1, false, true> : knn_tc_filter_kernel<2, false, true>)
                                      : (QH == 1 ? knn_tc_filter_kernel<1, false, false> : knn_tc_filter_kernel<2, false, false>);
         if (wide) B200_TRY(allow_smem(knn_tc_wide_kernel<false>, kFilterSmemMax));
