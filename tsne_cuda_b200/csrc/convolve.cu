@@ -175,8 +175,13 @@ __device__ __forceinline__ float kernel_value(int row, int j, float h, float cmi
     // node coordinates in float exactly as the reference forms them, summed and inverted in double (nbodyfft.cu:175-195)
     const float x1 = cmin + h / 2, y1 = cmin + h / 2 + row * h, y2 = cmin + h / 2 + j * h;
     const float da = x1 - y1, db = x1 - y2;
-    const double s = 1.0 + (double)(da * da) + (double)(db * db);
-    return (float)(1.0 / (s * s));
+    const double s = 1.0 + (double)(da * da) + (double)(db * db), t = s * s;
+    if (t > 1e37) return (float)(1.0 / t);
+    // 1 / t by two Newton-Raphson steps from the float reciprocal (off by less than 2^-21): 2^-42, then 2^-84 and one rounding,
+    // so the double that a division gives unless 1 / t lies within 2^-31 of an ulp of a tie.  A division's special cases
+    // put a lane's 28 values in one chain: iteration at 1 500 and 5 000 points 36.5 against 35.0 us.
+    const double r = (double)__fdividef(1.0f, (float)t), r1 = fma(r, fma(-t, r, 1.0), r);
+    return (float)fma(r1, fma(-t, r1, 1.0), r1);
 }
 // completes a lane's half of an even sequence: v[r], r < 14, holds x[28 r + l]; the rest is x[784 - (28 r + l)]
 __device__ __forceinline__ void mirror_input(float2 (&v)[kR], int lane)
