@@ -116,7 +116,7 @@ int b200tsne_knn(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t 
                  int64_t db_hi, int32_t *ids, float *d2, int device);
 
 /* How the last b200tsne_knn call of this thread ran: whether the tensor-core path was used, how many rows
- * its proof could not certify (recomputed by the SIMT search) and the largest observed filter error as a
+ * its proof could not certify (recomputed by exact distances) and the largest observed filter error as a
  * fraction of the assumed bound.  No counterpart in the reference. */
 int b200tsne_knn_last_stats(int *tensor_core, int *rows_recomputed, float *filter_error_ratio);
 

@@ -27,7 +27,7 @@ def test_knn_bit_exact(engine, oracle_cpu, n, d, k):
 @pytest.mark.parametrize("pairs", ["bf16", "tf32"])
 @pytest.mark.parametrize("n,d,k", [(3000, 50, 90), (70000, 30, 150), (420000, 50, 90)])
 def test_knn_tensor_core_paths(engine, oracle_cpu, monkeypatch, n, d, k, pairs):
-    """Online threshold (small), sample -> full (medium) and sample -> strided -> full (large) variants of the
+    """Sample -> full (small and medium) and sample -> strided -> full (large) variants of the
     tensor-core search, with both operand forms of the filter (bf16 pairs are the default): exact on sampled
     queries, and the SIMT fallback is only needed for a few rows."""
     from tsne_cuda_b200 import datasets

@@ -112,7 +112,7 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
 int mbar_wait_selftest(int timeout_ms, float *waited_ms, cudaStream_t st);   // see b200tsne_selftest_bounded_waits
 struct KnnStats {
     int tensor_core = 0;            // 1 when the tensor-core path ran
-    int rows_recomputed = 0;        // rows the proof could not certify, recomputed by the SIMT search
+    int rows_recomputed = 0;        // rows the proof could not certify, recomputed by another search
     float filter_error_ratio = 0;   // largest observed filter error on the candidates / assumed bound
 };
 // X: [N][D] row-major on the device; picks the path, handles the fallback rows, synchronises `st`.

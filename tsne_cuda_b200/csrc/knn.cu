@@ -1,4 +1,5 @@
-// Exact k-nearest-neighbour search, SIMT path.
+// Exact k-nearest-neighbour search: the choice of the path, and the search that keeps a list per query while the database
+// streams by (the others: knn_tc.cu, knn_dense.cu).
 //
 // Replaces the reference's FAISS IVF-Flat call (src/util/distance_utils.cu:79-121, approximate, with
 // results returned to the host as int64 and re-uploaded) by an exact search that stays on the device
@@ -389,8 +390,8 @@ constexpr int64_t kDenseMaxRows = 32768;
 static bool list_pays(int64_t rows, int64_t nd, int K) { return (double)rows * (double)nd > 1e7 * K * sqrt((double)K); }
 
 // Exact search of queries [q_lo,q_hi) against database rows [db_lo,db_hi) of X ([N][D], device),
-// choosing the tensor-core path where it applies and falling back to the SIMT search for the rows it
-// cannot certify.  Unfilled slots keep (INT_MAX, +inf); see launch_knn_finalize.
+// choosing the tensor-core path where it applies and recomputing the rows it cannot certify by one of the
+// other two.  Unfilled slots keep (INT_MAX, +inf); see launch_knn_finalize.
 int knn_search(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo, int64_t db_hi,
                int32_t *ids, float *d2, KnnStats *stats, cudaStream_t st, const PointCells *pc)
 {

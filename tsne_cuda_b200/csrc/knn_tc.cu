@@ -2,7 +2,7 @@
 // dimension in shared memory (D <= 63) and a chunked one for wider points (knn_tc_wide_kernel).
 //
 // Replaces the reference's FAISS IVF-Flat call (src/util/distance_utils.cu:79-121, approximate).
-// The result is the same as the SIMT search of knn.cu: ids ordered by the canonical fp32 distance
+// The result is the same as that of knn.cu's search: ids ordered by the canonical fp32 distance
 // (sequential, unfused) with ties broken by index.  It is obtained in three steps:
 //
 //  1. Filter.  Ranking keys  key_ij = |x_j|^2 - 2 x_i.x_j  come straight out of the tensor cores: the
@@ -15,13 +15,13 @@
 //     TMEM lane each per query tile) and
 //     walks the database in tiles of 128 points; each epilogue thread compares its row of the
 //     accumulator tile with a per-query threshold and appends the rare survivors to the query's
-//     candidate buffer with plain stores; the L = K + slack best are kept.  No N x N matrix is written.
-//  2. Re-rank.  The canonical distance of the L candidates is evaluated exactly and they are ordered by
-//     (distance, id).
-//  3. Proof.  Every point that is not a candidate has a key >= T (the largest key in the list), hence a
+//     candidate buffer with plain stores, about 3 L of them (L = 128 or 256).  No N x N matrix is written.
+//  2. Re-rank.  The canonical distance of the candidates that can be among the K best (their key is within twice the
+//     filter's error of the K-th smallest; at most L) is evaluated exactly and they are ordered by (distance, id).
+//  3. Proof.  Every point that is not evaluated has a key >= T (the threshold, or the smallest one left out), hence a
 //     canonical distance >= (|x_i|^2 + T - E)(1 - theta) with E bounding the filter's error and theta the
 //     rounding of the canonical sum.  If the K-th candidate distance is strictly below that bound the
-//     first K candidates are provably the exact answer; otherwise the row is flagged and recomputed by
+//     first K are provably the exact answer; otherwise the row is flagged and recomputed by
 //     an exact search.  The observed filter error on the candidates is checked against E as well.
 //
 // Operand staging: the prepared operands live in global memory as ready-made shared-memory images, one per 128-row tile
@@ -1018,7 +1018,7 @@ knn_tc_filter_kernel(const float *__restrict__ img_q, const float *__restrict__ 
 // stages of 96 KB: 5 to 9 % slower, 50 000 x 1 024 14.4 against 13.8 ms a scan).  After the
 // last chunk of a unit the sixteen epilogue warps (query tile x database tile x TMEM lane quarter) compare
 // the keys with the fixed thresholds exactly as in the narrow kernel; the next unit's MMAs wait until the
-// accumulators have been read.  Fixed thresholds only (a small database goes to the SIMT search).
+// accumulators have been read.
 constexpr int kWideKC = 16;                       // words of 32 bits per row, chunk and part (32 bf16 values, 16 TF32) = 2 MMA K steps
 constexpr int kWideSwizzle = 64;                  // bytes of such a row: the swizzle of the bf16 images
 constexpr uint32_t kWideChunkBytes = kWideKC * 1024;   // hi + lo of one tile and chunk
@@ -1446,7 +1446,8 @@ template <int EPL> __device__ __forceinline__ void warp_sort(unsigned long long 
 // is so large that more than L remain, the L smallest.  32 rows at a time are staged with asynchronous copies, VEC floats
 // each, whole or 32 dimensions wide in two stages: whole lines per request, where a lane that walks a row of its own
 // touches 32 lines with each.  A lane then reads its row from shared memory and sums in the canonical order.
-// Measured with the pass that used to write the L best out first: LATER.
+// Measured, selection included, before (addresses computed per copy, ranking by counting) and now: 60,000 x 784 5.1 -> 2.6 ms,
+// 50,000 x 1,024 7.7 -> 3.9, 10^6 x 50 15.2 -> 10.6, 100,003 x 96 (K = 32) 1.0 now.
 // EPL: evaluated candidates a lane sorts (L = 32 EPL); the buffer holds up to 8 L.
 template <int VEC, int EPL>
 __global__ void __launch_bounds__(kRerankWarps * 32, EPL <= 4 ? 6 : 4)
@@ -1976,7 +1977,7 @@ static ScanParts scan_parts(int blocks, int tiles, int share, int limit, int sms
 
 // X: [N][D] row-major (device).  ids/d2: [(q_hi-q_lo)][K].  n_failed_host receives the number of rows
 // whose proof did not close; their global row indices are in failed_list (device, first n entries) and
-// the caller recomputes them with the SIMT search.  Returns after the kernels are queued, except for
+// the caller recomputes them (knn_search).  Returns after the kernels are queued, except for
 // the small synchronous read of the counters.
 int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t q_hi, int64_t db_lo, int64_t db_hi, const PointCells &pc,
                   int32_t *ids, float *d2, void *workspace, int **failed_list, int *n_failed_host, float *err_ratio_host,
@@ -2107,11 +2108,10 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
         }
         return 0;
     };
-    // Three levels, each fixing the threshold of the next:
-    //  A  rank ~10 of a few thousand sample points spread over the database -> tau_A,
-    //     chosen so that ~300 points of sample B beat it;
-    //  B  every kSampleStride-th tile against tau_A;
-    //  C  everything against tau_B = the key of rank ~3L/kSampleStride in sample B: ~3L points beat it.
+    // Up to three levels, each fixing the threshold of the next:
+    //  A  a rank up to 16 of a sample of up to 16,384 points spread over the database -> tau_A;
+    //  B  (large databases) every kSampleStride-th tile against a tau_A that ~300 points of it beat;
+    //  C  everything against tau_A, or against the key of rank ~3L/kSampleStride in B: ~3L points beat either.
     // Before each scan the cells are tested against the thresholds it will use; a skipped cell holds no
     // point below them, so the candidate sets (and the sample statistics) are those of a full scan.
     // (the wide kernel strides over units of two tiles: the same 1/kSampleStride of the database)
