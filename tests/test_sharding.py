@@ -97,10 +97,17 @@ def _worker(rank, world, port, q):
         Fr_full, Z_full = cpu.repulsive(Y)
         assert abs((float(z) - N) - Z_full) / abs(Z_full) < 1e-5
         assert rel_l2(Fr[:, lo:hi], Fr_full[:, lo:hi]) < 1e-5
+        # what the engine does instead of that exchange, over peer memory and over collectives: every rank sums charges
+        # times potentials over the nodes of the grid it holds, in double
+        Z = None
+        for grid in (w.numpy().reshape(-1, 4), w_slices):
+            c, p = grid.astype(np.float64), yt.astype(np.float64).reshape(-1, 4)     # (count, x, y, r^2)
+            Z = float(((c[:, 0] + c[:, 3]) * p[:, 0] - 2 * (c[:, 1] * p[:, 1] + c[:, 2] * p[:, 2]) + c[:, 0] * p[:, 3]).sum()) - N
+            assert abs(Z - Z_full) / abs(Z_full) < 1e-5
         Fa = cpu.attractive(P, ids_full, Y, lo, hi)
         g = np.ones((2, N), np.float32)
         u = np.zeros((2, N), np.float32)
-        Ynew, _, _ = cpu.apply_forces(Y, Fa, Fr, g, u, 100.0, float(z) - N, 0.5, 12.0)
+        Ynew, _, _ = cpu.apply_forces(Y, Fa, Fr, g, u, 100.0, Z, 0.5, 12.0)
         mine = np.zeros((2, chunk), np.float32)
         mine[:, :hi - lo] = Ynew[:, lo:hi]
         parts = [torch.zeros((2, chunk)) for _ in range(world)]
