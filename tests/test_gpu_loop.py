@@ -125,11 +125,11 @@ def _steps(engine, monkeypatch, n, graphs, per_call, decay):
 def test_a_schedule_that_changes_at_every_call_is_not_captured_every_time(engine, monkeypatch, n, per_call):
     """A block is captured when it serves again: calls that each bring another learning rate take the time of direct
     launches (a capture and an executable in each call: 2.4 to 3.7 times that; the bar leaves half for a busy host), and
-    calls that repeat a schedule end up below it."""
+    calls that repeat a schedule end up below it (0.6 to 0.9 of it; a tenth for the host)."""
     direct, a = _steps(engine, monkeypatch, n, False, per_call, True)
     changing, b = _steps(engine, monkeypatch, n, True, per_call, True)
     repeated, _ = _steps(engine, monkeypatch, n, True, per_call, False)
     # the bars of the test above: an iteration's forces round to 1e-7 in no fixed order and the loop carries it on, so
     # after up to 180 of them (57 there) momentum is held to 1e-4, which another eta in one call (2 %) exceeds by far
     assert rel_l2(a[0], b[0]) < 1e-6 and rel_l2(a[1], b[1]) < 1e-4 and a[3] == b[3]
-    assert changing < 1.5 * direct and repeated < direct
+    assert changing < 1.5 * direct and repeated < 1.1 * direct
