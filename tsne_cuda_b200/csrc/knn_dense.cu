@@ -102,12 +102,12 @@ __device__ __forceinline__ int block_sum(int v, int *buf)
 constexpr unsigned kInfBits = 0x7f800000u;   // distances are >= 0: their bits order like them; NaN lies above and never ranks
 constexpr int kMaxDenseK = 512;
 
-// One block per (query, segment).  The n values of segment s of query q start at val + q * ld + s * seg; with `ids` they
+// One block per (query, segment).  The n values of segment s of query q start at val + q * ld + s * seg; with `ids` (IDS) they
 // carry the ids at the same place (equal values in ascending order of id), else value j has id id_lo + s * seg + j.  The K
 // smallest by (value, id), ascending, go to out row (q * segments + s), or, with out_rows, to row out_rows[q] - out_base;
 // slots without a value get (+inf, INT_MAX), and where such slots of shorter lists come in again (ids given) they are no
 // values: a neighbour infinitely far away is one, and precedes them.  KPT * 256 >= seg.
-template <int KPT>
+template <int KPT, bool IDS>
 __global__ void __launch_bounds__(kThreads)
 dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ ids, long long ld, long long n_total, long long seg, int id_lo,
                     int K, const int *__restrict__ out_rows, long long out_base, float *__restrict__ out_d, int32_t *__restrict__ out_i)
@@ -127,7 +127,7 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
     for (int j = 0; j < KPT; j++) {
         const int e = j * kThreads + tid;
         key[j] = e < n ? __float_as_uint(val[base + e]) : 0xffffffffu;
-        if (ids && key[j] == kInfBits && ids[base + e] == INT_MAX) key[j] = 0xffffffffu;
+        if (IDS && key[j] == kInfBits && ids[base + e] == INT_MAX) key[j] = 0xffffffffu;
         if (key[j] <= kInfBits) { lo = min(lo, key[j]); hi = max(hi, key[j]); valid++; }
     }
     lo = __reduce_min_sync(0xffffffffu, lo);
@@ -154,7 +154,7 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
         }
         v = b;
     }
-    auto id_of = [&](int e) { return ids ? ids[base + e] : (int32_t)(id_lo + s * seg + e); };
+    auto id_of = [&](int e) { return IDS ? ids[base + e] : (int32_t)(id_lo + s * seg + e); };
     auto keep = [&](int slot, int j) {
         s_key[slot] = (unsigned long long)key[j] << 32 | (unsigned)id_of(j * kThreads + tid);
     };
@@ -204,6 +204,7 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
 
 constexpr long long kMaxSegment = 48 * kThreads;   // values one block selects from (12,288)
 
+template <bool IDS>
 int launch_select(const float *val, const int32_t *ids, long long ld, long long n, long long seg, int segments, long long nq, int id_lo, int K,
                   const int *out_rows, long long out_base, float *out_d, int32_t *out_i, cudaStream_t st)
 {
@@ -215,11 +216,11 @@ int launch_select(const float *val, const int32_t *ids, long long ld, long long 
         const int *r = out_rows ? out_rows + q : nullptr;
         float *od = out_rows ? out_d : out_d + q * segments * K;
         int32_t *oi = out_rows ? out_i : out_i + q * segments * K;
-        if (longest <= 4 * kThreads) dense_select_kernel<4><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
-        else if (longest <= 8 * kThreads) dense_select_kernel<8><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
-        else if (longest <= 16 * kThreads) dense_select_kernel<16><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
-        else if (longest <= 32 * kThreads) dense_select_kernel<32><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
-        else dense_select_kernel<48><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        if (longest <= 4 * kThreads) dense_select_kernel<4, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        else if (longest <= 8 * kThreads) dense_select_kernel<8, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        else if (longest <= 16 * kThreads) dense_select_kernel<16, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        else if (longest <= 32 * kThreads) dense_select_kernel<32, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        else dense_select_kernel<48, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
         B200_CUDA(cudaGetLastError());
     }
     return 0;
@@ -279,22 +280,22 @@ int knn_dense(const float *X, int D, int K, int64_t q_lo, int64_t nq, const int 
         int32_t *final_i = q_index ? ids : ids + q * K;
         B200_TRY(launch_distances(X, D, q_lo + q, m, index, db_lo, nd, dist, ld, st));
         if (segments == 1) {
-            B200_TRY(launch_select(dist, nullptr, ld, nd, seg, 1, m, (int)db_lo, K, index, out_base, final_d, final_i, st));
+            B200_TRY(launch_select<false>(dist, nullptr, ld, nd, seg, 1, m, (int)db_lo, K, index, out_base, final_d, final_i, st));
             continue;
         }
         // the best of every segment, then of those lists (a level more while they are too long for a block)
-        B200_TRY(launch_select(dist, nullptr, ld, nd, seg, segments, m, (int)db_lo, K, nullptr, 0, part_d[0], part_i[0], st));
+        B200_TRY(launch_select<false>(dist, nullptr, ld, nd, seg, segments, m, (int)db_lo, K, nullptr, 0, part_d[0], part_i[0], st));
         long long lists = segments;
         int from = 0;
         while (lists * K > kMaxSegment) {
             const long long per = kMaxSegment / K;   // lists that one block merges
             const long long next = (lists + per - 1) / per;
-            B200_TRY(launch_select(part_d[from], part_i[from], lists * K, lists * K, per * K, (int)next, m, 0, K, nullptr, 0, part_d[from ^ 1],
+            B200_TRY(launch_select<true>(part_d[from], part_i[from], lists * K, lists * K, per * K, (int)next, m, 0, K, nullptr, 0, part_d[from ^ 1],
                                    part_i[from ^ 1], st));
             lists = next;
             from ^= 1;
         }
-        B200_TRY(launch_select(part_d[from], part_i[from], lists * K, lists * K, lists * K, 1, m, 0, K, index, out_base, final_d, final_i, st));
+        B200_TRY(launch_select<true>(part_d[from], part_i[from], lists * K, lists * K, lists * K, 1, m, 0, K, index, out_base, final_d, final_i, st));
     }
     return 0;
 }
@@ -303,9 +304,9 @@ int knn_dense(const float *X, int D, int K, int64_t q_lo, int64_t nq, const int 
 int knn_dense_load()
 {
     cudaFuncAttributes a;
-    const void *kernels[] = {(const void *)dense_distance_kernel<1>, (const void *)dense_distance_kernel<4>, (const void *)dense_select_kernel<4>,
-                             (const void *)dense_select_kernel<8>,   (const void *)dense_select_kernel<16>,  (const void *)dense_select_kernel<32>,
-                             (const void *)dense_select_kernel<48>};
+    const void *kernels[] = {(const void *)dense_distance_kernel<1>, (const void *)dense_distance_kernel<4>, (const void *)dense_select_kernel<4, false>,
+                             (const void *)dense_select_kernel<8, false>,   (const void *)dense_select_kernel<16, false>,  (const void *)dense_select_kernel<32, false>,
+                             (const void *)dense_select_kernel<48, false>};
     for (const void *k : kernels) B200_CUDA(cudaFuncGetAttributes(&a, k));
     return 0;
 }
@@ -320,7 +321,7 @@ int knn_dense_in_scratch(const float *X, int64_t N, int D, int K, float *scratch
     for (int64_t q = 0; q < N; q += round) {
         const int64_t m = std::min<int64_t>(round, N - q);
         B200_TRY(launch_distances(X, D, q, m, nullptr, 0, N, scratch, ld, st));
-        B200_TRY(launch_select(scratch, nullptr, ld, N, N, 1, m, 0, K, nullptr, 0, d2 + q * K, ids + q * K, st));
+        B200_TRY(launch_select<false>(scratch, nullptr, ld, N, N, 1, m, 0, K, nullptr, 0, d2 + q * K, ids + q * K, st));
     }
     return 0;
 }
