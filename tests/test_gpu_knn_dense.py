@@ -34,6 +34,25 @@ def test_host_points(engine, oracle_cpu, n, d, k, ties):
     assert np.array_equal(ids[lo:], ids_o) and np.array_equal(d2[lo:], d2_o)
 
 
+# groups of four threads, of one, none (K = 48 / 49, 192 / 193); as many keys a thread as a kernel has registers for, and one more
+@pytest.mark.parametrize("k", [47, 48, 49, 192, 193])
+@pytest.mark.parametrize("n", [256, 2047, 6144, 6145])
+@pytest.mark.parametrize("equal", [0, 600])
+def test_selection_by_a_bound(engine, oracle_cpu, n, k, equal):
+    """Without ties, and with more equal distances below the bound than there is room for: decided by the index."""
+    import torch
+    X = _points(n, 3, n + k, False)
+    X[n - min(n, equal):] = X[-1]
+    Xd = torch.from_numpy(X).cuda()
+    ids = torch.empty(n, k, dtype=torch.int32, device="cuda")
+    d2 = torch.empty(n, k, dtype=torch.float32, device="cuda")
+    engine.check(engine.lib.b200tsne_knn_noalloc(Xd.data_ptr(), n, 3, k, ids.data_ptr(), d2.data_ptr(), 0))
+    torch.cuda.synchronize()
+    lo = max(0, n - 300)
+    ids_o, d2_o = oracle_cpu.knn(X, k, q_lo=lo, q_hi=n)
+    assert np.array_equal(ids.cpu().numpy()[lo:], ids_o) and np.array_equal(d2.cpu().numpy()[lo:], d2_o)
+
+
 @pytest.mark.parametrize("n,d,k,ties", [(300, 2, 4, False), (4099, 64, 16, False), (4099, 3, 60, True), (12288, 7, 32, True),
                                         (12289, 7, 32, True), (2000, 1000, 9, False)])
 def test_device_points_without_allocation(engine, oracle_cpu, n, d, k, ties):

@@ -5,9 +5,9 @@
 // search could not certify, and callers that must not allocate.  A search that keeps a running list per query
 // (knn_exact_kernel) serves 64 queries per block and inserts survivors one at a time: at 1,500 points that is 24 blocks on
 // 148 SMs, and half of the time goes into insertions.  Here the distances are a plain tiled product over all SMs (three
-// unfused fp32 instructions per pair and dimension, the bound), and the selection is a bisection on the bits of keys
-// held in registers.  Measured on B200 (start of the path / now):
-// 4,099 points of 64 dimensions, K = 16: 1.69 / 0.31 ms; 1,500 x 20, K = 32: 1.63 / 0.06 ms; five rows of 60,000 x 784:
+// unfused fp32 instructions per pair and dimension, the bound), and the selection ranks the few keys, held in registers, that
+// lie below a bound from the smallest keys of groups (many equal keys, K > 192: bisection on the keys' bits).  Measured on B200 (lists / now):
+// 4,099 points of 64 dimensions, K = 16: 1.69 / 0.21 ms; 1,500 x 20, K = 32: 1.63 / 0.03 ms; five rows of 60,000 x 784:
 // 4.4 / 0.4 ms.
 #include <limits.h>
 
@@ -101,6 +101,7 @@ __device__ __forceinline__ int block_sum(int v, int *buf)
 
 constexpr unsigned kInfBits = 0x7f800000u;   // distances are >= 0: their bits order like them; NaN lies above and never ranks
 constexpr int kMaxDenseK = 512;
+constexpr int kGroupMaxK = 192;   // with 256 groups, about 256 ln(256 / (256 - K)) keys lie at or below the bound: 355
 
 // One block per (query, segment).  The n values of segment s of query q start at val + q * ld + s * seg; with `ids` (IDS) they
 // carry the ids at the same place (equal values in ascending order of id), else value j has id id_lo + s * seg + j.  The K
@@ -113,6 +114,8 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
                     int K, const int *__restrict__ out_rows, long long out_base, float *__restrict__ out_d, int32_t *__restrict__ out_i)
 {
     __shared__ unsigned long long s_key[kMaxDenseK];
+    __shared__ __align__(16) unsigned s_min[kThreads];
+    __shared__ unsigned s_bound;
     __shared__ int s_sum[2][kThreads / 32];
     __shared__ unsigned s_lo[kThreads / 32], s_hi[kThreads / 32];
     __shared__ int s_n, s_before;
@@ -130,10 +133,65 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
         if (IDS && key[j] == kInfBits && ids[base + e] == INT_MAX) key[j] = 0xffffffffu;
         if (key[j] <= kInfBits) { lo = min(lo, key[j]); hi = max(hi, key[j]); valid++; }
     }
+    auto id_of = [&](int e) { return IDS ? ids[base + e] : (int32_t)(id_lo + s * seg + e); };
+    auto composed = [&](int j) { return (unsigned long long)key[j] << 32 | (unsigned)id_of(j * kThreads + tid); };
+    const long long row = out_rows ? out_rows[q] - out_base : q * gridDim.x + s;
+    if (tid == 0) { s_n = 0; s_before = 0; s_bound = 0xffffffffu; }
+    // The K-th smallest of the smallest keys of disjoint groups bounds the K-th smallest key from above, and little more than K
+    // keys lie below it.  Four barriers instead of the bisection's thirty: whole search of 4,099 x 64, K = 16 318 -> 226 us,
+    // 1,500 x 20, K = 32 33.3 -> 25.2, 9,000 x 40 1,095 -> 840.
+    if (K <= kGroupMaxK) {
+        // groups of four threads while they are several times K: ranking them is that much shorter
+        const bool fours = K <= kGroupMaxK / 4;
+        unsigned m = lo;
+        if (fours) {
+            m = min(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = min(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        }
+        const int groups = fours ? kThreads / 4 : kThreads;
+        s_min[fours ? tid >> 2 : tid] = m;
+        __syncthreads();
+        if (tid < groups) {
+            m = s_min[tid];
+            int at_or_below = 0;
+#pragma unroll 4
+            for (int u = 0; u < groups; u += 4) {
+                const uint4 o = *reinterpret_cast<const uint4 *>(s_min + u);
+                at_or_below += (o.x <= m) + (o.y <= m) + (o.z <= m) + (o.w <= m);
+            }
+            m = __reduce_min_sync(0xffffffffu, at_or_below >= K ? m : 0xffffffffu);
+            if (lane == 0) atomicMin(&s_bound, m);
+        }
+        __syncthreads();
+        const unsigned bound = s_bound;
+        if (bound <= kInfBits) {   // else fewer than K groups have a key at all
+#pragma unroll
+            for (int j = 0; j < KPT; j++)
+                if (key[j] <= bound) {
+                    const int slot = atomicAdd(&s_n, 1);
+                    if (slot < kMaxDenseK) s_key[slot] = composed(j);
+                }
+            __syncthreads();
+            const int below = s_n;
+            if (below <= kMaxDenseK) {
+                for (int e = tid; e < below; e += kThreads) {
+                    const unsigned long long mine = s_key[e];
+                    int rank = 0;
+                    for (int u = 0; u < below; u++) rank += s_key[u] < mine;
+                    if (rank < K) {
+                        out_d[row * K + rank] = __uint_as_float((unsigned)(mine >> 32));
+                        out_i[row * K + rank] = (int32_t)(unsigned)mine;
+                    }
+                }
+                return;
+            }
+            __syncthreads();   // many equal keys: more than there is room for
+            if (tid == 0) s_n = 0;
+        }
+    }
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
     if (lane == 0) { s_lo[warp] = lo; s_hi[warp] = hi; }
-    if (tid == 0) { s_n = 0; s_before = 0; }
     int turn = 0;
     valid = block_sum(valid, s_sum[turn++ & 1]);
 #pragma unroll
@@ -154,15 +212,11 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
         }
         v = b;
     }
-    auto id_of = [&](int e) { return IDS ? ids[base + e] : (int32_t)(id_lo + s * seg + e); };
-    auto keep = [&](int slot, int j) {
-        s_key[slot] = (unsigned long long)key[j] << 32 | (unsigned)id_of(j * kThreads + tid);
-    };
     const bool ties = valid > K && at_most > K;   // more keys equal to v than there is room for: the first in order of id
     if (valid > 0) {
 #pragma unroll
         for (int j = 0; j < KPT; j++)
-            if (key[j] <= kInfBits && (ties ? key[j] < v : key[j] <= v)) keep(atomicAdd(&s_n, 1), j);
+            if (key[j] <= kInfBits && (ties ? key[j] < v : key[j] <= v)) s_key[atomicAdd(&s_n, 1)] = composed(j);
     }
     __syncthreads();
     if (ties) {
@@ -187,7 +241,6 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
     __syncthreads();
     // rank by counting: K is at most a few hundred
     const int got = min(valid, K);
-    const long long row = out_rows ? out_rows[q] - out_base : q * gridDim.x + s;
     for (int e = tid; e < K; e += kThreads) {
         if (e < got) {
             const unsigned long long mine = s_key[e];
@@ -219,6 +272,7 @@ int launch_select(const float *val, const int32_t *ids, long long ld, long long 
         if (longest <= 4 * kThreads) dense_select_kernel<4, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
         else if (longest <= 8 * kThreads) dense_select_kernel<8, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
         else if (longest <= 16 * kThreads) dense_select_kernel<16, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        else if (longest <= 24 * kThreads) dense_select_kernel<24, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
         else if (longest <= 32 * kThreads) dense_select_kernel<32, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
         else dense_select_kernel<48, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
         B200_CUDA(cudaGetLastError());
@@ -248,6 +302,15 @@ int launch_distances(const float *X, int D, int64_t q_lo, int64_t nq, const int 
 long long padded(long long nd) { return (nd + kTileP - 1) / kTileP * kTileP; }
 }  // namespace
 
+// Queries of one round of several: alike, in whole blocks of 64, where `most` would leave a short last round (4,099 x 64: five
+// rounds of 832, three blocks of distances an SM in each, instead of four of 960 and one of 259: 226 -> 211 us).
+static int64_t even_round(int64_t nq, int64_t most)
+{
+    if (nq <= most || most < 64) return most;
+    const int64_t rounds = (nq + most - 1) / most;
+    return std::min(most, ((nq + rounds - 1) / rounds + 63) / 64 * 64);
+}
+
 bool knn_dense_supported(int K) { return K <= kMaxDenseK; }
 
 // Queries [q_lo, q_lo + nq), or the nq rows that q_index lists, against database rows [db_lo, db_hi); the list of query
@@ -265,6 +328,7 @@ int knn_dense(const float *X, int D, int K, int64_t q_lo, int64_t nq, const int 
     // blocks, the second with three queries: 3,000 rows 49 ms against 33)
     int64_t round = std::max<int64_t>(1, std::min<int64_t>(nq, (1ll << 26) / ld));
     if (round < nq && round >= 16) round -= round % (round >= 64 ? 64 : 16);
+    round = even_round(nq, round);
     float *dist = nullptr, *part_d[2] = {nullptr, nullptr};
     int32_t *part_i[2] = {nullptr, nullptr};
     B200_TRY(tmp.alloc((void **)&dist, sizeof(float) * (size_t)round * ld));
@@ -305,7 +369,8 @@ int knn_dense_load()
 {
     cudaFuncAttributes a;
     const void *kernels[] = {(const void *)dense_distance_kernel<1>, (const void *)dense_distance_kernel<4>, (const void *)dense_select_kernel<4, false>,
-                             (const void *)dense_select_kernel<8, false>,   (const void *)dense_select_kernel<16, false>,  (const void *)dense_select_kernel<32, false>,
+                             (const void *)dense_select_kernel<8, false>,   (const void *)dense_select_kernel<16, false>,
+                             (const void *)dense_select_kernel<24, false>, (const void *)dense_select_kernel<32, false>,
                              (const void *)dense_select_kernel<48, false>};
     for (const void *k : kernels) B200_CUDA(cudaFuncGetAttributes(&a, k));
     return 0;
@@ -316,8 +381,9 @@ int knn_dense_load()
 int knn_dense_in_scratch(const float *X, int64_t N, int D, int K, float *scratch, long long floats, int32_t *ids, float *d2, cudaStream_t st)
 {
     const long long ld = padded(N);
-    const int64_t round = floats / ld / 64 * 64;
-    if (N > kMaxSegment || !knn_dense_supported(K) || round < 64) return -1;
+    const int64_t most = floats / ld / 64 * 64;
+    if (N > kMaxSegment || !knn_dense_supported(K) || most < 64) return -1;
+    const int64_t round = even_round(N, most);
     for (int64_t q = 0; q < N; q += round) {
         const int64_t m = std::min<int64_t>(round, N - q);
         B200_TRY(launch_distances(X, D, q, m, nullptr, 0, N, scratch, ld, st));
