@@ -171,19 +171,23 @@ __global__ void twiddle_init_kernel(float2 *tw)
 __device__ __forceinline__ int column_of(int k) { return k < kC ? k : kM - k; }
 __device__ __forceinline__ int slot_of(int k) { return k < kC ? 0 : 1; }
 
-// ---- spectrum of the kernel, first axis: two real rows per warp ----
+// ---- spectrum of the kernel, first axis: a row per warp.  Two rows could share a transform, but a lane then evaluates 28
+// values instead of 14, and the evaluation is as long as the transform: iteration at 1,500 / 5,000 / 20,011 points
+// 34.4 / 37.1 / 39.5 -> 32.4 / 34.5 / 38.4 us. ----
 __device__ __forceinline__ float kernel_value(int row, int j, float h, float cmin)
 {
     // node coordinates in float exactly as the reference forms them, summed and inverted in double (nbodyfft.cu:175-195)
     const float x1 = cmin + h / 2, y1 = cmin + h / 2 + row * h, y2 = cmin + h / 2 + j * h;
     const float da = x1 - y1, db = x1 - y2;
     const double s = 1.0 + (double)(da * da) + (double)(db * db), t = s * s;
-    if (t > 1e37) return (float)(1.0 / t);
     // 1 / t by two Newton-Raphson steps from the float reciprocal (off by less than 2^-21): 2^-42, then 2^-84 and one rounding,
-    // so the double that a division gives unless 1 / t lies within 2^-31 of an ulp of a tie.  A division's special cases
-    // put a lane's 28 values in one chain: iteration at 1 500 and 5 000 points 36.5 against 35.0 us.
-    const double r = (double)__fdividef(1.0f, (float)t), r1 = fma(r, fma(-t, r, 1.0), r);
-    return (float)fma(r1, fma(-t, r1, 1.0), r1);
+    // so the double that a division gives unless 1 / t lies within 2^-31 of an ulp of a tie.  Beyond the range of floats
+    // scaled by a power of two.  No branch: a lane's values are independent, and a branch in each (a division's special cases,
+    // a range check) puts them in one chain.
+    const bool big = t > 1e37;
+    const double ts = big ? t * 0x1p-160 : t;
+    const double r = (double)__fdividef(1.0f, (float)ts), r1 = fma(r, fma(-ts, r, 1.0), r), r2 = fma(r1, fma(-ts, r1, 1.0), r1);
+    return (float)(t > 1e78 ? 0.0 : big ? r2 * 0x1p-160 : r2);
 }
 // completes a lane's half of an even sequence: v[r], r < 14, holds x[28 r + l]; the rest is x[784 - (28 r + l)]
 __device__ __forceinline__ void mirror_input(float2 (&v)[kR], int lane)
@@ -208,7 +212,7 @@ spectrum_rows_kernel(float *__restrict__ Rk, const IterState *state, int slot, c
     __shared__ float2 exch[kSpecWarps][kEx];
     copy_twiddles<kSpecWarps * 32>(tws, tw);
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    const int row = 2 * (blockIdx.x * kSpecWarps + wi);
+    const int row = blockIdx.x * kSpecWarps + wi;
     const GridGeom g = load_geom(state, slot);
     const float h = g.box_width / (float)kInterp;
     float2 v[kR];
@@ -216,7 +220,8 @@ spectrum_rows_kernel(float *__restrict__ Rk, const IterState *state, int slot, c
     for (int r = 0; r < kHalf; r++) {
         const int j = kR * r + lane;
         const bool in = lane < kR && j < kG;
-        v[r] = make_float2(in ? kernel_value(row, j, h, g.cmin) : 0.0f, in ? kernel_value(row + 1, j, h, g.cmin) : 0.0f);
+        const float value = kernel_value(row, j, h, g.cmin);   // evaluated in all lanes: no branch around it
+        v[r] = make_float2(in ? value : 0.0f, 0.0f);
     }
     mirror_input(v, lane);
     copies_done();
@@ -227,7 +232,6 @@ spectrum_rows_kernel(float *__restrict__ Rk, const IterState *state, int slot, c
         const int k = kR * r + lane;
         if (k < kRkStride) {
             Rk[(size_t)row * kRkStride + k] = v[r].x;
-            if (row + 1 < kG) Rk[(size_t)(row + 1) * kRkStride + k] = v[r].y;
         }
     }
 }
@@ -416,7 +420,7 @@ int fft_workspace_init(FftWorkspace *ws, void *mem, cudaStream_t st)
 
 int launch_kernel_spectrum(const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st)
 {
-    constexpr int row_blocks = (kG / 2 + kSpecWarps - 1) / kSpecWarps, col_blocks = ((kC + 1) / 2 + kSpecWarps - 1) / kSpecWarps;
+    constexpr int row_blocks = (kG + kSpecWarps - 1) / kSpecWarps, col_blocks = ((kC + 1) / 2 + kSpecWarps - 1) / kSpecWarps;
     spectrum_rows_kernel<<<row_blocks, kSpecWarps * 32, 0, st>>>(ws.Rk, state, slot, ws.tw);
     B200_CUDA(cudaGetLastError());
     spectrum_columns_kernel<<<col_blocks, kSpecWarps * 32, 0, st>>>(ws.Rk, ws.Kh, ws.tw);
