@@ -992,6 +992,11 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
     // when the copy holds all rows, one in three when it holds a rank's share; B200TSNE_ATTRACTIVE_BLOCKS overrides.
     static const int want_blocks = getenv("B200TSNE_ATTRACTIVE_BLOCKS") ? atoi(getenv("B200TSNE_ATTRACTIVE_BLOCKS")) : 0;
     sms = want_blocks > 0 ? std::min(sms, want_blocks) : (b.rows == b.N ? sms - sms / 9 : sms - sms / 3);
+    // A small graph keeps fewer SMs from the pipeline, which is what the iteration waits for there: about sixteen chunks a warp
+    // (1 us each) are done before the potentials are.  Blocks 132 / 48 / 24 / 12 / 6, us an iteration: 1,500 x 32 (400
+    // chunks) 34.8 / 31.4 / 31.0 / 31.0 / 30.9; 5,000 x 90 (3,500) 39.5 / 31.9 / 31.3 / 31.3 / 31.4; 20,011 x 90 (14,100)
+    // 39.8 / 34.6 / 34.2 / 42.5 / 72.1; 60,000 x 90 (42,000) on 132 / 96 / 64 51.6 / 49.2 / 48.5.
+    if (want_blocks <= 0) sms = std::min(sms, std::max(6, b.C / (16 * kBlockedThreads / 32)));
     const int grid = std::max(1, std::min(sms, b.C));
     attractive_blocked_kernel<<<grid, kBlockedThreads, (size_t)b.T * sizeof(float2), st>>>(s, Yp, Yown, b.N, Fp);
     if (b.extra_C > 0) {   // the reverse-only entries of a truly symmetric P add to the same forces

@@ -48,6 +48,7 @@ void set_destroy(StreamSet *s)
     if (s->ev_t1) cudaEventDestroy(s->ev_t1);
     if (s->stream) cudaStreamDestroy(s->stream);
     if (s->stream2) cudaStreamDestroy(s->stream2);
+    if (s->stream3) cudaStreamDestroy(s->stream3);
     if (s->h_state) cudaFreeHost(s->h_state);
     delete s;
 }
@@ -56,6 +57,7 @@ int set_create(StreamSet *s)
 {
     B200_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     B200_CUDA(cudaStreamCreateWithFlags(&s->stream2, cudaStreamNonBlocking));
+    B200_CUDA(cudaStreamCreateWithFlags(&s->stream3, cudaStreamNonBlocking));
     B200_CUDA(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming));
     B200_CUDA(cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming));
     B200_CUDA(cudaEventCreateWithFlags(&s->ev_spectrum, cudaEventDisableTiming));
@@ -226,7 +228,8 @@ void stream_set_release(StreamSet *s)
         delete s;
         return;
     }
-    const bool fine = cudaStreamSynchronize(s->stream) == cudaSuccess && cudaStreamSynchronize(s->stream2) == cudaSuccess;
+    const bool fine = cudaStreamSynchronize(s->stream) == cudaSuccess && cudaStreamSynchronize(s->stream2) == cudaSuccess &&
+                      cudaStreamSynchronize(s->stream3) == cudaSuccess;
     if (fine) {
         std::lock_guard<std::mutex> hold(g_lock);
         int idle = 0;

@@ -21,7 +21,7 @@ unsigned long long context_id();
 struct StreamSet {
     int device = -1;
     unsigned long long context = 0;   // its handles are of this context
-    cudaStream_t stream = nullptr, stream2 = nullptr;
+    cudaStream_t stream = nullptr, stream2 = nullptr, stream3 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     IterState *h_state = nullptr;   // pinned
     // Executable graphs that finished sessions left behind.  Instantiating one of 16 iterations takes 1.3 ms (now and

@@ -33,6 +33,7 @@ struct Session {
     StreamSet *host = nullptr;       // the streams, events and pinned memory below come from here
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;  // attractive force overlaps the grid pipeline
+    cudaStream_t stream3 = nullptr;  // and so does the kernel's spectrum
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     DeviceArena arena;
 
