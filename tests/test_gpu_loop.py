@@ -133,3 +133,21 @@ def test_a_schedule_that_changes_at_every_call_is_not_captured_every_time(engine
     # after up to 180 of them (57 there) momentum is held to 1e-4, which another eta in one call (2 %) exceeds by far
     assert rel_l2(a[0], b[0]) < 1e-6 and rel_l2(a[1], b[1]) < 1e-4 and a[3] == b[3]
     assert changing < 1.5 * direct and repeated < 1.1 * direct
+
+
+@pytest.mark.parametrize("n", [1, 33, 21845, 21846])
+def test_state_goes_in_and_out_unchanged(engine, n):
+    """Both sides of the largest state that crosses in one piece; a second state right behind the first."""
+    P, ids, rng = _graph(n, 3, n)
+    a, b = [[rng.normal(0, 1, (2, n)).astype(np.float32) for _ in range(3)] for _ in range(2)]
+    with engine.Session(n, 3) as s:
+        s.set_affinities(P, ids)
+        s.set_state(*a, 4)
+        s.set_state(*b, 7)
+        got = s.get_state()
+        assert got[3] == 7 and all(np.array_equal(x, y) for x, y in zip(got, b))
+        assert np.array_equal(s.get_embedding(), b[0])
+        s.set_state(*a, 9)
+        s.run(1)
+        Y, u, _, step = s.get_state()
+        assert step == 10 and np.array_equal(Y, a[0] + u)    # the step was taken from the first state

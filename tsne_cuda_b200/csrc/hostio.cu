@@ -50,6 +50,7 @@ void set_destroy(StreamSet *s)
     if (s->stream2) cudaStreamDestroy(s->stream2);
     if (s->stream3) cudaStreamDestroy(s->stream3);
     if (s->h_state) cudaFreeHost(s->h_state);
+    if (s->io) cudaFreeHost(s->io);
     delete s;
 }
 
@@ -64,6 +65,7 @@ int set_create(StreamSet *s)
     B200_CUDA(cudaEventCreate(&s->ev_t0));
     B200_CUDA(cudaEventCreate(&s->ev_t1));
     B200_CUDA(cudaMallocHost((void **)&s->h_state, sizeof(IterState)));
+    B200_CUDA(cudaMallocHost((void **)&s->io, StreamSet::kIoBytes));
     return 0;
 }
 

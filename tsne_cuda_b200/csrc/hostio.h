@@ -24,6 +24,9 @@ struct StreamSet {
     cudaStream_t stream = nullptr, stream2 = nullptr, stream3 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     IterState *h_state = nullptr;   // pinned
+    // Pinned memory that kernels read and write across the bus: the state of a small map in one piece (Session::small_state).
+    static constexpr size_t kIoBytes = (size_t)512 << 10;
+    float *io = nullptr;
     // Executable graphs that finished sessions left behind.  Instantiating one of 16 iterations takes 1.3 ms (now and
     // then 100 on a busy host) and destroying it another; updating one of the same shape takes 0.1 ms.  They hold stale
     // addresses and are only launched after an update.

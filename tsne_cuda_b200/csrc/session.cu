@@ -250,6 +250,42 @@ int Session::set_optimizer_soa(const float *momentum_host, const float *gains_ho
     return 0;
 }
 
+bool Session::small_state() const
+{
+    return rows() == N && !(comm && comm->world > 1) && sizeof(float) * 6 * (size_t)N <= StreamSet::kIoBytes;
+}
+
+int Session::set_small_state(const float *Y_host, const float *momentum_host, const float *gains_host, int at_step)
+{
+    B200_CUDA(cudaSetDevice(device));
+    B200_CUDA(cudaStreamSynchronize(stream));   // an earlier state may still be on its way out of the same memory
+    const size_t block = 2 * (size_t)N;
+    memcpy(host->io, Y_host, sizeof(float) * block);
+    memcpy(host->io + block, momentum_host, sizeof(float) * block);
+    memcpy(host->io + 2 * block, gains_host, sizeof(float) * block);
+    step = at_step;
+    done_seen = 0;
+    B200_TRY(launch_state_reset(state, stream));
+    B200_TRY(launch_load_state(host->io, Y2, u, gains, N, state_order(), state, step & 1, stream));
+    B200_CUDA(cudaMemsetAsync(w, 0, sizeof(float4) * kG * kG, stream));
+    launches += 2;
+    return 0;
+}
+
+// null arrays are not asked for
+int Session::get_small_state(float *Y_host, float *momentum_host, float *gains_host)
+{
+    B200_CUDA(cudaSetDevice(device));
+    B200_TRY(launch_store_state(Y_host ? Y2 : nullptr, momentum_host ? u : nullptr, gains_host ? gains : nullptr, host->io, N, state_order(), stream));
+    B200_CUDA(cudaStreamSynchronize(stream));
+    const size_t block = 2 * (size_t)N;
+    float *to[3] = {Y_host, momentum_host, gains_host};
+    for (int k = 0; k < 3; k++)
+        if (to[k]) memcpy(to[k], host->io + k * block, sizeof(float) * block);
+    launches += 1;
+    return 0;
+}
+
 namespace {
 // Times the stages of one iteration when stage timers are on (serialised on one stream).
 struct StageClock {

@@ -129,6 +129,45 @@ __global__ void aos_to_soa_kernel(const float2 *aos, float *soa, long long N, co
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) { const long long j = perm ? perm[i] : i; const float2 v = aos[i]; soa[j] = v.x; soa[N + j] = v.y; }
 }
+__global__ void __launch_bounds__(256)
+load_state_kernel(const float *io, float2 *Y2, float2 *u2, float2 *gains2, long long N, const int32_t *perm, IterState *state, int slot)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    float mn = INFINITY, mx = -INFINITY;
+    if (i < N) {
+        const long long j = perm ? perm[i] : i;
+        const float2 y = make_float2(io[j], io[N + j]);
+        Y2[i] = y;
+        u2[i] = make_float2(io[2 * N + j], io[3 * N + j]);
+        gains2[i] = make_float2(io[4 * N + j], io[5 * N + j]);
+        mn = fminf(y.x, y.y);
+        mx = fmaxf(y.x, y.y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((threadIdx.x & 31) == 0 && mn <= mx) {
+        atomicMin(&state->min_enc[slot], enc_float(mn));
+        atomicMax(&state->max_enc[slot], enc_float(mx));
+    }
+}
+__global__ void __launch_bounds__(256)
+store_state_kernel(const float2 *Y2, const float2 *u2, const float2 *gains2, float *io, long long N, const int32_t *perm)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    const long long j = perm ? perm[i] : i;
+    const float2 *from[3] = {Y2, u2, gains2};
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+        if (from[a]) {
+            const float2 v = from[a][i];
+            io[2 * a * N + j] = v.x;
+            io[(2 * a + 1) * N + j] = v.y;
+        }
+}
 // dst[q] = src[perm[q]] (gather) or dst[perm[q]] = src[q] (scatter)
 __global__ void reorder_pairs_kernel(const float2 *src, float2 *dst, long long N, const int32_t *perm, int scatter)
 {
@@ -184,6 +223,22 @@ int launch_aos_to_soa(const float2 *aos, float *soa, int64_t N, cudaStream_t st,
 {
     if (N <= 0) return 0;
     aos_to_soa_kernel<<<nblk(N, 256), 256, 0, st>>>(aos, soa, N, perm);
+    B200_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int launch_load_state(const float *io, float2 *Y2, float2 *u2, float2 *gains2, int64_t N, const int32_t *perm, IterState *state, int slot,
+                      cudaStream_t st)
+{
+    if (N <= 0) return 0;
+    load_state_kernel<<<nblk(N, 256), 256, 0, st>>>(io, Y2, u2, gains2, N, perm, state, slot);
+    B200_CUDA(cudaGetLastError());
+    return 0;
+}
+int launch_store_state(const float2 *Y2, const float2 *u2, const float2 *gains2, float *io, int64_t N, const int32_t *perm, cudaStream_t st)
+{
+    if (N <= 0) return 0;
+    store_state_kernel<<<nblk(N, 256), 256, 0, st>>>(Y2, u2, gains2, io, N, perm);
     B200_CUDA(cudaGetLastError());
     return 0;
 }
