@@ -7,7 +7,7 @@
 // 148 SMs, and half of the time goes into insertions.  Here the distances are a plain tiled product over all SMs (three
 // unfused fp32 instructions per pair and dimension, the bound), and the selection ranks the few keys, held in registers, that
 // lie below a bound from the smallest keys of groups (many equal keys, K > 192: bisection on the keys' bits).  Measured on B200 (lists / now):
-// 4,099 points of 64 dimensions, K = 16: 1.69 / 0.21 ms; 1,500 x 20, K = 32: 1.63 / 0.03 ms; five rows of 60,000 x 784:
+// 4,099 points of 64 dimensions, K = 16: 1.69 / 0.20 ms; 1,500 x 20, K = 32: 1.63 / 0.03 ms; five rows of 60,000 x 784:
 // 4.4 / 0.4 ms.
 #include <limits.h>
 
@@ -22,22 +22,47 @@ constexpr int kTileP = 128;    // database points per tile
 constexpr int kDims = 32;      // dimensions per shared-memory chunk
 constexpr int kThreads = 256;
 
+// Two canonical operations at a time: each half rounds as the single instruction does.  The square is a fused operation with
+// -0, an argument of the kernel: of a packed product and a packed sum the compiler makes one rounding.  The fp32 pipe is as
+// busy as with single instructions, but half as many are issued: 4,099 x 64, K = 16 211 -> 201 us,
+// 10,000 x 100, K = 40 1,943 -> 1,827 (whole searches).
+constexpr unsigned long long kMinusZero2 = 0x8000000080000000ull;
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void add_square2(unsigned long long &acc, unsigned long long q, unsigned long long minus_p, unsigned long long minus_zero)
+{
+    asm("{\n\t.reg .b64 t;\n\t"
+        "add.rn.f32x2 t, %1, %2;\n\tfma.rn.f32x2 t, t, t, %3;\n\tadd.rn.f32x2 %0, %0, t;\n\t}"
+        : "+l"(acc)
+        : "l"(q), "l"(minus_p), "l"(minus_zero));
+}
+
 // dist[q * ld + p] = canonical distance (sequential over the dimensions, every operation rounded) of query q of the list
 // and database row db_lo + p.  QT queries and eight points a thread, 16 QT queries and 128 points a block.
 template <int QT>
 __global__ void __launch_bounds__(kThreads)
 dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long long nq, const int *__restrict__ q_index, long long db_lo,
-                      long long nd, float *__restrict__ dist, long long ld)
+                      long long nd, float *__restrict__ dist, long long ld, unsigned long long minus_zero)
 {
     constexpr int kTileQ = 16 * QT, kQs = kTileQ + 4, kPs = kTileP + 4;
     __shared__ __align__(16) float Qs[kDims][kQs], Ps[kDims][kPs];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31, warp = tid >> 5;
     const long long p0 = (long long)blockIdx.x * kTileP, q0 = (long long)blockIdx.y * kTileQ;
-    float acc[QT][8];
+    unsigned long long acc[QT][4];
 #pragma unroll
     for (int a = 0; a < QT; a++)
 #pragma unroll
-        for (int b = 0; b < 8; b++) acc[a][b] = 0.0f;
+        for (int b = 0; b < 4; b++) acc[a][b] = 0ull;
     for (int d0 = 0; d0 < D; d0 += kDims) {
         const int dlen = min(kDims, D - d0);
         __syncthreads();
@@ -51,7 +76,7 @@ dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long l
         for (int p = warp; p < kTileP; p += kThreads / 32) {
             float v = 0.0f;
             if (p0 + p < nd && lane < dlen) v = X[(db_lo + p0 + p) * D + d0 + lane];
-            Ps[lane][p] = v;
+            Ps[lane][p] = -v;   // the difference as a sum
         }
         __syncthreads();
 #pragma unroll 4
@@ -66,14 +91,13 @@ dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long l
             }
             const float4 pa = *reinterpret_cast<const float4 *>(&Ps[d][tx * 4]);
             const float4 pb = *reinterpret_cast<const float4 *>(&Ps[d][64 + tx * 4]);
-            const float pv[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
+            const unsigned long long pv[4] = {pack2(pa.x, pa.y), pack2(pa.z, pa.w), pack2(pb.x, pb.y), pack2(pb.z, pb.w)};
 #pragma unroll
-            for (int a = 0; a < QT; a++)
+            for (int a = 0; a < QT; a++) {
+                const unsigned long long qq = pack2(qv[a], qv[a]);
 #pragma unroll
-                for (int b = 0; b < 8; b++) {
-                    const float t = __fsub_rn(qv[a], pv[b]);
-                    acc[a][b] = __fadd_rn(acc[a][b], __fmul_rn(t, t));
-                }
+                for (int b = 0; b < 4; b++) add_square2(acc[a][b], qq, pv[b], minus_zero);
+            }
         }
     }
     // (rows of dist are padded to whole tiles: every store stays inside)
@@ -82,8 +106,9 @@ dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long l
         const long long q = q0 + ty * QT + a;
         if (q >= nq) continue;
         float *row = dist + q * ld + p0;
-        *reinterpret_cast<float4 *>(row + tx * 4) = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
-        *reinterpret_cast<float4 *>(row + 64 + tx * 4) = make_float4(acc[a][4], acc[a][5], acc[a][6], acc[a][7]);
+        const float2 d0 = unpack2(acc[a][0]), d1 = unpack2(acc[a][1]), d2 = unpack2(acc[a][2]), d3 = unpack2(acc[a][3]);
+        *reinterpret_cast<float4 *>(row + tx * 4) = make_float4(d0.x, d0.y, d1.x, d1.y);
+        *reinterpret_cast<float4 *>(row + 64 + tx * 4) = make_float4(d2.x, d2.y, d3.x, d3.y);
     }
 }
 
@@ -290,10 +315,10 @@ int launch_distances(const float *X, int D, int64_t q_lo, int64_t nq, const int 
         for (int64_t q = 0; q < nq; q += 65535 * 64) {
             const int64_t m = std::min<int64_t>(65535 * 64, nq - q);
             dense_distance_kernel<4><<<dim3(tiles, (unsigned)((m + 63) / 64)), kThreads, 0, st>>>(X, D, q_lo + q, m, q_index ? q_index + q : nullptr,
-                                                                                               db_lo, nd, dist + q * ld, ld);
+                                                                                               db_lo, nd, dist + q * ld, ld, kMinusZero2);
         }
     } else {
-        dense_distance_kernel<1><<<dim3(tiles, (unsigned)((nq + 15) / 16)), kThreads, 0, st>>>(X, D, q_lo, nq, q_index, db_lo, nd, dist, ld);
+        dense_distance_kernel<1><<<dim3(tiles, (unsigned)((nq + 15) / 16)), kThreads, 0, st>>>(X, D, q_lo, nq, q_index, db_lo, nd, dist, ld, kMinusZero2);
     }
     B200_CUDA(cudaGetLastError());
     return 0;
