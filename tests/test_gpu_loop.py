@@ -151,3 +151,39 @@ def test_state_goes_in_and_out_unchanged(engine, n):
         s.run(1)
         Y, u, _, step = s.get_state()
         assert step == 10 and np.array_equal(Y, a[0] + u)    # the step was taken from the first state
+
+
+@pytest.mark.parametrize("n", [2000, 21846])
+@pytest.mark.parametrize("where", ["YMG", "Y", "G"])
+def test_state_in_device_memory(engine, n, where):
+    """Arrays of a state may stand in device memory, some or all of them, at any size."""
+    import ctypes as C
+
+    import torch
+    P, ids, rng = _graph(n, 3, n)
+    host = [rng.normal(0, 1, (2, n)).astype(np.float32) for _ in range(3)]
+
+    def at(arrays):
+        return [C.cast(a.data_ptr() if torch.is_tensor(a) else a.ctypes.data, C.POINTER(C.c_float)) for a in arrays]
+
+    def there(arrays):
+        return [torch.from_numpy(a).cuda() if k in where else a.copy() for k, a in zip("YMG", arrays)]
+
+    with engine.Session(n, 3) as s:
+        s.set_affinities(P, ids)
+        given = there(host)
+        torch.cuda.synchronize()
+        engine.check(engine.lib.b200tsne_session_set_state(s._h, *at(given), 4))
+        got = s.get_state()
+        assert got[3] == 4 and all(np.array_equal(a, b) for a, b in zip(got, host))
+        out = there([np.zeros_like(a) for a in host])
+        torch.cuda.synchronize()
+        step = C.c_int()
+        engine.check(engine.lib.b200tsne_session_get_state(s._h, *at(out), C.byref(step)))
+        torch.cuda.synchronize()
+        assert step.value == 4 and all(np.array_equal(torch.as_tensor(a).cpu().numpy(), b) for a, b in zip(out, host))
+        Y = there([np.zeros_like(host[0])])[0]
+        torch.cuda.synchronize()
+        engine.check(engine.lib.b200tsne_session_get_embedding(s._h, at([Y])[0]))
+        torch.cuda.synchronize()
+        assert np.array_equal(torch.as_tensor(Y).cpu().numpy(), host[0])

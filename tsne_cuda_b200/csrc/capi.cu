@@ -455,13 +455,13 @@ int b200tsne_session_set_embedding(b200tsne_session *h, const float *Y, int rese
 int b200tsne_session_get_embedding(b200tsne_session *h, float *Y)
 {
     if (!h || !Y) { set_error("session_get_embedding: invalid arguments"); return B200TSNE_ERR_INVALID; }
-    return h->s.small_state() ? h->s.get_small_state(Y, nullptr, nullptr) : h->s.get_embedding_soa(Y);
+    return h->s.small_state(Y, nullptr, nullptr) ? h->s.get_small_state(Y, nullptr, nullptr) : h->s.get_embedding_soa(Y);
 }
 
 int b200tsne_session_get_state(b200tsne_session *h, float *Y, float *momentum, float *gains, int *step)
 {
     if (!h) { set_error("session_get_state: null session"); return B200TSNE_ERR_INVALID; }
-    if (h->s.small_state()) {
+    if (h->s.small_state(Y, momentum, gains)) {
         if (Y || momentum || gains) B200_TRY(h->s.get_small_state(Y, momentum, gains));
     } else {
         if (Y) B200_TRY(h->s.get_embedding_soa(Y));
@@ -480,7 +480,7 @@ int b200tsne_session_set_state(b200tsne_session *h, const float *Y, const float 
         set_error("session_set_state: in a sharded session the step must keep the parity of the current step");
         return B200TSNE_ERR_UNSUPPORTED;
     }
-    if (momentum && gains && s.small_state()) return s.set_small_state(Y, momentum, gains, step);
+    if (momentum && gains && s.small_state(Y, momentum, gains)) return s.set_small_state(Y, momentum, gains, step);
     s.step = step;                       // set_embedding prepares the min/max slot of this step
     B200_TRY(s.set_embedding_soa(Y, false));
     return s.set_optimizer_soa(momentum, gains);

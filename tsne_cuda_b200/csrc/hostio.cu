@@ -139,15 +139,16 @@ void stage_release(Stage *g)
     stage_destroy(g);
 }
 
-bool pageable(const void *p)
+cudaMemoryType memory_type(const void *p)
 {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         (void)cudaGetLastError();
-        return true;
+        return cudaMemoryTypeUnregistered;
     }
-    return a.type == cudaMemoryTypeUnregistered;
+    return a.type;
 }
+bool pageable(const void *p) { return memory_type(p) == cudaMemoryTypeUnregistered; }
 
 int lanes_for(size_t bytes)
 {
@@ -181,6 +182,12 @@ template <class F> cudaError_t on_lanes(int lanes, int device, F body)
 }
 
 }  // namespace
+
+bool plain_host(const void *p)
+{
+    const cudaMemoryType t = memory_type(p);
+    return t == cudaMemoryTypeUnregistered || t == cudaMemoryTypeHost;
+}
 
 unsigned long long context_id()
 {

@@ -52,6 +52,8 @@ void graph_exec_release(StreamSet *s, cudaGraphExec_t exec, unsigned long long s
 int copy_in(void *dst_device, const void *src_host, size_t bytes, cudaStream_t st);
 int copy_out(void *dst_host, const void *src_device, size_t bytes, cudaStream_t st);
 
+bool plain_host(const void *p);   // host memory, pinned or not: neither device nor managed memory, which a copy takes as well
+
 void host_pools_release(int device);   // idle sets and staging memory of one device
 
 }  // namespace b200

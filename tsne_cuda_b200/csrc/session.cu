@@ -250,9 +250,12 @@ int Session::set_optimizer_soa(const float *momentum_host, const float *gains_ho
     return 0;
 }
 
-bool Session::small_state() const
+bool Session::small_state(const void *Y, const void *momentum, const void *gains) const
 {
-    return rows() == N && !(comm && comm->world > 1) && sizeof(float) * 6 * (size_t)N <= StreamSet::kIoBytes;
+    if (rows() != N || (comm && comm->world > 1) || sizeof(float) * 6 * (size_t)N > StreamSet::kIoBytes) return false;
+    for (const void *p : {Y, momentum, gains})
+        if (p && !plain_host(p)) return false;
+    return true;
 }
 
 int Session::set_small_state(const float *Y_host, const float *momentum_host, const float *gains_host, int at_step)

@@ -147,7 +147,8 @@ struct Session {
     // the three arrays from and to pageable memory, each with a kernel and a wait, are most of a call that runs an iteration
     // or two: 2,000 points, state in, one iteration,
     // state out 183 -> 117 us; 5,000 points, state in, 200 iterations, embedding out 7.08 -> 6.52 ms.
-    bool small_state() const;
+    // The host reads and writes the caller's arrays itself, so those in device or managed memory (null: not given) go by copies.
+    bool small_state(const void *Y, const void *momentum, const void *gains) const;
     int set_small_state(const float *Y_host, const float *momentum_host, const float *gains_host, int at_step);
     int get_small_state(float *Y_host, float *momentum_host, float *gains_host);
     int iterate(int n_iters, float min_gradient_norm, float *elapsed_ms, int *iters_done);
