@@ -216,7 +216,7 @@ int b200tsne_session_get_embedding(b200tsne_session *s, float *Y);
 /* Checkpoint and resume of the loop: the embedding (2N floats SoA, all points), the owned rows' momentum (the
  * reference's old_forces) and gains (2 * rows floats SoA each; NULL = skip) and the iteration number, which
  * selects momentum, exaggeration and the spread-order refresh.  Like the embedding of the calls above, the arrays may stand
- * in host or device memory.  A session restored with set_state continues as the saved one would have.  Replaces: TSNE_INIT::RESUME (src/include/options.h:24), which the reference
+ * in host or device memory; both calls return when the state has arrived.  A session restored with set_state continues as the saved one would have.  Replaces: TSNE_INIT::RESUME (src/include/options.h:24), which the reference
  * declares for this purpose but implements as a copy of the points alone (src/fit_tsne.cu:205-217). */
 int b200tsne_session_get_state(b200tsne_session *s, float *Y, float *momentum, float *gains, int *step);
 int b200tsne_session_set_state(b200tsne_session *s, const float *Y, const float *momentum, const float *gains, int step);

@@ -187,3 +187,22 @@ def test_state_in_device_memory(engine, n, where):
         engine.check(engine.lib.b200tsne_session_get_embedding(s._h, at([Y])[0]))
         torch.cuda.synchronize()
         assert np.array_equal(torch.as_tensor(Y).cpu().numpy(), host[0])
+
+
+@pytest.mark.parametrize("n", [2000, 21845, 21846])
+def test_set_state_returns_when_the_state_has_arrived(engine, n):
+    """Nothing is left on the device when set_state returns: waiting for it takes what waiting for an idle device does (half
+    a megabyte still on its way: 30 us more)."""
+    import torch
+    P, ids, rng = _graph(n, 3, n)
+    a = [rng.normal(0, 1, (2, n)).astype(np.float32) for _ in range(3)]
+    left, idle = [], []
+    with engine.Session(n, 3) as s:
+        s.set_affinities(P, ids)
+        for _ in range(301):
+            s.set_state(*a, 4)
+            for t in (left, idle):
+                t0 = time.perf_counter()
+                torch.cuda.synchronize()
+                t.append(time.perf_counter() - t0)
+    assert sorted(left)[150] < 1.5 * sorted(idle)[150] + 2e-6

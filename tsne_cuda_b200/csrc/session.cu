@@ -261,7 +261,6 @@ bool Session::small_state(const void *Y, const void *momentum, const void *gains
 int Session::set_small_state(const float *Y_host, const float *momentum_host, const float *gains_host, int at_step)
 {
     B200_CUDA(cudaSetDevice(device));
-    B200_CUDA(cudaStreamSynchronize(stream));   // an earlier state may still be on its way out of the same memory
     const size_t block = 2 * (size_t)N;
     memcpy(host->io, Y_host, sizeof(float) * block);
     memcpy(host->io + block, momentum_host, sizeof(float) * block);
@@ -271,6 +270,9 @@ int Session::set_small_state(const float *Y_host, const float *momentum_host, co
     B200_TRY(launch_state_reset(state, stream));
     B200_TRY(launch_load_state(host->io, Y2, u, gains, N, state_order(), state, step & 1, stream));
     B200_CUDA(cudaMemsetAsync(w, 0, sizeof(float4) * kG * kG, stream));
+    // like the copying path: the call's work and its errors are its own (left queued, 8 us of a set_state, run(1), get_state
+    // of 110 moved into the next call), and the pinned memory is free for the next state
+    B200_CUDA(cudaStreamSynchronize(stream));
     launches += 2;
     return 0;
 }
