@@ -2,10 +2,14 @@
 reference kernel's golden output, the CPU oracle, the live reference kernel and the row-major kernel.
 Arithmetic to match: ComputePijxQijKernelV3 + reduce_sum_kernel, src/kernels/attr_forces.cu:129-184.
 Bar: 1e-5 relative L2, as for the row-major kernel."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
-from conftest import mixture, rel_l2
+from conftest import ROOT, mixture, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -155,3 +159,41 @@ def test_state_in_cell_order_and_in_natural_order_agree(engine, oracle_cpu, monk
         s.set_state(Ya, ma, ga, step_a)
         Y2, m2, g2, st2 = s.get_state()
         assert np.array_equal(Y2, Ya) and np.array_equal(m2, ma) and np.array_equal(g2, ga) and st2 == step_a
+
+
+TIMES = """
+import numpy as np
+from tsne_cuda_b200 import _lib as e
+n, k = int(%r), 90
+rng = np.random.default_rng(1)
+X = (rng.normal(0, 10, (4, 50))[np.arange(n) %% 4] + rng.normal(0, 1, (n, 50))).astype(np.float32)
+Y = rng.normal(0, 10, (2, n)).astype(np.float32)
+with e.Session(n, k) as s:
+    s.affinities_from_points(X, 30.0, 1e-3)
+    s.set_schedule(10.0, 12.0, 250, 0.5, 0.8)
+    loop = []
+    for _ in range(7):
+        s.set_state(Y, np.zeros_like(Y), np.ones_like(Y), 500)
+        loop.append(s.run(96)[0] / 96)
+    s.enable_stage_timers(True)
+    total = [0.0]
+    for _ in range(61):
+        s.run(1)
+        total.append(s.stage_times()["attractive"][0])
+    print(sorted(loop)[3] * 1e3, float(np.median(np.diff(total))) * 1e3)
+"""
+
+
+def _times(n, blocks):
+    """(microseconds of a settled iteration, of the attractive stage alone)"""
+    env = dict(os.environ)
+    env.pop("B200TSNE_ATTRACTIVE_BLOCKS", None)
+    if blocks:
+        env["B200TSNE_ATTRACTIVE_BLOCKS"] = str(blocks)
+    out = subprocess.run([sys.executable, "-c", TIMES % n], check=True, cwd=ROOT, timeout=200, env=env, capture_output=True, text=True).stdout
+    return [float(x) for x in out.split()[-2:]]
+
+
+def test_the_attractive_stage_alone_takes_the_sms(engine):
+    """With nothing beside it a small graph is spread over as many SMs as a large one (18 us on 132, 28 on 27 of them)."""
+    assert _times(20011, 0)[1] < 1.25 * _times(20011, 132)[1]

@@ -958,7 +958,7 @@ int blocked_attractive_build(BlockedAttractive *b, DeviceArena &arena, const flo
 // (Reading the force in cell order from the update kernel and letting it keep the cell-ordered embedding current
 // instead of these two conversion kernels was measured on one GPU: the update kernel's three scattered 8-byte
 // accesses per point cost it 148 us more - 169 instead of 21 - against the 17 us the conversions take.)
-int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, float2 *F2, cudaStream_t st, bool in_cell_order)
+int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, float2 *F2, cudaStream_t st, bool in_cell_order, bool beside_grid)
 {
     if (!b.ready) { set_error("attractive: the blocked copy of P was not built"); return -1; }
     if (in_cell_order && b.rows != b.N) { set_error("attractive: the cell order as the caller's order needs all rows"); return -1; }
@@ -996,7 +996,9 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
     // (1 us each) are done before the potentials are.  Blocks 132 / 48 / 24 / 12 / 6, us an iteration: 1,500 x 32 (400
     // chunks) 34.8 / 31.4 / 31.0 / 31.0 / 30.9; 5,000 x 90 (3,500) 39.5 / 31.9 / 31.3 / 31.3 / 31.4; 20,011 x 90 (14,100)
     // 39.8 / 34.6 / 34.2 / 42.5 / 72.1; 60,000 x 90 (42,000) on 132 / 96 / 64 51.6 / 49.2 / 48.5.
-    if (want_blocks <= 0) sms = std::min(sms, std::max(6, b.C / (16 * kBlockedThreads / 32)));
+    // Not where nothing runs beside it (20,011 x 90 alone: 18 us on 132 blocks, 28 on 27), nor for a rank's share, whose counts
+    // above were measured without it.
+    if (want_blocks <= 0 && beside_grid && b.rows == b.N) sms = std::min(sms, std::max(6, b.C / (16 * kBlockedThreads / 32)));
     const int grid = std::max(1, std::min(sms, b.C));
     attractive_blocked_kernel<<<grid, kBlockedThreads, (size_t)b.T * sizeof(float2), st>>>(s, Yp, Yown, b.N, Fp);
     if (b.extra_C > 0) {   // the reverse-only entries of a truly symmetric P add to the same forces

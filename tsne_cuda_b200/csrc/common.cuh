@@ -184,7 +184,9 @@ int blocked_attractive_build(BlockedAttractive *b, DeviceArena &arena, const flo
                              int64_t row_lo, int64_t row_hi, const int32_t *perm, const ExtraEntries *extra, cudaStream_t st);
 int launch_exclusive_scan_i32(int *data, int64_t n, cudaStream_t st);   // in place; small arrays (one block)
 // in_cell_order: Y2 and F2 are in the copy's own point order (one GPU): no conversion before or after the kernel
-int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, float2 *F2, cudaStream_t st, bool in_cell_order = false);
+// beside_grid: the grid pipeline runs at the same time
+int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, float2 *F2, cudaStream_t st, bool in_cell_order = false,
+                              bool beside_grid = false);
 
 // repulsive.cu
 struct FftWorkspace {

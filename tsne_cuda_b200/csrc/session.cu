@@ -442,7 +442,7 @@ int Session::one_iteration(int norm_mode, float stop_norm)
 
 int Session::attractive(cudaStream_t st)
 {
-    if (blocked.ready) return launch_attractive_blocked(blocked, Y2, Fattr, st, resident);
+    if (blocked.ready) return launch_attractive_blocked(blocked, Y2, Fattr, st, resident, /*beside_grid=*/!stage_timers);
     B200_TRY(launch_attractive(P, ids, Y2, N, K, row_lo, row_hi, Fattr, st));
     if (extra.count > 0) B200_TRY(launch_attractive_extra(extra.ptr, extra.ids, extra.val, Y2, N, row_lo, row_hi, Fattr, st));
     return 0;
