@@ -197,3 +197,9 @@ def _times(n, blocks):
 def test_the_attractive_stage_alone_takes_the_sms(engine):
     """With nothing beside it a small graph is spread over as many SMs as a large one (18 us on 132, 28 on 27 of them)."""
     assert _times(20011, 0)[1] < 1.25 * _times(20011, 132)[1]
+
+
+def test_a_settled_map_of_middle_size_is_not_slower_on_fewer_sms(engine):
+    """45,000 points, settled: 43 us an iteration on 132 SMs, 38 where one wave of the columns pass fits beside the attractive
+    kernel, 45 on a number of SMs in between."""
+    assert _times(45000, 0)[0] < 0.97 * _times(45000, 132)[0]

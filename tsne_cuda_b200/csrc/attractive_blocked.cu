@@ -855,6 +855,44 @@ int build_stream(StreamOut *out, DeviceArena &arena, DeviceArena &tmp, WalkArgs 
 }
 }  // namespace
 
+static int device_sms(int *sms)
+{
+    static int cached[64] = {0};
+    int dev = 0;
+    B200_CUDA(cudaGetDevice(&dev));
+    *sms = 148;
+    if (dev >= 0 && dev < 64) {
+        if (!cached[dev]) B200_CUDA(cudaDeviceGetAttribute(&cached[dev], cudaDevAttrMultiProcessorCount, dev));
+        *sms = cached[dev];
+    }
+    return 0;
+}
+
+// Blocks (SMs) of the attractive kernel of an iteration on one GPU, whose grid pipeline runs beside it on the SMs that are left.
+// A small graph is done before the potentials are, so the pipeline is what the iteration waits for, and its longest
+// kernel, the columns pass, has 393 blocks, four to an SM: on 99 SMs or more one wave, on fewer two.  So the graph takes a block per sixteen
+// chunks a warp (1 us each) and at most the SMs that one wave leaves (49 of 148), while it is done in the time that the
+// pipeline and the update need: 12 us a launch and 1 us a chunk of a warp, up to 48 us.  A larger graph takes what it takes
+// at any size (one SM in nine left, see launch_attractive_blocked): between the two the columns wait for a second wave as well.
+// us an iteration, exaggerated / settled, 90 neighbours (703 chunks per 1,000 points), on 24 | 49 | 64 | 80 | 96 | 132 blocks:
+//   20,011  34.0 / 34.0 | 34.4 / 34.5 | 34.0 / 33.9 | 35.3 / 35.1 | 36.9 / 36.9 | 39.2 / 39.2
+//   45,000  49.0 / 50.4 | 46.0 / 37.8 | 47.0 / 44.7 | 46.7 / 44.0 | 46.7 / 41.7 | 50.5 / 43.2
+//   60,000  59.0 / 60.3 | 48.7 / 40.7 | 47.8 / 44.8 | 48.3 / 44.8 | 48.8 / 44.9 | 51.0 / 45.2
+//   80,000  76.3 / 77.4 | 50.9 / 48.5 | 54.0 / 51.9 | 51.4 / 49.4 | 54.0 / 50.2 | 53.2 / 48.9
+//   100,000 93.3 / 93.7 | 55.3 / 55.9 | 61.0 / 51.0 | 54.9 / 51.9 | 54.4 / 53.8 | 56.2 / 51.6
+// (5,000: 31.3 on 6 to 24 blocks, 39.5 on 132.)  The entries of a truly symmetric P come in a second launch behind the
+// first, so both streams count, and 12 us less are left: 20,011 points on 24 | 32 | 49 | 132 blocks 45.0 | 36.8 | 35.3 | 42.2; 30,011 on 49 |
+// 80 | 132 40.1 | 41.2 | 45.0.  Larger ones were best between the two counts, 45,000 settled on 49 | 80 | 132 53.8 | 47.9 | 51.7, 60,000 63.1 |
+// 51.8 | 55.3: sixteen chunks a warp of the first stream, 24 of both.
+static int blocks_beside_grid(int sms, int wave_sms, long long C, long long extra_C)
+{
+    constexpr long long warps = kBlockedThreads / 32;
+    const long long most = sms - sms / 9, spare = std::min<long long>(most, sms - wave_sms);
+    const long long all = C + extra_C;
+    if (all <= spare * warps * (extra_C > 0 ? 24 : 36)) return (int)std::max(6ll, std::min(spare, all / (16 * warps)));
+    return (int)(extra_C > 0 ? std::min(most, std::max(C / (16 * warps), all / (24 * warps))) : most);
+}
+
 // Builds the blocked copy of the owned rows' fixed-width P and, with `extra`, a second stream from a variable-width
 // list of further entries of the same rows (the reverse-only edges of a truly symmetric P).  perm (device, [N];
 // null = identity) is the order of the points; persistent buffers come from `arena`.  On return b->ready says
@@ -946,6 +984,10 @@ int blocked_attractive_build(BlockedAttractive *b, DeviceArena &arena, const flo
     b->C = main_stream.C; b->E = main_stream.E; b->groups = main_stream.groups;
     b->extra_ev = extra_stream.ev; b->extra_ec = extra_stream.ec; b->extra_chunk_row0 = extra_stream.chunk_row0;
     b->extra_tile_chunk0 = extra_stream.tile_chunk0; b->extra_C = extra_stream.C; b->extra_E = extra_stream.E;
+    int sms = 0, wave_sms = 0;
+    B200_TRY(device_sms(&sms));
+    B200_TRY(convolve_wave_sms(&wave_sms));
+    b->beside_blocks = blocks_beside_grid(sms, wave_sms, b->C, b->extra_C);
     b->perm = perm; b->own_perm = own_perm; b->own_pos = own_pos;
     b->Yp = Yp; b->Yown = Yown; b->Fp = Fp;
     b->ntiles = ntiles; b->T = T;
@@ -973,16 +1015,8 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
     BlockedStream s;
     s.ev = b.ev; s.ec = b.ec; s.chunk_row0 = b.chunk_row0; s.tile_chunk0 = b.tile_chunk0;
     s.ntiles = b.ntiles; s.T = b.T; s.C = b.C;
-    int sms = 148;
-    {
-        static int cached[64] = {0};
-        int dev = 0;
-        B200_CUDA(cudaGetDevice(&dev));
-        if (dev >= 0 && dev < 64) {
-            if (!cached[dev]) B200_CUDA(cudaDeviceGetAttribute(&cached[dev], cudaDevAttrMultiProcessorCount, dev));
-            sms = cached[dev];
-        }
-    }
+    int sms = 0;
+    B200_TRY(device_sms(&sms));
     // A block fills its SM (1,024 threads, all registers, 224 KB of shared memory), so the grid pipeline that runs
     // beside this kernel on the other stream only gets the SMs this kernel leaves alone.  Measured at N = 10^6,
     // K = 90 on 148 SMs, one GPU: 148 blocks 3,645 iterations/s (attractive stage 175 us), 140: 3,906, 132: 3,962
@@ -992,13 +1026,9 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
     // when the copy holds all rows, one in three when it holds a rank's share; B200TSNE_ATTRACTIVE_BLOCKS overrides.
     static const int want_blocks = getenv("B200TSNE_ATTRACTIVE_BLOCKS") ? atoi(getenv("B200TSNE_ATTRACTIVE_BLOCKS")) : 0;
     sms = want_blocks > 0 ? std::min(sms, want_blocks) : (b.rows == b.N ? sms - sms / 9 : sms - sms / 3);
-    // A small graph keeps fewer SMs from the pipeline, which is what the iteration waits for there: about sixteen chunks a warp
-    // (1 us each) are done before the potentials are.  Blocks 132 / 48 / 24 / 12 / 6, us an iteration: 1,500 x 32 (400
-    // chunks) 34.8 / 31.4 / 31.0 / 31.0 / 30.9; 5,000 x 90 (3,500) 39.5 / 31.9 / 31.3 / 31.3 / 31.4; 20,011 x 90 (14,100)
-    // 39.8 / 34.6 / 34.2 / 42.5 / 72.1; 60,000 x 90 (42,000) on 132 / 96 / 64 51.6 / 49.2 / 48.5.
-    // Not where nothing runs beside it (20,011 x 90 alone: 18 us on 132 blocks, 28 on 27), nor for a rank's share, whose counts
-    // above were measured without it.
-    if (want_blocks <= 0 && beside_grid && b.rows == b.N) sms = std::min(sms, std::max(6, b.C / (16 * kBlockedThreads / 32)));
+    // Beside the pipeline a small graph takes fewer (see blocks_beside_grid), but not where nothing runs beside it (20,011 x 90
+    // alone: 18 us on 132 blocks, 28 on 27), nor for a rank's share, whose counts above were measured without that rule.
+    if (want_blocks <= 0 && beside_grid && b.rows == b.N) sms = b.beside_blocks;
     const int grid = std::max(1, std::min(sms, b.C));
     attractive_blocked_kernel<<<grid, kBlockedThreads, (size_t)b.T * sizeof(float2), st>>>(s, Yp, Yown, b.N, Fp);
     if (b.extra_C > 0) {   // the reverse-only entries of a truly symmetric P add to the same forces

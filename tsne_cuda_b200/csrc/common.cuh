@@ -174,6 +174,7 @@ struct BlockedAttractive {
     float2 *Yp = nullptr, *Yown = nullptr, *Fp = nullptr;
     int ntiles = 0, T = 0, C = 0;
     int64_t E = 0, groups = 0, N = 0, row_lo = 0, rows = 0;
+    int beside_blocks = 0;            // of the kernel where the grid pipeline runs at the same time and the copy holds all rows
     float entries_per_group = 0.0f;   // of the sampled rows, under the chosen order
     bool ready = false;
     void clear();
@@ -214,6 +215,7 @@ int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, int32
 // needs both; the last pass adds sum_i Z_i over all charges to state->zsum[slot] and clears w when asked to
 int launch_kernel_spectrum(const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
 int launch_convolve_rows(const float4 *w, const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
+int convolve_wave_sms(int *sms);   // SMs that hold all blocks of the columns pass at once
 int launch_convolve(float4 *w, float4 *ytilde, IterState *state, int slot, const FftWorkspace &ws, bool zero_w, cudaStream_t st);
 int launch_gather(const float2 *Y2, int64_t row_lo, int64_t row_hi, const IterState *state, int slot, InterpConsts ic,
                   const float4 *ytilde, float2 *Frep2, cudaStream_t st);
