@@ -53,6 +53,60 @@ def test_selection_by_a_bound(engine, oracle_cpu, n, k, equal):
     assert np.array_equal(ids.cpu().numpy()[lo:], ids_o) and np.array_equal(d2.cpu().numpy()[lo:], d2_o)
 
 
+def _awkward(n, d, kind):
+    """Points for which the smallest keys of the selection's groups say little about the K-th smallest key."""
+    rng = np.random.default_rng(n + d)
+    if kind == "period":                                     # a class's points stand 256 rows apart
+        return (rng.normal(0, 10, (256, d))[np.arange(n) % 256] + rng.normal(0, 1, (n, d))).astype(np.float32)
+    if kind == "binary":
+        return rng.integers(0, 2, (n, d)).astype(np.float32)
+    X = rng.normal(0, 1, (n, d)).astype(np.float32)          # "copies": most points are one
+    X[rng.random(n) < 0.8] = X[0]
+    return X
+
+
+def _noalloc(engine, Xd, k):
+    import torch
+    ids = torch.empty(len(Xd), k, dtype=torch.int32, device="cuda")
+    d2 = torch.empty(len(Xd), k, dtype=torch.float32, device="cuda")
+    engine.check(engine.lib.b200tsne_knn_noalloc(Xd.data_ptr(), *Xd.shape, k, ids.data_ptr(), d2.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    return ids, d2
+
+
+# fewer keys than are ranked at once; a full block of places and one more; both sides of every number of keys a thread holds
+@pytest.mark.parametrize("k", [16, 48, 90, 192, 300])
+@pytest.mark.parametrize("n", [100, 256, 257, 1024, 1025, 4096, 4097, 6145, 8192, 8193, 12288])
+@pytest.mark.parametrize("kind", ["period", "binary", "copies"])
+def test_selection_where_the_bound_is_loose(engine, oracle_cpu, kind, n, k):
+    import torch
+    X, k = _awkward(n, 7, kind), min(k, n)
+    ids, d2 = _noalloc(engine, torch.from_numpy(X).cuda(), k)
+    lo = max(0, n - 100)
+    ids_o, d2_o = oracle_cpu.knn(X, k, q_lo=lo, q_hi=n)
+    assert np.array_equal(ids.cpu().numpy()[lo:], ids_o) and np.array_equal(d2.cpu().numpy()[lo:], d2_o)
+
+
+@pytest.mark.parametrize("n,d,k", [(4099, 16, 90), (9000, 40, 16)])
+@pytest.mark.parametrize("kind", ["period", "binary", "copies"])
+def test_points_with_a_period_or_copies_take_no_longer(engine, kind, n, d, k):
+    """Neither neighbours at equal steps in the array nor many equal distances cost more than a fifth (1.6 and 1.45 times as long
+    where the bound is thrown away for them)."""
+    import torch
+    took = []
+    for X in (np.random.default_rng(1).normal(0, 1, (n, d)).astype(np.float32), _awkward(n, d, kind)):
+        Xd, times = torch.from_numpy(X).cuda(), []
+        for _ in range(9):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(5):
+                _noalloc(engine, Xd, k)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        took.append(sorted(times)[4])
+    assert took[1] < 1.2 * took[0]
+
+
 @pytest.mark.parametrize("n,d,k,ties", [(300, 2, 4, False), (4099, 64, 16, False), (4099, 3, 60, True), (12288, 7, 32, True),
                                         (12289, 7, 32, True), (2000, 1000, 9, False)])
 def test_device_points_without_allocation(engine, oracle_cpu, n, d, k, ties):

@@ -6,7 +6,7 @@
 // (knn_exact_kernel) serves 64 queries per block and inserts survivors one at a time: at 1,500 points that is 24 blocks on
 // 148 SMs, and half of the time goes into insertions.  Here the distances are a plain tiled product over all SMs (three
 // unfused fp32 instructions per pair and dimension, the bound), and the selection ranks the few keys, held in registers, that
-// lie below a bound from the smallest keys of groups (many equal keys, K > 192: bisection on the keys' bits).  Measured on B200 (lists / now):
+// lie below a bound from the smallest keys of groups (short rows, long lists: bisection on the keys' bits).  Measured on B200 (lists / now):
 // 4,099 points of 64 dimensions, K = 16: 1.69 / 0.20 ms; 1,500 x 20, K = 32: 1.63 / 0.03 ms; five rows of 60,000 x 784:
 // 4.4 / 0.4 ms.
 #include <limits.h>
@@ -126,21 +126,31 @@ __device__ __forceinline__ int block_sum(int v, int *buf)
 
 constexpr unsigned kInfBits = 0x7f800000u;   // distances are >= 0: their bits order like them; NaN lies above and never ranks
 constexpr int kMaxDenseK = 512;
-constexpr int kGroupMaxK = 192;   // with 256 groups, about 256 ln(256 / (256 - K)) keys lie at or below the bound: 355
+constexpr int kFewMore = 64;      // keys beyond K that are ranked rather than sorted out by further rounds of bisection
+// Lists of up to kFoursMaxK take the groups of the bound from four threads' keys each, longer ones from one thread's, and beyond kGroupMaxK, or
+// in rows of at most 2,048 keys, none: 256 smallest keys are ranked whatever the row's length (1,500 x 20, K = 90 39.5 us by a bound,
+// 35 by bisection, 2,047 x 20, K = 150 66 / 54, 3,000 x 20, K = 150 118 / 118), and ranking the 256 ln(256 / (256 - K)) or so that lie at or
+// below the bound takes their number's square (9,000 x 20, K = 150 758 / 887, K = 192 929 / 928).
+constexpr int kFoursMaxK = 48;
+constexpr int kGroupMaxK = 160;
+
+// Blocks an SM: what the keys leave registers for (unasked, the compiler took 64 instead of 48 for 24 keys, 201 -> 209 us at 4,099 x 64).
+constexpr int select_blocks(int kpt) { return kpt > 32 ? 3 : kpt > 16 ? 4 : kpt > 8 ? 5 : kpt > 4 ? 6 : 8; }
 
 // One block per (query, segment).  The n values of segment s of query q start at val + q * ld + s * seg; with `ids` (IDS) they
 // carry the ids at the same place (equal values in ascending order of id), else value j has id id_lo + s * seg + j.  The K
 // smallest by (value, id), ascending, go to out row (q * segments + s), or, with out_rows, to row out_rows[q] - out_base;
 // slots without a value get (+inf, INT_MAX), and where such slots of shorter lists come in again (ids given) they are no
 // values: a neighbour infinitely far away is one, and precedes them.  KPT * 256 >= seg.
-template <int KPT, bool IDS>
-__global__ void __launch_bounds__(kThreads)
+// LONG: lists of more than kFoursMaxK.
+template <int KPT, bool IDS, bool LONG>
+__global__ void __launch_bounds__(kThreads, select_blocks(KPT))
 dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ ids, long long ld, long long n_total, long long seg, int id_lo,
                     int K, const int *__restrict__ out_rows, long long out_base, float *__restrict__ out_d, int32_t *__restrict__ out_i)
 {
     __shared__ unsigned long long s_key[kMaxDenseK];
-    __shared__ __align__(16) unsigned s_min[kThreads];
-    __shared__ unsigned s_bound;
+    __shared__ __align__(16) unsigned s_min[kThreads], s_four[kThreads / 4];
+    __shared__ unsigned s_bound, s_least;
     __shared__ int s_sum[2][kThreads / 32];
     __shared__ unsigned s_lo[kThreads / 32], s_hi[kThreads / 32];
     __shared__ int s_n, s_before;
@@ -149,53 +159,65 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
     const long long base = q * ld + s * seg;
     const int n = (int)min(seg, n_total - s * seg);
     unsigned key[KPT];
-    unsigned lo = 0xffffffffu, hi = 0u;
-    int valid = 0;
+    unsigned lo = 0xffffffffu;
 #pragma unroll
     for (int j = 0; j < KPT; j++) {
         const int e = j * kThreads + tid;
         key[j] = e < n ? __float_as_uint(val[base + e]) : 0xffffffffu;
         if (IDS && key[j] == kInfBits && ids[base + e] == INT_MAX) key[j] = 0xffffffffu;
-        if (key[j] <= kInfBits) { lo = min(lo, key[j]); hi = max(hi, key[j]); valid++; }
+        lo = min(lo, key[j]);
+        // A group's smallest key so far goes from thread to thread of the warp.  Were a group the keys of one thread, points whose
+        // neighbours stand 256 apart (classes in turn, lines of a raster) would have whole classes in one group, and a bound with
+        // thousands of keys below: 4,099 x 16, K = 90 255 us, so 155; 9,000 x 40, K = 16 1,166, so 784 (without a period: 151, 798).
+        if (LONG || (j & 1)) lo = __shfl_sync(0xffffffffu, lo, (lane + 5) & 31);
     }
     auto id_of = [&](int e) { return IDS ? ids[base + e] : (int32_t)(id_lo + s * seg + e); };
     auto composed = [&](int j) { return (unsigned long long)key[j] << 32 | (unsigned)id_of(j * kThreads + tid); };
     const long long row = out_rows ? out_rows[q] - out_base : q * gridDim.x + s;
-    if (tid == 0) { s_n = 0; s_before = 0; s_bound = 0xffffffffu; }
+    if (tid == 0) { s_n = 0; s_before = 0; s_bound = s_least = 0xffffffffu; }
+    unsigned hi = 0u;
+    int known = 0;   // 1: hi is a key with at least K keys <= it; 2: and it is the K-th smallest
     // The K-th smallest of the smallest keys of disjoint groups bounds the K-th smallest key from above, and little more than K
-    // keys lie below it.  Four barriers instead of the bisection's thirty: whole search of 4,099 x 64, K = 16 318 -> 226 us,
-    // 1,500 x 20, K = 32 33.3 -> 25.2, 9,000 x 40 1,095 -> 840.
-    if (K <= kGroupMaxK) {
-        // groups of four threads while they are several times K: ranking them is that much shorter
-        const bool fours = K <= kGroupMaxK / 4;
-        unsigned m = lo;
-        if (fours) {
-            m = min(m, __shfl_xor_sync(0xffffffffu, m, 1));
-            m = min(m, __shfl_xor_sync(0xffffffffu, m, 2));
-        }
-        const int groups = fours ? kThreads / 4 : kThreads;
-        s_min[fours ? tid >> 2 : tid] = m;
+    // keys lie below it.  Three barriers instead of the bisection's thirty: whole search of 4,099 x 64, K = 16 317 -> 226 us,
+    // 1,500 x 20, K = 32 33 -> 25, 9,000 x 40 1,095 -> 840.
+    if (!LONG || (KPT > 8 && K <= kGroupMaxK)) {
+        constexpr int groups = LONG ? kThreads : kThreads / 4;
+        s_min[tid] = lo;
         __syncthreads();
         if (tid < groups) {
-            m = s_min[tid];
+            unsigned m = s_min[tid];
+            if constexpr (!LONG) {   // the same lane of four warps; this is two warps' work
+                const unsigned *const four = s_min + warp * 128 + lane;
+                m = min(min(four[0], four[32]), min(four[64], four[96]));
+                s_four[tid] = m;
+                asm volatile("bar.sync 1, %0;" ::"n"(kThreads / 4) : "memory");
+            }
+            const unsigned *const all = LONG ? s_min : s_four;
             int at_or_below = 0;
 #pragma unroll 4
             for (int u = 0; u < groups; u += 4) {
-                const uint4 o = *reinterpret_cast<const uint4 *>(s_min + u);
+                const uint4 o = *reinterpret_cast<const uint4 *>(all + u);
                 at_or_below += (o.x <= m) + (o.y <= m) + (o.z <= m) + (o.w <= m);
             }
+            const unsigned least = __reduce_min_sync(0xffffffffu, m);
             m = __reduce_min_sync(0xffffffffu, at_or_below >= K ? m : 0xffffffffu);
-            if (lane == 0) atomicMin(&s_bound, m);
+            if (lane == 0) { atomicMin(&s_bound, m); atomicMin(&s_least, least); }
         }
         __syncthreads();
         const unsigned bound = s_bound;
-        if (bound <= kInfBits) {   // else fewer than K groups have a key at all
+        // 0: fewer than K groups have a key at all; 2: K groups have the smallest key of the row (copies of a point: 9,000 x 40, K = 16,
+        // four points in five equal, 1,391 -> 850 us)
+        known = bound > kInfBits ? 0 : bound == s_least ? 2 : 1;
+        if (known == 1) {
+            // one trip to the shared counter a thread (one a key: 9,000 x 20, K = 150 797 us, so 758; 6,145 x 20, K = 40 282, so 265)
+            int mine_below = 0;
 #pragma unroll
-            for (int j = 0; j < KPT; j++)
-                if (key[j] <= bound) {
-                    const int slot = atomicAdd(&s_n, 1);
-                    if (slot < kMaxDenseK) s_key[slot] = composed(j);
-                }
+            for (int j = 0; j < KPT; j++) mine_below += key[j] <= bound;
+            int slot = mine_below > 0 ? atomicAdd(&s_n, mine_below) : 0;
+            if (mine_below > 0 && slot + mine_below <= kMaxDenseK)
+#pragma unroll
+                for (int j = 0; j < KPT; j++)
+                    if (key[j] <= bound) s_key[slot++] = composed(j);
             __syncthreads();
             const int below = s_n;
             if (below <= kMaxDenseK) {
@@ -210,34 +232,41 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
                 }
                 return;
             }
-            __syncthreads();   // many equal keys: more than there is room for
+            __syncthreads();   // more than there is room for
             if (tid == 0) s_n = 0;
         }
+        if (known) hi = bound;
     }
+    int valid = 0;
+#pragma unroll
+    for (int j = 0; j < KPT; j++)
+        if (key[j] <= kInfBits) { valid++; if (!known) hi = max(hi, key[j]); }
     lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (!known) hi = __reduce_max_sync(0xffffffffu, hi);
     if (lane == 0) { s_lo[warp] = lo; s_hi[warp] = hi; }
     int turn = 0;
     valid = block_sum(valid, s_sum[turn++ & 1]);
 #pragma unroll
     for (int w = 0; w < kThreads / 32; w++) { lo = min(lo, s_lo[w]); hi = max(hi, s_hi[w]); }
-    // v: the smallest bound with at least K keys <= v
-    int at_most = valid;
-    unsigned v = hi;
-    if (valid > K) {
+    // v: a bound with at least K keys <= v, few enough to rank, or else (ties) the K-th smallest key itself
+    const int few = min(K + kFewMore, kMaxDenseK);
+    bool ties = valid > few;
+    unsigned v = ties ? hi : kInfBits;
+    if (ties && known < 2) {
         unsigned a = lo, b = hi;
+        bool first = known;   // the bound often is the K-th smallest key, one of many equal ones: the largest key below it first
         while (a < b) {
-            const unsigned mid = a + ((b - a) >> 1);
+            const unsigned mid = first ? b - 1 : a + ((b - a) >> 1);
+            first = false;
             int c = 0;
 #pragma unroll
             for (int j = 0; j < KPT; j++) c += key[j] <= mid;
             c = block_sum(c, s_sum[turn++ & 1]);
-            if (c >= K) { b = mid; at_most = c; if (c == K) break; }
+            if (c >= K) { b = mid; if (c <= few) { ties = false; valid = c; break; } }
             else a = mid + 1;
         }
         v = b;
     }
-    const bool ties = valid > K && at_most > K;   // more keys equal to v than there is room for: the first in order of id
     if (valid > 0) {
 #pragma unroll
         for (int j = 0; j < KPT; j++)
@@ -264,26 +293,27 @@ dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ i
         }
     }
     __syncthreads();
-    // rank by counting: K is at most a few hundred
-    const int got = min(valid, K);
-    for (int e = tid; e < K; e += kThreads) {
-        if (e < got) {
-            const unsigned long long mine = s_key[e];
-            int rank = 0;
-            for (int u = 0; u < got; u++) rank += s_key[u] < mine;
+    // rank by counting: a few hundred keys at most
+    const int got = ties ? K : valid;
+    for (int e = tid; e < got; e += kThreads) {
+        const unsigned long long mine = s_key[e];
+        int rank = 0;
+        for (int u = 0; u < got; u++) rank += s_key[u] < mine;
+        if (rank < K) {
             out_d[row * K + rank] = __uint_as_float((unsigned)(mine >> 32));
             out_i[row * K + rank] = (int32_t)(unsigned)mine;
-        } else {
-            out_d[row * K + e] = INFINITY;
-            out_i[row * K + e] = INT_MAX;
         }
+    }
+    for (int e = got + tid; e < K; e += kThreads) {
+        out_d[row * K + e] = INFINITY;
+        out_i[row * K + e] = INT_MAX;
     }
 }
 
 constexpr long long kMaxSegment = 48 * kThreads;   // values one block selects from (12,288)
 
-template <bool IDS>
-int launch_select(const float *val, const int32_t *ids, long long ld, long long n, long long seg, int segments, long long nq, int id_lo, int K,
+template <bool IDS, bool LONG>
+int launch_select_as(const float *val, const int32_t *ids, long long ld, long long n, long long seg, int segments, long long nq, int id_lo, int K,
                   const int *out_rows, long long out_base, float *out_d, int32_t *out_i, cudaStream_t st)
 {
     const long long longest = std::min(n, seg);
@@ -294,15 +324,24 @@ int launch_select(const float *val, const int32_t *ids, long long ld, long long 
         const int *r = out_rows ? out_rows + q : nullptr;
         float *od = out_rows ? out_d : out_d + q * segments * K;
         int32_t *oi = out_rows ? out_i : out_i + q * segments * K;
-        if (longest <= 4 * kThreads) dense_select_kernel<4, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
-        else if (longest <= 8 * kThreads) dense_select_kernel<8, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
-        else if (longest <= 16 * kThreads) dense_select_kernel<16, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
-        else if (longest <= 24 * kThreads) dense_select_kernel<24, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
-        else if (longest <= 32 * kThreads) dense_select_kernel<32, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
-        else dense_select_kernel<48, IDS><<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi);
+        auto launch = [&](auto kernel) { kernel<<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi); };
+        if (longest <= 4 * kThreads) launch(dense_select_kernel<4, IDS, LONG>);
+        else if (longest <= 8 * kThreads) launch(dense_select_kernel<8, IDS, LONG>);
+        else if (longest <= 16 * kThreads) launch(dense_select_kernel<16, IDS, LONG>);
+        else if (longest <= 24 * kThreads) launch(dense_select_kernel<24, IDS, LONG>);
+        else if (longest <= 32 * kThreads) launch(dense_select_kernel<32, IDS, LONG>);
+        else launch(dense_select_kernel<48, IDS, LONG>);
         B200_CUDA(cudaGetLastError());
     }
     return 0;
+}
+
+template <bool IDS>
+int launch_select(const float *val, const int32_t *ids, long long ld, long long n, long long seg, int segments, long long nq, int id_lo, int K,
+                  const int *out_rows, long long out_base, float *out_d, int32_t *out_i, cudaStream_t st)
+{
+    const auto as = K > kFoursMaxK ? launch_select_as<IDS, true> : launch_select_as<IDS, false>;
+    return as(val, ids, ld, n, seg, segments, nq, id_lo, K, out_rows, out_base, out_d, out_i, st);
 }
 
 int launch_distances(const float *X, int D, int64_t q_lo, int64_t nq, const int *q_index, int64_t db_lo, int64_t nd, float *dist, long long ld,
@@ -389,16 +428,24 @@ int knn_dense(const float *X, int D, int K, int64_t q_lo, int64_t nq, const int 
     return 0;
 }
 
+template <bool LONG> static int load_select()
+{
+    cudaFuncAttributes a;
+    const void *kernels[] = {(const void *)dense_select_kernel<4, false, LONG>,  (const void *)dense_select_kernel<8, false, LONG>,
+                             (const void *)dense_select_kernel<16, false, LONG>, (const void *)dense_select_kernel<24, false, LONG>,
+                             (const void *)dense_select_kernel<32, false, LONG>, (const void *)dense_select_kernel<48, false, LONG>};
+    for (const void *k : kernels) B200_CUDA(cudaFuncGetAttributes(&a, k));
+    return 0;
+}
+
 // loads every kernel that knn_dense_in_scratch may launch (a look at its attributes does)
 int knn_dense_load()
 {
     cudaFuncAttributes a;
-    const void *kernels[] = {(const void *)dense_distance_kernel<1>, (const void *)dense_distance_kernel<4>, (const void *)dense_select_kernel<4, false>,
-                             (const void *)dense_select_kernel<8, false>,   (const void *)dense_select_kernel<16, false>,
-                             (const void *)dense_select_kernel<24, false>, (const void *)dense_select_kernel<32, false>,
-                             (const void *)dense_select_kernel<48, false>};
+    const void *kernels[] = {(const void *)dense_distance_kernel<1>, (const void *)dense_distance_kernel<4>};
     for (const void *k : kernels) B200_CUDA(cudaFuncGetAttributes(&a, k));
-    return 0;
+    B200_TRY(load_select<false>());
+    return load_select<true>();
 }
 
 // The same for all points against all, in scratch of `floats` floats that the caller owns; -1 when it is too small for
