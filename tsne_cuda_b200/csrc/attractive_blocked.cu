@@ -871,9 +871,10 @@ static int device_sms(int *sms)
 // Blocks (SMs) of the attractive kernel of an iteration on one GPU, whose grid pipeline runs beside it on the SMs that are left.
 // A small graph is done before the potentials are, so the pipeline is what the iteration waits for, and its longest
 // kernel, the columns pass, has 393 blocks, four to an SM: on 99 SMs or more one wave, on fewer two.  So the graph takes a block per sixteen
-// chunks a warp (1 us each) and at most the SMs that one wave leaves (49 of 148), while it is done in the time that the
-// pipeline and the update need: 12 us a launch and 1 us a chunk of a warp, up to 48 us.  A larger graph takes what it takes
-// at any size (one SM in nine left, see launch_attractive_blocked): between the two the columns wait for a second wave as well.
+// chunks a warp (1 us each) and at most what leaves 101 SMs (47 of 148: with 99 a block of another kernel that ends late still makes a second
+// wave, 60,000 images on 46 | 47 | 48 | 49 blocks 47.0 / 42.5 | 46.9 / 41.7 | 47.0 / 41.0 | 48.3 / 41.6 us exaggerated / settled), while it
+// is done in the time that the pipeline and the update need: 12 us a launch and 1 us a chunk of a warp, up to 48 us.  A larger graph takes
+// what it takes at any size (one SM in nine left, see launch_attractive_blocked): in between the columns wait for a second wave as well.
 // us an iteration, exaggerated / settled, 90 neighbours (703 chunks per 1,000 points), on 24 | 49 | 64 | 80 | 96 | 132 blocks:
 //   20,011  34.0 / 34.0 | 34.4 / 34.5 | 34.0 / 33.9 | 35.3 / 35.1 | 36.9 / 36.9 | 39.2 / 39.2
 //   45,000  49.0 / 50.4 | 46.0 / 37.8 | 47.0 / 44.7 | 46.7 / 44.0 | 46.7 / 41.7 | 50.5 / 43.2
@@ -887,7 +888,7 @@ static int device_sms(int *sms)
 static int blocks_beside_grid(int sms, int wave_sms, long long C, long long extra_C)
 {
     constexpr long long warps = kBlockedThreads / 32;
-    const long long most = sms - sms / 9, spare = std::min<long long>(most, sms - wave_sms);
+    const long long most = sms - sms / 9, spare = std::min<long long>(most, sms - wave_sms - 2);
     const long long all = C + extra_C;
     if (all <= spare * warps * (extra_C > 0 ? 24 : 36)) return (int)std::max(6ll, std::min(spare, all / (16 * warps)));
     return (int)(extra_C > 0 ? std::min(most, std::max(C / (16 * warps), all / (24 * warps))) : most);
