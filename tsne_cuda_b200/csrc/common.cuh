@@ -238,9 +238,8 @@ int launch_soa_to_aos(const float *soa, float2 *aos, int64_t N, cudaStream_t st,
 int launch_aos_to_soa(const float2 *aos, float *soa, int64_t N, cudaStream_t st, const int32_t *perm = nullptr);
 // A small map's state between the device and memory that the host shares with it, block-wise [2][N] each: embedding, momentum,
 // gains one after the other (load: and the embedding's min/max into a slot that has been reset; store: null arrays left out)
-int launch_load_state(const float *io, float2 *Y2, float2 *u2, float2 *gains2, int64_t N, const int32_t *perm, IterState *state, int slot,
-                      cudaStream_t st);
-int launch_store_state(const float2 *Y2, const float2 *u2, const float2 *gains2, float *io, int64_t N, const int32_t *perm, cudaStream_t st);
+int launch_load_state(const float *io, float2 *Y2, float2 *u2, float2 *gains2, int64_t N, IterState *state, int slot, cudaStream_t st);
+int launch_store_state(const float2 *Y2, const float2 *u2, const float2 *gains2, float *io, int64_t N, cudaStream_t st);
 // dst[q] = src[perm[q]], or with scatter dst[perm[q]] = src[q]
 int launch_reorder_pairs(const float2 *src, float2 *dst, int64_t N, const int32_t *perm, bool scatter, cudaStream_t st);
 int launch_fill(float *p, float v, int64_t n, cudaStream_t st);

@@ -65,7 +65,6 @@ int set_create(StreamSet *s)
     B200_CUDA(cudaEventCreate(&s->ev_t0));
     B200_CUDA(cudaEventCreate(&s->ev_t1));
     B200_CUDA(cudaMallocHost((void **)&s->h_state, sizeof(IterState)));
-    B200_CUDA(cudaMallocHost((void **)&s->io, StreamSet::kIoBytes));
     return 0;
 }
 
@@ -228,6 +227,15 @@ bool stream_set_alive(const StreamSet *s)
 {
     if (cudaSetDevice(s->device) != cudaSuccess) (void)cudaGetLastError();   // an error that stays: the handles are still valid
     return s->context == context_id();
+}
+
+float *stream_set_io(StreamSet *s)
+{
+    if (!s->io && cudaMallocHost((void **)&s->io, StreamSet::kIoBytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        s->io = nullptr;
+    }
+    return s->io;
 }
 
 void stream_set_release(StreamSet *s)

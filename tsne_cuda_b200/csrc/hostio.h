@@ -25,6 +25,8 @@ struct StreamSet {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     IterState *h_state = nullptr;   // pinned
     // Pinned memory that kernels read and write across the bus: the state of a small map in one piece (Session::small_state).
+    // The size bounds what is held pinned; it is no crossover (21,845 points, the most that it holds: state in, one iteration,
+    // state out 278 -> 184 us).  Made at first use: 20 us, but 1.2 ms where the driver has to pin a new block for it.
     static constexpr size_t kIoBytes = (size_t)512 << 10;
     float *io = nullptr;
     // Executable graphs that finished sessions left behind.  Instantiating one of 16 iterations takes 1.3 ms (now and
@@ -37,7 +39,8 @@ struct StreamSet {
     std::vector<KeptExec> execs;
 };
 int stream_set_acquire(StreamSet **out, int device);   // makes `device` current
-void stream_set_release(StreamSet *s);                 // waits for both streams; null is fine
+void stream_set_release(StreamSet *s);                 // waits for its streams; null is fine
+float *stream_set_io(StreamSet *s);                    // `io`; null when it cannot be had
 bool stream_set_alive(const StreamSet *s);             // its context still is the device's; makes the device current
 
 // An executable for `graph`: a kept one of the same shape, updated, else a new one; null if neither can be had.

@@ -250,12 +250,15 @@ int Session::set_optimizer_soa(const float *momentum_host, const float *gains_ho
     return 0;
 }
 
+// (the order of the points does not matter at these sizes, so the state is in the caller's)
+static_assert(StreamSet::kIoBytes / (6 * sizeof(float)) <= (size_t)kAttractiveTile, "a state in one piece is in natural order");
+
 bool Session::small_state(const void *Y, const void *momentum, const void *gains) const
 {
     if (rows() != N || (comm && comm->world > 1) || sizeof(float) * 6 * (size_t)N > StreamSet::kIoBytes) return false;
     for (const void *p : {Y, momentum, gains})
         if (p && !plain_host(p)) return false;
-    return true;
+    return stream_set_io(host) != nullptr;
 }
 
 int Session::set_small_state(const float *Y_host, const float *momentum_host, const float *gains_host, int at_step)
@@ -268,7 +271,7 @@ int Session::set_small_state(const float *Y_host, const float *momentum_host, co
     step = at_step;
     done_seen = 0;
     B200_TRY(launch_state_reset(state, stream));
-    B200_TRY(launch_load_state(host->io, Y2, u, gains, N, state_order(), state, step & 1, stream));
+    B200_TRY(launch_load_state(host->io, Y2, u, gains, N, state, step & 1, stream));
     B200_CUDA(cudaMemsetAsync(w, 0, sizeof(float4) * kG * kG, stream));
     // like the copying path: the call's work and its errors are its own (left queued, 8 us of a set_state, run(1), get_state
     // of 110 moved into the next call), and the pinned memory is free for the next state
@@ -281,7 +284,7 @@ int Session::set_small_state(const float *Y_host, const float *momentum_host, co
 int Session::get_small_state(float *Y_host, float *momentum_host, float *gains_host)
 {
     B200_CUDA(cudaSetDevice(device));
-    B200_TRY(launch_store_state(Y_host ? Y2 : nullptr, momentum_host ? u : nullptr, gains_host ? gains : nullptr, host->io, N, state_order(), stream));
+    B200_TRY(launch_store_state(Y_host ? Y2 : nullptr, momentum_host ? u : nullptr, gains_host ? gains : nullptr, host->io, N, stream));
     B200_CUDA(cudaStreamSynchronize(stream));
     const size_t block = 2 * (size_t)N;
     float *to[3] = {Y_host, momentum_host, gains_host};

@@ -130,16 +130,15 @@ __global__ void aos_to_soa_kernel(const float2 *aos, float *soa, long long N, co
     if (i < N) { const long long j = perm ? perm[i] : i; const float2 v = aos[i]; soa[j] = v.x; soa[N + j] = v.y; }
 }
 __global__ void __launch_bounds__(256)
-load_state_kernel(const float *io, float2 *Y2, float2 *u2, float2 *gains2, long long N, const int32_t *perm, IterState *state, int slot)
+load_state_kernel(const float *io, float2 *Y2, float2 *u2, float2 *gains2, long long N, IterState *state, int slot)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     float mn = INFINITY, mx = -INFINITY;
     if (i < N) {
-        const long long j = perm ? perm[i] : i;
-        const float2 y = make_float2(io[j], io[N + j]);
+        const float2 y = make_float2(io[i], io[N + i]);
         Y2[i] = y;
-        u2[i] = make_float2(io[2 * N + j], io[3 * N + j]);
-        gains2[i] = make_float2(io[4 * N + j], io[5 * N + j]);
+        u2[i] = make_float2(io[2 * N + i], io[3 * N + i]);
+        gains2[i] = make_float2(io[4 * N + i], io[5 * N + i]);
         mn = fminf(y.x, y.y);
         mx = fmaxf(y.x, y.y);
     }
@@ -154,18 +153,17 @@ load_state_kernel(const float *io, float2 *Y2, float2 *u2, float2 *gains2, long 
     }
 }
 __global__ void __launch_bounds__(256)
-store_state_kernel(const float2 *Y2, const float2 *u2, const float2 *gains2, float *io, long long N, const int32_t *perm)
+store_state_kernel(const float2 *Y2, const float2 *u2, const float2 *gains2, float *io, long long N)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    const long long j = perm ? perm[i] : i;
     const float2 *from[3] = {Y2, u2, gains2};
 #pragma unroll
     for (int a = 0; a < 3; a++)
         if (from[a]) {
             const float2 v = from[a][i];
-            io[2 * a * N + j] = v.x;
-            io[(2 * a + 1) * N + j] = v.y;
+            io[2 * a * N + i] = v.x;
+            io[(2 * a + 1) * N + i] = v.y;
         }
 }
 // dst[q] = src[perm[q]] (gather) or dst[perm[q]] = src[q] (scatter)
@@ -227,18 +225,17 @@ int launch_aos_to_soa(const float2 *aos, float *soa, int64_t N, cudaStream_t st,
     return 0;
 }
 
-int launch_load_state(const float *io, float2 *Y2, float2 *u2, float2 *gains2, int64_t N, const int32_t *perm, IterState *state, int slot,
-                      cudaStream_t st)
+int launch_load_state(const float *io, float2 *Y2, float2 *u2, float2 *gains2, int64_t N, IterState *state, int slot, cudaStream_t st)
 {
     if (N <= 0) return 0;
-    load_state_kernel<<<nblk(N, 256), 256, 0, st>>>(io, Y2, u2, gains2, N, perm, state, slot);
+    load_state_kernel<<<nblk(N, 256), 256, 0, st>>>(io, Y2, u2, gains2, N, state, slot);
     B200_CUDA(cudaGetLastError());
     return 0;
 }
-int launch_store_state(const float2 *Y2, const float2 *u2, const float2 *gains2, float *io, int64_t N, const int32_t *perm, cudaStream_t st)
+int launch_store_state(const float2 *Y2, const float2 *u2, const float2 *gains2, float *io, int64_t N, cudaStream_t st)
 {
     if (N <= 0) return 0;
-    store_state_kernel<<<nblk(N, 256), 256, 0, st>>>(Y2, u2, gains2, io, N, perm);
+    store_state_kernel<<<nblk(N, 256), 256, 0, st>>>(Y2, u2, gains2, io, N);
     B200_CUDA(cudaGetLastError());
     return 0;
 }
