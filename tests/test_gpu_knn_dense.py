@@ -34,6 +34,21 @@ def test_host_points(engine, oracle_cpu, n, d, k, ties):
     assert np.array_equal(ids[lo:], ids_o) and np.array_equal(d2[lo:], d2_o)
 
 
+@pytest.mark.parametrize("scale", [1e-19, 1e-20, 1e-21, 1e-22, 1e-23])
+@pytest.mark.parametrize("n,d,k", [(300, 7, 20), (1500, 20, 32), (4099, 5, 50)])
+def test_squares_at_the_end_of_the_range(engine, oracle_cpu, n, d, k, scale):
+    """Squares that are subnormal or round to zero, where a fused operation could round otherwise than a product: blocks of 64
+    queries, of 16 (at most 48 in all), and the search without allocation."""
+    import torch
+    X = (np.random.default_rng(n).normal(0, 1, (n, d)) * scale).astype(np.float32)
+    ids_o, d2_o = oracle_cpu.knn(X, k, q_lo=n - 200, q_hi=n)
+    for q_lo in (n - 200, n - 48, n - 1):
+        ids, d2 = engine.knn(X, k, q_lo=q_lo, q_hi=n)
+        assert np.array_equal(ids, ids_o[q_lo - n:]) and np.array_equal(d2, d2_o[q_lo - n:])
+    ids, d2 = _noalloc(engine, torch.from_numpy(X).cuda(), k)
+    assert np.array_equal(ids.cpu().numpy()[-200:], ids_o) and np.array_equal(d2.cpu().numpy()[-200:], d2_o)
+
+
 # groups of four threads, of one, none (K = 48 / 49, 192 / 193); as many keys a thread as a kernel has registers for, and one more
 @pytest.mark.parametrize("k", [47, 48, 49, 192, 193])
 @pytest.mark.parametrize("n", [256, 2047, 6144, 6145])

@@ -231,6 +231,23 @@ def test_repulsive_odd_sizes_vs_oracle(engine, oracle_cpu, n, scale):
         assert abs(Z - Z_o) <= 1e-4 * abs(Z_o) + 1e-3
 
 
+@pytest.mark.parametrize("spread", [1e9, 1e10, 1e15, 9.5e18])
+def test_kernel_values_beyond_the_range_of_floats(engine, spread):
+    """Nodes so far apart that the kernel's denominator leaves the range of floats (from 1.8e9 on) or squares overflow: all
+    values but the one at distance zero are below 1e-26, so the potentials are the charges.  Rounding: transforms of 784 points,
+    four of them in turn, 1e-6."""
+    n = 300
+    Y = (np.random.default_rng(3).uniform(-0.45, 0.45, (2, n)) * spread).astype(np.float32)
+    box = 2 * spread / 130
+    Y[:, 0], Y[:, 1] = (-spread, 0.5 * box), (spread, -0.5 * box)
+    _, _, w, yt = engine.repulsive(Y, True)
+    assert np.isfinite(w).all() and np.isfinite(yt).all()
+    for plane in range(4):
+        # beyond 1e15 the squares cannot be scaled to the counts any more, whose transform they share
+        if plane > 0 or spread < 1e15:
+            assert rel_l2(yt[..., plane], w[..., plane]) < 1e-5
+
+
 # ------------------------------------------------------------------------------------- live reference
 def test_stages_vs_live_reference_kernels(engine, oracle_cpu):
     from oracle import ref

@@ -36,8 +36,10 @@ def test_values_beyond_the_range_of_floats():
     rng = np.random.default_rng(2)
     for x in np.concatenate([10.0 ** rng.uniform(37, 78, 2000), [1.0000001e37, 8.5e37, 1.7e38, 3.5e38, 1.4e45, 2.9e45, 1e78]]):
         t = float(x) * 2.0 ** -160
-        r = float(np.float32(1) / np.float32(t))
-        assert 0 < r < 2.0 ** 126                             # CUDA's fast division: exact to two units in this range
-        r1 = fma(r, fma(-t, r, 1.0), r)
-        r2 = fma(r1, fma(-t, r1, 1.0), r1)
-        assert np.float32(r2 * 2.0 ** -160) == np.float32(1.0 / float(x))
+        assert 2.0 ** -126 < t < 2.0 ** 126                   # the divisors for which CUDA's fast division is within two units
+        exact = float(np.float32(1) / np.float32(t))
+        for ulps in (-2, 0, 2):
+            r = exact * (1 + ulps * 2.0 ** -23)
+            r1 = fma(r, fma(-t, r, 1.0), r)
+            r2 = fma(r1, fma(-t, r1, 1.0), r1)
+            assert np.float32(r2 * 2.0 ** -160) == np.float32(1.0 / float(x))
