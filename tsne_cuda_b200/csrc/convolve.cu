@@ -13,8 +13,8 @@
 //    one-dimensional transform the fourteen leading registers of a lane hold all of the input (forward) or all of the
 //    wanted output (inverse): the other half of the butterflies is left out at compile time.
 //  * The kernel is centred at index 0 and even in both axes, so its spectrum is real and even.  It depends on the
-//    embedding through the box width alone: two small kernels (spectrum_rows, spectrum_columns) prepare it on the other
-//    stream while the points are sorted and spread.  Two real rows share a complex transform, and the spectrum of
+//    embedding through the box width alone: two small kernels (spectrum_rows, spectrum_columns) prepare it on a stream of
+//    their own while the points are sorted and spread.  Two real columns share a complex transform, and the spectrum of
 //    column c serves column 784 - c as well.
 //  * Column c, its mirror image 784 - c, and both planes stand side by side in the workspace (32 bytes per row): one
 //    block transforms the four of them, every access is a whole sector, and the product with the spectrum never leaves
@@ -25,8 +25,8 @@
 //
 // Bound: about 5,300 warp transforms of 1,100 issue slots are 10,000 cycles of all 592 schedulers, 5 us; the rest is the
 // load latency of three dependent kernels.  Measured on B200, each kernel alone with warm caches: rows 5.2, columns 10.4,
-// rows back 7.2 us, beside them on the other stream 7 + 6 us for the spectrum (the three passes over 1024-point
-// transforms, with the kernel as a third plane, took 7.5, 20 and 7 us).
+// rows back 7.2 us (the three passes over 1024-point transforms, with the kernel as a third plane, took 7.5, 20 and 7 us);
+// cold, under the profiler, 7.1, 12.5 and 8.7, and beside them 6.4 + 7.6 for the spectrum.
 // Rounding: the repulsive force is as far from float64 as with the 1024-point transforms (1e-7 to 4e-7 of its norm for compact
 // maps, 7e-6 at spread 10); the sum of Z 1e-7 to 3e-7 for compact maps, where it was 0.5e-7 to 1.5e-7, and the same elsewhere.
 #include "grid_geom.cuh"
@@ -174,8 +174,8 @@ __device__ __forceinline__ int column_of(int k) { return k < kC ? k : kM - k; }
 __device__ __forceinline__ int slot_of(int k) { return k < kC ? 0 : 1; }
 
 // ---- spectrum of the kernel, first axis: a row per warp.  Two rows could share a transform, but a lane then evaluates 28
-// values instead of 14, and the evaluation is as long as the transform: iteration at 1,500 / 5,000 / 20,011 points
-// 34.4 / 37.1 / 39.5 -> 32.4 / 34.5 / 38.4 us. ----
+// values instead of 14, and the evaluation is as long as the transform: settled iteration at 1,500 / 20,011 / 45,000 points
+// 32.8 / 35.0 / 39.0 us with two rows, 32.2 / 34.6 / 38.2 with one. ----
 __device__ __forceinline__ float kernel_value(int row, int j, float h, float cmin)
 {
     // node coordinates in float exactly as the reference forms them, summed and inverted in double (nbodyfft.cu:175-195)

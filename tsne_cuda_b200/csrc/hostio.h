@@ -26,7 +26,7 @@ struct StreamSet {
     IterState *h_state = nullptr;   // pinned
     // Pinned memory that kernels read and write across the bus: the state of a small map in one piece (Session::small_state).
     // The size bounds what is held pinned; it is no crossover (21,845 points, the most that it holds: state in, one iteration,
-    // state out 278 -> 184 us).  Made at first use: 20 us, but 1.2 ms where the driver has to pin a new block for it.
+    // state out 278 -> 168 us).  Made at first use: 20 us, but 1.2 ms where the driver has to pin a new block for it.
     static constexpr size_t kIoBytes = (size_t)512 << 10;
     float *io = nullptr;
     // Executable graphs that finished sessions left behind.  Instantiating one of 16 iterations takes 1.3 ms (now and

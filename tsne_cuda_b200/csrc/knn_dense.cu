@@ -5,7 +5,7 @@
 // search could not certify, and callers that must not allocate.  A search that keeps a running list per query
 // (knn_exact_kernel) serves 64 queries per block and inserts survivors one at a time: at 1,500 points that is 24 blocks on
 // 148 SMs, and half of the time goes into insertions.  Here the distances are a plain tiled product over all SMs (three
-// unfused fp32 instructions per pair and dimension, the bound), and the selection ranks the few keys, held in registers, that
+// rounded fp32 operations per pair and dimension, issued for two pairs at a time, the bound), and the selection ranks the few keys, held in registers, that
 // lie below a bound from the smallest keys of groups (short rows, long lists: bisection on the keys' bits).  Measured on B200 (lists / now):
 // 4,099 points of 64 dimensions, K = 16: 1.69 / 0.20 ms; 1,500 x 20, K = 32: 1.63 / 0.03 ms; five rows of 60,000 x 784:
 // 4.4 / 0.4 ms.
