@@ -49,9 +49,10 @@ def test_squares_at_the_end_of_the_range(engine, oracle_cpu, n, d, k, scale):
     assert np.array_equal(ids.cpu().numpy()[-200:], ids_o) and np.array_equal(d2.cpu().numpy()[-200:], d2_o)
 
 
-# groups of four threads, of one, none (K = 48 / 49, 192 / 193); as many keys a thread as a kernel has registers for, and one more
-@pytest.mark.parametrize("k", [47, 48, 49, 192, 193])
-@pytest.mark.parametrize("n", [256, 2047, 6144, 6145])
+# groups of four threads, of one, none (K = 48 / 49, 160 / 161); rows that bisect beyond K = 48 and longer ones; both sides of the
+# numbers of keys a thread holds (test_selection_where_the_bound_is_loose has the others)
+@pytest.mark.parametrize("k", [47, 48, 49, 160, 161, 192, 193])
+@pytest.mark.parametrize("n", [256, 2047, 2048, 2049, 6144, 6145, 12288])
 @pytest.mark.parametrize("equal", [0, 600])
 def test_selection_by_a_bound(engine, oracle_cpu, n, k, equal):
     """Without ties, and with more equal distances below the bound than there is room for: decided by the index."""
