@@ -191,7 +191,7 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
 
 // repulsive.cu
 struct FftWorkspace {
-    float4 *A;      // [kG rows][columns 0 .. kM/2][2] row-transformed charges (see convolve.cu)
+    float4 *A;      // [columns 0 .. kM/2][four rows][8] row-transformed charges (see convolve.cu)
     float4 *B;      // the same after the column pass
     float2 *tw;     // [28][28] twiddles e^{-2 pi i k l / kM}
     float *Rk, *Kh; // row-transformed kernel; its spectrum by column

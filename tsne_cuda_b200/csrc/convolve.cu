@@ -16,17 +16,19 @@
 //    embedding through the box width alone: two small kernels (spectrum_rows, spectrum_columns) prepare it on a stream of
 //    their own while the points are sorted and spread.  Two real columns share a complex transform, and the spectrum of
 //    column c serves column 784 - c as well.
-//  * Column c, its mirror image 784 - c, and both planes stand side by side in the workspace (32 bytes per row): one
-//    block transforms the four of them, every access is a whole sector, and the product with the spectrum never leaves
-//    the SM.
+//  * Column c, its mirror image 784 - c, and both planes are one block of the column pass, and the product with the spectrum
+//    never leaves the SM.  Between the passes four rows of these four columns are one line of 128 bytes: a block of the row
+//    passes has four rows, and every block reads and writes whole lines.
 //  * The last pass also sums the normalisation on the grid: sum_i Z_i is the bilinear form of charges and potentials
 //    (each point's Z_i is interpolated from the potentials with the weights its charges were spread with), so it needs
 //    neither a pass over the points nor an exchange between ranks that hold the summed grid.
 //
-// Bound: about 5,300 warp transforms of 1,100 issue slots are 10,000 cycles of all 592 schedulers, 5 us; the rest is the
-// load latency of three dependent kernels.  Measured on B200, each kernel alone with warm caches: rows 5.2, columns 10.4,
-// rows back 7.2 us (the three passes over 1024-point transforms, with the kernel as a third plane, took 7.5, 20 and 7 us);
-// cold, under the profiler, 7.1, 12.5 and 8.7, and beside them 6.4 + 7.6 for the spectrum.
+// Bound: three kernels whose blocks each run once: the loads at their start, an exchange and the stores at their end take as
+// long as the transforms, and in those the fp32 pipe is three quarters busy (columns pass: 4,900 cycles of packed and scalar
+// arithmetic per scheduler in 6,500).  Measured on B200 inside an iteration of 5,000 points: rows 5.1, columns 6.9, rows
+// back 6.2 us.  With a row (390 blocks of two warps) as the unit of the row passes, so that the column pass read and wrote
+// 32 bytes per row (every load and store of a warp 28 different lines), and scalar arithmetic: 4.8, 9.8, 6.2.  Iteration at
+// 1,500 / 5,000 / 20,011 points 31.1 -> 29.1, 32.1 -> 29.4, 34.4 -> 31.2 us; 60,000 exaggerated 46.2 -> 43.9.
 // Rounding: the repulsive force is as far from float64 as with the 1024-point transforms (1e-7 to 4e-7 of its norm for compact
 // maps, 7e-6 at spread 10); the sum of Z 1e-7 to 3e-7 for compact maps, where it was 0.5e-7 to 1.5e-7, and the same elsewhere.
 #include "grid_geom.cuh"
@@ -46,13 +48,44 @@ constexpr int kExStride = kR + 1;            // float2 per row of the exchange b
 constexpr int kEx = kR * kExStride;
 static_assert(kM == kR * kR && kM >= 2 * kG - 1 && kR * kHalf >= kG && kR * (kHalf - 1) < kG, "transform length");
 
-__device__ __forceinline__ float2 operator+(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 operator-(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+// Sums and products with a real coefficient act on both halves of a complex number alike: one packed instruction each, with
+// the results of the two it stands for.  The fp32 pipe is as fast either way; the issue slots go to everything else.
+__device__ __forceinline__ uint64_t pack(float2 a)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack(uint64_t r)
+{
+    float2 a;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+    return a;
+}
+__device__ __forceinline__ float2 operator+(float2 a, float2 b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack(a)), "l"(pack(b)));
+    return unpack(r);
+}
 // a + c * t, a real coefficient
-__device__ __forceinline__ float2 axpy(float c, float2 t, float2 a) { return make_float2(fmaf(c, t.x, a.x), fmaf(c, t.y, a.y)); }
-// -i b (forward) or +i b (inverse)
-template <bool INV> __device__ __forceinline__ float2 turn(float2 b) { return INV ? make_float2(-b.y, b.x) : make_float2(b.y, -b.x); }
+__device__ __forceinline__ float2 axpy(float c, float2 t, float2 a)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack(make_float2(c, c))), "l"(pack(t)), "l"(pack(a)));
+    return unpack(r);
+}
+__device__ __forceinline__ float2 operator-(float2 a, float2 b) { return axpy(-1.0f, b, a); }
+__device__ __forceinline__ float2 times(float c, float2 t)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack(make_float2(c, c))), "l"(pack(t)));
+    return unpack(r);
+}
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+// a plus or minus b turned by -90 degrees (forward) or +90 (inverse)
+template <bool INV> __device__ __forceinline__ float2 add_turned(float2 a, float2 b) { return INV ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, a.y - b.x); }
+template <bool INV> __device__ __forceinline__ float2 sub_turned(float2 a, float2 b) { return add_turned<!INV>(a, b); }
 
 // Seven-point transform, natural order.  Z1..Z6: the input of that index is zero.
 template <bool INV, bool Z0, bool Z1, bool Z2, bool Z3, bool Z4, bool Z5, bool Z6> __device__ __forceinline__ void dft7(float2 (&v)[7])
@@ -69,7 +102,7 @@ template <bool INV, bool Z0, bool Z1, bool Z2, bool Z3, bool Z4, bool Z5, bool Z
     if (!none1) {
         sum = Z0 ? t1 : sum + t1;
         a1 = axpy(c1, t1, a1); a2 = axpy(c2, t1, a2); a3 = axpy(c3, t1, a3);
-        b1 = make_float2(s1 * d1.x, s1 * d1.y); b2 = make_float2(s2 * d1.x, s2 * d1.y); b3 = make_float2(s3 * d1.x, s3 * d1.y);
+        b1 = times(s1, d1); b2 = times(s2, d1); b3 = times(s3, d1);
     }
     if (!none2) {
         sum = sum + t2;
@@ -81,11 +114,10 @@ template <bool INV, bool Z0, bool Z1, bool Z2, bool Z3, bool Z4, bool Z5, bool Z
         a1 = axpy(c3, t3, a1); a2 = axpy(c1, t3, a2); a3 = axpy(c2, t3, a3);
         b1 = axpy(s3, d3, b1); b2 = axpy(-s1, d3, b2); b3 = axpy(s2, d3, b3);
     }
-    const float2 i1 = turn<INV>(b1), i2 = turn<INV>(b2), i3 = turn<INV>(b3);
     v[0] = sum;
-    v[1] = a1 + i1; v[6] = a1 - i1;
-    v[2] = a2 + i2; v[5] = a2 - i2;
-    v[3] = a3 + i3; v[4] = a3 - i3;
+    v[1] = add_turned<INV>(a1, b1); v[6] = sub_turned<INV>(a1, b1);
+    v[2] = add_turned<INV>(a2, b2); v[5] = sub_turned<INV>(a2, b2);
+    v[3] = add_turned<INV>(a3, b3); v[4] = sub_turned<INV>(a3, b3);
 }
 
 // input b of the a-th seven-point transform of fft28 is one of the zeros
@@ -107,11 +139,11 @@ template <bool INV, int NZ> __device__ __forceinline__ void fft28(float2 (&v)[kR
 #pragma unroll
     for (int kb = 0; kb < 7; kb++) {
         const float2 p = y[0][kb] + y[2][kb], m = y[0][kb] - y[2][kb];
-        const float2 q = y[1][kb] + y[3][kb], r = turn<INV>(y[1][kb] - y[3][kb]);
+        const float2 q = y[1][kb] + y[3][kb], r = y[1][kb] - y[3][kb];
         v[(8 * kb) % 28] = p + q;
-        v[(21 + 8 * kb) % 28] = m + r;
+        v[(21 + 8 * kb) % 28] = add_turned<INV>(m, r);
         v[(42 + 8 * kb) % 28] = p - q;
-        v[(63 + 8 * kb) % 28] = m - r;
+        v[(63 + 8 * kb) % 28] = sub_turned<INV>(m, r);
     }
 }
 
@@ -265,115 +297,130 @@ spectrum_columns_kernel(const float *__restrict__ Rk, float *__restrict__ Kh, co
     }
 }
 
-// ---- first pass: a row of the charge grid, both planes ----
-__global__ void __launch_bounds__(64)
+// ---- workspace between the passes ----
+// Column pair c (a column, its mirror image, both planes: q = 0 .. 3) and four rows are a line of 128 bytes; the lines of a
+// column pair follow one another.  A block of the row passes has four rows, so it writes or reads whole lines, and a block of
+// the column pass has one column pair: 12.5 KB in one piece.  Inside its line the place of (row, q) turns with the line, so
+// that a half warp that reads one q of sixteen rows meets sixteen bank pairs.
+constexpr int kRowsBlock = 4, kLines = (kG + kRowsBlock - 1) / kRowsBlock, kLine = 4 * kRowsBlock;   // kLine: float2
+static_assert(kLines * kRowsBlock == kR * kHalf, "rows beyond the grid are the zeros of a transform");
+__device__ __forceinline__ int place_in_line(int q, int line, int row) { return kRowsBlock * ((q + line) & 3) + (row & (kRowsBlock - 1)); }
+constexpr int kStageLine = kLine + 2;   // float2 per line in shared memory of the row passes: columns apart in their banks
+
+constexpr int kRowThreads = 2 * kRowsBlock * 32;   // a warp per row and plane
+constexpr size_t kStageBytes = sizeof(float2) * kC * kStageLine, kRowExBytes = sizeof(float2) * 2 * kRowsBlock * kEx;
+constexpr size_t kRowsSmem = sizeof(float2) * kM + (kStageBytes > kRowExBytes ? kStageBytes : kRowExBytes);
+constexpr size_t kBackSmem = kRowsSmem + sizeof(float4) * kRowsBlock * kG;
+
+// ---- first pass: four rows of the charge grid, both planes ----
+__global__ void __launch_bounds__(kRowThreads)
 fft_rows_forward_kernel(const float4 *__restrict__ w, float4 *__restrict__ A, const IterState *state, int slot, const float2 *__restrict__ tw)
 {
-    __shared__ __align__(16) float2 tws[kM], out[2][kC][2];   // out[plane][column][slot]
-    __shared__ float2 exch[2][kEx];
-    const int lane = threadIdx.x & 31, plane = threadIdx.x >> 5, row = blockIdx.x;
-    copy_twiddles<64>(tws, tw);
+    extern __shared__ __align__(16) float2 smem[];
+    float2 *tws = smem, *stage = smem + kM;   // the lines, once the exchange is over
+    const int lane = threadIdx.x & 31, plane = (threadIdx.x >> 5) & 1, row = kRowsBlock * blockIdx.x + (threadIdx.x >> 6);
+    copy_twiddles<kRowThreads>(tws, tw);
     const float2 *wrow = reinterpret_cast<const float2 *>(w + (size_t)row * kG) + plane;   // .xy or .zw of each node
     float2 v[kR];
 #pragma unroll
     for (int r = 0; r < kHalf; r++) {
         const int j = kR * r + lane;
-        v[r] = (lane < kR && j < kG) ? wrow[2 * j] : make_float2(0.0f, 0.0f);
+        v[r] = (lane < kR && j < kG && row < kG) ? wrow[2 * j] : make_float2(0.0f, 0.0f);
     }
     const float imag_scale = plane == 1 ? load_geom(state, slot).r2_scale : 1.0f;
 #pragma unroll
     for (int r = 0; r < kHalf; r++) v[r].y *= imag_scale;
     copies_done();
-    fft784_warp<false, kHalf>(v, exch[plane], tws, lane);
+    fft784_warp<false, kHalf>(v, stage + (threadIdx.x >> 5) * kEx, tws, lane);
+    __syncthreads();
     if (lane < kR) {
 #pragma unroll
         for (int r = 0; r < kR; r++) {
             const int k = kR * r + lane;
-            out[plane][column_of(k)][slot_of(k)] = v[r];
+            stage[column_of(k) * kStageLine + place_in_line(2 * plane + slot_of(k), blockIdx.x, row)] = v[r];
         }
     }
     __syncthreads();
-    float4 *dst = A + (size_t)row * kC * 2;
-#pragma unroll
-    for (int u = threadIdx.x; u < 2 * kC; u += 64) dst[u] = *reinterpret_cast<const float4 *>(out[u & 1][u >> 1]);
+#pragma unroll 4
+    for (int u = threadIdx.x; u < kC * kLine / 2; u += kRowThreads) {
+        const int c = u / (kLine / 2), part = u % (kLine / 2);
+        A[((size_t)c * kLines + blockIdx.x) * (kLine / 2) + part] = *reinterpret_cast<const float4 *>(stage + c * kStageLine + 2 * part);
+    }
 }
 
 // ---- second pass: column c, its mirror image, both planes: forward, product with the spectrum, inverse ----
-constexpr size_t kColsSmem = sizeof(float2) * (kM + 4 * kEx + 4 * kG) + sizeof(float) * kM;
+constexpr size_t kColsSmem = sizeof(float2) * (kM + 4 * kEx + kLines * kLine) + sizeof(float) * kM;
 __global__ void __launch_bounds__(128)
-fft_columns_kernel(const float2 *__restrict__ A, const float *__restrict__ Kh, float4 *__restrict__ B, const float2 *__restrict__ tw)
+fft_columns_kernel(const float4 *__restrict__ A, const float *__restrict__ Kh, float4 *__restrict__ B, const float2 *__restrict__ tw)
 {
     extern __shared__ __align__(16) float2 smem[];
-    float2 *tws = smem, *ex = smem + kM + (threadIdx.x >> 5) * kEx, *out = smem + kM + 4 * kEx;
-    float *spec = reinterpret_cast<float *>(smem + kM + 4 * kEx + 4 * kG);
+    float2 *tws = smem, *ex = smem + kM + (threadIdx.x >> 5) * kEx, *lines = smem + kM + 4 * kEx;
+    float *spec = reinterpret_cast<float *>(lines + kLines * kLine);
     const int lane = threadIdx.x & 31, q = threadIdx.x >> 5, c = blockIdx.x;
-    float2 v[kR];
-#pragma unroll
-    for (int r = 0; r < kHalf; r++) {
-        const int row = kR * r + lane;
-        v[r] = (lane < kR && row < kG) ? A[((size_t)row * kC + c) * 4 + q] : make_float2(0.0f, 0.0f);
-    }
+    constexpr int n4 = kLines * kLine / 2;
+    copy_floats<128>(reinterpret_cast<float *>(lines), reinterpret_cast<const float *>(A + (size_t)c * n4), n4);
     copy_twiddles<128>(tws, tw);
     copy_floats<128>(spec, Kh + (size_t)c * kM, kM / 4);
     copies_done();
-    fft784_warp<false, kHalf>(v, ex, tws, lane);
     const int sl = min(lane, kR - 1);
+    float2 *mine = lines + (sl / kRowsBlock) * kLine;   // rows 28 r + lane: 7 r lines further on; a warp has its q to itself
+    float2 v[kR];
 #pragma unroll
-    for (int r = 0; r < kR; r++) {
-        const float k = spec[kR * r + sl];
-        v[r].x *= k;
-        v[r].y *= k;
+    for (int r = 0; r < kHalf; r++) {
+        v[r] = mine[r * (kR / kRowsBlock) * kLine + place_in_line(q, r * (kR / kRowsBlock) + sl / kRowsBlock, sl)];
     }
+    fft784_warp<false, kHalf>(v, ex, tws, lane);
+#pragma unroll
+    for (int r = 0; r < kR; r++) v[r] = times(spec[kR * r + sl], v[r]);
     fft784_warp<true, kR>(v, ex, tws, lane);
     if (lane < kR) {
 #pragma unroll
-        for (int r = 0; r < kHalf; r++) {
-            const int row = kR * r + lane;
-            if (row < kG) out[q * kG + row] = v[r];
-        }
+        for (int r = 0; r < kHalf; r++) mine[r * (kR / kRowsBlock) * kLine + place_in_line(q, r * (kR / kRowsBlock) + sl / kRowsBlock, sl)] = v[r];
     }
     __syncthreads();
+    float4 *dst = B + (size_t)c * n4;
+    const float4 *out = reinterpret_cast<const float4 *>(lines);
 #pragma unroll
-    for (int row = threadIdx.x; row < kG; row += 128) {
-        const float2 a = out[row], b = out[kG + row], e = out[2 * kG + row], f = out[3 * kG + row];
-        float4 *dst = B + ((size_t)row * kC + c) * 2;
-        dst[0] = make_float4(a.x, a.y, b.x, b.y);
-        dst[1] = make_float4(e.x, e.y, f.x, f.y);
-    }
+    for (int u = threadIdx.x; u < n4; u += 128) dst[u] = out[u];
 }
 
-// ---- third pass: a row of potentials, both planes; the grid's share of sum_i Z_i ----
-__global__ void __launch_bounds__(64)
+// ---- third pass: four rows of potentials, both planes; the grid's share of sum_i Z_i ----
+__global__ void __launch_bounds__(kRowThreads)
 fft_rows_inverse_kernel(const float4 *__restrict__ B, float4 *__restrict__ w, float4 *__restrict__ ytilde, IterState *state, int slot,
                         const float2 *__restrict__ tw, int zero_w)
 {
-    __shared__ __align__(16) float2 tws[kM], in[2][kC][2];   // in[plane][column][slot]
-    __shared__ __align__(16) float4 charge[kG];
-    __shared__ float2 exch[2][kEx];
-    const int lane = threadIdx.x & 31, plane = threadIdx.x >> 5, row = blockIdx.x;
-    const float4 *src = B + (size_t)row * kC * 2;
-    float4 *wrow = w + (size_t)row * kG;
-    for (int u = threadIdx.x; u < 2 * kC; u += 64) copy16(in[u & 1][u >> 1], src + u);
-    copy_twiddles<64>(tws, tw);
-    for (int j = threadIdx.x; j < kG; j += 64) copy16(charge + j, wrow + j);
+    extern __shared__ __align__(16) float2 smem[];
+    float2 *tws = smem, *stage = smem + kM;   // the lines, before the exchange
+    float4 *charges = reinterpret_cast<float4 *>(smem) + (kBackSmem - sizeof(float4) * kRowsBlock * kG) / sizeof(float4);
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, plane = wi & 1, row = kRowsBlock * blockIdx.x + (wi >> 1);
+    for (int u = threadIdx.x; u < kC * kLine / 2; u += kRowThreads) {
+        const int c = u / (kLine / 2), part = u % (kLine / 2);
+        copy16(stage + c * kStageLine + 2 * part, B + ((size_t)c * kLines + blockIdx.x) * (kLine / 2) + part);
+    }
+    copy_twiddles<kRowThreads>(tws, tw);
+    float4 *wrows = w + (size_t)kRowsBlock * blockIdx.x * kG;
+    const int nodes = min(kRowsBlock, kG - kRowsBlock * (int)blockIdx.x) * kG;
+    for (int j = threadIdx.x; j < nodes; j += kRowThreads) copy16(charges + j, wrows + j);
     const float scale = 1.0f / ((float)kM * (float)kM);
     const float imag_scale = plane == 1 ? scale * load_geom(state, slot).r2_unscale : scale;
     copies_done();
     if (zero_w)
-        for (int j = threadIdx.x; j < kG; j += 64) wrow[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int j = threadIdx.x; j < nodes; j += kRowThreads) wrows[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float2 v[kR];
 #pragma unroll
     for (int r = 0; r < kR; r++) {
         const int k = kR * r + min(lane, kR - 1);
-        v[r] = in[plane][column_of(k)][slot_of(k)];
+        v[r] = stage[column_of(k) * kStageLine + place_in_line(2 * plane + slot_of(k), blockIdx.x, row)];
     }
-    fft784_warp<true, kR>(v, exch[plane], tws, lane);
+    __syncthreads();
+    fft784_warp<true, kR>(v, stage + wi * kEx, tws, lane);
     float2 *out = reinterpret_cast<float2 *>(ytilde + (size_t)row * kG) + plane;
+    const float4 *charge = charges + (wi >> 1) * kG;
     double z = 0.0;
 #pragma unroll
     for (int r = 0; r < kHalf; r++) {
         const int j = kR * r + lane;
-        if (lane < kR && j < kG) {
+        if (lane < kR && j < kG && row < kG) {
             const float2 p = make_float2(v[r].x * scale, v[r].y * imag_scale);
             out[2 * j] = p;
             // node = (x, y, count, r^2) charges and potentials:
@@ -386,12 +433,14 @@ fft_rows_inverse_kernel(const float4 *__restrict__ B, float4 *__restrict__ w, fl
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-    __shared__ double other;
-    if (threadIdx.x == 32) other = z;
+    __shared__ double zs[2 * kRowsBlock];
+    if (lane == 0) zs[wi] = z;
     __syncthreads();
     if (threadIdx.x == 0) {
-        atomicAdd(&state->zsum[slot], z + other);
-        if (row == 0) {   // recycle the other slot's min/max and this slot's norm for this iteration's update
+#pragma unroll
+        for (int k = 1; k < 2 * kRowsBlock; k++) z += zs[k];
+        atomicAdd(&state->zsum[slot], z);
+        if (blockIdx.x == 0) {   // recycle the other slot's min/max and this slot's norm for this iteration's update
             state->min_enc[slot ^ 1] = 0xffffffffu;
             state->max_enc[slot ^ 1] = 0u;
             state->unorm2[slot] = 0.0;
@@ -403,18 +452,20 @@ fft_rows_inverse_kernel(const float4 *__restrict__ B, float4 *__restrict__ w, fl
 
 size_t fft_workspace_bytes()
 {
-    return sizeof(float4) * (size_t)kG * kC * 2 * 2 + sizeof(float) * ((size_t)kG * kRkStride + (size_t)kC * kM) + sizeof(float2) * kM;
+    return sizeof(float2) * (size_t)kC * kLines * kLine * 2 + sizeof(float) * ((size_t)kG * kRkStride + (size_t)kC * kM) + sizeof(float2) * kM;
 }
 
 int fft_workspace_init(FftWorkspace *ws, void *mem, cudaStream_t st)
 {
     char *p = static_cast<char *>(mem);
-    ws->A = reinterpret_cast<float4 *>(p); p += sizeof(float4) * (size_t)kG * kC * 2;
-    ws->B = reinterpret_cast<float4 *>(p); p += sizeof(float4) * (size_t)kG * kC * 2;
+    ws->A = reinterpret_cast<float4 *>(p); p += sizeof(float2) * (size_t)kC * kLines * kLine;
+    ws->B = reinterpret_cast<float4 *>(p); p += sizeof(float2) * (size_t)kC * kLines * kLine;
     ws->tw = reinterpret_cast<float2 *>(p); p += sizeof(float2) * kM;
     ws->Kh = reinterpret_cast<float *>(p); p += sizeof(float) * (size_t)kC * kM;
     ws->Rk = reinterpret_cast<float *>(p);
-    static_assert(kColsSmem <= 48 * 1024, "columns pass: three blocks to an SM, and no more than a kernel may have unasked");
+    B200_CUDA(cudaFuncSetAttribute(fft_rows_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem));
+    B200_CUDA(cudaFuncSetAttribute(fft_rows_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBackSmem));
+    static_assert(kColsSmem <= 48 * 1024, "columns pass: no more than a kernel may have unasked");
     twiddle_init_kernel<<<(kM + 255) / 256, 256, 0, st>>>(ws->tw);
     B200_CUDA(cudaGetLastError());
     return 0;
@@ -440,16 +491,16 @@ int launch_kernel_spectrum(const IterState *state, int slot, const FftWorkspace 
 
 int launch_convolve_rows(const float4 *w, const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st)
 {
-    fft_rows_forward_kernel<<<kG, 64, 0, st>>>(w, ws.A, state, slot, ws.tw);
+    fft_rows_forward_kernel<<<kLines, kRowThreads, kRowsSmem, st>>>(w, ws.A, state, slot, ws.tw);
     B200_CUDA(cudaGetLastError());
     return 0;
 }
 
 int launch_convolve(float4 *w, float4 *ytilde, IterState *state, int slot, const FftWorkspace &ws, bool zero_w, cudaStream_t st)
 {
-    fft_columns_kernel<<<kC, 128, kColsSmem, st>>>(reinterpret_cast<const float2 *>(ws.A), ws.Kh, ws.B, ws.tw);
+    fft_columns_kernel<<<kC, 128, kColsSmem, st>>>(ws.A, ws.Kh, ws.B, ws.tw);
     B200_CUDA(cudaGetLastError());
-    fft_rows_inverse_kernel<<<kG, 64, 0, st>>>(ws.B, w, ytilde, state, slot, ws.tw, zero_w ? 1 : 0);
+    fft_rows_inverse_kernel<<<kLines, kRowThreads, kBackSmem, st>>>(ws.B, w, ytilde, state, slot, ws.tw, zero_w ? 1 : 0);
     B200_CUDA(cudaGetLastError());
     return 0;
 }
