@@ -43,7 +43,7 @@ namespace {
 constexpr int kR = 28;                       // kM = kR * kR
 constexpr int kHalf = kR / 2;                // registers that hold a 390-point input or output: 28 * 14 >= 390
 constexpr int kC = kM / 2 + 1;               // distinct columns of an even spectrum: 0 .. 392
-constexpr int kRkStride = kC + 1;            // row of Rk, padded to whole pairs of columns
+constexpr int kRkStride = (kC + 15) / 16 * 16;   // row of Rk: whole groups of the columns that a block of the second axis takes
 constexpr int kExStride = kR + 1;            // float2 per row of the exchange buffer (odd: no bank conflicts)
 constexpr int kEx = kR * kExStride;
 static_assert(kM == kR * kR && kM >= 2 * kG - 1 && kR * kHalf >= kG && kR * (kHalf - 1) < kG, "transform length");
@@ -270,33 +270,6 @@ spectrum_rows_kernel(float *__restrict__ Rk, const IterState *state, int slot, c
     }
 }
 
-// ---- second axis: two real columns per warp; Kh[c][k] ----
-__global__ void __launch_bounds__(kSpecWarps * 32)
-spectrum_columns_kernel(const float *__restrict__ Rk, float *__restrict__ Kh, const float2 *__restrict__ tw)
-{
-    __shared__ __align__(16) float2 tws[kM];
-    __shared__ float2 exch[kSpecWarps][kEx];
-    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    const int c = 2 * (blockIdx.x * kSpecWarps + wi);
-    float2 v[kR];
-#pragma unroll
-    for (int r = 0; r < kHalf; r++) {
-        const int row = kR * r + lane;
-        v[r] = (lane < kR && row < kG && c < kC) ? *reinterpret_cast<const float2 *>(Rk + (size_t)row * kRkStride + c) : make_float2(0.0f, 0.0f);
-    }
-    copy_twiddles<kSpecWarps * 32>(tws, tw);
-    mirror_input(v, lane);
-    copies_done();
-    fft784_warp<false, kR>(v, exch[wi], tws, lane);
-    if (c >= kC || lane >= kR) return;
-#pragma unroll
-    for (int r = 0; r < kR; r++) {
-        const int k = kR * r + lane;
-        Kh[(size_t)c * kM + k] = v[r].x;
-        if (c + 1 < kC) Kh[(size_t)(c + 1) * kM + k] = v[r].y;
-    }
-}
-
 // ---- workspace between the passes ----
 // Column pair c (a column, its mirror image, both planes: q = 0 .. 3) and four rows are a line of 128 bytes; the lines of a
 // column pair follow one another.  A block of the row passes has four rows, so it writes or reads whole lines, and a block of
@@ -312,11 +285,51 @@ constexpr size_t kStageBytes = sizeof(float2) * kC * kStageLine, kRowExBytes = s
 constexpr size_t kRowsSmem = sizeof(float2) * kM + (kStageBytes > kRowExBytes ? kStageBytes : kRowExBytes);
 constexpr size_t kBackSmem = kRowsSmem + sizeof(float4) * kRowsBlock * kG;
 
-// ---- first pass: four rows of the charge grid, both planes ----
+// ---- spectrum, second axis: sixteen columns per block, two real ones per warp; Kh[c][k] ----
+constexpr int kSpecCols = 2 * kRowThreads / 32, kSpecBlocks = kRkStride / kSpecCols;
+constexpr int kSpecRow = kSpecCols + 4;   // floats per row in shared memory
+static_assert(kRkStride % kSpecCols == 0 && kSpecBlocks * kSpecCols >= kC, "columns of the spectrum");
+static_assert(sizeof(float) * kG * kSpecRow <= kStageBytes, "the columns fit where the lines are staged");
+__device__ __forceinline__ void spectrum_columns(float2 *smem, const float *__restrict__ Rk, float *__restrict__ Kh, const float2 *__restrict__ tw, int block)
+{
+    float2 *tws = smem, *ex = smem + kM + (threadIdx.x >> 5) * kEx;
+    float *cols = reinterpret_cast<float *>(smem + kM);   // before the exchange
+    const int lane = threadIdx.x & 31, own = 2 * (threadIdx.x >> 5), c = kSpecCols * block + own;
+    for (int u = threadIdx.x; u < kG * kSpecCols / 4; u += kRowThreads) {
+        const int row = u / (kSpecCols / 4), part = u % (kSpecCols / 4);
+        copy16(cols + row * kSpecRow + 4 * part, Rk + (size_t)row * kRkStride + kSpecCols * block + 4 * part);
+    }
+    copy_twiddles<kRowThreads>(tws, tw);
+    copies_done();
+    float2 v[kR];
+#pragma unroll
+    for (int r = 0; r < kHalf; r++) {
+        const int row = kR * r + lane;
+        v[r] = (lane < kR && row < kG) ? *reinterpret_cast<const float2 *>(cols + row * kSpecRow + own) : make_float2(0.0f, 0.0f);
+    }
+    __syncthreads();
+    mirror_input(v, lane);
+    fft784_warp<false, kR>(v, ex, tws, lane);
+    if (c >= kC || lane >= kR) return;
+#pragma unroll
+    for (int r = 0; r < kR; r++) {
+        const int k = kR * r + lane;
+        Kh[(size_t)c * kM + k] = v[r].x;
+        if (c + 1 < kC) Kh[(size_t)(c + 1) * kM + k] = v[r].y;
+    }
+}
+
+// ---- first pass: four rows of the charge grid, both planes; the blocks after those take the spectrum's second axis, on SMs
+// that would idle ----
 __global__ void __launch_bounds__(kRowThreads)
-fft_rows_forward_kernel(const float4 *__restrict__ w, float4 *__restrict__ A, const IterState *state, int slot, const float2 *__restrict__ tw)
+fft_rows_forward_kernel(const float4 *__restrict__ w, float4 *__restrict__ A, const float *__restrict__ Rk, float *__restrict__ Kh,
+                        const IterState *state, int slot, const float2 *__restrict__ tw)
 {
     extern __shared__ __align__(16) float2 smem[];
+    if (blockIdx.x >= kLines) {
+        spectrum_columns(smem, Rk, Kh, tw, blockIdx.x - kLines);
+        return;
+    }
     float2 *tws = smem, *stage = smem + kM;   // the lines, once the exchange is over
     const int lane = threadIdx.x & 31, plane = (threadIdx.x >> 5) & 1, row = kRowsBlock * blockIdx.x + (threadIdx.x >> 6);
     copy_twiddles<kRowThreads>(tws, tw);
@@ -481,17 +494,14 @@ int convolve_wave_sms(int *sms)
 
 int launch_kernel_spectrum(const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st)
 {
-    constexpr int row_blocks = (kG + kSpecWarps - 1) / kSpecWarps, col_blocks = ((kC + 1) / 2 + kSpecWarps - 1) / kSpecWarps;
-    spectrum_rows_kernel<<<row_blocks, kSpecWarps * 32, 0, st>>>(ws.Rk, state, slot, ws.tw);
-    B200_CUDA(cudaGetLastError());
-    spectrum_columns_kernel<<<col_blocks, kSpecWarps * 32, 0, st>>>(ws.Rk, ws.Kh, ws.tw);
+    spectrum_rows_kernel<<<(kG + kSpecWarps - 1) / kSpecWarps, kSpecWarps * 32, 0, st>>>(ws.Rk, state, slot, ws.tw);
     B200_CUDA(cudaGetLastError());
     return 0;
 }
 
 int launch_convolve_rows(const float4 *w, const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st)
 {
-    fft_rows_forward_kernel<<<kLines, kRowThreads, kRowsSmem, st>>>(w, ws.A, state, slot, ws.tw);
+    fft_rows_forward_kernel<<<kLines + kSpecBlocks, kRowThreads, kRowsSmem, st>>>(w, ws.A, ws.Rk, ws.Kh, state, slot, ws.tw);
     B200_CUDA(cudaGetLastError());
     return 0;
 }

@@ -363,7 +363,7 @@ int Session::one_iteration(int norm_mode, float stop_norm)
         B200_CUDA(cudaStreamWaitEvent(stream3, ev_fork, 0));
         B200_TRY(launch_kernel_spectrum(state, slot, fft, stream3));
         B200_CUDA(cudaEventRecord(ev_spectrum, stream3));
-        launches += 2;
+        launches += 1;
     }
 
     // The embedding reshuffles quickly while it is being exaggerated and slowly afterwards: sort every
@@ -398,10 +398,10 @@ int Session::one_iteration(int norm_mode, float stop_norm)
     clk.begin(stream);
     float4 *charges = p2p ? w_sum : w;
     if (stage_timers) B200_TRY(launch_kernel_spectrum(state, slot, fft, stream));
+    else B200_CUDA(cudaStreamWaitEvent(stream, ev_spectrum, 0));
     B200_TRY(launch_convolve_rows(charges, state, slot, fft, stream));
-    if (!stage_timers) B200_CUDA(cudaStreamWaitEvent(stream, ev_spectrum, 0));
     B200_TRY(launch_convolve(charges, ytilde, state, slot, fft, !p2p, stream));   // sums Z over ALL points on the grid: no exchange
-    clk.end(stream, kStConvolve, stage_timers ? 5 : 3);
+    clk.end(stream, kStConvolve, stage_timers ? 4 : 3);
     const bool fused = !multi && !stage_timers;   // the update interpolates the repulsive force itself
     if (!fused) {
         clk.begin(stream);
