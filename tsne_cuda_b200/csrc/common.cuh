@@ -49,7 +49,7 @@ struct IterState {
 // Lagrange constants evaluated on the host exactly as the reference does (src/fit_tsne.cu:303-320).
 struct InterpConsts {
     float sp[kInterp];
-    float den[kInterp];
+    float den[kInterp], den_inv[kInterp];
 };
 InterpConsts make_interp_consts();
 

@@ -147,11 +147,37 @@ template <bool INV, int NZ> __device__ __forceinline__ void fft28(float2 (&v)[kR
     }
 }
 
+// Everything a block needs besides the values of its own transforms goes to shared memory with asynchronous copies, all
+// in flight at once: a loop of loads and stores waits for L2 once per round (seven to thirteen rounds here), which cost
+// more than the transforms.
+__device__ __forceinline__ void copy16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// What is needed first is a batch of its own: copies arrive at 64 bytes a cycle, and the transform starts on the first batch.
+__device__ __forceinline__ void end_batch() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LATER> __device__ __forceinline__ void copies_done()   // all but the last LATER batches are there, for the whole block
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(LATER) : "memory");
+    __syncthreads();
+}
+template <int THREADS> __device__ __forceinline__ void copy_floats(float *dst, const float *__restrict__ src, int n4)   // n4 times four
+{
+    for (int k = threadIdx.x; k < n4; k += THREADS) copy16(dst + 4 * k, src + 4 * k);
+}
+template <int THREADS> __device__ __forceinline__ void copy_twiddles(float2 *tws, const float2 *__restrict__ tw)
+{
+    copy_floats<THREADS>(reinterpret_cast<float *>(tws), reinterpret_cast<const float *>(tw), kM / 2);
+}
+
 // 784-point transform by one warp.  In: lane l < 28 holds x[28 r + l] in v[r] (zero from r = NZ on).  Out: lane l holds
-// X[l + 28 r] in v[r], the same pattern.  ex: kEx float2 of this warp; tws[k * 28 + l] = e^{-2 pi i k l / 784}.
-template <bool INV, int NZ> __device__ __forceinline__ void fft784_warp(float2 (&v)[kR], float2 *ex, const float2 *tws, int lane)
+// X[l + 28 r] in v[r], the same pattern.  ex: kEx float2 of this warp; tws[k * 28 + l] = e^{-2 pi i k l / 784}, there
+// when twiddles_ready() returns.
+template <bool INV, int NZ, class READY>
+__device__ __forceinline__ void fft784_warp(float2 (&v)[kR], float2 *ex, const float2 *tws, int lane, READY twiddles_ready)
 {
     fft28<INV, NZ>(v);
+    twiddles_ready();
     if (lane < kR) {
         ex[lane] = v[0];
 #pragma unroll
@@ -167,27 +193,6 @@ template <bool INV, int NZ> __device__ __forceinline__ void fft784_warp(float2 (
     for (int n = 0; n < kR; n++) v[n] = row[n];
     __syncwarp();
     fft28<INV, kR>(v);
-}
-
-// Everything a block needs besides the values of its own transforms goes to shared memory with asynchronous copies, all
-// in flight at once: a loop of loads and stores waits for L2 once per round (seven to thirteen rounds here), which cost
-// more than the transforms.
-__device__ __forceinline__ void copy16(void *dst, const void *src)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copies_done()
-{
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-}
-template <int THREADS> __device__ __forceinline__ void copy_floats(float *dst, const float *__restrict__ src, int n4)   // n4 times four
-{
-    for (int k = threadIdx.x; k < n4; k += THREADS) copy16(dst + 4 * k, src + 4 * k);
-}
-template <int THREADS> __device__ __forceinline__ void copy_twiddles(float2 *tws, const float2 *__restrict__ tw)
-{
-    copy_floats<THREADS>(reinterpret_cast<float *>(tws), reinterpret_cast<const float *>(tw), kM / 2);
 }
 
 __global__ void twiddle_init_kernel(float2 *tw)
@@ -245,6 +250,7 @@ spectrum_rows_kernel(float *__restrict__ Rk, const IterState *state, int slot, c
     __shared__ __align__(16) float2 tws[kM];
     __shared__ float2 exch[kSpecWarps][kEx];
     copy_twiddles<kSpecWarps * 32>(tws, tw);
+    end_batch();
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
     const int row = blockIdx.x * kSpecWarps + wi;
     const GridGeom g = load_geom(state, slot);
@@ -258,8 +264,7 @@ spectrum_rows_kernel(float *__restrict__ Rk, const IterState *state, int slot, c
         v[r] = make_float2(in ? value : 0.0f, 0.0f);
     }
     mirror_input(v, lane);
-    copies_done();
-    fft784_warp<false, kR>(v, exch[wi], tws, lane);
+    fft784_warp<false, kR>(v, exch[wi], tws, lane, copies_done<0>);
     if (row >= kG || lane >= kR) return;
 #pragma unroll
     for (int r = 0; r <= kHalf; r++) {
@@ -299,17 +304,18 @@ __device__ __forceinline__ void spectrum_columns(float2 *smem, const float *__re
         const int row = u / (kSpecCols / 4), part = u % (kSpecCols / 4);
         copy16(cols + row * kSpecRow + 4 * part, Rk + (size_t)row * kRkStride + kSpecCols * block + 4 * part);
     }
+    end_batch();
     copy_twiddles<kRowThreads>(tws, tw);
-    copies_done();
+    end_batch();
+    copies_done<1>();
     float2 v[kR];
 #pragma unroll
     for (int r = 0; r < kHalf; r++) {
         const int row = kR * r + lane;
         v[r] = (lane < kR && row < kG) ? *reinterpret_cast<const float2 *>(cols + row * kSpecRow + own) : make_float2(0.0f, 0.0f);
     }
-    __syncthreads();
     mirror_input(v, lane);
-    fft784_warp<false, kR>(v, ex, tws, lane);
+    fft784_warp<false, kR>(v, ex, tws, lane, copies_done<0>);
     if (c >= kC || lane >= kR) return;
 #pragma unroll
     for (int r = 0; r < kR; r++) {
@@ -333,6 +339,7 @@ fft_rows_forward_kernel(const float4 *__restrict__ w, float4 *__restrict__ A, co
     float2 *tws = smem, *stage = smem + kM;   // the lines, once the exchange is over
     const int lane = threadIdx.x & 31, plane = (threadIdx.x >> 5) & 1, row = kRowsBlock * blockIdx.x + (threadIdx.x >> 6);
     copy_twiddles<kRowThreads>(tws, tw);
+    end_batch();
     const float2 *wrow = reinterpret_cast<const float2 *>(w + (size_t)row * kG) + plane;   // .xy or .zw of each node
     float2 v[kR];
 #pragma unroll
@@ -343,8 +350,7 @@ fft_rows_forward_kernel(const float4 *__restrict__ w, float4 *__restrict__ A, co
     const float imag_scale = plane == 1 ? load_geom(state, slot).r2_scale : 1.0f;
 #pragma unroll
     for (int r = 0; r < kHalf; r++) v[r].y *= imag_scale;
-    copies_done();
-    fft784_warp<false, kHalf>(v, stage + (threadIdx.x >> 5) * kEx, tws, lane);
+    fft784_warp<false, kHalf>(v, stage + (threadIdx.x >> 5) * kEx, tws, lane, copies_done<0>);
     __syncthreads();
     if (lane < kR) {
 #pragma unroll
@@ -372,9 +378,12 @@ fft_columns_kernel(const float4 *__restrict__ A, const float *__restrict__ Kh, f
     const int lane = threadIdx.x & 31, q = threadIdx.x >> 5, c = blockIdx.x;
     constexpr int n4 = kLines * kLine / 2;
     copy_floats<128>(reinterpret_cast<float *>(lines), reinterpret_cast<const float *>(A + (size_t)c * n4), n4);
+    end_batch();
     copy_twiddles<128>(tws, tw);
+    end_batch();
     copy_floats<128>(spec, Kh + (size_t)c * kM, kM / 4);
-    copies_done();
+    end_batch();
+    copies_done<2>();
     const int sl = min(lane, kR - 1);
     float2 *mine = lines + (sl / kRowsBlock) * kLine;   // rows 28 r + lane: 7 r lines further on; a warp has its q to itself
     float2 v[kR];
@@ -382,10 +391,11 @@ fft_columns_kernel(const float4 *__restrict__ A, const float *__restrict__ Kh, f
     for (int r = 0; r < kHalf; r++) {
         v[r] = mine[r * (kR / kRowsBlock) * kLine + place_in_line(q, r * (kR / kRowsBlock) + sl / kRowsBlock, sl)];
     }
-    fft784_warp<false, kHalf>(v, ex, tws, lane);
+    fft784_warp<false, kHalf>(v, ex, tws, lane, copies_done<1>);
+    copies_done<0>();
 #pragma unroll
     for (int r = 0; r < kR; r++) v[r] = times(spec[kR * r + sl], v[r]);
-    fft784_warp<true, kR>(v, ex, tws, lane);
+    fft784_warp<true, kR>(v, ex, tws, lane, [] {});
     if (lane < kR) {
 #pragma unroll
         for (int r = 0; r < kHalf; r++) mine[r * (kR / kRowsBlock) * kLine + place_in_line(q, r * (kR / kRowsBlock) + sl / kRowsBlock, sl)] = v[r];
@@ -410,23 +420,26 @@ fft_rows_inverse_kernel(const float4 *__restrict__ B, float4 *__restrict__ w, fl
         const int c = u / (kLine / 2), part = u % (kLine / 2);
         copy16(stage + c * kStageLine + 2 * part, B + ((size_t)c * kLines + blockIdx.x) * (kLine / 2) + part);
     }
+    end_batch();
     copy_twiddles<kRowThreads>(tws, tw);
+    end_batch();
     float4 *wrows = w + (size_t)kRowsBlock * blockIdx.x * kG;
     const int nodes = min(kRowsBlock, kG - kRowsBlock * (int)blockIdx.x) * kG;
     for (int j = threadIdx.x; j < nodes; j += kRowThreads) copy16(charges + j, wrows + j);
+    end_batch();
     const float scale = 1.0f / ((float)kM * (float)kM);
     const float imag_scale = plane == 1 ? scale * load_geom(state, slot).r2_unscale : scale;
-    copies_done();
-    if (zero_w)
-        for (int j = threadIdx.x; j < nodes; j += kRowThreads) wrows[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    copies_done<2>();
     float2 v[kR];
 #pragma unroll
     for (int r = 0; r < kR; r++) {
         const int k = kR * r + min(lane, kR - 1);
         v[r] = stage[column_of(k) * kStageLine + place_in_line(2 * plane + slot_of(k), blockIdx.x, row)];
     }
-    __syncthreads();
-    fft784_warp<true, kR>(v, stage + wi * kEx, tws, lane);
+    fft784_warp<true, kR>(v, stage + wi * kEx, tws, lane, copies_done<1>);   // (a barrier: the lines have been read)
+    copies_done<0>();
+    if (zero_w)
+        for (int j = threadIdx.x; j < nodes; j += kRowThreads) wrows[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float2 *out = reinterpret_cast<float2 *>(ytilde + (size_t)row * kG) + plane;
     const float4 *charge = charges + (wi >> 1) * kG;
     double z = 0.0;

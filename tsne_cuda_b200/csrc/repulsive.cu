@@ -29,6 +29,7 @@ InterpConsts make_interp_consts()
         c.den[i] = 1;
         for (int j = 0; j < kInterp; j++)
             if (i != j) c.den[i] *= c.sp[i] - c.sp[j];
+        c.den_inv[i] = 1 / c.den[i];
     }
     return c;
 }
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(256) minmax_kernel(const float2 *__restrict__ 
 // each run issues the nine vector reductions.
 __device__ __forceinline__ int axis_box(float c, const GridGeom &g)
 {
-    int idx = (int)((c - g.cmin) / g.box_width);
+    int idx = (int)in_boxes(c - g.cmin, g);
     idx = max(0, idx);
     return min(kBoxes - 1, idx);
 }
@@ -193,6 +194,7 @@ spread_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows,
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const bool take = lane + d <= run_end;
+            if (!__any_sync(0xffffffffu, take)) break;   // no run is that long
 #pragma unroll
             for (int a = 0; a < kInterp; a++)
 #pragma unroll
@@ -208,7 +210,8 @@ spread_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows,
 }
 
 // No order, no merging: a point per thread (few points, see kSpreadPerLane).
-__global__ void __launch_bounds__(128)
+constexpr int kSpreadSmallThreads = 32;
+__global__ void __launch_bounds__(kSpreadSmallThreads)
 spread_direct_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows, const IterState *state, int slot, InterpConsts ic,
                      float4 *__restrict__ w)
 {
@@ -412,8 +415,8 @@ int launch_spread(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_
 {
     const long long n = row_hi - row_lo;
     if (n <= 0) return 0;
-    if (!order && n <= kSpreadDirectMax) spread_direct_kernel<<<nblk(n, 128), 128, 0, st>>>(Y2, row_lo, n, state, slot, ic, w);
-    else if (n <= kSpreadSingleMax) spread_kernel<1><<<nblk(n, 256), 256, 0, st>>>(Y2, row_lo, n, order, state, slot, ic, w, hist);
+    if (!order && n <= kSpreadDirectMax) spread_direct_kernel<<<nblk(n, kSpreadSmallThreads), kSpreadSmallThreads, 0, st>>>(Y2, row_lo, n, state, slot, ic, w);
+    else if (n <= kSpreadSingleMax) spread_kernel<1><<<nblk(n, 64), 64, 0, st>>>(Y2, row_lo, n, order, state, slot, ic, w, hist);
     else spread_kernel<kSpreadPerLane><<<nblk((n + kSpreadPerLane - 1) / kSpreadPerLane, 256), 256, 0, st>>>(Y2, row_lo, n, order, state, slot, ic, w, hist);
     B200_CUDA(cudaGetLastError());
     return 0;

@@ -40,8 +40,8 @@ __device__ __forceinline__ void step_point(float2 &y, const float2 fa, const flo
 // 2 us at 1 500 points and 5 at 200 000.)
 // norm_mode 1: unorm2[slot] = sum of squared updates.  2: and nothing is changed any more once the previous iteration's
 // norm is below stop_norm (the iterations the host has queued beyond the reference's stop leave the state alone).
-template <bool GATHER>
-__global__ void __launch_bounds__(256)
+template <bool GATHER, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 update_kernel(const float2 *Y2, UpdateTargets dst, const float2 *__restrict__ Fa, const float2 *__restrict__ Fr,
               const float4 *__restrict__ ytilde, InterpConsts ic, float2 *__restrict__ gains, float2 *__restrict__ u2, long long row_lo,
               long long n_rows, long long n_total, IterState *state, int slot, float eta, float momentum, float exaggeration,
@@ -71,26 +71,29 @@ update_kernel(const float2 *Y2, UpdateTargets dst, const float2 *__restrict__ Fa
         nrm = u.x * u.x + u.y * u.y;
         bad = !(isfinite(y.x) && isfinite(y.y));
     }
+    // order-preserving encodings: one reduction instruction each (a coordinate that is no number counts for neither)
+    unsigned emn = __reduce_min_sync(0xffffffffu, enc_float(fminf(INFINITY, mn))), emx = __reduce_max_sync(0xffffffffu, enc_float(fmaxf(-INFINITY, mx)));
+    if (norm_mode) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (norm_mode) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+        for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
     }
     bad = __any_sync(0xffffffffu, bad);
-    __shared__ float s_mn[8], s_mx[8], s_n[8];
-    __shared__ int s_bad[8];
+    constexpr int kWarps = THREADS / 32;
+    __shared__ unsigned s_mn[kWarps], s_mx[kWarps];
+    __shared__ float s_n[kWarps];
+    __shared__ int s_bad[kWarps];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) { s_mn[w] = mn; s_mx[w] = mx; s_n[w] = nrm; s_bad[w] = bad; }
+    if (lane == 0) { s_mn[w] = emn; s_mx[w] = emx; s_n[w] = nrm; s_bad[w] = bad; }
     __syncthreads();
     if (threadIdx.x == 0) {
         double tot = 0.0;
-        for (int k = 0; k < 8; k++) {
-            mn = fminf(mn, s_mn[k]); mx = fmaxf(mx, s_mx[k]); tot += (double)s_n[k]; bad |= s_bad[k];
+#pragma unroll
+        for (int k = 0; k < kWarps; k++) {
+            emn = min(emn, s_mn[k]); emx = max(emx, s_mx[k]); tot += (double)s_n[k]; bad |= s_bad[k];
         }
-        if (mn <= mx) {
-            atomicMin(&state->min_enc[slot ^ 1], enc_float(mn));
-            atomicMax(&state->max_enc[slot ^ 1], enc_float(mx));
+        if (emn <= emx) {
+            atomicMin(&state->min_enc[slot ^ 1], emn);
+            atomicMax(&state->max_enc[slot ^ 1], emx);
         }
         if (norm_mode && !stopped) atomicAdd(&state->unorm2[slot], tot);
         if (bad) state->bad = 1;
@@ -180,6 +183,7 @@ __global__ void fill_kernel(float *p, float v, long long n)
     if (i < n) p[i] = v;
 }
 
+constexpr long long kUpdateSmallMax = 148 * 256;
 inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 }  // namespace
 
@@ -188,14 +192,19 @@ int launch_update(const float2 *Y2, const UpdateTargets &dst, const float2 *Fatt
                   float momentum, float exaggeration, int norm_mode, float stop_norm, cudaStream_t st)
 {
     const long long n_rows = row_hi - row_lo;
-    // even an empty shard must run one block so that the state slots are recycled
-    const unsigned blocks = n_rows > 0 ? nblk(n_rows, 256) : 1;
-    if (ytilde)
-        update_kernel<true><<<blocks, 256, 0, st>>>(Y2, dst, Fattr2, nullptr, ytilde, ic, gains2, u2, row_lo, n_rows, N, state, slot, eta,
-                                                    momentum, exaggeration, norm_mode, stop_norm);
+    // Even an empty shard must run one block so that the state slots are recycled.  A warp's nine node reads touch up to 32
+    // lines each, which the SM serves one by one: blocks of two warps as long as larger ones would leave SMs idle.
+    const bool small = n_rows <= kUpdateSmallMax;
+    const unsigned blocks = n_rows > 0 ? nblk(n_rows, small ? 64 : 256) : 1;
+    if (ytilde && small)
+        update_kernel<true, 64><<<blocks, 64, 0, st>>>(Y2, dst, Fattr2, nullptr, ytilde, ic, gains2, u2, row_lo, n_rows, N, state, slot, eta,
+                                                       momentum, exaggeration, norm_mode, stop_norm);
+    else if (ytilde)
+        update_kernel<true, 256><<<blocks, 256, 0, st>>>(Y2, dst, Fattr2, nullptr, ytilde, ic, gains2, u2, row_lo, n_rows, N, state, slot, eta,
+                                                         momentum, exaggeration, norm_mode, stop_norm);
     else
-        update_kernel<false><<<blocks, 256, 0, st>>>(Y2, dst, Fattr2, Frep2, nullptr, ic, gains2, u2, row_lo, n_rows, N, state, slot, eta,
-                                                     momentum, exaggeration, norm_mode, stop_norm);
+        update_kernel<false, 256><<<n_rows > 0 ? nblk(n_rows, 256) : 1, 256, 0, st>>>(Y2, dst, Fattr2, Frep2, nullptr, ic, gains2, u2, row_lo, n_rows, N, state, slot, eta,
+                                                          momentum, exaggeration, norm_mode, stop_norm);
     B200_CUDA(cudaGetLastError());
     return 0;
 }
