@@ -613,6 +613,13 @@ permute_kernel(const float2 *__restrict__ Y2, const int32_t *__restrict__ perm, 
         Fp[q] = make_float2(0.0f, 0.0f);
     }
 }
+// the forces of an iteration whose points are in the copy's order.  One block an SM: as many as the rows need stand in the way
+// of the kernel that follows, whose blocks want a whole SM each (10^6 points 224 -> 231 us an iteration).
+constexpr int kClearBlocks = 148;
+__global__ void __launch_bounds__(256) clear_forces_kernel(float2 *Fp, long long rows)
+{
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < rows; q += (long long)gridDim.x * blockDim.x) Fp[q] = make_float2(0.0f, 0.0f);
+}
 __global__ void __launch_bounds__(256)
 unpermute_kernel(const float2 *__restrict__ Fp, const int32_t *__restrict__ own_pos, long long row_lo, long long rows, float2 *__restrict__ F2)
 {
@@ -658,7 +665,7 @@ __device__ __forceinline__ float2 tile_at(const float2 *tile, unsigned byte_offs
 }
 
 __device__ __forceinline__ void process_chunk(ChunkSet &w, const float2 *__restrict__ tile, const float2 *__restrict__ Yown,
-                                              float2 *__restrict__ Fp, int lane)
+                                              float2 *Fp, int lane)
 {
     const bool head = w.c.x & 0x8000u;
     const unsigned hm = __ballot_sync(0xffffffffu, head);
@@ -700,13 +707,19 @@ __device__ __forceinline__ void process_chunk(ChunkSet &w, const float2 *__restr
 
 __global__ void __launch_bounds__(kBlockedThreads, 1)
 attractive_blocked_kernel(BlockedStream b, const float2 *__restrict__ Yp, const float2 *__restrict__ Yown, long long N,
-                          float2 *__restrict__ Fp)
+                          float2 *Fp)
 {
     extern __shared__ float2 tile[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int nwarps = kBlockedThreads / 32;
     const int c_lo = (int)((long long)b.C * blockIdx.x / gridDim.x), c_hi = (int)((long long)b.C * (blockIdx.x + 1) / gridDim.x);
-    if (c_lo >= c_hi) return;
+    // Launched behind the clear of the forces, it may run beside it up to its first addition: positions and stream are what the
+    // clear found.
+    bool cleared = false;
+    if (c_lo >= c_hi) {
+        after_previous();
+        return;
+    }
     int t = 0;
     {
         int lo = 0, hi = b.ntiles;
@@ -733,6 +746,8 @@ attractive_blocked_kernel(BlockedStream b, const float2 *__restrict__ Yp, const 
             for (int i = threadIdx.x; i < n4; i += kBlockedThreads) dst[i] = __ldg(src + i);
             if ((cnt & 1) && threadIdx.x == 0) tile[cnt - 1] = Yp[base + cnt - 1];
         }
+        if (!cleared) after_previous();
+        cleared = true;
         __syncthreads();
         for (; cc < c_end; cc += nwarps) {
             ChunkSet cur = next;
@@ -1011,7 +1026,7 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
     const float2 *Yp = in_cell_order ? Y2 : b.Yp, *Yown = in_cell_order ? Y2 : b.Yown;
     float2 *Fp = in_cell_order ? F2 : b.Fp;
     const unsigned gN = (unsigned)((std::max(b.N, b.rows) + 255) / 256);
-    if (in_cell_order) B200_CUDA(cudaMemsetAsync(F2, 0, sizeof(float2) * (size_t)b.rows, st));
+    if (in_cell_order) clear_forces_kernel<<<(unsigned)std::min<int64_t>((b.rows + 255) / 256, kClearBlocks), 256, 0, st>>>(F2, b.rows);
     else permute_kernel<<<gN, 256, 0, st>>>(Y2, b.perm, b.N, b.Yp, b.own_perm, b.rows, b.Yown, b.Fp);
     BlockedStream s;
     s.ev = b.ev; s.ec = b.ec; s.chunk_row0 = b.chunk_row0; s.tile_chunk0 = b.tile_chunk0;
@@ -1031,7 +1046,8 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
     // alone: 18 us on 132 blocks, 28 on 27), nor for a rank's share, whose counts above were measured without that rule.
     if (want_blocks <= 0 && beside_grid && b.rows == b.N) sms = b.beside_blocks;
     const int grid = std::max(1, std::min(sms, b.C));
-    attractive_blocked_kernel<<<grid, kBlockedThreads, (size_t)b.T * sizeof(float2), st>>>(s, Yp, Yown, b.N, Fp);
+    if (in_cell_order) B200_CUDA(launch_chained(attractive_blocked_kernel, grid, kBlockedThreads, (size_t)b.T * sizeof(float2), st, s, Yp, Yown, b.N, Fp));
+    else attractive_blocked_kernel<<<grid, kBlockedThreads, (size_t)b.T * sizeof(float2), st>>>(s, Yp, Yown, b.N, Fp);   // (its positions come from the kernel before)
     if (b.extra_C > 0) {   // the reverse-only entries of a truly symmetric P add to the same forces
         BlockedStream x = s;
         x.ev = b.extra_ev; x.ec = b.extra_ec; x.chunk_row0 = b.extra_chunk_row0; x.tile_chunk0 = b.extra_tile_chunk0; x.C = b.extra_C;

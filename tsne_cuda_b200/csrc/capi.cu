@@ -331,7 +331,7 @@ int b200tsne_repulsive(const float *Y, int64_t N, float *Frep, float *Z, float *
     B200_TRY(launch_state_reset(st, sg.st));
     B200_TRY(launch_minmax_init(dY2, N, st, 0, sg.st));
     const InterpConsts ic = make_interp_consts();
-    B200_TRY(launch_spread(dY2, 0, N, nullptr, nullptr, st, 0, ic, dw, sg.st));
+    B200_TRY(launch_spread(dY2, 0, N, nullptr, nullptr, st, 0, ic, dw, nullptr, sg.st));
     if (w_out) B200_TRY(down(w_out, reinterpret_cast<float *>(dw), (size_t)kG * kG * 4, sg.st));
     B200_TRY(launch_kernel_spectrum(st, 0, ws, sg.st));
     B200_TRY(launch_convolve_rows(dw, st, 0, ws, sg.st));

@@ -72,6 +72,33 @@ __host__ __device__ inline float dec_float(unsigned int e)
 #endif
 }
 
+// ---- chained launches ----
+// A kernel of the iteration's chain may be placed on the SMs while the one before it in its stream still runs.  What it does
+// before after_previous() touches constants only; that call returns when the kernel before has ended and its stores are
+// visible, so completion stays as transitive as with plain launches: every thread that touches anything else makes the call,
+// and a block that leaves early makes it too.  let_next_start() allows the next one to be placed once all blocks have made
+// it; without it, when all have ended.  Pointers to what an earlier kernel wrote are not __restrict__: the compiler would be
+// free to read through them before that call.
+#ifdef __CUDACC__
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_chained(void (*kernel)(KArgs...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st, Args... args)
+{
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+#endif
+
 // ---- kernel launchers (all asynchronous on `st`; pointers are device memory) ----
 
 // knn.cu
@@ -207,12 +234,14 @@ constexpr long long kSpreadSingleMax = 131072;   // up to here a lane takes one 
 // order: local row indices sorted by box (null = natural order); see launch_order_refresh
 // hist (optional): the sort's counters, cleared on the way for the next sort
 int launch_spread(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order, int32_t *hist, const IterState *state,
-                  int slot, InterpConsts ic, float4 *w, cudaStream_t st);
+                  int slot, InterpConsts ic, float4 *w, const FftWorkspace *spectrum, cudaStream_t st);
+// spectrum (optional): the same launch does what launch_kernel_spectrum does; possible where a lane takes one point
+inline bool spread_takes_spectrum(int64_t n) { return n > 0 && n <= kSpreadSingleMax; }
 int launch_order_identity(int32_t *order, int64_t n, cudaStream_t st);
 int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, int32_t *order, int32_t *previous, int32_t *keys,
                          int32_t *hist, const IterState *state, int slot, cudaStream_t st);
-// convolve.cu: the kernel's spectrum (needs the slot's min/max only), the first pass over the charges, and the rest, which
-// needs both; the last pass adds sum_i Z_i over all charges to state->zsum[slot] and clears w when asked to
+// convolve.cu: the kernel's spectrum along its first axis (needs the slot's min/max only), the first pass over the charges and
+// the spectrum's second axis, and the rest; the last pass adds sum_i Z_i over all charges to state->zsum[slot] and clears w when asked to
 int launch_kernel_spectrum(const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
 int launch_convolve_rows(const float4 *w, const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
 int convolve_wave_sms(int *sms);   // SMs that hold all blocks of the columns pass at once

@@ -67,18 +67,25 @@ __device__ __forceinline__ void axis_weights(float c, const GridGeom &g, const I
     box = idx;
 }
 
+__device__ __forceinline__ float4 load_node(const float4 *p)   // volatile: a point's nodes are asked for one right after the other
+{
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 // the point's repulsive force before the division by Z, interpolated from the potentials
-__device__ __forceinline__ float2 repulsive_force(float2 y, const GridGeom &g, const InterpConsts &ic, const float4 *__restrict__ ytilde)
+__device__ __forceinline__ float2 repulsive_force(float2 y, const GridGeom &g, const InterpConsts &ic, const float4 *ytilde)
 {
     int bx, by;
     float Lx[kInterp], Ly[kInterp];
     axis_weights(y.x, g, ic, bx, Lx);
     axis_weights(y.y, g, ic, by, Ly);
-    float4 v[kInterp][kInterp];   // all nodes are on their way before the first is used
+    float4 v[kInterp][kInterp];
 #pragma unroll
     for (int a = 0; a < kInterp; a++)
 #pragma unroll
-        for (int b = 0; b < kInterp; b++) v[a][b] = ytilde[(size_t)(bx * kInterp + a) * kG + (by * kInterp + b)];
+        for (int b = 0; b < kInterp; b++) v[a][b] = load_node(ytilde + (size_t)(bx * kInterp + a) * kG + (by * kInterp + b));
     float p1 = 0.0f, p2 = 0.0f, p3 = 0.0f;
 #pragma unroll
     for (int a = 0; a < kInterp; a++) {

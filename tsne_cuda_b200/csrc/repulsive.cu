@@ -13,7 +13,7 @@
 //    r^2-charge) = two packed complex numbers, so a point issues 9 vector reductions instead of 36
 //    scalar atomics.
 //  * The convolution is in convolve.cu.
-#include "grid_geom.cuh"
+#include "fft784.cuh"
 
 #include <algorithm>
 
@@ -108,7 +108,8 @@ __device__ __forceinline__ int axis_box(float c, const GridGeom &g)
 // the points collide so rarely that sorting (three kernels, 15 us) costs more than it saves, and up to kSpreadDirectMax
 // even the shuffles do.  Whole iteration, exaggerated / settled: 5 000 points sorted every time 47 / 41 us, one by one
 // 37 / 37; 20 011 points sorted 44 / 42, merged in natural order 41 / 41, one by one 57 / 42; 60 000 points sorted
-// 54 / 49, natural order 61 / 49.
+// 54 / 49, natural order 61 / 49.  (Both kinds of small spread take blocks of two warps, which leave no SM idle, and the
+// merge ends with the longest run.)
 constexpr int kSpreadPerLane = 4;
 
 __device__ __forceinline__ void spread_flush(float4 *__restrict__ w, int bx, int by, const float (&v)[kInterp][kInterp][4])
@@ -123,19 +124,35 @@ __device__ __forceinline__ void spread_flush(float4 *__restrict__ w, int bx, int
 }
 
 // the counters of the next sort (a clear of its own would be one more node of the chain)
-__device__ __forceinline__ void clear_histogram(int32_t *hist)
+__device__ __forceinline__ void clear_histogram(int32_t *hist, int block, int blocks)
 {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < kBoxes * kBoxes; k += gridDim.x * blockDim.x) hist[k] = 0;
+    for (int k = block * blockDim.x + threadIdx.x; k < kBoxes * kBoxes; k += blocks * blockDim.x) hist[k] = 0;
 }
+
+// What the first blocks of a small map's spread do: the first axis of the kernel's spectrum, which needs the bounding box like
+// the spread and is needed by the kernel after it.  A stream of its own starts when the update has ended; this launch is on
+// its way by then.
+struct SpectrumRows {
+    float *Rk;
+    const float2 *tw;
+    int blocks;   // 0: not here
+};
+constexpr int kSpreadSmallThreads = kSpecWarps * 32;
 
 // hist (optional): the sort's counters, cleared here for the next one
 template <int PER_LANE>
-__global__ void __launch_bounds__(256)
-spread_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows, const int32_t *__restrict__ order,
-              const IterState *state, int slot, InterpConsts ic, float4 *__restrict__ w, int32_t *__restrict__ hist)
+__global__ void __launch_bounds__(PER_LANE == 1 ? kSpreadSmallThreads : 256)
+spread_kernel(const float2 *Y2, long long row_lo, long long n_rows, const int32_t *order, const IterState *state, int slot, InterpConsts ic,
+              float4 *w, int32_t *hist, SpectrumRows spec)
 {
-    if (hist) clear_histogram(hist);
-    const long long t0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * PER_LANE;
+    if (PER_LANE == 1 && blockIdx.x < spec.blocks) {
+        spectrum_rows(spec.Rk, state, slot, spec.tw, blockIdx.x);
+        return;
+    }
+    const int block = PER_LANE == 1 ? blockIdx.x - spec.blocks : blockIdx.x;
+    after_previous();
+    if (hist) clear_histogram(hist, block, PER_LANE == 1 ? gridDim.x - spec.blocks : gridDim.x);
+    const long long t0 = ((long long)block * blockDim.x + threadIdx.x) * PER_LANE;
     const int lane = threadIdx.x & 31;
     const GridGeom g = load_geom(state, slot);
     int key = -1, bx = 0, by = 0;
@@ -210,15 +227,18 @@ spread_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows,
 }
 
 // No order, no merging: a point per thread (few points, see kSpreadPerLane).
-constexpr int kSpreadSmallThreads = 32;
 __global__ void __launch_bounds__(kSpreadSmallThreads)
-spread_direct_kernel(const float2 *__restrict__ Y2, long long row_lo, long long n_rows, const IterState *state, int slot, InterpConsts ic,
-                     float4 *__restrict__ w)
+spread_direct_kernel(const float2 *Y2, long long row_lo, long long n_rows, const IterState *state, int slot, InterpConsts ic, float4 *w, SpectrumRows spec)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x < spec.blocks) {
+        spectrum_rows(spec.Rk, state, slot, spec.tw, blockIdx.x);
+        return;
+    }
+    const long long t = (long long)(blockIdx.x - spec.blocks) * blockDim.x + threadIdx.x;
+    after_previous();
     if (t >= n_rows) return;
-    const GridGeom g = load_geom(state, slot);
     const float2 y = Y2[row_lo + t];
+    const GridGeom g = load_geom(state, slot);
     int bx, by;
     float Lx[kInterp], Ly[kInterp];
     axis_weights(y.x, g, ic, bx, Lx);
@@ -411,14 +431,21 @@ int launch_state_swap(IterState *state, cudaStream_t st)
 }
 
 int launch_spread(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order, int32_t *hist, const IterState *state,
-                  int slot, InterpConsts ic, float4 *w, cudaStream_t st)
+                  int slot, InterpConsts ic, float4 *w, const FftWorkspace *spectrum, cudaStream_t st)
 {
     const long long n = row_hi - row_lo;
+    SpectrumRows spec = {nullptr, nullptr, 0};
+    if (spectrum) spec = {spectrum->Rk, spectrum->tw, kSpecRowBlocks};
+    if (spectrum && !spread_takes_spectrum(n)) return -1;
     if (n <= 0) return 0;
-    if (!order && n <= kSpreadDirectMax) spread_direct_kernel<<<nblk(n, kSpreadSmallThreads), kSpreadSmallThreads, 0, st>>>(Y2, row_lo, n, state, slot, ic, w);
-    else if (n <= kSpreadSingleMax) spread_kernel<1><<<nblk(n, 64), 64, 0, st>>>(Y2, row_lo, n, order, state, slot, ic, w, hist);
-    else spread_kernel<kSpreadPerLane><<<nblk((n + kSpreadPerLane - 1) / kSpreadPerLane, 256), 256, 0, st>>>(Y2, row_lo, n, order, state, slot, ic, w, hist);
-    B200_CUDA(cudaGetLastError());
+    if (!order && n <= kSpreadDirectMax)
+        B200_CUDA(launch_chained(spread_direct_kernel, spec.blocks + nblk(n, kSpreadSmallThreads), kSpreadSmallThreads, 0, st, Y2, row_lo, n, state, slot, ic, w, spec));
+    else if (n <= kSpreadSingleMax)
+        B200_CUDA(launch_chained(spread_kernel<1>, spec.blocks + nblk(n, kSpreadSmallThreads), kSpreadSmallThreads, 0, st, Y2, row_lo, n, order, state, slot, ic, w,
+                                 hist, spec));
+    else
+        B200_CUDA(launch_chained(spread_kernel<kSpreadPerLane>, nblk((n + kSpreadPerLane - 1) / kSpreadPerLane, 256), 256, 0, st, Y2, row_lo, n, order, state,
+                                 slot, ic, w, hist, spec));
     return 0;
 }
 

@@ -2,11 +2,11 @@
 // points to affinities, and the gradient loop (reference: the body of tsnecuda::RunTsne,
 // src/fit_tsne.cu:84-166 for the set-up and :402-580 for the loop).
 //
-// One iteration on one GPU is eight kernels and a clear (three more where the spread order is refreshed) and no host
-// synchronisation:
+// One iteration on one GPU is seven kernels (one more in a large map, three more where the spread order is refreshed) and no
+// host synchronisation:
 //   stream  : [order x3] -> spread -> FFT rows -> FFT columns -> FFT rows^-1 --> update (interpolates the repulsive force)
 //   stream2 : clear forces -> attractive ---------------------------------------^
-//   stream3 : kernel spectrum x2 -> (FFT columns)
+//   stream3 : kernel spectrum of a large map -> (FFT rows); the spread's launch has a small map's
 // A sharded run, and one whose stages are timed, gathers the repulsive force in a kernel of its own before the update.
 // The embedding's min/max and the normalisation sum travel between kernels in device memory
 // (IterState), so the two per-iteration host round trips of the reference do not exist.
@@ -334,6 +334,7 @@ int Session::one_iteration(int norm_mode, float stop_norm)
     const bool p2p = multi && px != nullptr;   // exchanges over peer memory instead of collectives
     StageClock clk(this);
     cudaStream_t sa = stage_timers ? stream : stream2;  // attractive stream
+    const bool spectrum_in_spread = !stage_timers && spread_takes_spectrum(rows());
     if (p2p) {
         // the grid buffer of the next iteration: the peers finished reading it before they signalled the
         // update this rank waited for at the end of the previous iteration
@@ -360,10 +361,13 @@ int Session::one_iteration(int norm_mode, float stop_norm)
         launches += attractive_launches();
         // The kernel's spectrum needs the bounding box only, like the attractive force, so the two start together: in front of
         // that force it delays it by 13 us (10^6 points, exaggerated / settled: 249 / 249 us an iteration, beside it 235 / 240).
-        B200_CUDA(cudaStreamWaitEvent(stream3, ev_fork, 0));
-        B200_TRY(launch_kernel_spectrum(state, slot, fft, stream3));
-        B200_CUDA(cudaEventRecord(ev_spectrum, stream3));
-        launches += 1;
+        // Small maps have it in the spread's launch.
+        if (!spectrum_in_spread) {
+            B200_CUDA(cudaStreamWaitEvent(stream3, ev_fork, 0));
+            B200_TRY(launch_kernel_spectrum(state, slot, fft, stream3));
+            B200_CUDA(cudaEventRecord(ev_spectrum, stream3));
+            launches += 1;
+        }
     }
 
     // The embedding reshuffles quickly while it is being exaggerated and slowly afterwards: sort every
@@ -378,7 +382,8 @@ int Session::one_iteration(int norm_mode, float stop_norm)
         clk.end(stream, kStOrder, 3);
     }
     clk.begin(stream);
-    B200_TRY(launch_spread(Y2, row_lo, row_hi, refresh > 0 ? order : nullptr, refresh > 0 ? box_hist : nullptr, state, slot, ic, w, stream));
+    B200_TRY(launch_spread(Y2, row_lo, row_hi, refresh > 0 ? order : nullptr, refresh > 0 ? box_hist : nullptr, state, slot, ic, w,
+                           spectrum_in_spread ? &fft : nullptr, stream));
     clk.end(stream, kStSpread, 1);
     if (p2p) {
         clk.begin(stream);
@@ -398,7 +403,7 @@ int Session::one_iteration(int norm_mode, float stop_norm)
     clk.begin(stream);
     float4 *charges = p2p ? w_sum : w;
     if (stage_timers) B200_TRY(launch_kernel_spectrum(state, slot, fft, stream));
-    else B200_CUDA(cudaStreamWaitEvent(stream, ev_spectrum, 0));
+    else if (!spectrum_in_spread) B200_CUDA(cudaStreamWaitEvent(stream, ev_spectrum, 0));
     B200_TRY(launch_convolve_rows(charges, state, slot, fft, stream));
     B200_TRY(launch_convolve(charges, ytilde, state, slot, fft, !p2p, stream));   // sums Z over ALL points on the grid: no exchange
     clk.end(stream, kStConvolve, stage_timers ? 4 : 3);

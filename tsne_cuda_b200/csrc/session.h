@@ -153,7 +153,7 @@ struct Session {
     int iterate(int n_iters, float min_gradient_norm, float *elapsed_ms, int *iters_done);
     int one_iteration(int norm_mode, float stop_norm);
     int attractive(cudaStream_t st);   // Fattr of the owned rows from the current embedding
-    int attractive_launches() const { return blocked.ready ? (resident ? 1 : 3) + (blocked.extra_C > 0) : 1 + (extra.count > 0); }
+    int attractive_launches() const { return blocked.ready ? (resident ? 2 : 3) + (blocked.extra_C > 0) : 1 + (extra.count > 0); }
     int affinities_from_points(const float *X_host, int D, float perplexity, float eps);
 };
 

@@ -42,26 +42,33 @@ __device__ __forceinline__ void step_point(float2 &y, const float2 fa, const flo
 // norm is below stop_norm (the iterations the host has queued beyond the reference's stop leave the state alone).
 template <bool GATHER, int THREADS>
 __global__ void __launch_bounds__(THREADS)
-update_kernel(const float2 *Y2, UpdateTargets dst, const float2 *__restrict__ Fa, const float2 *__restrict__ Fr,
-              const float4 *__restrict__ ytilde, InterpConsts ic, float2 *__restrict__ gains, float2 *__restrict__ u2, long long row_lo,
-              long long n_rows, long long n_total, IterState *state, int slot, float eta, float momentum, float exaggeration,
+update_kernel(const float2 *Y2, UpdateTargets dst, const float2 *Fa, const float2 *Fr, const float4 *ytilde, InterpConsts ic, float2 *gains,
+              float2 *u2, long long row_lo, long long n_rows, long long n_total, IterState *state, int slot, float eta, float momentum, float exaggeration,
               int norm_mode, float stop_norm)
 {
-    const double zsum = state->zsum[slot];
-    const float Z = (float)zsum - (float)n_total;
-    const bool stopped = norm_mode == 2 && (float)sqrt(state->unorm2[slot ^ 1]) < stop_norm;
-    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    after_previous();
+    // Everything that does not depend on a position is loaded before anything is computed: the positions' nodes are the second
+    // round trip to L2 then (900 cycles each here) and not the fourth.
+    const long long r = (long long)blockIdx.x * THREADS + threadIdx.x, i = row_lo + r;
+    const bool mine = r < n_rows;
+    float2 y = make_float2(0.0f, 0.0f), g = y, u = y, fa = y, fr = y;
+    if (mine) {
+        y = Y2[i]; g = gains[r]; u = u2[r];
+        fa = __ldcs(Fa + i);
+        if (!GATHER) fr = __ldcs(Fr + i);
+    }
+    const double zsum = state->zsum[slot], last_norm2 = state->unorm2[slot ^ 1];
+    const GridGeom geom = load_geom(state, slot);
     float mn = INFINITY, mx = -INFINITY, nrm = 0.0f;
     int bad = 0;
-    if (r < n_rows) {
-        const long long i = row_lo + r;
-        float2 y = Y2[i], g = gains[r], u = u2[r];
-        const float2 fa = __ldcs(Fa + i);
-        const float2 fr = GATHER ? repulsive_force(y, load_geom(state, slot), ic, ytilde) : __ldcs(Fr + i);
+    const bool stopped = norm_mode == 2 && (float)sqrt(last_norm2) < stop_norm;
+    if (mine) {
+        if (GATHER) fr = repulsive_force(y, geom, ic, ytilde);
+        const float Z = (float)zsum - (float)n_total;
         if (!stopped) {
             step_point(y, fa, fr, g, u, eta, Z, momentum, exaggeration);
 #pragma unroll
-            for (int t = 0; t < kMaxUpdateTargets; t++)
+            for (int t = 0; t < (GATHER ? 1 : kMaxUpdateTargets); t++)   // (GATHER: one GPU)
                 if (t < dst.n) dst.p[t][i] = y;
             gains[r] = g;
             u2[r] = u;
@@ -195,17 +202,13 @@ int launch_update(const float2 *Y2, const UpdateTargets &dst, const float2 *Fatt
     // Even an empty shard must run one block so that the state slots are recycled.  A warp's nine node reads touch up to 32
     // lines each, which the SM serves one by one: blocks of two warps as long as larger ones would leave SMs idle.
     const bool small = n_rows <= kUpdateSmallMax;
-    const unsigned blocks = n_rows > 0 ? nblk(n_rows, small ? 64 : 256) : 1;
-    if (ytilde && small)
-        update_kernel<true, 64><<<blocks, 64, 0, st>>>(Y2, dst, Fattr2, nullptr, ytilde, ic, gains2, u2, row_lo, n_rows, N, state, slot, eta,
-                                                       momentum, exaggeration, norm_mode, stop_norm);
-    else if (ytilde)
-        update_kernel<true, 256><<<blocks, 256, 0, st>>>(Y2, dst, Fattr2, nullptr, ytilde, ic, gains2, u2, row_lo, n_rows, N, state, slot, eta,
-                                                         momentum, exaggeration, norm_mode, stop_norm);
-    else
-        update_kernel<false, 256><<<n_rows > 0 ? nblk(n_rows, 256) : 1, 256, 0, st>>>(Y2, dst, Fattr2, Frep2, nullptr, ic, gains2, u2, row_lo, n_rows, N, state, slot, eta,
-                                                          momentum, exaggeration, norm_mode, stop_norm);
-    B200_CUDA(cudaGetLastError());
+    const auto chained = [&](auto kernel) {
+        const unsigned threads = small ? 64 : 256;
+        return launch_chained(kernel, n_rows > 0 ? nblk(n_rows, threads) : 1, threads, 0, st, Y2, dst, Fattr2, Frep2, ytilde, ic, gains2, u2, row_lo, n_rows, N,
+                              state, slot, eta, momentum, exaggeration, norm_mode, stop_norm);
+    };
+    if (ytilde) B200_CUDA(chained(small ? update_kernel<true, 64> : update_kernel<true, 256>));
+    else B200_CUDA(chained(small ? update_kernel<false, 64> : update_kernel<false, 256>));
     return 0;
 }
 
