@@ -884,29 +884,22 @@ static int device_sms(int *sms)
 }
 
 // Blocks (SMs) of the attractive kernel of an iteration on one GPU, whose grid pipeline runs beside it on the SMs that are left.
-// A small graph is done before the potentials are, so the pipeline is what the iteration waits for, and its longest
-// kernel, the columns pass, has 393 blocks, four to an SM: on 99 SMs or more one wave, on fewer two.  So the graph takes a block per sixteen
-// chunks a warp (1 us each) and at most what leaves 101 SMs (47 of 148: with 99 a block of another kernel that ends late still makes a second
-// wave, 60,000 images on 46 | 47 | 48 | 49 blocks 47.0 / 42.5 | 46.9 / 41.7 | 47.0 / 41.0 | 48.3 / 41.6 us exaggerated / settled), while it
-// is done in the time that the pipeline and the update need: 12 us a launch and 1 us a chunk of a warp, up to 48 us.  A larger graph takes
-// what it takes at any size (one SM in nine left, see launch_attractive_blocked): in between the columns wait for a second wave as well.
-// us an iteration, exaggerated / settled, 90 neighbours (703 chunks per 1,000 points), on 24 | 49 | 64 | 80 | 96 | 132 blocks:
-//   20,011  34.0 / 34.0 | 34.4 / 34.5 | 34.0 / 33.9 | 35.3 / 35.1 | 36.9 / 36.9 | 39.2 / 39.2
-//   45,000  49.0 / 50.4 | 46.0 / 37.8 | 47.0 / 44.7 | 46.7 / 44.0 | 46.7 / 41.7 | 50.5 / 43.2
-//   60,000  59.0 / 60.3 | 48.7 / 40.7 | 47.8 / 44.8 | 48.3 / 44.8 | 48.8 / 44.9 | 51.0 / 45.2
-//   80,000  76.3 / 77.4 | 50.9 / 48.5 | 54.0 / 51.9 | 51.4 / 49.4 | 54.0 / 50.2 | 53.2 / 48.9
-//   100,000 93.3 / 93.7 | 55.3 / 55.9 | 61.0 / 51.0 | 54.9 / 51.9 | 54.4 / 53.8 | 56.2 / 51.6
-// (5,000: 31.3 on 6 to 24 blocks, 39.5 on 132.)  The entries of a truly symmetric P come in a second launch behind the
-// first, so both streams count, and 12 us less are left: 20,011 points on 24 | 32 | 49 | 132 blocks 45.0 | 36.8 | 35.3 | 42.2; 30,011 on 49 |
-// 80 | 132 40.1 | 41.2 | 45.0.  Larger ones were best between the two counts, 45,000 settled on 49 | 80 | 132 53.8 | 47.9 | 51.7, 60,000 63.1 |
-// 51.8 | 55.3: sixteen chunks a warp of the first stream, 24 of both.
-static int blocks_beside_grid(int sms, int wave_sms, long long C, long long extra_C)
+// A chunk of the stream is 0.034 us of an SM; what the pipeline has to do beside it is 1,200 us of one, 3,200 where the iteration
+// sorts its points: the SMs are divided in the proportion of the two, which is where both end together.  (At most six short of all:
+// the pipeline's last kernel is a chain of its own.)  us an iteration, exaggerated (sorting in each iteration from 32,768 points
+// on) / settled, 90 neighbours (703 chunks per 1,000 points, 816 at 10^6), by the number of blocks:
+//   20,011     24 | 47 | 80              26.6 / 26.6 | 27.0 / 26.9 | 27.6 / 27.5
+//   40,000     47 | 64 | 96              40.2 / 31.2 | 39.9 / 31.0 | 39.3 / 32.5
+//   60,000     47 | 64 | 80 | 96         43.2 / 38.5 | 42.9 / 34.1 | 43.2 / 34.0 | 43.5 / 37.2
+//   100,000    64 | 80 | 96 | 132        48.7 / 48.2 | 48.3 / 43.2 | 49.9 / 42.1 | 50.4 / 45.0
+//   200,000    96 | 112 | 128 | 132      62.6 / 61.9 | 63.9 / 62.6 | 66.6 / 61.6 | 73.1 / 62.1
+//   600,000    120 | 124 | 130 | 138     144.3 / 147.3 | 141.6 / 145.1 | 141.1 / 138.7 | 148.5 / 135.6
+//   10^6       128 | 132 | 136 | 142     228.5 / 235.1 | 224.9 / 231.2 | 236.0 / 228.6 | 236.8 / 221.0
+// The entries of a truly symmetric P come in a second launch behind the first, so both streams count.
+static int blocks_beside_grid(int sms, long long chunks, bool sorts)
 {
-    constexpr long long warps = kBlockedThreads / 32;
-    const long long most = sms - sms / 9, spare = std::min<long long>(most, sms - wave_sms - 2);
-    const long long all = C + extra_C;
-    if (all <= spare * warps * (extra_C > 0 ? 24 : 36)) return (int)std::max(6ll, std::min(spare, all / (16 * warps)));
-    return (int)(extra_C > 0 ? std::min(most, std::max(C / (16 * warps), all / (24 * warps))) : most);
+    const long long pipeline = sorts ? 96000 : 35500;   // chunks that take as long
+    return (int)std::max(6ll, std::min<long long>(sms - 6, sms * chunks / (chunks + pipeline)));
 }
 
 // Builds the blocked copy of the owned rows' fixed-width P and, with `extra`, a second stream from a variable-width
@@ -1000,10 +993,6 @@ int blocked_attractive_build(BlockedAttractive *b, DeviceArena &arena, const flo
     b->C = main_stream.C; b->E = main_stream.E; b->groups = main_stream.groups;
     b->extra_ev = extra_stream.ev; b->extra_ec = extra_stream.ec; b->extra_chunk_row0 = extra_stream.chunk_row0;
     b->extra_tile_chunk0 = extra_stream.tile_chunk0; b->extra_C = extra_stream.C; b->extra_E = extra_stream.E;
-    int sms = 0, wave_sms = 0;
-    B200_TRY(device_sms(&sms));
-    B200_TRY(convolve_wave_sms(&wave_sms));
-    b->beside_blocks = blocks_beside_grid(sms, wave_sms, b->C, b->extra_C);
     b->perm = perm; b->own_perm = own_perm; b->own_pos = own_pos;
     b->Yp = Yp; b->Yown = Yown; b->Fp = Fp;
     b->ntiles = ntiles; b->T = T;
@@ -1016,7 +1005,7 @@ int blocked_attractive_build(BlockedAttractive *b, DeviceArena &arena, const flo
 // (Reading the force in cell order from the update kernel and letting it keep the cell-ordered embedding current
 // instead of these two conversion kernels was measured on one GPU: the update kernel's three scattered 8-byte
 // accesses per point cost it 148 us more - 169 instead of 21 - against the 17 us the conversions take.)
-int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, float2 *F2, cudaStream_t st, bool in_cell_order, bool beside_grid)
+int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, float2 *F2, cudaStream_t st, bool in_cell_order, BesideGrid beside)
 {
     if (!b.ready) { set_error("attractive: the blocked copy of P was not built"); return -1; }
     if (in_cell_order && b.rows != b.N) { set_error("attractive: the cell order as the caller's order needs all rows"); return -1; }
@@ -1033,6 +1022,7 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
     s.ntiles = b.ntiles; s.T = b.T; s.C = b.C;
     int sms = 0;
     B200_TRY(device_sms(&sms));
+    const int all_sms = sms;
     // A block fills its SM (1,024 threads, all registers, 224 KB of shared memory), so the grid pipeline that runs
     // beside this kernel on the other stream only gets the SMs this kernel leaves alone.  Measured at N = 10^6,
     // K = 90 on 148 SMs, one GPU: 148 blocks 3,645 iterations/s (attractive stage 175 us), 140: 3,906, 132: 3,962
@@ -1042,9 +1032,11 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
     // when the copy holds all rows, one in three when it holds a rank's share; B200TSNE_ATTRACTIVE_BLOCKS overrides.
     static const int want_blocks = getenv("B200TSNE_ATTRACTIVE_BLOCKS") ? atoi(getenv("B200TSNE_ATTRACTIVE_BLOCKS")) : 0;
     sms = want_blocks > 0 ? std::min(sms, want_blocks) : (b.rows == b.N ? sms - sms / 9 : sms - sms / 3);
-    // Beside the pipeline a small graph takes fewer (see blocks_beside_grid), but not where nothing runs beside it (20,011 x 90
-    // alone: 18 us on 132 blocks, 28 on 27), nor for a rank's share, whose counts above were measured without that rule.
-    if (want_blocks <= 0 && beside_grid && b.rows == b.N) sms = b.beside_blocks;
+    // Beside the pipeline of one GPU the SMs are divided by what either has to do (blocks_beside_grid), but not where nothing runs
+    // beside it (20,011 x 90 alone: 18 us on 132 blocks, 28 on 27), nor for a rank's share, whose counts above were measured
+    // without that rule.
+    if (want_blocks <= 0 && beside != BesideGrid::nothing && b.rows == b.N)
+        sms = blocks_beside_grid(all_sms, (long long)b.C + b.extra_C, beside == BesideGrid::sorting);
     const int grid = std::max(1, std::min(sms, b.C));
     if (in_cell_order) B200_CUDA(launch_chained(attractive_blocked_kernel, grid, kBlockedThreads, (size_t)b.T * sizeof(float2), st, s, Yp, Yown, b.N, Fp));
     else attractive_blocked_kernel<<<grid, kBlockedThreads, (size_t)b.T * sizeof(float2), st>>>(s, Yp, Yown, b.N, Fp);   // (its positions come from the kernel before)

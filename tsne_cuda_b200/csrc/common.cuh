@@ -201,7 +201,6 @@ struct BlockedAttractive {
     float2 *Yp = nullptr, *Yown = nullptr, *Fp = nullptr;
     int ntiles = 0, T = 0, C = 0;
     int64_t E = 0, groups = 0, N = 0, row_lo = 0, rows = 0;
-    int beside_blocks = 0;            // of the kernel where the grid pipeline runs at the same time and the copy holds all rows
     float entries_per_group = 0.0f;   // of the sampled rows, under the chosen order
     bool ready = false;
     void clear();
@@ -212,9 +211,10 @@ int blocked_attractive_build(BlockedAttractive *b, DeviceArena &arena, const flo
                              int64_t row_lo, int64_t row_hi, const int32_t *perm, const ExtraEntries *extra, cudaStream_t st);
 int launch_exclusive_scan_i32(int *data, int64_t n, cudaStream_t st);   // in place; small arrays (one block)
 // in_cell_order: Y2 and F2 are in the copy's own point order (one GPU): no conversion before or after the kernel
-// beside_grid: the grid pipeline runs at the same time
+// beside: what runs at the same time (the grid pipeline of an iteration that sorts its points, or one that does not)
+enum class BesideGrid { nothing, sorting, settled };
 int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, float2 *F2, cudaStream_t st, bool in_cell_order = false,
-                              bool beside_grid = false);
+                              BesideGrid beside = BesideGrid::nothing);
 
 // repulsive.cu
 struct FftWorkspace {
@@ -244,7 +244,6 @@ int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, int32
 // the spectrum's second axis, and the rest; the last pass adds sum_i Z_i over all charges to state->zsum[slot] and clears w when asked to
 int launch_kernel_spectrum(const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
 int launch_convolve_rows(const float4 *w, const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
-int convolve_wave_sms(int *sms);   // SMs that hold all blocks of the columns pass at once
 int launch_convolve(float4 *w, float4 *ytilde, IterState *state, int slot, const FftWorkspace &ws, bool zero_w, cudaStream_t st);
 int launch_gather(const float2 *Y2, int64_t row_lo, int64_t row_hi, const IterState *state, int slot, InterpConsts ic,
                   const float4 *ytilde, float2 *Frep2, cudaStream_t st);

@@ -43,8 +43,6 @@
 
 #include <math.h>
 
-#include <algorithm>
-
 namespace b200 {
 namespace {
 
@@ -294,14 +292,6 @@ int fft_workspace_init(FftWorkspace *ws, void *mem, cudaStream_t st)
     static_assert(kColsSmem <= 48 * 1024, "columns pass: no more than a kernel may have unasked");
     twiddle_init_kernel<<<(kM + 255) / 256, 256, 0, st>>>(ws->tw);
     B200_CUDA(cudaGetLastError());
-    return 0;
-}
-
-int convolve_wave_sms(int *sms)
-{
-    int per_sm = 0;
-    B200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fft_columns_kernel, 128, kColsSmem));
-    *sms = (kC + std::max(per_sm, 1) - 1) / std::max(per_sm, 1);
     return 0;
 }
 

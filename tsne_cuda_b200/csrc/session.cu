@@ -341,17 +341,10 @@ int Session::one_iteration(int norm_mode, float stop_norm)
         B200_CUDA(cudaMemsetAsync(px->w_local(px->parity ^ 1), 0, sizeof(float4) * kG * kG, stream));
     }
 
-    // The attractive kernel and the grid pipeline run side by side, the kernel with one block per SM on 8/9 of the SMs for a
-    // large graph, on fewer for a small one (blocks_beside_grid), whose iteration is the pipeline's chain.  What follows is
-    // the large graph.  Timestamps taken inside the kernels at N = 10^6 (one GPU), before the transforms had 784 points and
-    // the update interpolated: the attractive kernel runs 190 us and ends 37 us before the
-    // update can start; the pipeline, 90 us when it has the GPU to itself, takes 229 us on the SMs that are left and
-    // is what the update waits for.  More SMs for the pipeline slow the attractive kernel by as much as they speed
-    // the pipeline up (124, 132 and 140 attractive blocks: 3 940, 3 955, 3 905 iterations/s): the iteration is bound
-    // by the SM time of its kernels, not by their overlap.  Neither a higher stream priority for the attractive
-    // kernel nor holding the pipeline back until its blocks are resident (they are within 8 us anyway) changed it.
-    // Inside the pipeline it is the spread that suffers: 118 us on the 16 spare SMs against 28 alone (scatter 37
-    // against 26; FFT and gather as when alone), 60 us when 32 SMs are spared, which costs the attractive kernel more.
+    // The attractive kernel and the grid pipeline run side by side and divide the SMs between them (blocks_beside_grid), so a
+    // large iteration is bound by the SM time of its kernels: at N = 10^6, settled, the update 32 us and the spread 20 on all
+    // SMs, then 170 us of the attractive kernel beside the rest of the pipeline.  A higher stream priority for the attractive
+    // kernel changed nothing.
     // An L2 evict-first policy on the attractive kernel's stream loads: +0.8 %, not kept.
     if (!stage_timers) {
         B200_CUDA(cudaEventRecord(ev_fork, stream));
@@ -452,7 +445,9 @@ int Session::one_iteration(int norm_mode, float stop_norm)
 
 int Session::attractive(cudaStream_t st)
 {
-    if (blocked.ready) return launch_attractive_blocked(blocked, Y2, Fattr, st, resident, /*beside_grid=*/!stage_timers);
+    // (an iteration that sorts once in a while leaves as many SMs as the others)
+    const BesideGrid beside = stage_timers ? BesideGrid::nothing : refresh_period(step) == 1 ? BesideGrid::sorting : BesideGrid::settled;
+    if (blocked.ready) return launch_attractive_blocked(blocked, Y2, Fattr, st, resident, beside);
     B200_TRY(launch_attractive(P, ids, Y2, N, K, row_lo, row_hi, Fattr, st));
     if (extra.count > 0) B200_TRY(launch_attractive_extra(extra.ptr, extra.ids, extra.val, Y2, N, row_lo, row_hi, Fattr, st));
     return 0;
