@@ -229,17 +229,20 @@ int launch_state_reset(IterState *state, cudaStream_t st);   // both slots, sums
 int launch_state_swap(IterState *state, cudaStream_t st);    // exchanges the two slots (a stop between iterations of other parity)
 int launch_minmax_init(const float2 *Y2, int64_t N, IterState *state, int slot, cudaStream_t st);
 constexpr long long kSpreadDirectMax = 8192;      // up to here points are spread one by one
-constexpr long long kSortMin = 32768;             // from here on the spread order is sorted (both: repulsive.cu)
+constexpr long long kSortMin = 32768;             // from here on the spread order is sorted (both: repulsive.cu),
+constexpr long long kSortEarlyMin = 3000;         // from here on while the embedding is being exaggerated,
+constexpr long long kSortEachFrom = 65536;        // from here on then in every iteration (session.cu)
 constexpr long long kSpreadSingleMax = 131072;   // up to here a lane takes one point of the order
-// order: local row indices sorted by box (null = natural order); see launch_order_refresh
+// order: local row indices sorted by box (null = natural order); see launch_order_count
 // hist (optional): the sort's counters, cleared on the way for the next sort
 int launch_spread(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order, int32_t *hist, const IterState *state,
                   int slot, InterpConsts ic, float4 *w, const FftWorkspace *spectrum, cudaStream_t st);
 // spectrum (optional): the same launch does what launch_kernel_spectrum does; possible where a lane takes one point
 inline bool spread_takes_spectrum(int64_t n) { return n > 0 && n <= kSpreadSingleMax; }
 int launch_order_identity(int32_t *order, int64_t n, cudaStream_t st);
-int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, int32_t *order, int32_t *previous, int32_t *keys,
-                         int32_t *hist, const IterState *state, int slot, cudaStream_t st);
+int launch_order_count(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order, int32_t *previous, int32_t *keys, int32_t *hist,
+                       const IterState *state, int slot, cudaStream_t st);
+int launch_order_scatter(int64_t n, int32_t *order, const int32_t *previous, const int32_t *keys, int32_t *hist, cudaStream_t st);
 // convolve.cu: the kernel's spectrum along its first axis (needs the slot's min/max only), the first pass over the charges and
 // the spectrum's second axis, and the rest; the last pass adds sum_i Z_i over all charges to state->zsum[slot] and clears w when asked to
 int launch_kernel_spectrum(const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);

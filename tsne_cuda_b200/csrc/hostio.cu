@@ -44,6 +44,8 @@ void set_destroy(StreamSet *s)
     if (s->ev_fork) cudaEventDestroy(s->ev_fork);
     if (s->ev_join) cudaEventDestroy(s->ev_join);
     if (s->ev_spectrum) cudaEventDestroy(s->ev_spectrum);
+    if (s->ev_spread) cudaEventDestroy(s->ev_spread);
+    if (s->ev_order) cudaEventDestroy(s->ev_order);
     if (s->ev_t0) cudaEventDestroy(s->ev_t0);
     if (s->ev_t1) cudaEventDestroy(s->ev_t1);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -62,6 +64,8 @@ int set_create(StreamSet *s)
     B200_CUDA(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming));
     B200_CUDA(cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming));
     B200_CUDA(cudaEventCreateWithFlags(&s->ev_spectrum, cudaEventDisableTiming));
+    B200_CUDA(cudaEventCreateWithFlags(&s->ev_spread, cudaEventDisableTiming));
+    B200_CUDA(cudaEventCreateWithFlags(&s->ev_order, cudaEventDisableTiming));
     B200_CUDA(cudaEventCreate(&s->ev_t0));
     B200_CUDA(cudaEventCreate(&s->ev_t1));
     B200_CUDA(cudaMallocHost((void **)&s->h_state, sizeof(IterState)));

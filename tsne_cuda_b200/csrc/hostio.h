@@ -22,7 +22,7 @@ struct StreamSet {
     int device = -1;
     unsigned long long context = 0;   // its handles are of this context
     cudaStream_t stream = nullptr, stream2 = nullptr, stream3 = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_spread = nullptr, ev_order = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     IterState *h_state = nullptr;   // pinned
     // Pinned memory that kernels read and write across the bus: the state of a small map in one piece (Session::small_state).
     // The size bounds what is held pinned; it is no crossover (21,845 points, the most that it holds: state in, one iteration,

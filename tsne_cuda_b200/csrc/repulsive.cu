@@ -457,10 +457,10 @@ int launch_order_identity(int32_t *order, int64_t n, cudaStream_t st)
     return 0;
 }
 
-// `order` sorted anew by the box of the points' current position; previous, keys: n ints of scratch each,
-// hist: kBoxes^2 counters, zero on entry (the spread that follows clears them again).
-int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, int32_t *order, int32_t *previous, int32_t *keys,
-                         int32_t *hist, const IterState *state, int slot, cudaStream_t st)
+// `order` sorted anew by the box of the points' current position, in two parts: the first only reads it.  previous, keys: n
+// ints of scratch each; hist: kBoxes^2 counters, zero on entry and used up afterwards (the spread clears them where it is told to).
+int launch_order_count(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_t *order, int32_t *previous, int32_t *keys, int32_t *hist,
+                       const IterState *state, int slot, cudaStream_t st)
 {
     const long long n = row_hi - row_lo;
     if (n <= 0) return 0;
@@ -469,6 +469,13 @@ int launch_order_refresh(const float2 *Y2, int64_t row_lo, int64_t row_hi, int32
     B200_CUDA(cudaGetLastError());
     order_scan_kernel<<<1, 1024, 0, st>>>(hist);
     B200_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int launch_order_scatter(int64_t n, int32_t *order, const int32_t *previous, const int32_t *keys, int32_t *hist, cudaStream_t st)
+{
+    if (n <= 0) return 0;
+    const long long n_thr = (n + kOrderPerThread - 1) / kOrderPerThread;
     order_scatter_kernel<<<nblk(n_thr, 256), 256, 0, st>>>(previous, keys, n, hist, order);
     B200_CUDA(cudaGetLastError());
     return 0;

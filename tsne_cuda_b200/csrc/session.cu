@@ -117,7 +117,7 @@ int Session::init(int64_t N_, int K_, int64_t lo, int64_t hi, int device_)
     // pipeline compete for the same load/store units rather than for block slots.)
     B200_TRY(stream_set_acquire(&host, device));
     stream = host->stream; stream2 = host->stream2; stream3 = host->stream3;
-    ev_fork = host->ev_fork; ev_join = host->ev_join; ev_spectrum = host->ev_spectrum; ev_t0 = host->ev_t0; ev_t1 = host->ev_t1;
+    ev_fork = host->ev_fork; ev_join = host->ev_join; ev_spectrum = host->ev_spectrum; ev_spread = host->ev_spread; ev_order = host->ev_order; ev_t0 = host->ev_t0; ev_t1 = host->ev_t1;
     h_state = host->h_state;
     arena.serve(stream);
     arena.serve(stream2);
@@ -136,8 +136,13 @@ int Session::init(int64_t N_, int K_, int64_t lo, int64_t hi, int device_)
     B200_TRY(launch_order_identity(order, rows(), stream));
     B200_CUDA(cudaMemsetAsync(box_hist, 0, sizeof(int32_t) * kBoxes * kBoxes, stream));
     if (rows() < kSortMin) order_refresh = 0;
-    if (const char *e = getenv("B200TSNE_ORDER_REFRESH")) order_refresh = atoi(e);
-    if (const char *e = getenv("B200TSNE_ORDER_REFRESH_EARLY")) order_refresh_early = std::max(1, atoi(e));
+    order_refresh_early = rows() >= kSortEachFrom ? 1 : rows() >= kSortMin ? 4 : rows() >= kSortEarlyMin ? 8 : 0;
+    if (const char *e = getenv("B200TSNE_ORDER_REFRESH")) {
+        order_refresh = std::max(0, atoi(e));
+        order_refresh_early = order_refresh == 0 ? 0 : std::max(1, order_refresh_early);
+    }
+    if (const char *e = getenv("B200TSNE_ORDER_REFRESH_EARLY")) order_refresh_early = order_refresh_early_sharded = std::max(1, atoi(e));
+    if (order_refresh == 0) order_refresh_early_sharded = 0;   // ranks sort in both phases or in neither
     if (const char *e = getenv("B200TSNE_GRAPHS")) use_graphs = atoi(e) != 0;
     B200_TRY(arena.alloc((void **)&Y2, sizeof(float2) * npad));
     B200_TRY(arena.alloc((void **)&Fattr, sizeof(float2) * npad));
@@ -184,7 +189,7 @@ void Session::destroy()
     arena.release();
     stream_set_release(host);
     host = nullptr;
-    h_state = nullptr; stream = stream2 = stream3 = nullptr; ev_fork = ev_join = ev_spectrum = ev_t0 = ev_t1 = nullptr;
+    h_state = nullptr; stream = stream2 = stream3 = nullptr; ev_fork = ev_join = ev_spectrum = ev_spread = ev_order = ev_t0 = ev_t1 = nullptr;
 }
 
 int Session::set_embedding_soa(const float *Y_host, bool reset)
@@ -324,7 +329,7 @@ struct StageClock {
 }  // namespace
 
 // norm_mode, stop_norm: see launch_update
-int Session::one_iteration(int norm_mode, float stop_norm)
+int Session::one_iteration(int norm_mode, float stop_norm, bool sorts)
 {
     const int slot = step & 1;
     const bool late = step >= force_magnify_iters;
@@ -363,21 +368,45 @@ int Session::one_iteration(int norm_mode, float stop_norm)
         }
     }
 
-    // The embedding reshuffles quickly while it is being exaggerated and slowly afterwards: sort every
-    // order_refresh_early iterations early, every order_refresh iterations later.  (Sorting the rows for iteration t + 1
+    // The embedding reshuffles quickly while it is being exaggerated and slowly afterwards, and a large one pays more for boxes
+    // that are mixed up than for a sort: more than kSortEachFrom points are sorted in every iteration early, fewer every
+    // fourth or eighth, and every eighth later (below kSortMin points not at all).  An iteration while exaggerated, from a
+    // blob / from a blob with a learning rate of n / 12 / from a layout:
+    //     points      natural order        every 8th            every 4th            every one (on the chain)
+    //     3,000       26.4 / 26.8 / 27.4   26.2 / 26.2 / 26.1
+    //     5,000       29.0 / 28.5 / 30.0   26.9 / 26.6 / 26.7
+    //     20,011      39.6 / 40.0 / 43.0   30.2 / 32.1 / 29.2   30.3 / 32.3 / 29.3
+    //     60,000      38.8 / 38.8 / 33.8   37.2 / 40.5 / 35.1   36.6 / 39.8 / 34.4   44.4 / 44.6 / 44.2
+    //     90,000                                                48.9 / 57.2 / 41.3   47.7 / 48.9 / 48.7
+    //     130,000                                               59.4 / 73.3 / 50.6   53.3 / 56.0 / 55.7
+    //     200,000     102 / 93 / 67        73.7 / 92.7 / 63.2   71.9 / 93.0 / 62.8   63.3 / 63.5 / 63.6
+    // (Sorting the rows for iteration t + 1
     // at the end of iteration t, while waiting for the other ranks, was measured on two GPUs: the next bounding box is only
     // known after that meeting, and boxes taken from the previous one - the embedding grows by more than a box
     // width per exaggerated iteration - break the runs of equal boxes: spread 61 us instead of 15.)
     const int refresh = refresh_period(step);
-    if (refresh > 0 && step % refresh == 0) {
+    // An order that is to serve several iterations may as well be one older: its sort is then off the chain, beside it.
+    const bool sorts_beside = sorts && refresh > 1 && !multi && !stage_timers;
+    if (sorts && !sorts_beside) {
         clk.begin(stream);
-        B200_TRY(launch_order_refresh(Y2, row_lo, row_hi, order, order_alt, order_keys, box_hist, state, slot, stream));
+        B200_TRY(launch_order_count(Y2, row_lo, row_hi, order, order_alt, order_keys, box_hist, state, slot, stream));
+        B200_TRY(launch_order_scatter(rows(), order, order_alt, order_keys, box_hist, stream));
         clk.end(stream, kStOrder, 3);
     }
     clk.begin(stream);
-    B200_TRY(launch_spread(Y2, row_lo, row_hi, refresh > 0 ? order : nullptr, refresh > 0 ? box_hist : nullptr, state, slot, ic, w,
+    B200_TRY(launch_spread(Y2, row_lo, row_hi, refresh > 0 ? order : nullptr, sorts && !sorts_beside ? box_hist : nullptr, state, slot, ic, w,
                            spectrum_in_spread ? &fft : nullptr, stream));
     clk.end(stream, kStSpread, 1);
+    if (sorts_beside) {
+        B200_CUDA(cudaEventRecord(ev_spread, stream));
+        B200_CUDA(cudaStreamWaitEvent(stream3, ev_fork, 0));
+        B200_TRY(launch_order_count(Y2, row_lo, row_hi, order, order_alt, order_keys, box_hist, state, slot, stream3));
+        B200_CUDA(cudaStreamWaitEvent(stream3, ev_spread, 0));   // it reads the order
+        B200_TRY(launch_order_scatter(rows(), order, order_alt, order_keys, box_hist, stream3));
+        B200_CUDA(cudaMemsetAsync(box_hist, 0, sizeof(int32_t) * kBoxes * kBoxes, stream3));
+        B200_CUDA(cudaEventRecord(ev_order, stream3));
+        launches += 3;
+    }
     if (p2p) {
         clk.begin(stream);
         if (grid_two_shot) {
@@ -412,6 +441,7 @@ int Session::one_iteration(int norm_mode, float stop_norm)
         clk.end(stream, kStAttractive, attractive_launches());
     } else {
         B200_CUDA(cudaStreamWaitEvent(stream, ev_join, 0));
+        if (sorts_beside) B200_CUDA(cudaStreamWaitEvent(stream, ev_order, 0));
     }
     clk.begin(stream);
     UpdateTargets dst;
@@ -493,10 +523,19 @@ void Session::drop_graphs()
     graphs.clear();
 }
 
+bool Session::sorts_at(int b, int block) const
+{
+    const int period = refresh_period(step);   // (a block is of one phase)
+    if (period <= 1) return period == 1;
+    if (block >= kGraphIters) return b % period == 0;
+    return b == 0 && since_sort >= (block > 1 ? 2 * period : period);
+}
+
 int Session::refresh_period(int at) const
 {
-    if (order_refresh <= 0) return 0;
-    return at < force_magnify_iters + 50 ? order_refresh_early : order_refresh;
+    const bool early = at < force_magnify_iters + 50;
+    if (!early) return order_refresh;
+    return comm && comm->world > 1 ? order_refresh_early_sharded : order_refresh_early;
 }
 
 // How many of the next iterations one graph covers; 0 when the next one has to be launched directly.  A graph holds
@@ -545,11 +584,11 @@ int Session::run_graph_block(int &iters, int remaining, int norm_mode, float sto
     key.momentum = late ? post_momentum : pre_momentum;
     key.norm_mode = norm_mode;
     key.stop_norm = stop_norm;
-    for (int b = 0; b < iters; b++) {   // which of the iterations sort
-        const int r = refresh_period(step + b);
-        if (r > 0 && (step + b) % r == 0) key.sorts |= 1u << b;
-    }
-    key.natural = refresh_period(step) == 0;
+    int last_sort = -1;
+    for (int b = 0; b < iters; b++)
+        if (sorts_at(b, iters)) { key.sorts |= 1u << b; last_sort = b; }
+    const int period = refresh_period(step);
+    key.nodes = (period == 0 ? kNatural : period == 1 ? kSortsEach : 0) | (spread_takes_spectrum(rows()) ? kSpectrumInSpread : 0);
     IterGraph *g = nullptr;
     for (IterGraph &have : graphs)
         if (have.same(key)) g = &have;
@@ -568,7 +607,7 @@ int Session::run_graph_block(int &iters, int remaining, int norm_mode, float sto
         cudaGraph_t graph = nullptr;
         B200_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         int rc = 0;
-        for (int b = 0; b < iters && rc == 0; b++) rc = one_iteration(norm_mode, stop_norm);
+        for (int b = 0; b < iters && rc == 0; b++) rc = one_iteration(norm_mode, stop_norm, key.sorts >> b & 1);
         const cudaError_t end = cudaStreamEndCapture(stream, &graph);
         key.launches = launches - launches0;
         step = step0;
@@ -587,6 +626,7 @@ int Session::run_graph_block(int &iters, int remaining, int norm_mode, float sto
     }
     B200_CUDA(cudaGraphLaunch(g->exec, stream));
     step += iters;
+    since_sort = last_sort < 0 ? since_sort + iters : iters - last_sort;
     launches += g->launches;
     return 0;
 }
@@ -617,7 +657,9 @@ int Session::iterate(int n_iters, float min_gradient_norm, float *elapsed_ms, in
             if (rc != 0) block = 0;
         }
         if (block == 0) {
-            B200_TRY(one_iteration(norm_mode, min_gradient_norm));
+            const bool sorts = sorts_at(0, 1);
+            since_sort = sorts ? 1 : since_sort + 1;
+            B200_TRY(one_iteration(norm_mode, min_gradient_norm, sorts));
             block = 1;
         }
         it += block;

@@ -34,7 +34,7 @@ struct Session {
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;  // attractive force overlaps the grid pipeline
     cudaStream_t stream3 = nullptr;  // and so does the kernel's spectrum
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_spectrum = nullptr, ev_spread = nullptr, ev_order = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     DeviceArena arena;
 
     // affinities (owned rows)
@@ -66,8 +66,9 @@ struct Session {
     float2 *u = nullptr;      // [rows]
     float *soa_tmp = nullptr; // [2N] staging for SoA <-> AoS conversion
     int32_t *order = nullptr, *order_alt = nullptr, *order_keys = nullptr, *box_hist = nullptr;  // spread order (owned rows)
-    int order_refresh_early = 1;  // the same while the embedding is still being exaggerated (and 50 iterations after)
-    int order_refresh = 8;    // iterations between two counting sorts of the spread order once the embedding has settled (0 = natural order)
+    // iterations between two counting sorts of the spread order once the embedding has settled, and while it is still being
+    // exaggerated and 50 iterations after, on one GPU and on one of several (0 = natural order)
+    int order_refresh = 8, order_refresh_early = 1, order_refresh_early_sharded = 1;
     // grid
     float4 *w = nullptr;      // [G][G]
     float4 *ytilde = nullptr; // [G][G]
@@ -107,16 +108,17 @@ struct Session {
     struct IterGraph {
         cudaGraphExec_t exec = nullptr;
         int iters = 0, parity = 0, norm_mode = 0;
-        bool late = false, natural = false;
+        bool late = false;
+        int nodes = 0;             // which kernels an iteration has beside the sorts' (kNatural, ...)
         unsigned sorts = 0;        // bit b: the b-th iteration sorts the spread order
         float eta = 0, exaggeration = 0, momentum = 0, stop_norm = 0;
         int64_t launches = 0;
         int asked = 0;             // of one without an executable: how many calls asked for it
         // what decides which nodes it has: an executable of the same shape can be updated instead of made anew
-        unsigned long long shape() const { return (unsigned long long)sorts << 32 | (unsigned)iters << 2 | (unsigned)natural << 1; }
+        unsigned long long shape() const { return (unsigned long long)sorts << 32 | (unsigned)iters << 4 | (unsigned)nodes; }
         bool same(const IterGraph &o) const
         {
-            return iters == o.iters && parity == o.parity && norm_mode == o.norm_mode && late == o.late && natural == o.natural &&
+            return iters == o.iters && parity == o.parity && norm_mode == o.norm_mode && late == o.late && nodes == o.nodes &&
                    sorts == o.sorts && eta == o.eta && exaggeration == o.exaggeration && momentum == o.momentum && stop_norm == o.stop_norm;
         }
     };
@@ -128,7 +130,12 @@ struct Session {
     static constexpr size_t kMaxGraphs = 24;
     std::vector<IterGraph> graphs, missed;   // with an executable; asked for lately, without one
     bool use_graphs = true;   // B200TSNE_GRAPHS=0 turns them off
+    static constexpr int kNatural = 1, kSortsEach = 2, kSpectrumInSpread = 4;
     int refresh_period(int at) const;   // iterations between two sorts of the spread order at step `at` (0: natural order)
+    // Does the b-th of `block` iterations launched together sort?  Large blocks sort at fixed places, so that one executable
+    // serves a phase; pairs, of which one that sorts is another executable, half as often; since_sort: iterations since the last.
+    bool sorts_at(int b, int block) const;
+    int since_sort = 1 << 20;
     int graph_block(int remaining) const;
     bool worth_capturing(const IterGraph &key, int remaining);
     int run_graph_block(int &iters, int remaining, int norm_mode, float stop_norm);
@@ -151,7 +158,7 @@ struct Session {
     int set_small_state(const float *Y_host, const float *momentum_host, const float *gains_host, int at_step);
     int get_small_state(float *Y_host, float *momentum_host, float *gains_host);
     int iterate(int n_iters, float min_gradient_norm, float *elapsed_ms, int *iters_done);
-    int one_iteration(int norm_mode, float stop_norm);
+    int one_iteration(int norm_mode, float stop_norm, bool sorts);
     int attractive(cudaStream_t st);   // Fattr of the owned rows from the current embedding
     int attractive_launches() const { return blocked.ready ? (resident ? 2 : 3) + (blocked.extra_C > 0) : 1 + (extra.count > 0); }
     int affinities_from_points(const float *X_host, int D, float perplexity, float eps);
