@@ -13,6 +13,7 @@
 
 #include "../../include/tsnecuda/fit_tsne.h"
 #include "../../include/tsnecuda_b200.h"
+#include "hostio.h"
 #include "session.h"
 
 namespace tsnecuda {
@@ -121,6 +122,7 @@ int run(Options &opt, GpuOptions &gpu_opt)
     std::thread y0_thread([&]() {
         y0_rc = initial_embedding(opt, y0);
         if (y0_rc != 0) y0_error = b200::last_error();
+        if (opt.return_style == RETURN_STYLE::ONCE) b200::populate_pages(opt.return_data, sizeof(float) * 2 * (size_t)N);
     });
     // kNN, max-normalisation, perplexity search and symmetrisation run back to back on the device;
     // the split between the two printed phases is only meaningful with stage timers on.

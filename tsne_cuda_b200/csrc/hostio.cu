@@ -3,6 +3,8 @@
 
 #include <cuda.h>
 #include <string.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -185,6 +187,19 @@ template <class F> cudaError_t on_lanes(int lanes, int device, F body)
 }
 
 }  // namespace
+
+void populate_pages(void *p, size_t bytes)
+{
+#ifdef MADV_POPULATE_WRITE
+    if (!p || bytes < kPopulateMin || !pageable(p)) return;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), lo = ((uintptr_t)p + page - 1) / page * page, hi = ((uintptr_t)p + bytes) / page * page;
+    // a failure (an old kernel, a mapping of another kind) leaves the faults to the copy
+    if (lo < hi) (void)madvise(reinterpret_cast<void *>(lo), hi - lo, MADV_POPULATE_WRITE);
+#else
+    (void)p;
+    (void)bytes;
+#endif
+}
 
 bool plain_host(const void *p)
 {

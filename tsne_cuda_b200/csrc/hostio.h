@@ -55,6 +55,12 @@ void graph_exec_release(StreamSet *s, cudaGraphExec_t exec, unsigned long long s
 int copy_in(void *dst_device, const void *src_host, size_t bytes, cudaStream_t st);
 int copy_out(void *dst_host, const void *src_device, size_t bytes, cudaStream_t st);
 
+// Gives a pageable buffer its pages ahead of a copy_out, while the device is busy with what will be copied: in fresh memory
+// the faults are a good part of the copy (100,003 x 96, K = 32, lists in fresh arrays: whole call 10.0 -> 9.0 ms).  The contents stay as they are; any
+// thread may call it; other kinds of memory and small buffers are left alone.
+constexpr size_t kPopulateMin = (size_t)2 << 20;
+void populate_pages(void *p, size_t bytes);
+
 bool plain_host(const void *p);   // host memory, pinned or not: neither device nor managed memory, which a copy takes as well
 
 void host_pools_release(int device);   // idle sets and staging memory of one device
