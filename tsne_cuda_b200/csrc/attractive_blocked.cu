@@ -899,7 +899,11 @@ static int device_sms(int *sms)
 static int blocks_beside_grid(int sms, long long chunks, bool sorts)
 {
     const long long pipeline = sorts ? 96000 : 35500;   // chunks that take as long
-    return (int)std::max(6ll, std::min<long long>(sms - 6, sms * chunks / (chunks + pipeline)));
+    const long long blocks = std::max(6ll, std::min<long long>(sms - 6, sms * chunks / (chunks + pipeline)));
+    // The longest kernel of the pipeline, the columns pass, has 393 blocks, four to an SM: a graph that is done in time on what
+    // leaves it 101 SMs (one wave) has no more (30,011 points on 47 | 55 blocks 27.7 | 29.7).
+    const long long spare = std::max(6, sms - 101);
+    return (int)(chunks <= 544 * spare ? std::min(blocks, spare) : blocks);
 }
 
 // Builds the blocked copy of the owned rows' fixed-width P and, with `extra`, a second stream from a variable-width
@@ -1001,6 +1005,14 @@ int blocked_attractive_build(BlockedAttractive *b, DeviceArena &arena, const flo
     return 0;
 }
 
+int free_beside_attractive(const BlockedAttractive &b, BesideGrid beside, int *free_sms)
+{
+    int sms = 0;
+    B200_TRY(device_sms(&sms));
+    *free_sms = !b.ready ? 0 : beside == BesideGrid::nothing ? sms : sms - blocks_beside_grid(sms, (long long)b.C + b.extra_C, beside == BesideGrid::sorting);
+    return 0;
+}
+
 // F2[row_lo + r] = attractive force of the owned rows on the embedding Y2 (three launches)
 // (Reading the force in cell order from the update kernel and letting it keep the cell-ordered embedding current
 // instead of these two conversion kernels was measured on one GPU: the update kernel's three scattered 8-byte
@@ -1020,9 +1032,9 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
     BlockedStream s;
     s.ev = b.ev; s.ec = b.ec; s.chunk_row0 = b.chunk_row0; s.tile_chunk0 = b.tile_chunk0;
     s.ntiles = b.ntiles; s.T = b.T; s.C = b.C;
-    int sms = 0;
-    B200_TRY(device_sms(&sms));
-    const int all_sms = sms;
+    int sms = 0, all_sms = 0;
+    B200_TRY(device_sms(&all_sms));
+    sms = all_sms;
     // A block fills its SM (1,024 threads, all registers, 224 KB of shared memory), so the grid pipeline that runs
     // beside this kernel on the other stream only gets the SMs this kernel leaves alone.  Measured at N = 10^6,
     // K = 90 on 148 SMs, one GPU: 148 blocks 3,645 iterations/s (attractive stage 175 us), 140: 3,906, 132: 3,962

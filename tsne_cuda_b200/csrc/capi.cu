@@ -349,7 +349,7 @@ int b200tsne_repulsive(const float *Y, int64_t N, float *Frep, float *Z, float *
     if (w_out) B200_TRY(down(w_out, reinterpret_cast<float *>(dw), (size_t)kG * kG * 4, sg.st));
     B200_TRY(launch_kernel_spectrum(st, 0, ws, sg.st));
     B200_TRY(launch_convolve_rows(dw, st, 0, ws, sg.st));
-    B200_TRY(launch_convolve(dw, dyt, st, 0, ws, false, sg.st));
+    B200_TRY(launch_convolve(dw, dyt, st, 0, ws, false, 0, sg.st));
     B200_TRY(launch_gather(dY2, 0, N, st, 0, ic, dyt, dF2, sg.st));
     B200_TRY(launch_aos_to_soa(dF2, dF, N, sg.st));
     B200_TRY(down(Frep, dF, (size_t)2 * N, sg.st));

@@ -215,6 +215,7 @@ int launch_exclusive_scan_i32(int *data, int64_t n, cudaStream_t st);   // in pl
 enum class BesideGrid { nothing, sorting, settled };
 int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, float2 *F2, cudaStream_t st, bool in_cell_order = false,
                               BesideGrid beside = BesideGrid::nothing);
+int free_beside_attractive(const BlockedAttractive &b, BesideGrid beside, int *sms);   // SMs that it leaves alone then
 
 // repulsive.cu
 struct FftWorkspace {
@@ -247,7 +248,8 @@ int launch_order_scatter(int64_t n, int32_t *order, const int32_t *previous, con
 // the spectrum's second axis, and the rest; the last pass adds sum_i Z_i over all charges to state->zsum[slot] and clears w when asked to
 int launch_kernel_spectrum(const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
 int launch_convolve_rows(const float4 *w, const IterState *state, int slot, const FftWorkspace &ws, cudaStream_t st);
-int launch_convolve(float4 *w, float4 *ytilde, IterState *state, int slot, const FftWorkspace &ws, bool zero_w, cudaStream_t st);
+// free_sms: SMs that no other kernel fills meanwhile, as far as known
+int launch_convolve(float4 *w, float4 *ytilde, IterState *state, int slot, const FftWorkspace &ws, bool zero_w, int free_sms, cudaStream_t st);
 int launch_gather(const float2 *Y2, int64_t row_lo, int64_t row_hi, const IterState *state, int slot, InterpConsts ic,
                   const float4 *ytilde, float2 *Frep2, cudaStream_t st);
 

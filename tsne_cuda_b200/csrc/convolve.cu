@@ -164,6 +164,11 @@ fft_rows_forward_kernel(const float4 *w, float4 *A, const float *Rk, float *Kh, 
 
 // ---- second pass: column c, its mirror image, both planes: forward, product with the spectrum, inverse ----
 constexpr size_t kColsSmem = sizeof(float2) * (kM + 4 * kEx + kLines * kLine) + sizeof(float) * kM;
+// What a block asks for where three to an SM are all there: the blocks come while the rows end, and the SMs that are free by
+// then would take four (1,500 / 5,000 points 24.0 -> 22.9 / 24.4 -> 23.5 us an iteration; with fewer SMs, of which some
+// have to take four, 20,011 points 27.2 -> 29.7).
+constexpr size_t kColsSmemThree = 72 * 1024;
+static_assert(kColsSmem <= kColsSmemThree && 4 * kColsSmemThree > 227 * 1024 && 3 * (kColsSmemThree + 1024) <= 227 * 1024, "three blocks to an SM");
 __global__ void __launch_bounds__(128)
 fft_columns_kernel(const float4 *A, const float *Kh, float4 *B, const float2 *__restrict__ tw)
 {
@@ -289,7 +294,7 @@ int fft_workspace_init(FftWorkspace *ws, void *mem, cudaStream_t st)
     ws->Rk = reinterpret_cast<float *>(p);
     B200_CUDA(cudaFuncSetAttribute(fft_rows_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem));
     B200_CUDA(cudaFuncSetAttribute(fft_rows_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBackSmem));
-    static_assert(kColsSmem <= 48 * 1024, "columns pass: no more than a kernel may have unasked");
+    B200_CUDA(cudaFuncSetAttribute(fft_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColsSmemThree));
     twiddle_init_kernel<<<(kM + 255) / 256, 256, 0, st>>>(ws->tw);
     B200_CUDA(cudaGetLastError());
     return 0;
@@ -308,9 +313,9 @@ int launch_convolve_rows(const float4 *w, const IterState *state, int slot, cons
     return 0;
 }
 
-int launch_convolve(float4 *w, float4 *ytilde, IterState *state, int slot, const FftWorkspace &ws, bool zero_w, cudaStream_t st)
+int launch_convolve(float4 *w, float4 *ytilde, IterState *state, int slot, const FftWorkspace &ws, bool zero_w, int free_sms, cudaStream_t st)
 {
-    B200_CUDA(launch_chained(fft_columns_kernel, kC, 128, kColsSmem, st, ws.A, ws.Kh, ws.B, ws.tw));
+    B200_CUDA(launch_chained(fft_columns_kernel, kC, 128, 3 * free_sms >= kC ? kColsSmemThree : kColsSmem, st, ws.A, ws.Kh, ws.B, ws.tw));
     B200_CUDA(launch_chained(fft_rows_inverse_kernel, kLines, kRowThreads, kBackSmem, st, ws.B, w, ytilde, state, slot, ws.tw, zero_w ? 1 : 0));
     return 0;
 }

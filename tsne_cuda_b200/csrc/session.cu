@@ -427,7 +427,9 @@ int Session::one_iteration(int norm_mode, float stop_norm, bool sorts)
     if (stage_timers) B200_TRY(launch_kernel_spectrum(state, slot, fft, stream));
     else if (!spectrum_in_spread) B200_CUDA(cudaStreamWaitEvent(stream, ev_spectrum, 0));
     B200_TRY(launch_convolve_rows(charges, state, slot, fft, stream));
-    B200_TRY(launch_convolve(charges, ytilde, state, slot, fft, !p2p, stream));   // sums Z over ALL points on the grid: no exchange
+    int free_sms = 0;
+    if (!multi) B200_TRY(free_beside_attractive(blocked, beside_attractive(), &free_sms));
+    B200_TRY(launch_convolve(charges, ytilde, state, slot, fft, !p2p, free_sms, stream));   // sums Z over ALL points on the grid: no exchange
     clk.end(stream, kStConvolve, stage_timers ? 4 : 3);
     const bool fused = !multi && !stage_timers;   // the update interpolates the repulsive force itself
     if (!fused) {
@@ -473,11 +475,15 @@ int Session::one_iteration(int norm_mode, float stop_norm, bool sorts)
     return 0;
 }
 
-int Session::attractive(cudaStream_t st)
+BesideGrid Session::beside_attractive() const
 {
     // (an iteration that sorts once in a while leaves as many SMs as the others)
-    const BesideGrid beside = stage_timers ? BesideGrid::nothing : refresh_period(step) == 1 ? BesideGrid::sorting : BesideGrid::settled;
-    if (blocked.ready) return launch_attractive_blocked(blocked, Y2, Fattr, st, resident, beside);
+    return stage_timers ? BesideGrid::nothing : refresh_period(step) == 1 ? BesideGrid::sorting : BesideGrid::settled;
+}
+
+int Session::attractive(cudaStream_t st)
+{
+    if (blocked.ready) return launch_attractive_blocked(blocked, Y2, Fattr, st, resident, beside_attractive());
     B200_TRY(launch_attractive(P, ids, Y2, N, K, row_lo, row_hi, Fattr, st));
     if (extra.count > 0) B200_TRY(launch_attractive_extra(extra.ptr, extra.ids, extra.val, Y2, N, row_lo, row_hi, Fattr, st));
     return 0;

@@ -159,6 +159,7 @@ struct Session {
     int get_small_state(float *Y_host, float *momentum_host, float *gains_host);
     int iterate(int n_iters, float min_gradient_norm, float *elapsed_ms, int *iters_done);
     int one_iteration(int norm_mode, float stop_norm, bool sorts);
+    BesideGrid beside_attractive() const;   // what runs beside the attractive kernel at this step
     int attractive(cudaStream_t st);   // Fattr of the owned rows from the current embedding
     int attractive_launches() const { return blocked.ready ? (resident ? 2 : 3) + (blocked.extra_C > 0) : 1 + (extra.count > 0); }
     int affinities_from_points(const float *X_host, int D, float perplexity, float eps);
