@@ -26,7 +26,8 @@
 // Bound: three kernels whose blocks each run once: the loads at their start, an exchange and the stores at their end take as
 // long as the transforms, and in those the fp32 pipe is three quarters busy (columns pass: 4,900 cycles of packed and scalar
 // arithmetic per scheduler in 6,500).  Measured on B200 inside an iteration of 5,000 points, from the end of the kernel before:
-// rows 3.5, columns 5.3, rows back 4.9 us, and 0.6 to 0.9 us between two of them.  What that came from, per iteration at
+// rows 3.5, columns 5.3, rows back 4.9 us, and 0.6 to 0.9 us between two of them (before the last
+// two steps below).  What that came from, per iteration at
 // 1,500 / 5,000 / 20,011 points:
 //   a row per block in the row passes (the column pass read and wrote 32 bytes of a line: every access of a warp touched 28
 //   different lines), scalar arithmetic, the spectrum in two kernels on a third stream                   31.1 / 32.1 / 34.4 us
@@ -34,6 +35,10 @@
 //   the spectrum's second axis beside the rows (it was what the column pass waited for, 1.5 us)          27.7 / 27.9 / 31.3
 //   copies in the order of their use; point kernels of small blocks (repulsive.cu, update.cu)            27.5 / 28.1 / 31.4
 //   chained launches, the spectrum's first axis beside the spread, loads before arithmetic in update.cu  24.0 / 24.1 / 26.9
+//   three blocks of the column pass to an SM where that places all of them                               23.0 / 23.4 / 27.1
+//   a lane's twiddles in registers, loaded before the kernel in front has ended                          21.7 / 22.2 / 26.1
+// A warp's transforms are 750 instructions in 2,800 cycles whether two or three of them share a scheduler, so blocks of three
+// rows on 130 SMs instead of four on 98 gained nothing (22.9 -> 23.3: the columns then meet bank conflicts).
 // Chained launches gain nothing where the next kernel may start too early: blocks of the column pass that are placed while
 // rows still run share the SMs unevenly (27.8 -> 29.0 with the permission at the start of each kernel, 26.7 at its end, 26.4
 // before its last stores).
@@ -64,7 +69,7 @@ __device__ __forceinline__ int slot_of(int k) { return k < kC ? 0 : 1; }
 __global__ void __launch_bounds__(kSpecWarps * 32)
 spectrum_rows_kernel(float *Rk, const IterState *state, int slot, const float2 *__restrict__ tw)
 {
-    spectrum_rows(Rk, state, slot, tw, blockIdx.x);
+    spectrum_rows<false>(Rk, state, slot, tw, blockIdx.x);
 }
 
 // ---- workspace between the passes ----
@@ -79,7 +84,7 @@ constexpr int kStageLine = kLine + 2;   // float2 per line in shared memory of t
 
 constexpr int kRowThreads = 2 * kRowsBlock * 32;   // a warp per row and plane
 constexpr size_t kStageBytes = sizeof(float2) * kC * kStageLine, kRowExBytes = sizeof(float2) * 2 * kRowsBlock * kEx;
-constexpr size_t kRowsSmem = sizeof(float2) * kM + (kStageBytes > kRowExBytes ? kStageBytes : kRowExBytes);
+constexpr size_t kRowsSmem = kStageBytes > kRowExBytes ? kStageBytes : kRowExBytes;
 constexpr size_t kBackSmem = kRowsSmem + sizeof(float4) * kRowsBlock * kG;
 
 // ---- spectrum, second axis: sixteen columns per block, two real ones per warp; Kh[c][k] ----
@@ -89,11 +94,11 @@ static_assert(kRkStride % kSpecCols == 0 && kSpecBlocks * kSpecCols >= kC, "colu
 static_assert(sizeof(float) * kG * kSpecRow <= kStageBytes, "the columns fit where the lines are staged");
 __device__ __forceinline__ void spectrum_columns(float2 *smem, const float *Rk, float *Kh, const float2 *__restrict__ tw, int block)
 {
-    float2 *tws = smem, *ex = smem + kM + (threadIdx.x >> 5) * kEx;
-    float *cols = reinterpret_cast<float *>(smem + kM);   // before the exchange
+    float2 *ex = smem + (threadIdx.x >> 5) * kEx;
+    float *cols = reinterpret_cast<float *>(smem);   // before the exchange
     const int lane = threadIdx.x & 31, own = 2 * (threadIdx.x >> 5), c = kSpecCols * block + own;
-    copy_twiddles<kRowThreads>(tws, tw);
-    end_batch();
+    Twiddles t;
+    load_twiddles(t, tw, lane);
     after_previous();
     for (int u = threadIdx.x; u < kG * kSpecCols / 4; u += kRowThreads) {
         const int row = u / (kSpecCols / 4), part = u % (kSpecCols / 4);
@@ -108,7 +113,7 @@ __device__ __forceinline__ void spectrum_columns(float2 *smem, const float *Rk, 
         v[r] = (lane < kR && row < kG) ? *reinterpret_cast<const float2 *>(cols + row * kSpecRow + own) : make_float2(0.0f, 0.0f);
     }
     mirror_input(v, lane);
-    fft784_warp<false, kR>(v, ex, tws, lane, [] { __syncthreads(); });   // the columns have been read
+    fft784_warp<false, kR>(v, ex, t, lane, [] { __syncthreads(); });   // the columns have been read
     let_next_start();
     if (c >= kC || lane >= kR) return;
 #pragma unroll
@@ -129,10 +134,10 @@ fft_rows_forward_kernel(const float4 *w, float4 *A, const float *Rk, float *Kh, 
         spectrum_columns(smem, Rk, Kh, tw, blockIdx.x - kLines);
         return;
     }
-    float2 *tws = smem, *stage = smem + kM;   // the lines, once the exchange is over
+    float2 *stage = smem;   // the lines, once the exchange is over
     const int lane = threadIdx.x & 31, plane = (threadIdx.x >> 5) & 1, row = kRowsBlock * blockIdx.x + (threadIdx.x >> 6);
-    copy_twiddles<kRowThreads>(tws, tw);
-    end_batch();
+    Twiddles t;
+    load_twiddles(t, tw, lane);
     after_previous();
     const float2 *wrow = reinterpret_cast<const float2 *>(w + (size_t)row * kG) + plane;   // .xy or .zw of each node
     float2 v[kR];
@@ -144,7 +149,7 @@ fft_rows_forward_kernel(const float4 *w, float4 *A, const float *Rk, float *Kh, 
     const float imag_scale = plane == 1 ? load_geom(state, slot).r2_scale : 1.0f;
 #pragma unroll
     for (int r = 0; r < kHalf; r++) v[r].y *= imag_scale;
-    fft784_warp<false, kHalf>(v, stage + (threadIdx.x >> 5) * kEx, tws, lane, copies_done<0>);
+    fft784_warp<false, kHalf>(v, stage + (threadIdx.x >> 5) * kEx, t, lane, [] {});
     let_next_start();
     __syncthreads();
     if (lane < kR) {
@@ -163,7 +168,7 @@ fft_rows_forward_kernel(const float4 *w, float4 *A, const float *Rk, float *Kh, 
 }
 
 // ---- second pass: column c, its mirror image, both planes: forward, product with the spectrum, inverse ----
-constexpr size_t kColsSmem = sizeof(float2) * (kM + 4 * kEx + kLines * kLine) + sizeof(float) * kM;
+constexpr size_t kColsSmem = sizeof(float2) * (4 * kEx + kLines * kLine) + sizeof(float) * kM;
 // What a block asks for where three to an SM are all there: the blocks come while the rows end, and the SMs that are free by
 // then would take four (1,500 / 5,000 points 24.0 -> 22.9 / 24.4 -> 23.5 us an iteration; with fewer SMs, of which some
 // have to take four, 20,011 points 27.2 -> 29.7).
@@ -173,12 +178,12 @@ __global__ void __launch_bounds__(128)
 fft_columns_kernel(const float4 *A, const float *Kh, float4 *B, const float2 *__restrict__ tw)
 {
     extern __shared__ __align__(16) float2 smem[];
-    float2 *tws = smem, *ex = smem + kM + (threadIdx.x >> 5) * kEx, *lines = smem + kM + 4 * kEx;
+    float2 *ex = smem + (threadIdx.x >> 5) * kEx, *lines = smem + 4 * kEx;
     float *spec = reinterpret_cast<float *>(lines + kLines * kLine);
     const int lane = threadIdx.x & 31, q = threadIdx.x >> 5, c = blockIdx.x;
     constexpr int n4 = kLines * kLine / 2;
-    copy_twiddles<128>(tws, tw);
-    end_batch();
+    Twiddles t;
+    load_twiddles(t, tw, lane);
     after_previous();
     copy_floats<128>(reinterpret_cast<float *>(lines), reinterpret_cast<const float *>(A + (size_t)c * n4), n4);
     end_batch();
@@ -192,11 +197,11 @@ fft_columns_kernel(const float4 *A, const float *Kh, float4 *B, const float2 *__
     for (int r = 0; r < kHalf; r++) {
         v[r] = mine[r * (kR / kRowsBlock) * kLine + place_in_line(q, r * (kR / kRowsBlock) + sl / kRowsBlock, sl)];
     }
-    fft784_warp<false, kHalf>(v, ex, tws, lane, [] {});
+    fft784_warp<false, kHalf>(v, ex, t, lane, [] {});
     copies_done<0>();
 #pragma unroll
     for (int r = 0; r < kR; r++) v[r] = times(spec[kR * r + sl], v[r]);
-    fft784_warp<true, kR>(v, ex, tws, lane, [] {});
+    fft784_warp<true, kR>(v, ex, t, lane, [] {});
     let_next_start();
     if (lane < kR) {
 #pragma unroll
@@ -214,11 +219,11 @@ __global__ void __launch_bounds__(kRowThreads)
 fft_rows_inverse_kernel(const float4 *B, float4 *w, float4 *ytilde, IterState *state, int slot, const float2 *__restrict__ tw, int zero_w)
 {
     extern __shared__ __align__(16) float2 smem[];
-    float2 *tws = smem, *stage = smem + kM;   // the lines, before the exchange
+    float2 *stage = smem;   // the lines, before the exchange
     float4 *charges = reinterpret_cast<float4 *>(smem) + (kBackSmem - sizeof(float4) * kRowsBlock * kG) / sizeof(float4);
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, plane = wi & 1, row = kRowsBlock * blockIdx.x + (wi >> 1);
-    copy_twiddles<kRowThreads>(tws, tw);
-    end_batch();
+    Twiddles t;
+    load_twiddles(t, tw, lane);
     after_previous();
     for (int u = threadIdx.x; u < kC * kLine / 2; u += kRowThreads) {
         const int c = u / (kLine / 2), part = u % (kLine / 2);
@@ -238,7 +243,7 @@ fft_rows_inverse_kernel(const float4 *B, float4 *w, float4 *ytilde, IterState *s
         const int k = kR * r + min(lane, kR - 1);
         v[r] = stage[column_of(k) * kStageLine + place_in_line(2 * plane + slot_of(k), blockIdx.x, row)];
     }
-    fft784_warp<true, kR>(v, stage + wi * kEx, tws, lane, [] { __syncthreads(); });   // the lines have been read
+    fft784_warp<true, kR>(v, stage + wi * kEx, t, lane, [] { __syncthreads(); });   // the lines have been read
     let_next_start();
     copies_done<0>();
     if (zero_w)

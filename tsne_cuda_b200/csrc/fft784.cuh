@@ -112,9 +112,9 @@ template <bool INV, int NZ> __device__ __forceinline__ void fft28(float2 (&v)[kR
     }
 }
 
-// Everything a block needs besides the values of its own transforms goes to shared memory with asynchronous copies, all
-// in flight at once: a loop of loads and stores waits for L2 once per round (seven to thirteen rounds here), which cost
-// more than the transforms.
+// What a block needs besides the values of its own transforms goes to shared memory with asynchronous copies, all in flight at
+// once: a loop of loads and stores waits for L2 once per round (seven to thirteen rounds here), which cost more than the
+// transforms.
 __device__ __forceinline__ void copy16(void *dst, const void *src)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -130,24 +130,36 @@ template <int THREADS> __device__ __forceinline__ void copy_floats(float *dst, c
 {
     for (int k = threadIdx.x; k < n4; k += THREADS) copy16(dst + 4 * k, src + 4 * k);
 }
-template <int THREADS> __device__ __forceinline__ void copy_twiddles(float2 *tws, const float2 *__restrict__ tw)
+
+// A lane's twiddles, e^{-2 pi i k l / 784} at tw[k * 28 + l], in registers: they are asked for before the kernel in front has
+// ended, serve both transforms of a column, and a transform then waits for its exchange alone (out of shared memory, one
+// by one between the products, 1,500 / 5,000 / 20,011 points 23.0 / 23.4 / 27.1 us an iteration; so 21.7 / 22.2 / 26.1).
+using Twiddles = float2[kR];
+__device__ __forceinline__ void load_twiddles(Twiddles &t, const float2 *__restrict__ tw, int lane)
 {
-    copy_floats<THREADS>(reinterpret_cast<float *>(tws), reinterpret_cast<const float *>(tw), kM / 2);
+#pragma unroll
+    for (int k = 1; k < kR; k++)   // volatile: here and not where they are used
+        asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(t[k].x), "=f"(t[k].y) : "l"(tw + k * kR + min(lane, kR - 1)));
 }
 
+// The same, each read where it is used: for a kernel whose other blocks want the registers.
+struct LateTwiddles {
+    const float2 *tw;
+    __device__ __forceinline__ float2 operator[](int k) const { return __ldg(tw + k * kR); }
+};
+
 // 784-point transform by one warp.  In: lane l < 28 holds x[28 r + l] in v[r] (zero from r = NZ on).  Out: lane l holds
-// X[l + 28 r] in v[r], the same pattern.  ex: kEx float2 of this warp; tws[k * 28 + l] = e^{-2 pi i k l / 784}, there
-// when twiddles_ready() returns.
-template <bool INV, int NZ, class READY>
-__device__ __forceinline__ void fft784_warp(float2 (&v)[kR], float2 *ex, const float2 *tws, int lane, READY twiddles_ready)
+// X[l + 28 r] in v[r], the same pattern.  ex: kEx float2 of this warp, free when exchange_free() returns.
+template <bool INV, int NZ, class TWIDDLES, class READY>
+__device__ __forceinline__ void fft784_warp(float2 (&v)[kR], float2 *ex, const TWIDDLES &t, int lane, READY exchange_free)
 {
     fft28<INV, NZ>(v);
-    twiddles_ready();
+    exchange_free();
     if (lane < kR) {
         ex[lane] = v[0];
 #pragma unroll
         for (int k = 1; k < kR; k++) {
-            float2 w = tws[k * kR + lane];
+            float2 w = t[k];
             if (INV) w.y = -w.y;
             ex[k * kExStride + lane] = cmul(v[k], w);
         }
@@ -195,13 +207,13 @@ __device__ __forceinline__ void mirror_input(float2 (&v)[kR], int lane)
 
 // block: rows kSpecWarps block .. of the kernel, a block of kSpecWarps warps
 constexpr int kSpecWarps = 2, kSpecRowBlocks = (kG + kSpecWarps - 1) / kSpecWarps;
+template <bool LATE>
 __device__ __forceinline__ void spectrum_rows(float *Rk, const IterState *state, int slot, const float2 *__restrict__ tw, int block)
 {
-    __shared__ __align__(16) float2 tws[kM];
     __shared__ float2 exch[kSpecWarps][kEx];
-    copy_twiddles<kSpecWarps * 32>(tws, tw);
-    end_batch();
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    Twiddles t;
+    if (!LATE) load_twiddles(t, tw, lane);
     const int row = block * kSpecWarps + wi;
     after_previous();
     const GridGeom g = load_geom(state, slot);
@@ -215,7 +227,8 @@ __device__ __forceinline__ void spectrum_rows(float *Rk, const IterState *state,
         v[r] = make_float2(in ? value : 0.0f, 0.0f);
     }
     mirror_input(v, lane);
-    fft784_warp<false, kR>(v, exch[wi], tws, lane, copies_done<0>);
+    if constexpr (LATE) fft784_warp<false, kR>(v, exch[wi], LateTwiddles{tw + min(lane, kR - 1)}, lane, [] {});
+    else fft784_warp<false, kR>(v, exch[wi], t, lane, [] {});
     if (row >= kG || lane >= kR) return;
 #pragma unroll
     for (int r = 0; r <= kHalf; r++) {

@@ -140,18 +140,26 @@ struct SpectrumRows {
 constexpr int kSpreadSmallThreads = kSpecWarps * 32;
 
 // hist (optional): the sort's counters, cleared here for the next one
-template <int PER_LANE>
+// SPECTRUM: the first blocks have the spectrum's rows, with their twiddles in registers or read late.  The former leaves room
+// for half as many blocks of points on an SM: an iteration at 20,011 / 30,011 / 60,000 / 100,000 points, exaggerated,
+// 26.3 / 27.2 / 34.7 / 49.0 us, read late 26.8 / 27.7 / 34.2 / 47.9.
+enum class SpreadSpectrum { none, late, registers };
+template <int PER_LANE, SpreadSpectrum SPECTRUM>
 __global__ void __launch_bounds__(PER_LANE == 1 ? kSpreadSmallThreads : 256)
 spread_kernel(const float2 *Y2, long long row_lo, long long n_rows, const int32_t *order, const IterState *state, int slot, InterpConsts ic,
               float4 *w, int32_t *hist, SpectrumRows spec)
 {
-    if (PER_LANE == 1 && blockIdx.x < spec.blocks) {
-        spectrum_rows(spec.Rk, state, slot, spec.tw, blockIdx.x);
-        return;
+    int block = blockIdx.x, blocks = gridDim.x;
+    if constexpr (SPECTRUM != SpreadSpectrum::none) {
+        if (block < spec.blocks) {
+            spectrum_rows<SPECTRUM == SpreadSpectrum::late>(spec.Rk, state, slot, spec.tw, block);
+            return;
+        }
+        block -= spec.blocks;
+        blocks -= spec.blocks;
     }
-    const int block = PER_LANE == 1 ? blockIdx.x - spec.blocks : blockIdx.x;
     after_previous();
-    if (hist) clear_histogram(hist, block, PER_LANE == 1 ? gridDim.x - spec.blocks : gridDim.x);
+    if (hist) clear_histogram(hist, block, blocks);
     const long long t0 = ((long long)block * blockDim.x + threadIdx.x) * PER_LANE;
     const int lane = threadIdx.x & 31;
     const GridGeom g = load_geom(state, slot);
@@ -231,7 +239,7 @@ __global__ void __launch_bounds__(kSpreadSmallThreads)
 spread_direct_kernel(const float2 *Y2, long long row_lo, long long n_rows, const IterState *state, int slot, InterpConsts ic, float4 *w, SpectrumRows spec)
 {
     if (blockIdx.x < spec.blocks) {
-        spectrum_rows(spec.Rk, state, slot, spec.tw, blockIdx.x);
+        spectrum_rows<false>(spec.Rk, state, slot, spec.tw, blockIdx.x);
         return;
     }
     const long long t = (long long)(blockIdx.x - spec.blocks) * blockDim.x + threadIdx.x;
@@ -441,10 +449,13 @@ int launch_spread(const float2 *Y2, int64_t row_lo, int64_t row_hi, const int32_
     if (!order && n <= kSpreadDirectMax)
         B200_CUDA(launch_chained(spread_direct_kernel, spec.blocks + nblk(n, kSpreadSmallThreads), kSpreadSmallThreads, 0, st, Y2, row_lo, n, state, slot, ic, w, spec));
     else if (n <= kSpreadSingleMax)
-        B200_CUDA(launch_chained(spread_kernel<1>, spec.blocks + nblk(n, kSpreadSmallThreads), kSpreadSmallThreads, 0, st, Y2, row_lo, n, order, state, slot, ic, w,
-                                 hist, spec));
+        B200_CUDA(launch_chained(!spectrum       ? spread_kernel<1, SpreadSpectrum::none>
+                                 : n < kSortMin ? spread_kernel<1, SpreadSpectrum::registers>
+                                                : spread_kernel<1, SpreadSpectrum::late>,
+                                 spec.blocks + nblk(n, kSpreadSmallThreads), kSpreadSmallThreads, 0,
+                                 st, Y2, row_lo, n, order, state, slot, ic, w, hist, spec));
     else
-        B200_CUDA(launch_chained(spread_kernel<kSpreadPerLane>, nblk((n + kSpreadPerLane - 1) / kSpreadPerLane, 256), 256, 0, st, Y2, row_lo, n, order, state,
+        B200_CUDA(launch_chained(spread_kernel<kSpreadPerLane, SpreadSpectrum::none>, nblk((n + kSpreadPerLane - 1) / kSpreadPerLane, 256), 256, 0, st, Y2, row_lo, n, order, state,
                                  slot, ic, w, hist, spec));
     return 0;
 }
