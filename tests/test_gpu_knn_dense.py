@@ -227,3 +227,42 @@ def test_against_the_list_search_on_every_row(engine, monkeypatch, n, d, k, ties
     monkeypatch.setenv("B200TSNE_KNN", "simt")
     ids_l, d2_l = engine.knn(X, k)
     assert np.array_equal(ids, ids_l) and np.array_equal(d2, d2_l)
+
+
+@pytest.mark.parametrize("n,d,k", [(700, 33, 20), (4099, 64, 16), (9000, 20, 150)])
+def test_a_search_between_the_kernels_that_write_and_clear_its_points(engine, n, d, k):
+    """The rounds of a search overlap with each other, but not with what the caller has queued before and after it in the
+    stream: queued, and captured with its producer."""
+    import torch
+    stream = torch.cuda.Stream()
+    source, X = torch.empty(n, d, device="cuda"), torch.empty(n, d, device="cuda")
+    ids, d2 = torch.empty(n, k, dtype=torch.int32, device="cuda"), torch.empty(n, k, device="cuda")
+
+    def search():
+        engine.check(engine.lib.b200tsne_knn_noalloc(X.data_ptr(), n, d, k, ids.data_ptr(), d2.data_ptr(), stream.cuda_stream))
+
+    def expect(points):
+        want_i, want_d = _noalloc(engine, points, k)
+        assert torch.equal(ids, want_i) and torch.equal(d2, want_d)
+
+    for _ in range(3):
+        with torch.cuda.stream(stream):
+            source.normal_()
+            slow = torch.ones(3000, 3000, device="cuda") @ torch.ones(3000, 3000, device="cuda")   # the points come late
+            torch.mul(source, slow[0, 0] / 3000, out=X)
+            search()
+            points = X.clone()
+            X.zero_()
+        torch.cuda.synchronize()
+        expect(points)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        torch.mul(source, 2.0, out=X)
+        search()
+        X.zero_()
+    for _ in range(3):
+        source.normal_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        expect(2.0 * source)

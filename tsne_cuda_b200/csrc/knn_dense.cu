@@ -7,7 +7,7 @@
 // 148 SMs, and half of the time goes into insertions.  Here the distances are a plain tiled product over all SMs (three
 // rounded fp32 operations per pair and dimension, issued for two pairs at a time, the bound), and the selection ranks the few keys, held in registers, that
 // lie below a bound from the smallest keys of groups (short rows, long lists: bisection on the keys' bits).  Measured on B200 (lists / now):
-// 4,099 points of 64 dimensions, K = 16: 1.69 / 0.20 ms; 1,500 x 20, K = 32: 1.63 / 0.03 ms; five rows of 60,000 x 784:
+// 4,099 points of 64 dimensions, K = 16: 1.69 / 0.18 ms; 1,500 x 20, K = 32: 1.63 / 0.03 ms; five rows of 60,000 x 784:
 // 4.4 / 0.4 ms.
 #include <limits.h>
 
@@ -27,12 +27,6 @@ constexpr int kThreads = 256;
 // busy as with single instructions, but half as many are issued: 4,099 x 64, K = 16 211 -> 201 us,
 // 10,000 x 100, K = 40 1,943 -> 1,827 (whole searches).
 constexpr unsigned long long kMinusZero2 = 0x8000000080000000ull;
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
 __device__ __forceinline__ float2 unpack2(unsigned long long v)
 {
     float2 r;
@@ -49,13 +43,20 @@ __device__ __forceinline__ void add_square2(unsigned long long &acc, unsigned lo
 
 // dist[q * ld + p] = canonical distance (sequential over the dimensions, every operation rounded) of query q of the list
 // and database row db_lo + p.  QT queries and eight points a thread, 16 QT queries and 128 points a block.
+// Bound: the fp32 pipe, which the packed operations of a dimension take for 96 cycles a warp.  So the next chunk of dimensions
+// is on its way while one is worked on, and a query's value stands twice in shared memory, as the operation wants it.
+// Launched behind the selection of the round before, it runs beside it up to its stores (see chained launches in common.cuh).
+// Whole searches, K in brackets, before and with these: 4,099 x 64 (16) 201 -> 181 us, 6,145 x 20 (40) 267 -> 204, 9,000 x 20 (150)
+// 743 -> 586, 10,000 x 100 (40) 1,800 -> 1,734, 12,288 x 32 (48) 1,125 -> 947, 3,000 x 33 (8) 91 -> 77; three blocks to an SM, as
+// one wave of a round of 832 queries wants (122 registers and two blocks: 184 us at 4,099 x 64).
 template <int QT>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 3)
 dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long long nq, const int *__restrict__ q_index, long long db_lo,
-                      long long nd, float *__restrict__ dist, long long ld, unsigned long long minus_zero)
+                      long long nd, float *dist, long long ld, unsigned long long minus_zero)
 {
-    constexpr int kTileQ = 16 * QT, kQs = kTileQ + 4, kPs = kTileP + 4;
-    __shared__ __align__(16) float Qs[kDims][kQs], Ps[kDims][kPs];
+    constexpr int kTileQ = 16 * QT, kQs = kTileQ + 2, kPs = kTileP + 4, kWarps = kThreads / 32;
+    __shared__ __align__(16) float2 Qs[kDims][kQs];
+    __shared__ __align__(16) float Ps[kDims][kPs];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31, warp = tid >> 5;
     const long long p0 = (long long)blockIdx.x * kTileP, q0 = (long long)blockIdx.y * kTileQ;
     unsigned long long acc[QT][4];
@@ -63,43 +64,51 @@ dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long l
     for (int a = 0; a < QT; a++)
 #pragma unroll
         for (int b = 0; b < 4; b++) acc[a][b] = 0ull;
+    // a warp reads 32 dimensions of one row at a time (coalesced) and stores them as a column
+    float qn[kTileQ / kWarps], pn[kTileP / kWarps];
+    auto fetch = [&](int d0) {
+        const bool in = lane < D - d0;
+#pragma unroll
+        for (int k = 0; k < kTileQ / kWarps; k++) {
+            const long long pos = q0 + warp + k * kWarps;
+            qn[k] = in && pos < nq ? X[(q_index ? (long long)q_index[pos] : q_lo + pos) * D + d0 + lane] : 0.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < kTileP / kWarps; k++) {
+            const long long pos = p0 + warp + k * kWarps;
+            pn[k] = in && pos < nd ? X[(db_lo + pos) * D + d0 + lane] : 0.0f;
+        }
+    };
+    fetch(0);
     for (int d0 = 0; d0 < D; d0 += kDims) {
         const int dlen = min(kDims, D - d0);
         __syncthreads();
-        // a warp reads 32 dimensions of one row at a time (coalesced) and stores them as a column
-        for (int q = warp; q < kTileQ; q += kThreads / 32) {
-            const long long pos = q0 + q;
-            float v = 0.0f;
-            if (pos < nq && lane < dlen) v = X[(q_index ? (long long)q_index[pos] : q_lo + pos) * D + d0 + lane];
-            Qs[lane][q] = v;
-        }
-        for (int p = warp; p < kTileP; p += kThreads / 32) {
-            float v = 0.0f;
-            if (p0 + p < nd && lane < dlen) v = X[(db_lo + p0 + p) * D + d0 + lane];
-            Ps[lane][p] = -v;   // the difference as a sum
-        }
+#pragma unroll
+        for (int k = 0; k < kTileQ / kWarps; k++) Qs[lane][warp + k * kWarps] = make_float2(qn[k], qn[k]);
+#pragma unroll
+        for (int k = 0; k < kTileP / kWarps; k++) Ps[lane][warp + k * kWarps] = -pn[k];   // the difference as a sum
         __syncthreads();
-#pragma unroll 4
+        if (d0 + kDims < D) fetch(d0 + kDims);
+#pragma unroll 8
         for (int d = 0; d < dlen; d++) {
-            float qv[QT];
+            unsigned long long qq[QT];
             if constexpr (QT == 4) {
-                const float4 q4 = *reinterpret_cast<const float4 *>(&Qs[d][ty * 4]);
-                qv[0] = q4.x; qv[1] = q4.y; qv[2] = q4.z; qv[3] = q4.w;
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(&Qs[d][ty * 4]), b = *reinterpret_cast<const ulonglong2 *>(&Qs[d][ty * 4 + 2]);
+                qq[0] = a.x; qq[1] = a.y; qq[2] = b.x; qq[3] = b.y;
             } else {
 #pragma unroll
-                for (int a = 0; a < QT; a++) qv[a] = Qs[d][ty * QT + a];
+                for (int a = 0; a < QT; a++) qq[a] = *reinterpret_cast<const unsigned long long *>(&Qs[d][ty * QT + a]);
             }
-            const float4 pa = *reinterpret_cast<const float4 *>(&Ps[d][tx * 4]);
-            const float4 pb = *reinterpret_cast<const float4 *>(&Ps[d][64 + tx * 4]);
-            const unsigned long long pv[4] = {pack2(pa.x, pa.y), pack2(pa.z, pa.w), pack2(pb.x, pb.y), pack2(pb.z, pb.w)};
+            const ulonglong2 pa = *reinterpret_cast<const ulonglong2 *>(&Ps[d][tx * 4]), pb = *reinterpret_cast<const ulonglong2 *>(&Ps[d][64 + tx * 4]);
+            const unsigned long long pv[4] = {pa.x, pa.y, pb.x, pb.y};
 #pragma unroll
-            for (int a = 0; a < QT; a++) {
-                const unsigned long long qq = pack2(qv[a], qv[a]);
+            for (int a = 0; a < QT; a++)
 #pragma unroll
-                for (int b = 0; b < 4; b++) add_square2(acc[a][b], qq, pv[b], minus_zero);
-            }
+                for (int b = 0; b < 4; b++) add_square2(acc[a][b], qq[a], pv[b], minus_zero);
         }
     }
+    let_next_start();
+    after_previous();   // the selection before this round reads dist
     // (rows of dist are padded to whole tiles: every store stays inside)
 #pragma unroll
     for (int a = 0; a < QT; a++) {
@@ -145,9 +154,11 @@ constexpr int select_blocks(int kpt) { return kpt > 32 ? 3 : kpt > 16 ? 4 : kpt 
 // LONG: lists of more than kFoursMaxK.
 template <int KPT, bool IDS, bool LONG>
 __global__ void __launch_bounds__(kThreads, select_blocks(KPT))
-dense_select_kernel(const float *__restrict__ val, const int32_t *__restrict__ ids, long long ld, long long n_total, long long seg, int id_lo,
-                    int K, const int *__restrict__ out_rows, long long out_base, float *__restrict__ out_d, int32_t *__restrict__ out_i)
+dense_select_kernel(const float *val, const int32_t *ids, long long ld, long long n_total, long long seg, int id_lo,
+                    int K, const int *__restrict__ out_rows, long long out_base, float *out_d, int32_t *out_i)
 {
+    let_next_start();   // the distances of the next round touch nothing of this one's before they wait
+    after_previous();
     __shared__ unsigned long long s_key[kMaxDenseK];
     __shared__ __align__(16) unsigned s_min[kThreads], s_four[kThreads / 4];
     __shared__ unsigned s_bound, s_least;
@@ -324,14 +335,15 @@ int launch_select_as(const float *val, const int32_t *ids, long long ld, long lo
         const int *r = out_rows ? out_rows + q : nullptr;
         float *od = out_rows ? out_d : out_d + q * segments * K;
         int32_t *oi = out_rows ? out_i : out_i + q * segments * K;
-        auto launch = [&](auto kernel) { kernel<<<grid, kThreads, 0, st>>>(v, i, ld, n, seg, id_lo, K, r, out_base, od, oi); };
+        cudaError_t launched = cudaSuccess;
+        auto launch = [&](auto kernel) { launched = launch_chained(kernel, grid, kThreads, 0, st, v, i, ld, n, seg, id_lo, K, r, out_base, od, oi); };
         if (longest <= 4 * kThreads) launch(dense_select_kernel<4, IDS, LONG>);
         else if (longest <= 8 * kThreads) launch(dense_select_kernel<8, IDS, LONG>);
         else if (longest <= 16 * kThreads) launch(dense_select_kernel<16, IDS, LONG>);
         else if (longest <= 24 * kThreads) launch(dense_select_kernel<24, IDS, LONG>);
         else if (longest <= 32 * kThreads) launch(dense_select_kernel<32, IDS, LONG>);
         else launch(dense_select_kernel<48, IDS, LONG>);
-        B200_CUDA(cudaGetLastError());
+        B200_CUDA(launched);
     }
     return 0;
 }
@@ -344,22 +356,28 @@ int launch_select(const float *val, const int32_t *ids, long long ld, long long 
     return as(val, ids, ld, n, seg, segments, nq, id_lo, K, out_rows, out_base, out_d, out_i, st);
 }
 
-int launch_distances(const float *X, int D, int64_t q_lo, int64_t nq, const int *q_index, int64_t db_lo, int64_t nd, float *dist, long long ld,
+// first: of a call.  What was queued before the call may write the points, so that launch waits for all of it; the later ones
+// find this call's selection in front.
+int launch_distances(const float *X, int D, int64_t q_lo, int64_t nq, const int *q_index, int64_t db_lo, int64_t nd, float *dist, long long ld, bool first,
                      cudaStream_t st)
 {
     if (nd <= 0) return 0;
+    const auto launch = [&](auto kernel, dim3 grid, int64_t q, int64_t m) {
+        const int *index = q_index ? q_index + q : nullptr;
+        if (!first) return launch_chained(kernel, grid, kThreads, 0, st, X, D, q_lo + q, m, index, db_lo, nd, dist + q * ld, ld, kMinusZero2);
+        kernel<<<grid, kThreads, 0, st>>>(X, D, q_lo + q, m, index, db_lo, nd, dist + q * ld, ld, kMinusZero2);
+        return cudaGetLastError();
+    };
     const unsigned tiles = (unsigned)((nd + kTileP - 1) / kTileP);
     // a short list of queries: 16 a block waste less of the tile
     if (nq > 48) {
         for (int64_t q = 0; q < nq; q += 65535 * 64) {
             const int64_t m = std::min<int64_t>(65535 * 64, nq - q);
-            dense_distance_kernel<4><<<dim3(tiles, (unsigned)((m + 63) / 64)), kThreads, 0, st>>>(X, D, q_lo + q, m, q_index ? q_index + q : nullptr,
-                                                                                               db_lo, nd, dist + q * ld, ld, kMinusZero2);
+            B200_CUDA(launch(dense_distance_kernel<4>, dim3(tiles, (unsigned)((m + 63) / 64)), q, m));
         }
     } else {
-        dense_distance_kernel<1><<<dim3(tiles, (unsigned)((nq + 15) / 16)), kThreads, 0, st>>>(X, D, q_lo, nq, q_index, db_lo, nd, dist, ld, kMinusZero2);
+        B200_CUDA(launch(dense_distance_kernel<1>, dim3(tiles, (unsigned)((nq + 15) / 16)), 0, nq));
     }
-    B200_CUDA(cudaGetLastError());
     return 0;
 }
 
@@ -406,7 +424,7 @@ int knn_dense(const float *X, int D, int K, int64_t q_lo, int64_t nq, const int 
         const int *index = q_index ? q_index + q : nullptr;
         float *final_d = q_index ? d2 : d2 + q * K;
         int32_t *final_i = q_index ? ids : ids + q * K;
-        B200_TRY(launch_distances(X, D, q_lo + q, m, index, db_lo, nd, dist, ld, st));
+        B200_TRY(launch_distances(X, D, q_lo + q, m, index, db_lo, nd, dist, ld, q == 0, st));
         if (segments == 1) {
             B200_TRY(launch_select<false>(dist, nullptr, ld, nd, seg, 1, m, (int)db_lo, K, index, out_base, final_d, final_i, st));
             continue;
@@ -458,7 +476,7 @@ int knn_dense_in_scratch(const float *X, int64_t N, int D, int K, float *scratch
     const int64_t round = even_round(N, most);
     for (int64_t q = 0; q < N; q += round) {
         const int64_t m = std::min<int64_t>(round, N - q);
-        B200_TRY(launch_distances(X, D, q, m, nullptr, 0, N, scratch, ld, st));
+        B200_TRY(launch_distances(X, D, q, m, nullptr, 0, N, scratch, ld, q == 0, st));
         B200_TRY(launch_select<false>(scratch, nullptr, ld, N, N, 1, m, 0, K, nullptr, 0, d2 + q * K, ids + q * K, st));
     }
     return 0;
