@@ -296,3 +296,23 @@ def test_normalisation_sums_the_grid_in_double(engine, n, spread, offset):
     w, yt = w.astype(np.float64), yt.astype(np.float64)
     z = ((w[..., 0] + w[..., 3]) * yt[..., 0] - 2 * w[..., 1] * yt[..., 1] - 2 * w[..., 2] * yt[..., 2] + w[..., 0] * yt[..., 3]).sum()
     assert abs((Z + n) - z) <= 2.0 ** -23 * z
+
+
+@pytest.mark.parametrize("kind", ["normal", "copies", "whole numbers"])
+@pytest.mark.parametrize("n,d,k", [(40, 3, 40), (3000, 4, 31), (3000, 7, 33), (9000, 20, 90)])
+def test_session_symmetrises_by_distance_as_the_stage_by_ids(engine, kind, n, d, k):
+    """A session finds a point in its neighbour's row by the distance, the stage call by reading the row: the same P bit for bit,
+    also where many neighbours stand at the same distance (copies, whole numbers)."""
+    rng = np.random.default_rng(n + k)
+    X = rng.normal(0, 1, (n, d)).astype(np.float32)
+    if kind == "copies":
+        X = np.ascontiguousarray(np.repeat(X[:n // 8], 8, axis=0))
+    elif kind == "whole numbers":
+        X = rng.integers(0, 3, (n, d)).astype(np.float32)
+    ids, d2 = engine.knn(X, k)
+    p, _, _ = engine.perplexity(d2, k / 4.0, 1e-3)
+    with engine.Session(len(X), k) as s:
+        s.affinities_from_points(X, k / 4.0, 1e-3)
+        P, ids_s = s.get_affinities()
+    assert np.array_equal(ids, ids_s)
+    assert np.array_equal(P, engine.symmetrize(p, ids), equal_nan=True)
