@@ -240,8 +240,8 @@ own_scatter_kernel(const int32_t *__restrict__ perm, long long N, long long row_
 // ---- walking the rows of a range: per-warp scratch ----
 constexpr int kWalkWarps = 1;
 constexpr int kMaxK = 1024;
-// MAXT tiles and MAXS slots per segment: the common case (up to 64 tiles, rows of up to 128 slots) has a scratch of
-// 3 KB, so that a block's one warp shares its SM with 31 others; the general one (1,024 of each) takes 38 KB and
+// MAXT tiles and MAXS slots per segment: the common case (up to 64 tiles, rows of up to 256 slots) has a scratch of
+// 4 KB, so that a block's one warp shares its SM with 31 others; the general one (1,024 of each) takes 38 KB and
 // five warps fill an SM (the walk is a chain of dependent round trips: 14 ms against 5 at N = 10^6, K = 90).
 template <int MAXT, int MAXS>
 struct WalkScratchT {
@@ -255,7 +255,8 @@ struct WalkScratchT {
     unsigned long long win[MAXT][2];
     int win_id[MAXT];              // absolute lane / 16 of win[.][0]
 };
-using WalkScratchSmall = WalkScratchT<64, 128>;
+constexpr int kSmallTiles = 64, kSmallSlots = 256;
+using WalkScratchSmall = WalkScratchT<kSmallTiles, kSmallSlots>;
 using WalkScratch = WalkScratchT<kMaxTiles, kMaxK>;
 // slot word: bits 16..25 tile, bit 30 first slot of its (row, tile) group; low 16 bits: rank inside the group in
 // slot order, later the cell (4 x lane of the group + entry) the slot's entry is written to
@@ -817,7 +818,11 @@ int build_stream(StreamOut *out, DeviceArena &arena, DeviceArena &tmp, WalkArgs 
     // and the set-up from 0.190 to 0.217 s (one lane per group walks the group's entries): it pays from 4,500
     // iterations on, so it is off unless B200TSNE_ATTRACTIVE_PLACE=1 asks for it.
     a.greedy = getenv("B200TSNE_ATTRACTIVE_PLACE") ? atoi(getenv("B200TSNE_ATTRACTIVE_PLACE")) : 0;
+    // Short ranges where there are few rows: a warp walks its rows one after the other, each a chain of round trips, and 64 rows to a
+    // warp are 469 warps on 148 SMs at 30,011 points.  A range looks at one row more than it has.  Both walks, us, 64 rows and now:
+    // 5,000 x 64 277 -> 18, 20,011 x 32 178 -> 32, 60,000 x 90 515 -> 153, 50,000 x 150 (the smaller scratch included) 1,530 -> 231.
     a.range_rows = 64;
+    while (a.range_rows > 2 && a.n_seg < 3552ll * a.range_rows) a.range_rows /= 2;
     while ((a.n_seg + a.range_rows - 1) / a.range_rows * ntiles > (1ll << 24)) a.range_rows *= 2;
     a.n_ranges = (a.n_seg + a.range_rows - 1) / a.range_rows;
 
@@ -826,7 +831,7 @@ int build_stream(StreamOut *out, DeviceArena &arena, DeviceArena &tmp, WalkArgs 
     B200_CUDA(cudaMemsetAsync(totals, 0, sizeof(h_tot), st));
     const long long n_samples = std::min<long long>(a.n_seg, 4096);
     // the small scratch when the tiles and the longest segment fit it
-    const bool small = ntiles <= 64 && a.max_len <= 128;
+    const bool small = ntiles <= kSmallTiles && a.max_len <= kSmallSlots;
     if (small) sample_kernel<WalkScratchSmall><<<(unsigned)((n_samples + kWalkWarps - 1) / kWalkWarps), kWalkWarps * 32, 0, st>>>(a, n_samples, totals);
     else sample_kernel<WalkScratch><<<(unsigned)((n_samples + kWalkWarps - 1) / kWalkWarps), kWalkWarps * 32, 0, st>>>(a, n_samples, totals);
     B200_CUDA(cudaGetLastError());
