@@ -1386,6 +1386,19 @@ __device__ __forceinline__ float canon_step(float acc, float x, float y)
     return __fadd_rn(acc, __fmul_rn(t, t));
 }
 
+// The rounded squares of two rounded differences: x - y as x + (-1) y, the square as a fused operation with -0, an argument of the
+// kernel (a packed product and the sum after it would get one rounding), each half as the single instruction rounds it.
+__device__ __forceinline__ float2 canon_squares(float2 x, float2 y, unsigned long long minus_zero)
+{
+    float2 q;
+    asm("{\n\t.reg .b64 a, b, m;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 m, 0xbf800000bf800000;\n\t"
+        "fma.rn.f32x2 a, b, m, a;\n\tfma.rn.f32x2 a, a, a, %6;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "=f"(q.x), "=f"(q.y)
+        : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "l"(minus_zero));
+    return q;
+}
+constexpr unsigned long long kMinusZero2 = 0x8000000080000000ull;
+
 constexpr int kRerankWarps = 4;
 constexpr int kMaxL = 256;
 constexpr int kRerankDims = 32;   // dimensions per stage of wide rows
@@ -1394,12 +1407,14 @@ constexpr int kRerankWhole = 64;  // rows of up to this many dimensions are stag
 // Staged rows are `stride` floats apart: a multiple of 4, but not of 8, so that 32 lanes read 16 bytes of a row of their own
 // without bank conflicts.
 __host__ __device__ constexpr int rerank_stride(int D) { const int d = D <= kRerankWhole ? (D + 3) / 4 * 4 : kRerankDims; return d % 8 == 0 ? d + 4 : d; }
-// one warp: one stage (two where the row is walked) of 32 candidate rows and the query; L evaluated candidates; 34 row
-// addresses
-__host__ __device__ constexpr size_t rerank_floats(int D, int L) { return (size_t)(D <= kRerankWhole ? 1 : 2) * 33 * rerank_stride(D) + 4 * (size_t)L + 68; }
+// Stages of a row that is walked: one hides its latency behind the other warps that its smaller share of shared memory makes room
+// for (16 -> 24 on an SM), two where the registers of 256 candidates allow 16 anyway (scan and selection apart, ms, two | one:
+// 100,003 x 96, K = 32 0.95 | 0.77, 60,000 x 784, K = 90 2.55 | 2.47, 50,000 x 1,024, K = 150 3.74 | 4.10).
+__host__ __device__ constexpr int rerank_stages(int D, int L) { return D <= kRerankWhole || L <= 128 ? 1 : 2; }
+// one warp: the stages of 32 candidate rows and the query; L evaluated candidates; 34 row addresses
+__host__ __device__ constexpr size_t rerank_floats(int D, int L) { return (size_t)rerank_stages(D, L) * 33 * rerank_stride(D) + 4 * (size_t)L + 68; }
 
-__host__ __device__ constexpr size_t rerank_floats_max(int L) { return rerank_floats(kRerankWhole + 1, L); }
-static_assert(rerank_floats_max(0) >= rerank_floats(kRerankWhole, 0), "rows that are walked take the most");
+__host__ __device__ constexpr size_t rerank_floats_max(int L) { return rerank_floats(kRerankWhole, L) > rerank_floats(kRerankWhole + 1, L) ? rerank_floats(kRerankWhole, L) : rerank_floats(kRerankWhole + 1, L); }
 
 template <int BYTES> __device__ __forceinline__ void async_copy(void *dst, const void *src)
 {
@@ -1447,7 +1462,8 @@ template <int EPL> __device__ __forceinline__ void warp_sort(unsigned long long 
 // each, whole or 32 dimensions wide in two stages: whole lines per request, where a lane that walks a row of its own
 // touches 32 lines with each.  A lane then reads its row from shared memory and sums in the canonical order.
 // Measured, selection included, before (addresses computed per copy, ranking by counting) and now: 60,000 x 784 5.1 -> 2.6 ms,
-// 50,000 x 1,024 7.7 -> 3.9, 10^6 x 50 15.2 -> 10.6, 100,003 x 96 (K = 32) 1.0 now.
+// 50,000 x 1,024 7.7 -> 3.9, 10^6 x 50 15.2 -> 10.6, 100,003 x 96 (K = 32) 1.0; with squares two at a time and one stage 2.5, 3.7 (two
+// stages), 10.2, 0.77.
 // EPL: evaluated candidates a lane sorts (L = 32 EPL); the buffer holds up to 8 L.
 template <int VEC, int EPL>
 __global__ void __launch_bounds__(kRerankWarps * 32, EPL <= 4 ? 6 : 4)
@@ -1456,10 +1472,11 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
                      const int *__restrict__ counts, const float *__restrict__ tau, int K, const double *__restrict__ norms_exact,
                      float err_scale, const float2 *__restrict__ res_q, const float *__restrict__ rho, int32_t *__restrict__ ids,
                      float *__restrict__ d2, int *__restrict__ failed, int *__restrict__ n_failed, float *__restrict__ max_err_ratio,
-                     const float *__restrict__ Xp)
+                     const float *__restrict__ Xp, unsigned long long minus_zero)
 {
     // Xp (optional): the database rows in list order, Xp[pos] = X[dblist[pos]]
     constexpr int L = 32 * EPL, SLOTS = 8 * EPL;
+    constexpr bool ahead = rerank_stages(kRerankWhole + 1, L) > 1;   // a row that is walked: the next stage is fetched while one is summed
     extern __shared__ __align__(16) float stage_mem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long q = (long long)blockIdx.x * kRerankWarps + w;
@@ -1476,7 +1493,7 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
     const bool whole = D <= kRerankWhole;
     float *stage = stage_mem + (size_t)w * rerank_floats(D, L);
     // evaluated candidates: distance bits and row id, row of `base`, filter key
-    unsigned long long *s_key = reinterpret_cast<unsigned long long *>(stage + (whole ? 1 : 2) * 33 * stride);
+    unsigned long long *s_key = reinterpret_cast<unsigned long long *>(stage + rerank_stages(D, L) * 33 * stride);
     int *s_src = reinterpret_cast<int *>(s_key + L);
     float *s_fkey = reinterpret_cast<float *>(s_src + L);
     const float **s_row = reinterpret_cast<const float **>(s_fkey + L);   // the rows of a group, then the query
@@ -1551,7 +1568,7 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
         s_row[lane] = lane < rows ? base + (size_t)s_src[g + lane] * D : xq;
         __syncwarp();
         auto fetch = [&](int c) {
-            float *to = stage + (size_t)(c & 1) * 33 * stride + sub * stride + col;
+            float *to = stage + (size_t)(ahead ? c & 1 : 0) * 33 * stride + sub * stride + col;
             const int d = c * width + col;
             if (col < width && d < D) {
 #pragma unroll 4
@@ -1564,22 +1581,22 @@ knn_tc_rerank_kernel(const float *__restrict__ X, int D, const int *__restrict__
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
         float acc = 0.0f;
-        fetch(0);
+        if (ahead) fetch(0);
         for (int c = 0; c < chunks; c++) {
-            if (c + 1 < chunks) {
+            if (!ahead) fetch(c);
+            if (ahead && c + 1 < chunks) {
                 fetch(c + 1);
                 asm volatile("cp.async.wait_group 1;" ::: "memory");
             } else {
                 asm volatile("cp.async.wait_group 0;" ::: "memory");
             }
             __syncwarp();
-            const float *x = query + (size_t)(c & 1) * 33 * stride, *y = mine + (size_t)(c & 1) * 33 * stride;
+            const float *x = query + (size_t)(ahead ? c & 1 : 0) * 33 * stride, *y = mine + (size_t)(ahead ? c & 1 : 0) * 33 * stride;
             auto four = [&](int d) {
                 const float4 u = *reinterpret_cast<const float4 *>(x + d), v = *reinterpret_cast<const float4 *>(y + d);
-                acc = canon_step(acc, u.x, v.x);
-                acc = canon_step(acc, u.y, v.y);
-                acc = canon_step(acc, u.z, v.z);
-                acc = canon_step(acc, u.w, v.w);
+                const float2 a = canon_squares(make_float2(u.x, u.y), make_float2(v.x, v.y), minus_zero);
+                const float2 b = canon_squares(make_float2(u.z, u.w), make_float2(v.z, v.w), minus_zero);
+                acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, a.x), a.y), b.x), b.y);
             };
             const int len = min(width, D - c * width);
             if (len == kRerankDims) {
@@ -2197,7 +2214,7 @@ int launch_knn_tc(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t
     B200_TRY(allow_smem(rerank, sizeof(float) * kRerankWarps * rerank_floats_max(L)));
     rerank<<<(unsigned)((nq + kRerankWarps - 1) / kRerankWarps), kRerankWarps * 32, rerank_smem, st>>>(
         X, D, w.qlist, w.dblist, q_lo, nq, cand, cap, counts, tau, K, w.norms_q, err_scale, bf16 ? w.res_q : nullptr,
-        reinterpret_cast<const float *>(counters + 4), ids, d2, failed, counters + 1, reinterpret_cast<float *>(counters + 3), xp);
+        reinterpret_cast<const float *>(counters + 4), ids, d2, failed, counters + 1, reinterpret_cast<float *>(counters + 3), xp, kMinusZero2);
     B200_CUDA(cudaGetLastError());
     knn_tc_collect_failed_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(failed, nq, w.qlist, flist, counters + 2);
     B200_CUDA(cudaGetLastError());
