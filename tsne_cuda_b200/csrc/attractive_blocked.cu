@@ -889,8 +889,8 @@ static int device_sms(int *sms)
 }
 
 // Blocks (SMs) of the attractive kernel of an iteration on one GPU, whose grid pipeline runs beside it on the SMs that are left.
-// A chunk of the stream is 0.034 us of an SM; what the pipeline has to do beside it is 1,200 us of one, 3,200 where the iteration
-// sorts its points: the SMs are divided in the proportion of the two, which is where both end together.  (At most six short of all:
+// A chunk of the stream is 0.034 us of an SM; what the pipeline has to do beside it is 1,200 us of one, 1,700 beside graphs of 36,000 to
+// 100,000 chunks, whose pipeline is what the iteration waits for, 3,200 where the iteration sorts its points: the SMs are divided in the proportion of the two, which is where both end together.  (At most six short of all:
 // the pipeline's last kernel is a chain of its own.)  us an iteration, exaggerated (sorting in each iteration from 32,768 points
 // on) / settled, 90 neighbours (703 chunks per 1,000 points, 816 at 10^6), by the number of blocks:
 //   20,011     24 | 47 | 80              26.6 / 26.6 | 27.0 / 26.9 | 27.6 / 27.5
@@ -900,10 +900,13 @@ static int device_sms(int *sms)
 //   200,000    96 | 112 | 128 | 132      62.6 / 61.9 | 63.9 / 62.6 | 66.6 / 61.6 | 73.1 / 62.1
 //   600,000    120 | 124 | 130 | 138     144.3 / 147.3 | 141.6 / 145.1 | 141.1 / 138.7 | 148.5 / 135.6
 //   10^6       128 | 132 | 136 | 142     228.5 / 235.1 | 224.9 / 231.2 | 236.0 / 228.6 | 236.8 / 221.0
+// Settled again, with the transforms as they are now: 60,000 on 60 | 68 | 72 | 80 | 88 33.5 | 32.3 | 33.1 | 33.1 | 36.6, 80,000 on 76 |
+// 80 | 84 | 88 36.9 | 36.5 | 35.6 | 38.2, 100,000 on 80 | 88 | 92 | 96 42.1 | 40.1 | 40.0 | 41.1.
 // The entries of a truly symmetric P come in a second launch behind the first, so both streams count.
 static int blocks_beside_grid(int sms, long long chunks, bool sorts)
 {
-    const long long pipeline = sorts ? 96000 : 35500;   // chunks that take as long
+    // chunks that take as long
+    const long long pipeline = sorts ? 96000 : chunks >= 36000 && chunks < 100000 ? 49000 : 35500;
     const long long blocks = std::max(6ll, std::min<long long>(sms - 6, sms * chunks / (chunks + pipeline)));
     // The longest kernel of the pipeline, the columns pass, has 393 blocks, four to an SM: a graph that is done in time on what
     // leaves it 101 SMs (one wave) has no more (30,011 points on 47 | 55 blocks 27.7 | 29.7).
