@@ -24,7 +24,7 @@ constexpr size_t kMaxKeptExecs = 16;   // executable graphs kept per set
 constexpr int kLanes = 8;
 constexpr size_t kChunk = (size_t)1 << 20;
 // Measured: 188 MB of points 19 ms by a plain copy, 7 ms in lanes; at 8 MB starting the threads costs what they save.
-constexpr size_t kStagedMin = (size_t)24 << 20;
+constexpr size_t kStagedMin = kPopulateEnd;
 constexpr int kMaxIdleStages = 2;                // 16 MiB of pinned memory each, kept per device
 
 struct Stage {
@@ -188,16 +188,19 @@ template <class F> cudaError_t on_lanes(int lanes, int device, F body)
 
 }  // namespace
 
-void populate_pages(void *p, size_t bytes)
+void populate_pages(void *p, size_t bytes, const std::atomic<bool> &stop)
 {
 #ifdef MADV_POPULATE_WRITE
-    if (!p || bytes < kPopulateMin || !pageable(p)) return;
+    if (!p || !worth_populating(bytes) || !pageable(p)) return;
     const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), lo = ((uintptr_t)p + page - 1) / page * page, hi = ((uintptr_t)p + bytes) / page * page;
+    constexpr uintptr_t piece = (uintptr_t)1 << 20;
     // a failure (an old kernel, a mapping of another kind) leaves the faults to the copy
-    if (lo < hi) (void)madvise(reinterpret_cast<void *>(lo), hi - lo, MADV_POPULATE_WRITE);
+    for (uintptr_t at = lo; at < hi && !stop.load(std::memory_order_relaxed); at += piece)
+        if (madvise(reinterpret_cast<void *>(at), std::min(piece, hi - at), MADV_POPULATE_WRITE) != 0) return;
 #else
     (void)p;
     (void)bytes;
+    (void)stop;
 #endif
 }
 
