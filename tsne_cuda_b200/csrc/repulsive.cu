@@ -104,12 +104,13 @@ __device__ __forceinline__ int axis_box(float c, const GridGeom &g)
 // lane's last (open) run is then combined with those of its neighbours as described above, so the 180
 // shuffles of the segmented reduction are paid once per 32 * kSpreadPerLane points.
 //
-// Fewer points leave most SMs idle with four points a lane: up to kSpreadSingleMax a lane takes one.  Below kSortMin
-// the points collide so rarely that sorting (three kernels, 15 us) costs more than it saves, and up to kSpreadDirectMax
-// even the shuffles do.  Whole iteration, exaggerated / settled: 5 000 points sorted every time 47 / 41 us, one by one
-// 37 / 37; 20 011 points sorted 44 / 42, merged in natural order 41 / 41, one by one 57 / 42; 60 000 points sorted
-// 54 / 49, natural order 61 / 49.  (Both kinds of small spread take blocks of two warps, which leave no SM idle, and the
-// merge ends with the longest run.)
+// Fewer points leave most SMs idle with four points a lane: up to kSpreadSingleMax a lane takes one.  Points without an
+// order, up to kSpreadDirectMax, are spread one by one, since in natural order the shuffles cost more than they save; the
+// sort (three kernels, 15 us) is on the chain from kSortEachFrom points on only, see the session.  Whole iteration,
+// exaggerated / settled, with the sort on the chain of every iteration: 5 000 points sorted 47 / 41 us, one by one 37 / 37;
+// 20 011 points sorted 44 / 42, merged in natural order 41 / 41, one by one 57 / 42; 60 000 points sorted 54 / 49, natural
+// order 61 / 49.  (Both kinds of small spread take blocks of two warps, which leave no SM idle, and the merge ends with the
+// longest run.)
 constexpr int kSpreadPerLane = 4;
 
 __device__ __forceinline__ void spread_flush(float4 *__restrict__ w, int bx, int by, const float (&v)[kInterp][kInterp][4])
