@@ -1,7 +1,8 @@
 // Gradient, gains and momentum update (reference: IntegrationKernel, src/kernels/apply_forces.cu:11-57)
 // fused with the min/max reduction the next iteration's grid needs (reference: thrust::minmax_element
 // + two host reads, src/fit_tsne.cu:430-432) and the optional update-norm reduction
-// (src/fit_tsne.cu:522-527).  Pure streaming kernel: 40 bytes read and 24 written per point.
+// (src/fit_tsne.cu:522-527).  40 bytes read and 24 written per point, and nine nodes of 16 bytes out of L2 where the repulsive
+// force is interpolated here (10^6 points: 32 us, 22 without).
 #include "grid_geom.cuh"
 
 namespace b200 {
