@@ -316,3 +316,24 @@ def test_session_symmetrises_by_distance_as_the_stage_by_ids(engine, kind, n, d,
         P, ids_s = s.get_affinities()
     assert np.array_equal(ids, ids_s)
     assert np.array_equal(P, engine.symmetrize(p, ids), equal_nan=True)
+
+
+def test_symmetrisation_of_points_at_equal_distances_takes_no_longer(engine):
+    """Binary features put most of a row at a few distances.  The set-up behind the search takes what it takes for the same points
+    moved apart by a hair (1.2 of it; rows walked through to find a point among its equals, 2.9)."""
+    n, d, k = 20000, 12, 150
+    rng = np.random.default_rng(0)
+    X = rng.integers(0, 2, (n, d)).astype(np.float32)
+    apart = X + rng.normal(0, 1e-3, X.shape).astype(np.float32)
+    took = []
+    for points in (X, apart):
+        with engine.Session(n, k) as s:
+            s.enable_stage_timers(True)
+            s.affinities_from_points(points, k / 3.0, 1e-3)
+            t = []
+            for _ in range(9):
+                before = s.stage_times()["affinities"][0]
+                s.affinities_from_points(points, k / 3.0, 1e-3)
+                t.append(s.stage_times()["affinities"][0] - before)
+            took.append(sorted(t)[4])
+    assert took[0] < 1.6 * took[1]

@@ -123,18 +123,29 @@ symmetrize_kernel(const float *__restrict__ p, const int32_t *__restrict__ ids, 
         const bool valid = (unsigned long long)j_mine < (unsigned long long)N;
         if constexpr (BY_DISTANCE) {
             // A neighbour whose own last one is nearer than this point does not have it in its row; in the others it stands
-            // among those at its distance.  A lane a neighbour: fewer sectors than the ids have, and 32 searches in flight.
+            // among those at its distance, by id (unfilled slots, id -1, last).  A lane a neighbour: fewer sectors than the ids
+            // have, and 32 searches in flight.
             const float d = valid ? d2[i * K + s_mine] : 0.0f;
             if (valid && d <= furthest[j_mine]) {
                 const float *dj = d2 + (long long)j_mine * K;
+                const int32_t *ij = ids + (long long)j_mine * K;
                 int lo = 0, hi = K;
                 while (lo < hi) {
                     const int mid = (lo + hi) >> 1;
                     if (dj[mid] < d) lo = mid + 1;
                     else hi = mid;
                 }
-                for (; lo < K && dj[lo] == d; lo++)
-                    if (ids[(long long)j_mine * K + lo] == (int32_t)i) acc_mine += p[(long long)j_mine * K + lo];
+                // Whole numbers and copies have most of a row at one distance, so its equals are searched too: 60,000 x 32 binary
+                // features, K = 150 0.73 ms (walked through 3.6, by ids alone 0.93, points without equals 0.17).
+                if (lo < K && ij[lo] != (int32_t)i) {
+                    hi = K;
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (dj[mid] == d && (uint32_t)ij[mid] < (uint32_t)i) lo = mid + 1;
+                        else hi = mid;
+                    }
+                }
+                if (lo < K && ij[lo] == (int32_t)i) acc_mine += p[(long long)j_mine * K + lo];
             }
             if (s_mine < K) P_rows[r * K + s_mine] = (float)((double)acc_mine / inv);
             continue;
