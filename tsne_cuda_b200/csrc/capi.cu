@@ -6,7 +6,6 @@
 #include <algorithm>
 #include <new>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "../../include/tsnecuda_b200.h"
@@ -83,31 +82,16 @@ int b200tsne_knn(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t 
     float *dX = nullptr, *dd = nullptr;
     int32_t *di = nullptr;
     const size_t nq = (size_t)(q_hi - q_lo);
-    struct Helper {
-        std::thread t;
-        std::atomic<bool> stop{false};
-        void end()
-        {
-            stop = true;
-            if (t.joinable()) t.join();
-        }
-        ~Helper() { end(); }
-    } helper;   // the lists' pages, while the points are copied and searched
-    if (worth_populating(sizeof(float) * nq * K)) try {
-        helper.t = std::thread([=, &helper] {
-            if (cudaSetDevice(device) != cudaSuccess) return;
-            populate_pages(ids, sizeof(int32_t) * nq * K, helper.stop);
-            populate_pages(d2, sizeof(float) * nq * K, helper.stop);
-        });
-    } catch (const std::exception &) {   // no thread to be had: the copy finds the pages itself
-    }
+    PagesAhead pages;   // the lists', while the points are copied and searched
+    const size_t list_bytes = sizeof(float) * nq * K;
+    if (worth_populating(list_bytes)) pages.start(pageable(ids) ? ids : nullptr, pageable(d2) ? d2 : nullptr, list_bytes);
     B200_TRY(up(a, &dX, X, (size_t)N * D, sg.st));
     B200_TRY(a.alloc((void **)&di, sizeof(int32_t) * std::max<size_t>(nq * K, 1)));
     B200_TRY(a.alloc((void **)&dd, sizeof(float) * std::max<size_t>(nq * K, 1)));
     B200_TRY(knn_search(dX, N, D, K, q_lo, q_hi, db_lo, db_hi, di, dd, &g_last_knn_stats, sg.st));
     B200_TRY(launch_knn_finalize(di, dd, (int64_t)nq * K, sg.st));
     B200_CUDA(cudaStreamSynchronize(sg.st));   // the lists are there
-    helper.end();
+    pages.end();
     B200_TRY(down(ids, di, nq * K, sg.st));
     B200_TRY(down(d2, dd, nq * K, sg.st));
     B200_CUDA(cudaStreamSynchronize(sg.st));

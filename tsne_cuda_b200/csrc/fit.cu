@@ -13,7 +13,6 @@
 
 #include "../../include/tsnecuda/fit_tsne.h"
 #include "../../include/tsnecuda_b200.h"
-#include "hostio.h"
 #include "session.h"
 
 namespace tsnecuda {
@@ -119,16 +118,13 @@ int run(Options &opt, GpuOptions &gpu_opt)
     std::vector<float> y0;
     std::string y0_error;
     int y0_rc = 0;
-    std::atomic<bool> searched{false};
     std::thread y0_thread([&]() {
         y0_rc = initial_embedding(opt, y0);
         if (y0_rc != 0) y0_error = b200::last_error();
-        if (opt.return_style == RETURN_STYLE::ONCE) b200::populate_pages(opt.return_data, sizeof(float) * 2 * (size_t)N, searched);
     });
     // kNN, max-normalisation, perplexity search and symmetrisation run back to back on the device;
     // the split between the two printed phases is only meaningful with stage timers on.
     const int aff_rc = s.affinities_from_points(opt.points, opt.num_dims, opt.perplexity, opt.perplexity_search_epsilon);
-    searched = true;
     y0_thread.join();
     if (aff_rc != 0) return aff_rc;
     if (verbose) std::cout << "done.\nComputing Pij matrix... " << std::endl;

@@ -3,8 +3,6 @@
 
 #include <cuda.h>
 #include <string.h>
-#include <sys/mman.h>
-#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -153,7 +151,6 @@ cudaMemoryType memory_type(const void *p)
     }
     return a.type;
 }
-bool pageable(const void *p) { return memory_type(p) == cudaMemoryTypeUnregistered; }
 
 int lanes_for(size_t bytes)
 {
@@ -188,21 +185,7 @@ template <class F> cudaError_t on_lanes(int lanes, int device, F body)
 
 }  // namespace
 
-void populate_pages(void *p, size_t bytes, const std::atomic<bool> &stop)
-{
-#ifdef MADV_POPULATE_WRITE
-    if (!p || !worth_populating(bytes) || !pageable(p)) return;
-    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), lo = ((uintptr_t)p + page - 1) / page * page, hi = ((uintptr_t)p + bytes) / page * page;
-    constexpr uintptr_t piece = (uintptr_t)1 << 20;
-    // a failure (an old kernel, a mapping of another kind) leaves the faults to the copy
-    for (uintptr_t at = lo; at < hi && !stop.load(std::memory_order_relaxed); at += piece)
-        if (madvise(reinterpret_cast<void *>(at), std::min(piece, hi - at), MADV_POPULATE_WRITE) != 0) return;
-#else
-    (void)p;
-    (void)bytes;
-    (void)stop;
-#endif
-}
+bool pageable(const void *p) { return memory_type(p) == cudaMemoryTypeUnregistered; }
 
 bool plain_host(const void *p)
 {

@@ -4,11 +4,10 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
-#include <atomic>
-
 #include <vector>
 
 #include "common.cuh"
+#include "pages.h"
 
 namespace b200 {
 
@@ -57,15 +56,7 @@ void graph_exec_release(StreamSet *s, cudaGraphExec_t exec, unsigned long long s
 int copy_in(void *dst_device, const void *src_host, size_t bytes, cudaStream_t st);
 int copy_out(void *dst_host, const void *src_device, size_t bytes, cudaStream_t st);
 
-// Gives a pageable buffer its pages ahead of a copy_out, while the device is busy with what will be copied: in fresh memory
-// the faults are a good part of the copy (100,003 x 96, K = 32, lists in fresh arrays: whole call 10.0 -> 9.0 ms).  The contents stay as they are; any
-// thread may call it; other kinds of memory, small buffers and those that several threads will fill are left alone (two
-// lists of 150 MB, pages made ahead of the threads: 28 -> 50 ms).  It looks at `stop` between pieces, so that whoever is ready
-// to copy does not wait for the rest.
-constexpr size_t kPopulateMin = (size_t)2 << 20, kPopulateEnd = (size_t)24 << 20;
-inline bool worth_populating(size_t bytes) { return bytes >= kPopulateMin && bytes < kPopulateEnd; }
-void populate_pages(void *p, size_t bytes, const std::atomic<bool> &stop);
-
+bool pageable(const void *p);     // host memory that CUDA knows nothing of
 bool plain_host(const void *p);   // host memory, pinned or not: neither device nor managed memory, which a copy takes as well
 
 void host_pools_release(int device);   // idle sets and staging memory of one device
