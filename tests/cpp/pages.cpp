@@ -73,6 +73,17 @@ int main()
         ahead.start(nullptr, nullptr, bytes);
         ahead.start(a, b, kPopulateMin - 1);
         CHECK(!ahead.started());
+        memset(a, 1, bytes);
+        memset(b, 1, bytes);
+        CHECK(!pages_missing(a, bytes) && !pages_missing(b + 1, bytes - 1));
+        ahead.start(a, b, bytes);   // nothing left to do
+        CHECK(!ahead.started());
+        char *half = map(bytes);
+        memset(half, 1, bytes / 4);
+        CHECK(pages_missing(half, bytes));
+        ahead.start(a, half, bytes);
+        CHECK(ahead.started());
+        ahead.end();
         for (int k = 0; k < 50; k++) {
             PagesAhead other;
             other.start(map(bytes), nullptr, bytes);

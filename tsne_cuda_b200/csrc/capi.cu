@@ -90,8 +90,10 @@ int b200tsne_knn(const float *X, int64_t N, int D, int K, int64_t q_lo, int64_t 
     B200_TRY(a.alloc((void **)&dd, sizeof(float) * std::max<size_t>(nq * K, 1)));
     B200_TRY(knn_search(dX, N, D, K, q_lo, q_hi, db_lo, db_hi, di, dd, &g_last_knn_stats, sg.st));
     B200_TRY(launch_knn_finalize(di, dd, (int64_t)nq * K, sg.st));
-    B200_CUDA(cudaStreamSynchronize(sg.st));   // the lists are there
-    pages.end();
+    if (pages.started()) {
+        B200_CUDA(cudaStreamSynchronize(sg.st));   // the lists are there
+        pages.end();
+    }
     B200_TRY(down(ids, di, nq * K, sg.st));
     B200_TRY(down(d2, dd, nq * K, sg.st));
     B200_CUDA(cudaStreamSynchronize(sg.st));

@@ -38,6 +38,19 @@ inline void populate_pages(void *p, size_t bytes, const std::atomic<bool> &stop)
 #endif
 }
 
+// Does the buffer lack pages?  Its first, middle and last whole page are looked at: a buffer that an earlier call has
+// filled needs no thread (starting one takes 25 us: 9,000 x 20, K = 60 into the same arrays 771 us with it, 745 without).
+inline bool pages_missing(const void *p, size_t bytes)
+{
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), lo = ((uintptr_t)p + page - 1) / page * page, hi = ((uintptr_t)p + bytes) / page * page;
+    if (!p || hi <= lo) return false;
+    for (const uintptr_t at : {lo, (lo + (hi - lo) / 2) / page * page, hi - page}) {
+        unsigned char in = 0;
+        if (mincore(reinterpret_cast<void *>(at), page, &in) == 0 && !(in & 1)) return true;
+    }
+    return false;
+}
+
 // A thread that populates up to two buffers of one size until it is told that the copy is due.
 class PagesAhead {
 public:
@@ -47,7 +60,7 @@ public:
     ~PagesAhead() { end(); }
     void start(void *a, void *b, size_t bytes)   // null: none
     {
-        if (thread_.joinable() || (!a && !b) || !worth_populating(bytes)) return;
+        if (thread_.joinable() || !worth_populating(bytes) || !(pages_missing(a, bytes) || pages_missing(b, bytes))) return;
         try {
             thread_ = std::thread([this, a, b, bytes] {
                 populate_pages(a, bytes, stop_);
