@@ -104,6 +104,41 @@ def test_blocks_of_iterations_and_single_steps_agree(engine):
         assert rel_l2(o[0], out[0][0]) < 1e-6 and rel_l2(o[1], out[0][1]) < 1e-4
 
 
+@pytest.mark.parametrize("n,step,refresh,early,chunks,sorts", [
+    (40000, 400, None, None, [64], 8),
+    (40000, 0, "0", "1", [64], 0),                           # natural order, whatever the other variable says
+    (20000, 0, None, "4", [64], 16),
+    (2999, 0, None, None, [64], 0),
+    (3000, 0, None, None, [64], 8),
+    (65535, 0, None, None, [64], 16),
+    (65536, 0, None, None, [64], 64),
+])
+def test_how_often_the_order_is_sorted(engine, monkeypatch, n, step, refresh, early, chunks, sorts):
+    """Counted in launches: a sort has three."""
+    P, ids, rng = _graph(n, 3, 4)
+    Y = rng.normal(0, 5.0, (2, n)).astype(np.float32)
+
+    def launches():
+        with engine.Session(n, 3) as s:
+            s.set_affinities(P, ids)
+            s.set_schedule(1e-3, 12.0, 250, 0.5, 0.8)
+            s.set_state(Y, np.zeros_like(Y), np.ones_like(Y), step)
+            before = s.launch_count()
+            for c in chunks:
+                s.run(c)
+            return s.launch_count() - before
+
+    for name, value in (("B200TSNE_ORDER_REFRESH", refresh), ("B200TSNE_ORDER_REFRESH_EARLY", early)):
+        if value is None:
+            monkeypatch.delenv(name, raising=False)
+        else:
+            monkeypatch.setenv(name, value)
+    got = launches()
+    monkeypatch.setenv("B200TSNE_ORDER_REFRESH", "0")
+    monkeypatch.delenv("B200TSNE_ORDER_REFRESH_EARLY", raising=False)
+    assert got - launches() == 3 * sorts
+
+
 def _steps(engine, monkeypatch, n, graphs, per_call, decay):
     monkeypatch.setenv("B200TSNE_GRAPHS", "1" if graphs else "0")
     P, ids, rng = _graph(n, 6, 8)

@@ -137,11 +137,14 @@ int Session::init(int64_t N_, int K_, int64_t lo, int64_t hi, int device_)
     B200_CUDA(cudaMemsetAsync(box_hist, 0, sizeof(int32_t) * kBoxes * kBoxes, stream));
     if (rows() < kSortMin) order_refresh = 0;
     order_refresh_early = rows() >= kSortEachFrom ? 1 : rows() >= kSortMin ? 4 : rows() >= kSortEarlyMin ? 8 : 0;
+    bool never = false;
     if (const char *e = getenv("B200TSNE_ORDER_REFRESH")) {
         order_refresh = std::max(0, atoi(e));
-        order_refresh_early = order_refresh == 0 ? 0 : std::max(1, order_refresh_early);
+        never = order_refresh == 0;
+        order_refresh_early = std::max(1, order_refresh_early);
     }
     if (const char *e = getenv("B200TSNE_ORDER_REFRESH_EARLY")) order_refresh_early = order_refresh_early_sharded = std::max(1, atoi(e));
+    if (never) order_refresh_early = 0;
     if (order_refresh == 0) order_refresh_early_sharded = 0;   // ranks sort in both phases or in neither
     if (const char *e = getenv("B200TSNE_GRAPHS")) use_graphs = atoi(e) != 0;
     B200_TRY(arena.alloc((void **)&Y2, sizeof(float2) * npad));
