@@ -105,6 +105,10 @@ def test_blocks_of_iterations_and_single_steps_agree(engine):
 
 
 @pytest.mark.parametrize("n,step,refresh,early,chunks,sorts", [
+    (40000, 400, "32", None, [64, 64], 4),                   # a period above a block's sixteen iterations
+    (40000, 400, "10", None, [160], 16),                     # one that does not divide them
+    (40000, 400, "10", None, [1] * 40, 4),
+    (40000, 400, "5", None, [2] * 20, 8),
     (40000, 400, None, None, [64], 8),
     (40000, 0, "0", "1", [64], 0),                           # natural order, whatever the other variable says
     (20000, 0, None, "4", [64], 16),

@@ -536,8 +536,11 @@ bool Session::sorts_at(int b, int block) const
 {
     const int period = refresh_period(step);   // (a block is of one phase)
     if (period <= 1) return period == 1;
-    if (block >= kGraphIters) return b % period == 0;
-    return b == 0 && since_sort >= (block > 1 ? 2 * period : period);
+    const bool fixed = kGraphIters % period == 0;
+    if (fixed && block >= kGraphIters) return b % period == 0;
+    if (fixed) return b == 0 && since_sort >= (block > 1 ? 2 * period : period);
+    const int first = std::max(0, period - since_sort);
+    return b >= first && (b - first) % period == 0;
 }
 
 int Session::refresh_period(int at) const
