@@ -229,6 +229,19 @@ def test_against_the_list_search_on_every_row(engine, monkeypatch, n, d, k, ties
     assert np.array_equal(ids, ids_l) and np.array_equal(d2, d2_l)
 
 
+@pytest.mark.parametrize("n,rows", [(2147, 2147), (2305, 2305), (2305, 48), (2305, 49), (20000, 48), (32768, 37)])
+@pytest.mark.parametrize("d", [1, 32, 33, 97])
+def test_distances_on_both_sides_of_four_blocks_to_an_sm(engine, monkeypatch, n, rows, d):
+    """592 blocks of 64 (16 from 48 rows on down) queries and 128 points on 148 SMs: 578, 703, 57, 19, 471 and 768 here."""
+    X = _points(n, d, n + d, False)
+    lo = (n - rows) // 2
+    ids, d2 = engine.knn(X, 240, lo, lo + rows)
+    assert engine.knn_last_stats()["tensor_core"] == 0
+    monkeypatch.setenv("B200TSNE_KNN", "simt")
+    ids_l, d2_l = engine.knn(X, 240, lo, lo + rows)
+    assert np.array_equal(ids, ids_l) and np.array_equal(d2, d2_l)
+
+
 @pytest.mark.parametrize("n,d,k", [(700, 33, 20), (4099, 64, 16), (9000, 20, 150)])
 def test_a_search_between_the_kernels_that_write_and_clear_its_points(engine, n, d, k):
     """The rounds of a search overlap with each other, but not with what the caller has queued before and after it in the

@@ -11,6 +11,8 @@
 // 4.4 / 0.4 ms.
 #include <limits.h>
 
+#include <type_traits>
+
 #include <algorithm>
 
 #include "session.h"
@@ -27,6 +29,12 @@ constexpr int kThreads = 256;
 // busy as with single instructions, but half as many are issued: 4,099 x 64, K = 16 211 -> 201 us,
 // 10,000 x 100, K = 40 1,943 -> 1,827 (whole searches).
 constexpr unsigned long long kMinusZero2 = 0x8000000080000000ull;
+__device__ __forceinline__ unsigned long long twice(float v)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
 __device__ __forceinline__ float2 unpack2(unsigned long long v)
 {
     float2 r;
@@ -43,19 +51,23 @@ __device__ __forceinline__ void add_square2(unsigned long long &acc, unsigned lo
 
 // dist[q * ld + p] = canonical distance (sequential over the dimensions, every operation rounded) of query q of the list
 // and database row db_lo + p.  QT queries and eight points a thread, 16 QT queries and 128 points a block.
-// Bound: the fp32 pipe, which the packed operations of a dimension take for 96 cycles a warp.  So the next chunk of dimensions
-// is on its way while one is worked on, and a query's value stands twice in shared memory, as the operation wants it.
-// Launched behind the selection of the round before, it runs beside it up to its stores (see chained launches in common.cuh).
-// Whole searches, K in brackets, before and with these: 4,099 x 64 (16) 201 -> 181 us, 6,145 x 20 (40) 267 -> 204, 9,000 x 20 (150)
-// 743 -> 586, 10,000 x 100 (40) 1,800 -> 1,734, 12,288 x 32 (48) 1,125 -> 947, 3,000 x 33 (8) 91 -> 77; three blocks to an SM, as
-// one wave of a round of 832 queries wants (122 registers and two blocks: 184 us at 4,099 x 64).
-template <int QT>
-__global__ void __launch_bounds__(kThreads, 3)
+// Bound: the fp32 pipe, which the packed operations of a dimension take for 96 cycles a warp.
+// AHEAD: the next chunk of dimensions is on its way in registers while one is worked on, and a query's value stands twice in
+// shared memory, as the operation wants it; three blocks to an SM, as one wave of a round of 832 queries wants (122 registers and
+// two blocks: 184 us at 4,099 x 64).  A launch of many waves hides the loads behind a fourth block instead and is bound by the
+// pipe alone.  The line is where all blocks find a place at once, four to an SM.  Searches, us, AHEAD | not, blocks of a launch in
+// brackets: 3,000 x 33, K = 8 (384) 72 | 83, 4,099 x 64, K = 16 (429) 176 | 208, 6,145 x 20, K = 40 (490) 200 | 210, 10,000 x 100, K = 40
+// (474) 1,728 | 1,715; K = 240 2,150 x 257 (578) 215 | 216, 2,300 x 257 (648) 253 | 245, 3,500 x 257 (1,540) 494 | 468, 12,288 x 97 (8,128)
+// 2,408 | 2,235.
+// Launched behind the selection of the round before, it runs beside it up to its stores (see chained launches in common.cuh): with
+// AHEAD 4,099 x 64 (16) 201 -> 181 us, 9,000 x 20 (150) 743 -> 586, 12,288 x 32 (48) 1,125 -> 947.
+template <int QT, bool AHEAD>
+__global__ void __launch_bounds__(kThreads, AHEAD ? 3 : 4)
 dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long long nq, const int *__restrict__ q_index, long long db_lo,
                       long long nd, float *dist, long long ld, unsigned long long minus_zero)
 {
-    constexpr int kTileQ = 16 * QT, kQs = kTileQ + 2, kPs = kTileP + 4, kWarps = kThreads / 32;
-    __shared__ __align__(16) float2 Qs[kDims][kQs];
+    constexpr int kTileQ = 16 * QT, kQs = kTileQ + (AHEAD ? 2 : 4), kPs = kTileP + 4, kWarps = kThreads / 32;
+    __shared__ __align__(16) std::conditional_t<AHEAD, float2, float> Qs[kDims][kQs];
     __shared__ __align__(16) float Ps[kDims][kPs];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31, warp = tid >> 5;
     const long long p0 = (long long)blockIdx.x * kTileP, q0 = (long long)blockIdx.y * kTileQ;
@@ -65,39 +77,54 @@ dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long l
 #pragma unroll
         for (int b = 0; b < 4; b++) acc[a][b] = 0ull;
     // a warp reads 32 dimensions of one row at a time (coalesced) and stores them as a column
-    float qn[kTileQ / kWarps], pn[kTileP / kWarps];
-    auto fetch = [&](int d0) {
+    auto query_at = [&](int k, int d0, bool in) {
+        const long long pos = q0 + warp + k * kWarps;
+        return in && pos < nq ? X[(q_index ? (long long)q_index[pos] : q_lo + pos) * D + d0 + lane] : 0.0f;
+    };
+    auto point_at = [&](int k, int d0, bool in) {
+        const long long pos = p0 + warp + k * kWarps;
+        return in && pos < nd ? X[(db_lo + pos) * D + d0 + lane] : 0.0f;
+    };
+    [[maybe_unused]] float qn[kTileQ / kWarps], pn[kTileP / kWarps];
+    [[maybe_unused]] auto fetch = [&](int d0) {
         const bool in = lane < D - d0;
 #pragma unroll
-        for (int k = 0; k < kTileQ / kWarps; k++) {
-            const long long pos = q0 + warp + k * kWarps;
-            qn[k] = in && pos < nq ? X[(q_index ? (long long)q_index[pos] : q_lo + pos) * D + d0 + lane] : 0.0f;
-        }
+        for (int k = 0; k < kTileQ / kWarps; k++) qn[k] = query_at(k, d0, in);
 #pragma unroll
-        for (int k = 0; k < kTileP / kWarps; k++) {
-            const long long pos = p0 + warp + k * kWarps;
-            pn[k] = in && pos < nd ? X[(db_lo + pos) * D + d0 + lane] : 0.0f;
-        }
+        for (int k = 0; k < kTileP / kWarps; k++) pn[k] = point_at(k, d0, in);
     };
-    fetch(0);
+    if constexpr (AHEAD) fetch(0);
     for (int d0 = 0; d0 < D; d0 += kDims) {
         const int dlen = min(kDims, D - d0);
         __syncthreads();
+        if constexpr (AHEAD) {
 #pragma unroll
-        for (int k = 0; k < kTileQ / kWarps; k++) Qs[lane][warp + k * kWarps] = make_float2(qn[k], qn[k]);
+            for (int k = 0; k < kTileQ / kWarps; k++) Qs[lane][warp + k * kWarps] = make_float2(qn[k], qn[k]);
 #pragma unroll
-        for (int k = 0; k < kTileP / kWarps; k++) Ps[lane][warp + k * kWarps] = -pn[k];   // the difference as a sum
+            for (int k = 0; k < kTileP / kWarps; k++) Ps[lane][warp + k * kWarps] = -pn[k];   // the difference as a sum
+        } else {
+#pragma unroll 4
+            for (int k = 0; k < kTileQ / kWarps; k++) Qs[lane][warp + k * kWarps] = query_at(k, d0, lane < dlen);
+#pragma unroll 4
+            for (int k = 0; k < kTileP / kWarps; k++) Ps[lane][warp + k * kWarps] = -point_at(k, d0, lane < dlen);
+        }
         __syncthreads();
-        if (d0 + kDims < D) fetch(d0 + kDims);
-#pragma unroll 8
+        if constexpr (AHEAD)
+            if (d0 + kDims < D) fetch(d0 + kDims);
+#pragma unroll (AHEAD ? 8 : 4)
         for (int d = 0; d < dlen; d++) {
             unsigned long long qq[QT];
-            if constexpr (QT == 4) {
+            if constexpr (!AHEAD) {
+                float qv[QT];
+                if constexpr (QT == 4) *reinterpret_cast<float4 *>(qv) = *reinterpret_cast<const float4 *>(&Qs[d][ty * 4]);
+                else qv[0] = Qs[d][ty];
+#pragma unroll
+                for (int a = 0; a < QT; a++) qq[a] = twice(qv[a]);
+            } else if constexpr (QT == 4) {
                 const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(&Qs[d][ty * 4]), b = *reinterpret_cast<const ulonglong2 *>(&Qs[d][ty * 4 + 2]);
                 qq[0] = a.x; qq[1] = a.y; qq[2] = b.x; qq[3] = b.y;
             } else {
-#pragma unroll
-                for (int a = 0; a < QT; a++) qq[a] = *reinterpret_cast<const unsigned long long *>(&Qs[d][ty * QT + a]);
+                qq[0] = *reinterpret_cast<const unsigned long long *>(&Qs[d][ty]);
             }
             const ulonglong2 pa = *reinterpret_cast<const ulonglong2 *>(&Ps[d][tx * 4]), pb = *reinterpret_cast<const ulonglong2 *>(&Ps[d][64 + tx * 4]);
             const unsigned long long pv[4] = {pa.x, pa.y, pb.x, pb.y};
@@ -369,14 +396,20 @@ int launch_distances(const float *X, int D, int64_t q_lo, int64_t nq, const int 
         return cudaGetLastError();
     };
     const unsigned tiles = (unsigned)((nd + kTileP - 1) / kTileP);
+    int device = 0, sms = 0;
+    B200_CUDA(cudaGetDevice(&device));
+    B200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const auto launch_tiles = [&](auto ahead, auto plain, unsigned rows, int64_t q, int64_t m) {
+        return launch((long long)tiles * rows <= 4ll * sms ? ahead : plain, dim3(tiles, rows), q, m);
+    };
     // a short list of queries: 16 a block waste less of the tile
     if (nq > 48) {
         for (int64_t q = 0; q < nq; q += 65535 * 64) {
             const int64_t m = std::min<int64_t>(65535 * 64, nq - q);
-            B200_CUDA(launch(dense_distance_kernel<4>, dim3(tiles, (unsigned)((m + 63) / 64)), q, m));
+            B200_CUDA(launch_tiles(dense_distance_kernel<4, true>, dense_distance_kernel<4, false>, (unsigned)((m + 63) / 64), q, m));
         }
     } else {
-        B200_CUDA(launch(dense_distance_kernel<1>, dim3(tiles, (unsigned)((nq + 15) / 16)), 0, nq));
+        B200_CUDA(launch_tiles(dense_distance_kernel<1, true>, dense_distance_kernel<1, false>, (unsigned)((nq + 15) / 16), 0, nq));
     }
     return 0;
 }
@@ -460,7 +493,8 @@ template <bool LONG> static int load_select()
 int knn_dense_load()
 {
     cudaFuncAttributes a;
-    const void *kernels[] = {(const void *)dense_distance_kernel<1>, (const void *)dense_distance_kernel<4>};
+    const void *kernels[] = {(const void *)dense_distance_kernel<1, true>, (const void *)dense_distance_kernel<1, false>, (const void *)dense_distance_kernel<4, true>,
+                             (const void *)dense_distance_kernel<4, false>};
     for (const void *k : kernels) B200_CUDA(cudaFuncGetAttributes(&a, k));
     B200_TRY(load_select<false>());
     return load_select<true>();
