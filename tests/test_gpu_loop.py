@@ -26,7 +26,8 @@ def _same(a, b):
     assert (np.abs(a[2] - b[2]) > 1e-5).mean() < 1e-4 and a[3] == b[3]
 
 
-# points one by one | merged in natural order | sorted, a point a lane | sorted, four a lane: both sides of every border
+# the first iteration: points one by one up to 2,999, a point a lane in the order as it is allocated up to 131,072, sorted from
+# 65,536 on; then four a lane
 @pytest.mark.parametrize("n", [1, 31, 8192, 8193, 32767, 32768, 131072, 131075])
 @pytest.mark.parametrize("spread", [1e-4, 20.0])
 def test_one_iteration_vs_oracle(engine, oracle_cpu, n, spread):
@@ -46,6 +47,58 @@ def test_one_iteration_vs_oracle(engine, oracle_cpu, n, spread):
     assert rel_l2(mom, mom_o) < 1.1e-4
     # the embedding rounds once more per coordinate
     assert np.abs(Y1 - Yo).max() < 1.1e-4 * np.linalg.norm(mom_o) + 2e-7 * np.abs(Yo).max()
+
+
+# Exaggerated: one by one below 3,000 points, then through an order that is sorted beside the chain every eighth iteration, from
+# 32,768 on every fourth, from 65,536 on on the chain in each.  Settled: one by one up to 8,192, merged in natural order below
+# 32,768, then sorted beside the chain.  Both sides of every border, after single steps, pairs and blocks.
+@pytest.mark.parametrize("n", [2999, 3000, 8192, 8193, 32767, 32768, 65535, 65536, 131072, 131075])
+@pytest.mark.parametrize("step", [0, 400])
+@pytest.mark.parametrize("before", [[1], [1] * 9, [2] * 9, [64, 2]])
+def test_an_iteration_through_a_refreshed_order_vs_oracle(engine, oracle_cpu, n, step, before):
+    """One more iteration from wherever some have led, so that it spreads the points in the order that those have sorted."""
+    P, ids, rng = _graph(n, 4, n)
+    Y = rng.normal(0, 1e-4 if step == 0 else 20.0, (2, n)).astype(np.float32)
+    Y[:, : n // 3] *= 0.02
+    with engine.Session(n, 4) as s:
+        s.set_affinities(P, ids)
+        s.set_schedule(100.0, 12.0, 250, 0.5, 0.8)
+        s.set_state(Y, np.zeros_like(Y), np.ones_like(Y), step)
+        for k in before:
+            s.run(k)
+        Y0, u0, g0, at = s.get_state()
+        s.run(1)
+        Y1, u1, g1, _ = s.get_state()
+    assert at == step + sum(before)
+    _, g_o, u_o, _ = oracle_cpu.iterate(P, ids, Y0, 1, 100.0, first_step=at, gains=g0, old=u0)
+    m = np.float32(0.5 if at < 250 else 0.8)
+    # the new part of the momentum is the forces', the rest rounds once
+    assert np.linalg.norm((u1 - m * u0) - (u_o - m * u0)) < 1.1e-4 * np.linalg.norm(u_o - m * u0) + 2.0 ** -23 * np.linalg.norm(u0)
+    assert (np.abs(g1 - g_o) > 1e-5).mean() < 1e-3 and np.abs(Y1 - (Y0 + u1)).max() <= 2.0 ** -23 * np.abs(Y1).max()
+
+
+@pytest.mark.parametrize("n", [3000, 8193, 32768, 65535])
+@pytest.mark.parametrize("step", [0, 400])
+def test_order_beside_the_chain_and_none_agree(engine, monkeypatch, n, step):
+    """40 iterations from a blob (settled: from a layout) through orders sorted beside the chain, sorted on it in each iteration,
+    and in natural order: up to the order of the sums, as between blocks and single steps below."""
+    P, ids, rng = _graph(n, 6, 6)
+    Y = rng.normal(0, 1e-4 if step == 0 else 5.0, (2, n)).astype(np.float32)
+    out = []
+    for refresh, early in ((None, None), ("1", "1"), ("0", None)):
+        for name, value in (("B200TSNE_ORDER_REFRESH", refresh), ("B200TSNE_ORDER_REFRESH_EARLY", early)):
+            if value is None:
+                monkeypatch.delenv(name, raising=False)
+            else:
+                monkeypatch.setenv(name, value)
+        with engine.Session(n, 6) as s:
+            s.set_affinities(P, ids)
+            s.set_schedule(1.0, 12.0, 250, 0.5, 0.8)
+            s.set_state(Y, np.zeros_like(Y), np.ones_like(Y), step)
+            s.run(40)
+            out.append(s.get_state())
+    for o in out[1:]:
+        assert rel_l2(o[0], out[0][0]) < 1e-6 and rel_l2(o[1], out[0][1]) < 1e-4
 
 
 @pytest.mark.parametrize("n", [700, 40000])
