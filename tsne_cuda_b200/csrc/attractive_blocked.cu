@@ -714,8 +714,8 @@ attractive_blocked_kernel(BlockedStream b, const float2 *__restrict__ Yp, const 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int nwarps = kBlockedThreads / 32;
     const int c_lo = (int)((long long)b.C * blockIdx.x / gridDim.x), c_hi = (int)((long long)b.C * (blockIdx.x + 1) / gridDim.x);
-    // Launched behind the clear of the forces, it may run beside it up to its first addition: positions and stream are what the
-    // clear found.
+    // Launched behind the clear of the forces, it may run beside it up to its first addition.  Positions and stream are read before
+    // that: the clear is an ordinary launch, so the update that wrote the positions had ended when it began.
     bool cleared = false;
     if (c_lo >= c_hi) {
         after_previous();
@@ -890,8 +890,9 @@ static int device_sms(int *sms)
 
 // Blocks (SMs) of the attractive kernel of an iteration on one GPU, whose grid pipeline runs beside it on the SMs that are left.
 // A chunk of the stream is 0.034 us of an SM; what the pipeline has to do beside it is 1,200 us of one, 1,700 beside graphs of 36,000 to
-// 100,000 chunks, whose pipeline is what the iteration waits for, 3,200 where the iteration sorts its points: the SMs are divided in the proportion of the two, which is where both end together.  (At most six short of all:
-// the pipeline's last kernel is a chain of its own.)  us an iteration, exaggerated (sorting in each iteration from 32,768 points
+// 100,000 chunks, whose pipeline is what the iteration waits for, 3,200 where the iteration sorts its points: the SMs are divided
+// in the proportion of the two, which is where both end together.  (At most six short of all: the pipeline's last kernel is a
+// chain of its own.)  us an iteration, exaggerated (sorting in each iteration from 32,768 points
 // on) / settled, 90 neighbours (703 chunks per 1,000 points, 816 at 10^6), by the number of blocks:
 //   20,011     24 | 47 | 80              26.6 / 26.6 | 27.0 / 26.9 | 27.6 / 27.5
 //   40,000     47 | 64 | 96              40.2 / 31.2 | 39.9 / 31.0 | 39.3 / 32.5
@@ -902,7 +903,13 @@ static int device_sms(int *sms)
 //   10^6       128 | 132 | 136 | 142     228.5 / 235.1 | 224.9 / 231.2 | 236.0 / 228.6 | 236.8 / 221.0
 // Settled again, with the transforms as they are now: 60,000 on 60 | 68 | 72 | 80 | 88 33.5 | 32.3 | 33.1 | 33.1 | 36.6, 80,000 on 76 |
 // 80 | 84 | 88 36.9 | 36.5 | 35.6 | 38.2, 100,000 on 80 | 88 | 92 | 96 42.1 | 40.1 | 40.0 | 41.1.
-// The entries of a truly symmetric P come in a second launch behind the first, so both streams count.
+// At the ends of that band the number of blocks jumps, the time does not (it has a minimum on either side, where the columns' last
+// wave is full), settled: 50,500 points by the rule (74 blocks) 31.8, on 64 31.8; 52,000 (62) 32.0, on 76 32.8; 139,000 (98) 48.2, on
+// 108 47.5; 146,000 (110) 48.4, on 100 48.0.  Best of 40 to 120 in steps of four, and the rule: 38,000 29.2, 29.8; 45,000 31.0, 31.0;
+// 90,000 37.8, 37.7; 120,000 44.0, 44.0; 139,000 46.7, 48.2; 146,000 46.9, 48.4; 170,000 52.6, 53.3.
+// The entries of a truly symmetric P come in a second launch behind the first, so both streams count: settled, 90 neighbours
+// and their mirror images, by the rule | best of 24 to 132: 20,011 points 29.2 | 29.1, 30,011 32.7 | 32.0, 45,000 41.7 | 37.3
+// (96 blocks), 60,000 44.6 | 42.2 (112), 100,000 57.5 | 58.5.
 static int blocks_beside_grid(int sms, long long chunks, bool sorts)
 {
     // chunks that take as long
@@ -1035,6 +1042,7 @@ int launch_attractive_blocked(const BlockedAttractive &b, const float2 *Y2, floa
     const float2 *Yp = in_cell_order ? Y2 : b.Yp, *Yown = in_cell_order ? Y2 : b.Yown;
     float2 *Fp = in_cell_order ? F2 : b.Fp;
     const unsigned gN = (unsigned)((std::max(b.N, b.rows) + 255) / 256);
+    // (an ordinary launch: the kernel behind it reads the positions before it waits)
     if (in_cell_order) clear_forces_kernel<<<(unsigned)std::min<int64_t>((b.rows + 255) / 256, kClearBlocks), 256, 0, st>>>(F2, b.rows);
     else permute_kernel<<<gN, 256, 0, st>>>(Y2, b.perm, b.N, b.Yp, b.own_perm, b.rows, b.Yown, b.Fp);
     BlockedStream s;

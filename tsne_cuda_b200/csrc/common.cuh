@@ -73,13 +73,36 @@ __host__ __device__ inline float dec_float(unsigned int e)
 }
 
 // ---- chained launches ----
-// A kernel of the iteration's chain may be placed on the SMs while the one before it in its stream still runs.  What it does
-// before after_previous() touches constants only; that call returns when the kernel before has ended and its stores are
-// visible, so completion stays as transitive as with plain launches: every thread that touches anything else makes the call,
-// and a block that leaves early makes it too.  let_next_start() allows the next one to be placed once all blocks have made
-// it; without it, when all have ended.  Pointers to what an earlier kernel wrote are not __restrict__: the compiler would be
-// free to read through them before that call.
+// A kernel of the iteration's chain may be placed on the SMs while the one before it in its stream still runs.
+// after_previous() returns when that one has ended and its stores are visible, so completion stays as transitive as with
+// plain launches: every thread that touches more than constants makes the call, and a block that leaves early makes it too.
+// let_next_start() allows the next one to be placed once all blocks have made it; without it, when all have ended.
+// Before after_previous() a kernel touches constants, and nothing else unless the launch in front of it is an ORDINARY one
+// and leaves alone what is read: that launch began after everything before it had ended, so what earlier kernels wrote is
+// there.  Two kernels rest on that, and neither launch in front of them may become a chained one:
+//   attractive_blocked_kernel   reads positions and its stream, behind clear_forces_kernel (writes the forces);
+//   dense_distance_kernel       reads points and the list of queries, behind a selection (writes lists) whose own predecessors,
+//                               back to the ordinary launch that a search begins with, write distances and lists only.
+// Pointers to what an earlier kernel wrote are not __restrict__ but there: the compiler would be free to read through them
+// before that call.
 #ifdef __CUDACC__
+// two floats in one register pair, as the packed instructions take them
+__device__ __forceinline__ unsigned long long pack(float2 a)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack(unsigned long long r)
+{
+    float2 a;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+    return a;
+}
+// Two zeros to add to a packed square, so that it is rounded for itself: of a packed product and a packed sum the compiler
+// makes one rounding, and it does so too where it can see that the sum is with zero, so kernels have this as an argument.
+constexpr unsigned long long kMinusZero2 = 0x8000000080000000ull;
+
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... KArgs, typename... Args>

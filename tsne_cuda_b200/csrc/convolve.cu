@@ -25,10 +25,8 @@
 //
 // Bound: three kernels whose blocks each run once: the loads at their start, an exchange and the stores at their end take as
 // long as the transforms, and in those the fp32 pipe is three quarters busy (columns pass: 4,900 cycles of packed and scalar
-// arithmetic per scheduler in 6,500).  Measured on B200 inside an iteration of 5,000 points, from the end of the kernel before:
-// rows 3.5, columns 5.3, rows back 4.9 us, and 0.6 to 0.9 us between two of them (before the last
-// two steps below).  What that came from, per iteration at
-// 1,500 / 5,000 / 20,011 points:
+// arithmetic per scheduler in 6,500).  Measured on B200 inside an iteration of 5,000 points (clock stamps): rows 3.3, columns 4.9,
+// rows back 4.6 us, and 0.7 to 1.1 us between two of them.  What that came from, per iteration at 1,500 / 5,000 / 20,011 points:
 //   a row per block in the row passes (the column pass read and wrote 32 bytes of a line: every access of a warp touched 28
 //   different lines), scalar arithmetic, the spectrum in two kernels on a third stream                   31.1 / 32.1 / 34.4 us
 //   four rows per block and whole lines between the passes, packed arithmetic                            29.1 / 29.4 / 31.2

@@ -15,35 +15,23 @@ static_assert(kM == kR * kR && kM >= 2 * kG - 1 && kR * kHalf >= kG && kR * (kHa
 
 // Sums and products with a real coefficient act on both halves of a complex number alike: one packed instruction each, with
 // the results of the two it stands for.  The fp32 pipe is as fast either way; the issue slots go to everything else.
-__device__ __forceinline__ uint64_t pack(float2 a)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
-    return r;
-}
-__device__ __forceinline__ float2 unpack(uint64_t r)
-{
-    float2 a;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
-    return a;
-}
 __device__ __forceinline__ float2 operator+(float2 a, float2 b)
 {
-    uint64_t r;
+    unsigned long long r;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack(a)), "l"(pack(b)));
     return unpack(r);
 }
 // a + c * t, a real coefficient
 __device__ __forceinline__ float2 axpy(float c, float2 t, float2 a)
 {
-    uint64_t r;
+    unsigned long long r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack(make_float2(c, c))), "l"(pack(t)), "l"(pack(a)));
     return unpack(r);
 }
 __device__ __forceinline__ float2 operator-(float2 a, float2 b) { return axpy(-1.0f, b, a); }
 __device__ __forceinline__ float2 times(float c, float2 t)
 {
-    uint64_t r;
+    unsigned long long r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack(make_float2(c, c))), "l"(pack(t)));
     return unpack(r);
 }

@@ -24,23 +24,9 @@ constexpr int kTileP = 128;    // database points per tile
 constexpr int kDims = 32;      // dimensions per shared-memory chunk
 constexpr int kThreads = 256;
 
-// Two canonical operations at a time: each half rounds as the single instruction does.  The square is a fused operation with
-// -0, an argument of the kernel: of a packed product and a packed sum the compiler makes one rounding.  The fp32 pipe is as
-// busy as with single instructions, but half as many are issued: 4,099 x 64, K = 16 211 -> 201 us,
+// Two canonical operations at a time: each half rounds as the single instruction does (kMinusZero2: common.cuh).  The fp32 pipe
+// is as busy as with single instructions, but half as many are issued: 4,099 x 64, K = 16 211 -> 201 us,
 // 10,000 x 100, K = 40 1,943 -> 1,827 (whole searches).
-constexpr unsigned long long kMinusZero2 = 0x8000000080000000ull;
-__device__ __forceinline__ unsigned long long twice(float v)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(unsigned long long v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
 __device__ __forceinline__ void add_square2(unsigned long long &acc, unsigned long long q, unsigned long long minus_p, unsigned long long minus_zero)
 {
     asm("{\n\t.reg .b64 t;\n\t"
@@ -119,7 +105,7 @@ dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long l
                 if constexpr (QT == 4) *reinterpret_cast<float4 *>(qv) = *reinterpret_cast<const float4 *>(&Qs[d][ty * 4]);
                 else qv[0] = Qs[d][ty];
 #pragma unroll
-                for (int a = 0; a < QT; a++) qq[a] = twice(qv[a]);
+                for (int a = 0; a < QT; a++) qq[a] = pack(make_float2(qv[a], qv[a]));
             } else if constexpr (QT == 4) {
                 const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(&Qs[d][ty * 4]), b = *reinterpret_cast<const ulonglong2 *>(&Qs[d][ty * 4 + 2]);
                 qq[0] = a.x; qq[1] = a.y; qq[2] = b.x; qq[3] = b.y;
@@ -142,7 +128,7 @@ dense_distance_kernel(const float *__restrict__ X, int D, long long q_lo, long l
         const long long q = q0 + ty * QT + a;
         if (q >= nq) continue;
         float *row = dist + q * ld + p0;
-        const float2 d0 = unpack2(acc[a][0]), d1 = unpack2(acc[a][1]), d2 = unpack2(acc[a][2]), d3 = unpack2(acc[a][3]);
+        const float2 d0 = unpack(acc[a][0]), d1 = unpack(acc[a][1]), d2 = unpack(acc[a][2]), d3 = unpack(acc[a][3]);
         *reinterpret_cast<float4 *>(row + tx * 4) = make_float4(d0.x, d0.y, d1.x, d1.y);
         *reinterpret_cast<float4 *>(row + 64 + tx * 4) = make_float4(d2.x, d2.y, d3.x, d3.y);
     }

@@ -1386,18 +1386,17 @@ __device__ __forceinline__ float canon_step(float acc, float x, float y)
     return __fadd_rn(acc, __fmul_rn(t, t));
 }
 
-// The rounded squares of two rounded differences: x - y as x + (-1) y, the square as a fused operation with -0, an argument of the
-// kernel (a packed product and the sum after it would get one rounding), each half as the single instruction rounds it.
+// The rounded squares of two rounded differences: x - y as x + (-1) y, the square as a fused operation with -0 (kMinusZero2:
+// common.cuh), each half as the single instruction rounds it.
 __device__ __forceinline__ float2 canon_squares(float2 x, float2 y, unsigned long long minus_zero)
 {
-    float2 q;
+    float2 q;   // (the moves are part of it: with pack() and unpack() the compiler spills more)
     asm("{\n\t.reg .b64 a, b, m;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 m, 0xbf800000bf800000;\n\t"
         "fma.rn.f32x2 a, b, m, a;\n\tfma.rn.f32x2 a, a, a, %6;\n\tmov.b64 {%0, %1}, a;\n\t}"
         : "=f"(q.x), "=f"(q.y)
         : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "l"(minus_zero));
     return q;
 }
-constexpr unsigned long long kMinusZero2 = 0x8000000080000000ull;
 
 constexpr int kRerankWarps = 4;
 constexpr int kMaxL = 256;
