@@ -227,6 +227,37 @@ def test_a_schedule_that_changes_at_every_call_is_not_captured_every_time(engine
     assert changing < 1.5 * direct and repeated < 1.1 * direct
 
 
+def test_a_session_after_many_kinds_of_others_finds_its_executables(engine):
+    """Sessions of several sizes, phases and steps leave more executables than the sixteen that are kept.  The first session of
+    another size pays for its own (3 ms on 5.6), the second finds them (its first run 1.03 of the others; made anew, 1.5)."""
+    def session(n):
+        P, ids, rng = _graph(n, 6, n)
+        Y = rng.normal(0, 5.0, (2, n)).astype(np.float32)
+        s = engine.Session(n, 6)
+        s.set_affinities(P, ids)
+        s.set_schedule(1.0, 12.0, 250, 0.5, 0.8)
+        return s, lambda step: s.set_state(Y, np.zeros_like(Y), np.ones_like(Y), step)
+
+    engine.release_cached_memory()                            # one set of streams, nothing kept
+    for n in (2000, 4000, 70000, 140000):
+        s, start = session(n)
+        with s:
+            for step in (0, 400):
+                start(step)
+                for per in [64, 64] + [1] * 20 + [2] * 20:
+                    s.run(per)
+    for _ in range(2):
+        s, start = session(40000)
+        with s:
+            t = []
+            for _ in range(7):
+                start(0)
+                t0 = time.perf_counter()
+                s.run(224)
+                t.append(time.perf_counter() - t0)
+    assert t[0] < 1.15 * sorted(t)[3]
+
+
 @pytest.mark.parametrize("n", [1, 33, 21845, 21846])
 def test_state_goes_in_and_out_unchanged(engine, n):
     """Both sides of the largest state that crosses in one piece; a second state right behind the first."""

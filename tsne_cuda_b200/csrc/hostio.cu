@@ -292,8 +292,17 @@ bool graph_exec_kept(const StreamSet *s, unsigned long long shape)
 
 void graph_exec_release(StreamSet *s, cudaGraphExec_t exec, unsigned long long shape)
 {
-    if (!s || s->execs.size() >= kMaxKeptExecs) cudaGraphExecDestroy(exec);
-    else s->execs.push_back({exec, shape});
+    if (!s) {
+        cudaGraphExecDestroy(exec);
+        return;
+    }
+    // The one that was used longest ago makes room: a new one takes 2 to 3 ms (16 iterations), and a program that goes on with
+    // what it does now would pay that in each of its sessions.
+    if (s->execs.size() >= kMaxKeptExecs) {
+        cudaGraphExecDestroy(s->execs.front().exec);
+        s->execs.erase(s->execs.begin());
+    }
+    s->execs.push_back({exec, shape});
 }
 
 int copy_in(void *dst, const void *src, size_t bytes, cudaStream_t st)

@@ -565,8 +565,8 @@ int Session::graph_block(int remaining) const
     return px ? 0 : 1;
 }
 
-// Capturing a block and having an executable for it costs 100 us (updated) to 400 (new) more than the launches it saves cost
-// once, so it has to serve again: blocks that this call repeats or that an earlier one asked for, single iterations (50 us
+// Capturing a block and having an executable for it costs 100 us (updated) to 400 (a new pair; sixteen iterations 2 to 3 ms) more
+// than the launches it saves cost once, so it has to serve again: blocks that this call repeats or that an earlier one asked for, single iterations (50 us
 // saved) that were asked for kSingleFrom times.  A caller that steps one by one and changes the schedule every time
 // never gets there (2,000 / 60,000 points, us per step: 286 / 436 with a capture each, 119 / 118 launched directly); the odd
 // iteration at the end of a short call does not pay for an executable of its own.
