@@ -75,13 +75,17 @@ int main()
         CHECK(!ahead.started());
         memset(a, 1, bytes);
         memset(b, 1, bytes);
-        CHECK(!pages_missing(a, bytes) && !pages_missing(b + 1, bytes - 1));
+        CHECK(pages_missing(a, bytes) == 0 && pages_missing(b + 1, bytes - 1) == 0);
         ahead.start(a, b, bytes);   // nothing left to do
         CHECK(!ahead.started());
-        char *half = map(bytes);
-        memset(half, 1, bytes / 4);
-        CHECK(pages_missing(half, bytes));
-        ahead.start(a, half, bytes);
+        // a few missing in the middle, and more of them
+        char *holes = map(kPopulateEnd);
+        memset(holes, 1, kPopulateEnd);
+        madvise(holes + 2000 * page, kPagesWorthAThread * page, MADV_DONTNEED);
+        CHECK(pages_missing(holes, kPopulateEnd - 1) == kPagesWorthAThread && pages_missing(holes + 1, bytes) == 0);
+        ahead.start(a, holes + 2001 * page, bytes);
+        CHECK(!ahead.started());
+        ahead.start(a, holes + 2000 * page - 1, bytes);
         CHECK(ahead.started());
         ahead.end();
         for (int k = 0; k < 50; k++) {
